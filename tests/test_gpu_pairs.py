@@ -1,0 +1,60 @@
+"""Pairwise queries at the edges of their kernels' work splits, against the
+CPU oracle (whole numbers: equal)."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+N = 6000
+
+
+@pytest.fixture(scope="module")
+def sg():
+    import __graft_entry__ as ge
+    ge.build()
+    import sstgraph_gb300
+    return sstgraph_gb300
+
+
+@pytest.fixture(scope="module")
+def graph(sg):
+    """Rows of every shape: hubs of many leaves, rows of one leaf at each
+    capacity, empty rows."""
+    rng = np.random.default_rng(3)
+    hubs = [np.stack([np.full(k, v), rng.choice(N, k, replace=False)], 1)
+            for v, k in ((0, 5900), (1, 3000), (2, 700), (3, 65))]
+    rest = [np.stack([np.full(k, 10 + k), rng.choice(N, k, replace=False)], 1)
+            for k in range(1, 41)]
+    noise = rng.integers(100, N - 100, (20000, 2))
+    edges = oracle.symmetrize(np.concatenate(hubs + rest + [noise]).astype(np.uint32))
+    g, o = sg.SparseMatrixV(N), oracle.OracleGraph(N)
+    g.insert_batch(edges)
+    o.insert_batch(edges)
+    return g, o
+
+
+def pairs_of(n):
+    rng = np.random.default_rng(n)
+    p = rng.integers(0, N, (n, 2)).astype(np.uint32)
+    hub = rng.random((n, 2)) < 0.3
+    p[hub] = rng.integers(0, 55, int(hub.sum()))
+    return p
+
+
+# 1 pair; a block's share and one more; the clusters' shares (2 blocks an SM,
+# 64 pairs a block at most) filled unevenly
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 303, 305, 513, 4099, 20011])
+@pytest.mark.parametrize("early", [False, True])
+def test_common_neighbors(graph, n, early):
+    g, o = graph
+    p = pairs_of(n)
+    if n > 4:
+        p[1] = (0, 1)    # two hubs
+        p[2] = (7, 7)    # a row with itself
+        p[3] = (N, 1)    # an id out of range
+        p[4] = (N - 1, 0)
+    got = g.common_neighbors_batch(p, early)
+    exp = [0 if max(a, b) >= N else o.common_neighbors(int(a), int(b), early) for a, b in p]
+    assert np.array_equal(got, np.array(exp, np.uint64))
