@@ -173,6 +173,44 @@ __device__ __forceinline__ uint32_t leaf_lower_bound(const uint32_t *p,
   return lo;
 }
 
+// Whether x (not kEmpty) is in the row of a segment, in few round trips: for
+// callers that look many ids up in one row, where the row's lines are near and
+// the chain of dependent loads is what costs (common neighbours: 136 -> 103 us
+// for 20,000 pairs at RMAT scale 18, against find_leaf and leaf_lower_bound).
+// The leaf search loads three heads a step (capacities are powers of two, so
+// the range quarters exactly), and all the leaf's slots load together, 16
+// bytes at a time: a segment of 4 slots or more starts on a 16-byte boundary,
+// and every slot past a leaf's ids holds kEmpty, so no count is needed first.
+// Lookups spread over a whole large graph are bound by the sectors they touch
+// and keep the narrow forms above (1e6 lookups at scale 24: 84 us a batch's
+// locate against 106 with this).
+__device__ __forceinline__ bool seg_has(const uint32_t *slots, uint64_t base,
+                                        uint32_t cap, uint32_t x) {
+  if (x == kEmpty) return false;
+  const uint32_t *p = slots + base;
+  if (cap < 4) return (cap > 0 && p[0] == x) || (cap > 1 && p[1] == x);
+  if (cap > kLeaf) {
+    uint32_t lo = 0, n = cap >> kLeafLog;  // the leaf is in [lo, lo + n)
+    for (; n >= 4; n >>= 2) {
+      const uint64_t q = (uint64_t)n << (kLeafLog - 2);  // slots of a quarter
+      const uint32_t *h = p + ((uint64_t)lo << kLeafLog);
+      const uint32_t h1 = h[q], h2 = h[2 * q], h3 = h[3 * q];
+      lo += ((uint32_t)(h1 <= x) + (h2 <= x) + (h3 <= x)) * (n >> 2);
+    }
+    if (n == 2) lo += p[(uint64_t)(lo + 1) << kLeafLog] <= x;
+    p += (uint64_t)lo << kLeafLog;
+  }
+  const uint4 *q = reinterpret_cast<const uint4 *>(p);
+  uint4 v[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    v[k] = 4u * k < cap ? q[k] : make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
+  bool r = false;
+#pragma unroll
+  for (int k = 0; k < 8; k++) r |= v[k].x == x || v[k].y == x || v[k].z == x || v[k].w == x;
+  return r;
+}
+
 }  // namespace sst
 
 #define SST_CUDA_TRY(expr)                                                    \

@@ -85,15 +85,6 @@ sst_status graph_copy_into(sst_graph *dst, sst_graph *src) {
 namespace {
 constexpr uint32_t kTcvChunkLeaves = 32;
 
-__device__ __forceinline__ bool probe(const DGraph &g, uint64_t base,
-                                      uint32_t cap, uint32_t deg, uint32_t x) {
-  uint32_t l = find_leaf(g.slots, base, cap, x);
-  uint32_t c = leaf_count(g, base, cap, deg, l);
-  const uint32_t *p = g.slots + base + ((uint64_t)l << kLeafLog);
-  uint32_t pos = leaf_lower_bound(p, c, x);
-  return pos < c && p[pos] == x;
-}
-
 __device__ __forceinline__ uint32_t leaves_of(uint32_t cap) {
   return cap == 0 ? 0 : (cap <= kLeaf ? 1 : cap >> kLeafLog);
 }
@@ -163,14 +154,14 @@ __global__ void k_tcv_count(DGraph g, const uint32_t *__restrict__ vs,
     const uint32_t s = g.deg[u] <= g.deg[w] ? u : w, o = s == u ? w : u;
     const uint64_t sbase = g.base[s], obase = g.base[o];
     const uint32_t scap = g.cap[s], sdeg = g.deg[s];
-    const uint32_t ocap = g.cap[o], odeg = g.deg[o];
+    const uint32_t ocap = g.cap[o];
     const uint32_t l0 = j * kTcvChunkLeaves;
     const uint32_t l1 = min(l0 + kTcvChunkLeaves, leaves_of(scap));
     uint32_t hits = 0;
     for (uint32_t l = l0; l < l1; l++) {
       const uint32_t c = leaf_count(g, sbase, scap, sdeg, l);
       if ((uint32_t)lane < c)
-        hits += probe(g, obase, ocap, odeg, g.slots[sbase + ((uint64_t)l << kLeafLog) + lane]);
+        hits += seg_has(g.slots, obase, ocap, g.slots[sbase + ((uint64_t)l << kLeafLog) + lane]);
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, d);

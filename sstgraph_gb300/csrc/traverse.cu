@@ -1173,16 +1173,6 @@ __global__ void k_tc_off(const uint64_t *__restrict__ vleaf,
 }
 
 // ------------------------------------------------------------- pairs
-__device__ __forceinline__ bool seg_has(const DGraph &g, uint64_t base, uint32_t cap,
-                                        uint32_t deg, uint32_t x) {
-  if (!cap) return false;
-  const uint32_t l = find_leaf(g.slots, base, cap, x);
-  const uint32_t c = leaf_count(g, base, cap, deg, l);
-  const uint32_t *p = g.slots + base + ((uint64_t)l << kLeafLog);
-  const uint32_t pos = leaf_lower_bound(p, c, x);
-  return pos < c && p[pos] == x;
-}
-
 // Common neighbours of pairs: every id of the shorter row is looked up in the
 // longer one.  On a skewed graph one pair of hubs holds more leaves than all
 // the rest (a thread per pair, the form before this, spent its time in the one
@@ -1201,7 +1191,7 @@ constexpr uint32_t kCommonPairs = 64;  // pairs of a block, at most
 
 struct CommonPair {
   uint64_t sbase, obase;  // the shorter and the longer row
-  uint32_t scap, sdeg, ocap, odeg;
+  uint32_t scap, sdeg, ocap;
   uint32_t lim;  // ids from here on do not count (early end)
 };
 
@@ -1226,8 +1216,8 @@ k_common(DGraph g, const uint32_t *__restrict__ pairs, uint64_t n, uint32_t per_
         const uint32_t da = g.deg[a], db = g.deg[b];
         const uint32_t s = da <= db ? a : b, o = s == a ? b : a;
         const uint32_t scap = g.cap[s];
-        s_pair[j] = CommonPair{g.base[s], g.base[o], scap,      min(da, db),
-                               g.cap[o],  max(da, db), early ? min(a, b) : kEmpty};
+        s_pair[j] = CommonPair{g.base[s],   g.base[o], scap,
+                               min(da, db), g.cap[o],  early ? min(a, b) : kEmpty};
         leaves = scap ? nleaves_of(scap) : 0;
       }
     }
@@ -1277,7 +1267,7 @@ k_common(DGraph g, const uint32_t *__restrict__ pairs, uint64_t n, uint32_t per_
                              ? g.slots[q.sbase + ((uint64_t)l << kLeafLog) + lane]
                              : kEmpty;
       if (__shfl_sync(full, x, 0) >= q.lim) break;  // this leaf and the rest
-      if (x < q.lim) hits += seg_has(g, q.obase, q.ocap, q.odeg, x);
+      if (x < q.lim) hits += seg_has(g.slots, q.obase, q.ocap, x);
     }
     hits = __reduce_add_sync(full, hits);
     if (lane == 0 && hits)

@@ -58,3 +58,23 @@ def test_common_neighbors(graph, n, early):
     got = g.common_neighbors_batch(p, early)
     exp = [0 if max(a, b) >= N else o.common_neighbors(int(a), int(b), early) for a, b in p]
     assert np.array_equal(got, np.array(exp, np.uint64))
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 20011])
+def test_has_batch(graph, n):
+    """Lookups in rows of every capacity, at and beside the ids they hold."""
+    g, o = graph
+    p = pairs_of(n)
+    off, cols = o.csr()
+    rng = np.random.default_rng(n + 1)
+    for i in range(0, n, 2):  # an id of the row, or the one before or after it
+        u = p[i, 0]
+        if off[u + 1] > off[u]:
+            x = int(cols[rng.integers(off[u], off[u + 1])]) + int(rng.integers(-1, 2))
+            p[i, 1] = min(max(x, 0), N - 1)
+    if n > 4:
+        p[1] = (0, 0xFFFFFFFF)  # the gap marker is no id
+        p[2] = (50, 0xFFFFFFFF)
+        p[3] = (N, 1)
+    exp = [p[i, 0] < N and p[i, 1] < N and o.has(int(p[i, 0]), int(p[i, 1])) for i in range(n)]
+    assert np.array_equal(g.has_batch(p), np.array(exp, np.uint8))
