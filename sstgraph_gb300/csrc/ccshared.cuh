@@ -1,8 +1,8 @@
 // Connected-components building blocks shared by the PMA graph
 // (traverse.cu) and the byte-width snapshot (compact.cu): the
 // layout-independent parts of Afforest (Sutton, Ben-Nun, Barak 2018).
-//  1. link every vertex to its first two neighbours (two rounds, each
-//     followed by compression);
+//  1. link every vertex to its first neighbours (the snapshot: two rounds of
+//     cc_link, each followed by compression; the graph: hooks, traverse.cu);
 //  2. sample 1024 vertices' roots and take the most frequent one, c: the
 //     largest component so far;
 //  3. link every edge of every vertex whose root is not c (on a symmetric
@@ -16,15 +16,10 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "primitives.cuh"
 
 namespace sst {
 namespace {
-
-__device__ __forceinline__ uint32_t cc_root(const uint32_t *par, uint32_t x) {
-  uint32_t p;
-  while ((p = __ldcg(par + x)) != x) x = p;
-  return x;
-}
 
 __global__ void k_iota(uint32_t *__restrict__ p, uint32_t n) {
   uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -76,44 +71,61 @@ __device__ __forceinline__ void cc_link(uint32_t *par, uint32_t u, uint32_t v,
   }
 }
 
-// the most frequent root among 1024 sampled vertices (ties: the smaller)
+// The most frequent root among 1024 sampled vertices (ties: the smaller).
+// One block: the roots meet in a shared hash table of counters (open
+// addressing, at most half full), so the kernel is two rounds of loads and a
+// reduction; sorting the 1024 roots took 55 block barriers.
+constexpr uint32_t kGiantSlots = 2048;
 __global__ void __launch_bounds__(1024) k_cc_giant(const uint32_t *__restrict__ par,
                                                    uint32_t n,
                                                    unsigned long long *__restrict__ out) {
-  __shared__ uint32_t lab[1024];
+  __shared__ uint32_t key[kGiantSlots], cnt[kGiantSlots];
   __shared__ unsigned long long best;
   const uint32_t t = threadIdx.x;
-  const uint32_t v = (uint32_t)(mix64(0x5EEDull + t) % n);
-  lab[t] = par[v];
+  pdl_wait();
+  const uint32_t root = par[(uint32_t)(mix64(0x5EEDull + t) % n)];
+  for (uint32_t i = t; i < kGiantSlots; i += 1024) {
+    key[i] = kEmpty;  // no vertex has this id
+    cnt[i] = 0;
+  }
   if (t == 0) best = 0;
   __syncthreads();
-  for (uint32_t k = 2; k <= 1024; k <<= 1)  // bitonic sort, ascending
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      const uint32_t o = t ^ j;
-      if (o > t) {
-        const uint32_t a = lab[t], b = lab[o];
-        const bool up = (t & k) == 0;
-        if ((a > b) == up) {
-          lab[t] = b;
-          lab[o] = a;
-        }
-      }
-      __syncthreads();
-    }
-  if (t == 0 || lab[t] != lab[t - 1]) {
-    uint32_t e = t + 1;
-    while (e < 1024 && lab[e] == lab[t]) e++;
-    // larger count first, then the smaller label
-    atomicMax(&best, ((unsigned long long)(e - t) << 32) | (0xFFFFFFFFu - lab[t]));
+  uint32_t h = (root * 0x9E3779B1u) >> 21;  // top 11 bits
+  for (;;) {
+    const uint32_t k = atomicCAS(&key[h], kEmpty, root);
+    if (k == kEmpty || k == root) break;
+    h = (h + 1) & (kGiantSlots - 1);
   }
+  // lanes of one warp that hold the same root add once
+  const uint32_t peers = __match_any_sync(0xffffffffu, root);
+  if ((t & 31) == (uint32_t)__ffs(peers) - 1) atomicAdd(&cnt[h], (uint32_t)__popc(peers));
+  __syncthreads();
+  // larger count first, then the smaller label
+  unsigned long long b = 0;
+  for (uint32_t i = t; i < kGiantSlots; i += 1024)
+    if (cnt[i]) b = max(b, ((unsigned long long)cnt[i] << 32) | (0xFFFFFFFFu - key[i]));
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, d));
+  if ((t & 31) == 0 && b) atomicMax(&best, b);
   __syncthreads();
   if (t == 0) out[0] = 0xFFFFFFFFu - (uint32_t)(best & 0xFFFFFFFFu);
 }
 
-__global__ void k_cc_compress(uint32_t *__restrict__ par, uint32_t n) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+// Every vertex to its root; with `hooks`, only if it is not zero.  Nothing is
+// linked meanwhile, so the parents may come through L1 (an old one is an
+// ancestor): most chains end at one hot root, and loads of it past L1 queue at
+// its L2 slice (2e6 vertices already compressed: 16 us that way, 8 us
+// this way).
+__global__ void k_cc_compress(uint32_t *par, uint32_t n,
+                              const unsigned long long *__restrict__ hooks) {
+  pdl_wait();
+  if (hooks && *hooks == 0) return;
+  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n) return;
-  par[v] = cc_root(par, v);
+  const uint32_t p = par[v];
+  uint32_t x = p, q;
+  while ((q = par[x]) != x) x = q;
+  if (x != p) par[v] = x;
 }
 
 }  // namespace

@@ -1358,7 +1358,7 @@ sst_status compact_cc(sst_compact *c, uint32_t *d_labels) {
   SST_LAUNCH(k_iota, blocks_for(n), kTB, 0, s, d_labels, n);
   for (uint32_t r = 0; r < 2; r++) {
     SST_LAUNCH(k_ccc_sample, blocks_for(n), kTB, 0, s, dc, r, d_labels, err);
-    SST_LAUNCH(k_cc_compress, blocks_for(n), kTB, 0, s, d_labels, n);
+    SST_LAUNCH(k_cc_compress, blocks_for(n), kTB, 0, s, d_labels, n, nullptr);
   }
   SST_LAUNCH(k_cc_giant, 1, 1024, 0, s, d_labels, n, giant);
   if (c->nsmall)
@@ -1367,7 +1367,7 @@ sst_status compact_cc(sst_compact *c, uint32_t *d_labels) {
   if (c->nchunks)
     SST_LAUNCH(k_ccc_rest_chunks, warp_blocks(c->nchunks), kTB, 0, s, dc, c->d_cv, c->d_c0,
                c->nchunks, giant, d_labels, err);
-  SST_LAUNCH(k_cc_compress, blocks_for(n), kTB, 0, s, d_labels, n);
+  SST_LAUNCH(k_cc_compress, blocks_for(n), kTB, 0, s, d_labels, n, nullptr);
   SST_CUDA_TRY(cudaMemcpyAsync(c->h_cnt, c->d_cnt, 16, cudaMemcpyDeviceToHost, s));
   SST_CUDA_TRY(cudaStreamSynchronize(s));
   SST_CUDA_TRY(cudaGetLastError());

@@ -849,17 +849,75 @@ __global__ void k_bfs_pull_chunks(DGraph g, const unsigned long long *__restrict
 }
 
 // ------------------------------------------------------------- cc
-// Afforest, with the helpers in ccshared.cuh
-// round r of the sampling: u links to its r-th neighbour in its first leaf
-__global__ void k_cc_sample(DGraph g, uint32_t r, uint32_t *__restrict__ par,
-                            unsigned long long *__restrict__ err) {
+// Afforest, with the helpers in ccshared.cuh, but the sampled links are hooks
+// without a loop.  Linking every vertex to its first two neighbours by find
+// and compare-and-swap (the form before) had 2e6 threads chase and extend
+// chains of fresh roots: 385 us a neighbour on a uniform graph of 2e6 vertices
+// and 14e6 stored edges, where all of the rounds below take 175 us together.  They
+// are bound by scattered 32-byte sectors: a row's first ids (read once, here),
+// and two parents a vertex and round.
+// The start: every vertex below its smallest neighbour (rows ascend), if that
+// is smaller.  A parent is smaller than its child, so the links are a forest.
+// nb keeps the next two neighbours (kEmpty: none) for the rounds.
+__global__ void k_cc_hook_first(DGraph g, uint32_t *__restrict__ par,
+                                uint32_t *__restrict__ nb1, uint32_t *__restrict__ nb2) {
+  pdl_wait();
   const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= g.n) return;
   const uint32_t cap = g.cap[u];
-  if (!cap) return;
-  const uint64_t base = g.base[u];
-  const uint32_t c0 = leaf_count(g, base, cap, g.deg[u], 0);
-  if (r < c0) cc_link(par, u, g.slots[base + r], err);
+  uint4 x = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
+  if (cap >= 4) {  // starts on a 16-byte boundary; slots past the ids hold kEmpty
+    x = *reinterpret_cast<const uint4 *>(g.slots + g.base[u]);
+  } else if (cap) {
+    const uint32_t *p = g.slots + g.base[u];
+    x.x = p[0];
+    if (cap > 1) x.y = p[1];
+  }
+  par[u] = min(u, x.x);
+  nb1[u] = x.y;
+  nb2[u] = x.z;
+}
+
+// A round, after a compression: of the roots of u and its two kept neighbours
+// the larger ones go below the smallest.  A root keeps the smallest that any
+// vertex offers it, and a parent that is read while it changes is an ancestor:
+// either way a tree only moves below a vertex of its own component with a
+// smaller id.  A hook that another one replaces is linked later: phase 3 takes
+// every edge of every vertex outside the largest component.
+// The first round, of every vertex, leaves 5e3 trees on that uniform graph.
+// Their roots would get hundreds of offers each, and atomics on one address
+// wait for each other (25 ns apiece: a second round of every vertex takes 240
+// us, of every 8th 74 us).  So on a large graph the second round takes every
+// 32nd vertex, the third every 512th, which joins the two or three trees that
+// then hold most vertices, and the last every vertex: 0.1% are outside the
+// largest tree after it (4% at average degree 2.4).  Below kCcSampledN there
+// are too few vertices for that, and launches cost more than the atomics.
+// When the second round finds nothing to hook the later ones return at once.
+// The parents come through L1: nearly all are one hot root, whose loads would
+// queue at one L2 slice, and a stale one is an ancestor too.
+constexpr uint32_t kCcSampledN = 1u << 17;
+constexpr int kCcMaxRounds = 4;
+constexpr uint32_t kCcStride[2][kCcMaxRounds] = {{1, 1, 0, 0}, {1, 32, 512, 1}};
+__global__ void k_cc_hook(const uint32_t *__restrict__ nb1, const uint32_t *__restrict__ nb2,
+                          uint32_t n, uint32_t stride, uint32_t *par,
+                          const unsigned long long *__restrict__ before,
+                          unsigned long long *__restrict__ hooks) {
+  pdl_wait();
+  if (before && *before == 0) return;
+  const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * stride;
+  bool hooked = false;
+  if (u < n) {
+    const uint32_t x = nb1[u], y = nb2[u];
+    const uint32_t a = par[u];
+    const uint32_t b = x != kEmpty ? par[x] : a;
+    const uint32_t c = y != kEmpty ? par[y] : a;
+    const uint32_t m = min(a, min(b, c));
+    // a look (past L1) before an atomic: an offer that is no better costs less
+    if (a > m && ld_par(par, a) > m) hooked |= atomicMin(&par[a], m) > m;
+    if (b > m && ld_par(par, b) > m) hooked |= atomicMin(&par[b], m) > m;
+    if (c > m && ld_par(par, c) > m) hooked |= atomicMin(&par[c], m) > m;
+  }
+  if (__syncthreads_or(hooked) && threadIdx.x == 0) *(volatile unsigned long long *)hooks = 1;
 }
 
 // phase 3, one-leaf vertices: thread per vertex
@@ -868,6 +926,7 @@ __global__ void k_cc_rest_small(DGraph g, const unsigned long long *__restrict__
                                 const unsigned long long *__restrict__ giant,
                                 uint32_t *__restrict__ par,
                                 unsigned long long *__restrict__ err) {
+  pdl_wait();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nsmall) return;
   const uint32_t u = small[i];
@@ -884,6 +943,7 @@ __global__ void k_cc_rest_chunks(DGraph g, const unsigned long long *__restrict_
                                  const unsigned long long *__restrict__ giant,
                                  uint32_t *__restrict__ par,
                                  unsigned long long *__restrict__ err) {
+  pdl_wait();
   const uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (c >= nchunks) return;
@@ -1607,22 +1667,31 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
   const uint32_t n = g->n;
   if (n == 0) return SST_OK;
   uint32_t *par = d_labels;
-  unsigned long long *giant = t->d_small, *err = t->d_small + 1;
-  SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, 16, s));
+  unsigned long long *giant = t->d_small, *err = t->d_small + 1, *hooks = t->d_small + 2;
+  SST_CUDA_TRY(t->qa.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->qb.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, (2 + kCcMaxRounds) * 8, s));
   const DGraph dg = g->view();
-  SST_LAUNCH(k_iota, blocks_for(n), kTB, 0, s, par, n);
-  for (uint32_t r = 0; r < 2; r++) {
-    SST_LAUNCH(k_cc_sample, blocks_for(n), kTB, 0, s, dg, r, par, err);
-    SST_LAUNCH(k_cc_compress, blocks_for(n), kTB, 0, s, par, n);
+  SST_LAUNCH_PDL(k_cc_hook_first, blocks_for(n), kTB, 0, s, dg, par, t->qa.p, t->qb.p);
+  SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n,
+                 static_cast<const unsigned long long *>(nullptr));
+  const bool sampled = n >= kCcSampledN;
+  for (int r = 0; r < (sampled ? 4 : 2); r++) {
+    const uint32_t stride = kCcStride[sampled][r];
+    SST_LAUNCH_PDL(k_cc_hook, blocks_for((n + stride - 1) / stride), kTB, 0, s, t->qa.p,
+                   t->qb.p, n, stride, par, r ? hooks + std::min(r - 1, 1) : nullptr,
+                   hooks + r);
+    SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, hooks + r);
   }
-  SST_LAUNCH(k_cc_giant, 1, 1024, 0, s, par, n, giant);
+  SST_LAUNCH_PDL(k_cc_giant, 1, 1024, 0, s, par, n, giant);
   if (t->nsmall)
-    SST_LAUNCH(k_cc_rest_small, blocks_for(t->nsmall), kTB, 0, s, dg, t->sdesc.p,
+    SST_LAUNCH_PDL(k_cc_rest_small, blocks_for(t->nsmall), kTB, 0, s, dg, t->sdesc.p,
                t->small.p, t->nsmall, giant, par, err);
   if (t->nchunks)
-    SST_LAUNCH(k_cc_rest_chunks, warp_blocks(t->nchunks), kTB, 0, s, dg, t->cdesc.p,
+    SST_LAUNCH_PDL(k_cc_rest_chunks, warp_blocks(t->nchunks), kTB, 0, s, dg, t->cdesc.p,
                t->cv.p, t->nchunks, giant, par, err);
-  SST_LAUNCH(k_cc_compress, blocks_for(n), kTB, 0, s, par, n);
+  SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n,
+                 static_cast<const unsigned long long *>(nullptr));
   SST_CUDA_TRY(cudaMemcpyAsync(t->h_small, t->d_small, 16, cudaMemcpyDeviceToHost, s));
   SST_CUDA_TRY(cudaStreamSynchronize(s));
   SST_CUDA_TRY(cudaGetLastError());
