@@ -13,6 +13,7 @@
 #include <cooperative_groups.h>
 #include <vector>
 
+#include "bfslevels.cuh"
 #include "ccshared.cuh"
 #include "prfixed.cuh"
 #include "tcshared.cuh"
@@ -84,6 +85,7 @@ struct TravState {
   DevBuf<double> inv_deg, ca, cb, partial;
   // bfs
   DevBuf<uint32_t> qa, qb, fbits, icnt, ioff, iv, il0;
+  DevBuf<unsigned long long> qitems;
   DevBuf<int32_t> depth_tmp, parent_tmp;
   // bc
   DevBuf<double> sigma, ratio;
@@ -110,6 +112,7 @@ struct TravState {
   int64_t pr_kernels = 0;      // kernels in the captured graph
   uint64_t *h_small = nullptr;  // pinned readback slots
   unsigned long long *d_small = nullptr;
+  void *d_bfs = nullptr;  // BfsCtl, zero between searches
 };
 
 // frees every buffer and the captured PageRank graph; the tuning stays, and
@@ -133,6 +136,7 @@ static void trav_buffers_release(TravState *t) {
   t->qb.release();
   t->fbits.release();
   t->icnt.release();
+  t->qitems.release();
   t->ioff.release();
   t->iv.release();
   t->il0.release();
@@ -181,6 +185,7 @@ void trav_release(sst_graph *g) {
   trav_buffers_release(t);
   if (t->h_small) cudaFreeHost(t->h_small);
   if (t->d_small) cudaFree(t->d_small);
+  if (t->d_bfs) cudaFree(t->d_bfs);
   delete t;
   g->trav = nullptr;
 }
@@ -194,7 +199,7 @@ uint64_t trav_device_bytes(const sst_graph *g) {
   add(t->sdesc.cap, 8); add(t->multi.cap, 4); add(t->big.cap, 4); add(t->small.cap, 4);
   add(t->flag.cap, 4); add(t->pos.cap, 4); add(t->inv_deg.cap, 8); add(t->ca.cap, 8);
   add(t->cb.cap, 8); add(t->partial.cap, 8); add(t->qa.cap, 4); add(t->qb.cap, 4);
-  add(t->fbits.cap, 4); add(t->icnt.cap, 4); add(t->ioff.cap, 4); add(t->iv.cap, 4);
+  add(t->fbits.cap, 4); add(t->qitems.cap, 8); add(t->icnt.cap, 4); add(t->ioff.cap, 4); add(t->iv.cap, 4);
   add(t->il0.cap, 4); add(t->depth_tmp.cap, 4); add(t->parent_tmp.cap, 4);
   add(t->sigma.cap, 8); add(t->ratio.cap, 8); add(t->lvl_list.cap, 4);
   add(t->lvl_cnt.cap, 4); add(t->par.cap, 4); add(t->toff.cap, 8); add(t->tlpre.cap, 8);
@@ -1345,6 +1350,8 @@ static TravState *state(sst_graph *g) {
     g->trav = new TravState();
     cudaMallocHost(&g->trav->h_small, 64 * sizeof(uint64_t));
     cudaMalloc(&g->trav->d_small, 64 * sizeof(unsigned long long));
+    cudaMalloc(&g->trav->d_bfs, sizeof(BfsCtl));
+    cudaMemsetAsync(g->trav->d_bfs, 0, sizeof(BfsCtl), g->stream);
   }
   return g->trav;
 }
@@ -1655,8 +1662,56 @@ static sst_status bfs_run(sst_graph *g, uint32_t src, int32_t *d_parents, int32_
   return SST_OK;
 }
 
+// blocks of a cooperative grid for `threads` threads of work: no more than the
+// work fills (see bfslevels.cuh), no more than fit at once
+static sst_status coop_grid(const sst_graph *g, const void *kernel, uint64_t threads,
+                            unsigned *grid) {
+  int per_sm = 0;
+  SST_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kCoopThreads, 0));
+  if (per_sm < 1) {
+    set_error_message("a traversal kernel does not fit the device");
+    return SST_EDEVICE;
+  }
+  const uint64_t most = (uint64_t)std::min(per_sm, kCoopPerSm) * g->sms;
+  *grid = (unsigned)std::min<uint64_t>(most, (threads + kCoopThreads - 1) / kCoopThreads + 1);
+  return SST_OK;
+}
+
 sst_status bfs(sst_graph *g, uint32_t src, int32_t *d_parents, int32_t *d_depths) {
-  return bfs_run(g, src, d_parents, d_depths, nullptr, nullptr);
+  sst_status st = ensure_lists(g);
+  if (st != SST_OK) return st;
+  TravState *t = g->trav;
+  cudaStream_t s = g->stream;
+  const uint32_t n = g->n;
+  // a row's push items are at most 32 / kBfsLeaves for each of its chunks in
+  // the lists (chunks of up to 32 leaves)
+  const uint64_t max_items = t->nchunks * (32 / kBfsLeaves) + 1;
+  SST_CUDA_TRY(t->qa.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->qitems.ensure(max_items));
+  SST_CUDA_TRY(t->fbits.ensure(n / 32 + 2));
+  if (!d_depths) {
+    SST_CUDA_TRY(t->depth_tmp.ensure(n));
+    d_depths = t->depth_tmp.p;
+  }
+  BfsCtl *ctl = reinterpret_cast<BfsCtl *>(t->d_bfs);
+  const BfsArgs a{g->view(), g->m,        src,        t->bfs_alpha, t->small.p,
+                  t->sdesc.p, t->nsmall,  t->cv.p,    t->cdesc.p,   t->nchunks,
+                  d_depths,  d_parents,   t->fbits.p, t->qa.p,      t->qitems.p,
+                  max_items, ctl, reinterpret_cast<unsigned long long *>(t->h_small)};
+  unsigned grid = 1;
+  st = coop_grid(g, reinterpret_cast<const void *>(k_bfs_levels),
+                 std::max(t->nsmall, 32 * t->nchunks), &grid);
+  if (st != SST_OK) return st;
+  SST_CUDA_TRY(launch_coop("k_bfs_levels", k_bfs_levels, grid, kCoopThreads, s, a));
+  SST_CUDA_TRY(cudaStreamSynchronize(s));
+  const uint64_t err = *(volatile uint64_t *)t->h_small;
+  if (err) {
+    set_error_message(err == 1   ? "BFS: a grid barrier timed out"
+                      : err == 2 ? "BFS: a level queue overflowed"
+                                 : "BFS exceeded n levels");
+    return err == 2 ? SST_EDEVICE : SST_ETIMEDOUT;
+  }
+  return SST_OK;
 }
 
 sst_status cc(sst_graph *g, uint32_t *d_labels) {
