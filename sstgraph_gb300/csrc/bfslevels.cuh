@@ -562,14 +562,365 @@ __device__ __forceinline__ void bfs_count(BfsCount *c, const BfsSum &sum) {
   }
 }
 
-__device__ __forceinline__ void bfs_levels(const BfsArgs &a) {
+// ------------------------------------------------------------ dependencies
+// Brandes' single-source dependencies in the same launch: path counts (sigma)
+// on the way down, beside the search itself, then the dependencies level by
+// level back up.
+//
+// An edge joins levels that differ by at most one, so a row of level d has
+// neighbours at d - 1, d and d + 1 only.  With one array for the even levels'
+// values and one for the odd levels', zero until a row is done, the sum over
+// all of a row's neighbours in the other parity's array is the sum over the
+// wanted level alone (the other one of that parity is still zero, and adding
+// zeros changes no bit): one gather an edge, where looking the depth up first
+// took one or two.
+//
+// The order of every row's sum is fixed, the same as the multi-source form's:
+// a one-leaf row in neighbour order; a multi-leaf row in chunks of kBcLeaves
+// leaves, each lane over its chunk's leaves in order, then the lanes by
+// shuffles, then the chunks in order.
+constexpr uint32_t kBcLeaves = 32;
+constexpr uint32_t kHubCap = kBcLeaves * kLeaf;  // a larger row is a hub: a warp a chunk
+
+// capacity classes of the multi-leaf rows, largest first: hubs, then 32 leaves
+// down to 2
+constexpr int kBcClasses = 6;
+__device__ __forceinline__ int bc_class(uint32_t cap) {
+  return cap > kHubCap ? 0 : __clz(cap) - __clz(kHubCap) + 1;
+}
+struct BcCtl {
+  uint32_t items;             // chunks of the hubs
+  uint32_t count[kBcClasses]; // rows of a class
+  uint32_t at[kBcClasses];    // rows of a class listed so far
+};
+
+struct BcArgs {
+  double *sigma;      // 2n: of even levels' rows, then of odd levels'
+  double *ratio;      // (1 + dependency) / sigma, likewise
+  double *dep;        // n, the result
+  const uint32_t *big;  // all multi-leaf rows
+  uint64_t nbig;
+  uint64_t max_hub;     // entries of the four hub arrays
+  uint2 *hub;           // hubs: row, first item
+  uint2 *hub_item;      // their chunks: hub, chunk
+  double *hub_part;     // a chunk's sum
+  uint32_t *hub_done;   // chunks summed, of a hub (zero between levels)
+  uint32_t *order;      // the other multi-leaf rows by capacity, largest first; nbig entries
+  BcCtl *bc;            // zero at launch and after
+  uint2 *level;         // per level: queue ends, multi-leaf rows' high bit = not in the queue
+};
+constexpr uint32_t kNotQueued = 1u << 31;
+
+constexpr int kBcFlight = 8;  // neighbours (or leaves) in flight
+
+// Row ids are read once a pass and leave L1 to the gathered values; those
+// change between levels, so they are not read through the read-only path.
+__device__ __forceinline__ uint32_t ld_id(const uint32_t *p) {
+  uint32_t v;
+  asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_id4(const uint32_t *p) {
+  uint4 v;
+  asm("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p));
+  return v;
+}
+// the sums of val over the one-leaf rows of a warp, a lane a row (deg = 0: none)
+__device__ __forceinline__ double bc_sum_rows(const BfsArgs &a, uint64_t base, uint32_t deg,
+                                              const double *val) {
+  const uint32_t *p = a.g.slots + base;
+  const bool wide = (base & 3) == 0;  // else a segment of one or two slots
+  double s = 0.0;
+  for (uint32_t j = 0; j < deg; j += kBcFlight) {
+    uint32_t x[kBcFlight];
+    if (wide) {
+      const uint4 q0 = ld_id4(p + j);
+      const uint4 q1 = j + 4 < deg ? ld_id4(p + j + 4) : q0;
+      x[0] = q0.x, x[1] = q0.y, x[2] = q0.z, x[3] = q0.w;
+      x[4] = q1.x, x[5] = q1.y, x[6] = q1.z, x[7] = q1.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < kBcFlight; k++) x[k] = k < 2 && j + k < deg ? p[k] : 0u;
+    }
+    double y[kBcFlight];
+#pragma unroll
+    for (int k = 0; k < kBcFlight; k++) y[k] = j + k < deg ? val[x[k]] : 0.0;
+#pragma unroll
+    for (int k = 0; k < kBcFlight; k++) s += y[k];
+  }
+  return s;
+}
+
+// the sum of val over leaves [l0, l1) of a multi-leaf row, by a warp (lane 0
+// has it); at most kBcLeaves of them
+__device__ __forceinline__ double bc_sum_leaves(const BfsArgs &a, uint64_t base, uint32_t l0,
+                                                uint32_t l1, const double *val) {
+  const uint32_t *p = a.g.slots + base + (threadIdx.x & 31);
+  double acc = 0.0;
+  for (uint32_t l = l0; l < l1; l += kBcFlight) {
+    uint32_t x[kBcFlight];
+#pragma unroll
+    for (int k = 0; k < kBcFlight; k++)
+      x[k] = l + k < l1 ? ld_id(p + ((uint64_t)(l + k) << kLeafLog)) : kEmpty;
+    double y[kBcFlight];
+#pragma unroll
+    for (int k = 0; k < kBcFlight; k++) y[k] = x[k] != kEmpty ? val[x[k]] : 0.0;
+#pragma unroll
+    for (int k = 0; k < kBcFlight; k++) acc += y[k];
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) acc += __shfl_down_sync(kFull, acc, d);
+  return acc;
+}
+
+// row v of level lvl has the sum s
+__device__ __forceinline__ void bc_finish(const BfsArgs &a, const BcArgs &b, uint32_t v, int lvl,
+                                          bool down, double s) {
+  const uint64_t i = (lvl & 1 ? (uint64_t)a.g.n : 0) + v;
+  if (down) {
+    b.sigma[i] = s;
+  } else {
+    const double sg = b.sigma[i], dv = sg * s;
+    b.dep[v] = dv;
+    b.ratio[i] = (1.0 + dv) / sg;
+  }
+}
+
+// Sums over lanes of R accumulators at once: afterwards lanes j * 32/R .. hold
+// accumulator j's sum, each the same sum as shuffling it down by 16, 8, 4, 2, 1
+// (an addition's two sides may change places).  The first log2(R) steps halve
+// the accumulators, so R of them take R - 1 + 5 - log2(R) additions, not 5R: a
+// warp's FP64 addition takes about 15 cycles of this device's pipe, which is
+// what bounds the wide levels (with a reduction and a division a row, by one
+// lane, the pipe was busy for 255 of 700 us at RMAT scale 20).
+template <int R>
+__device__ __forceinline__ double bc_reduce(double (&acc)[R]) {
+  const int lane = threadIdx.x & 31;
+  int d = 16;
+#pragma unroll
+  for (int r = R / 2; r > 0; r >>= 1, d >>= 1) {
+    const bool up = lane & d;
+#pragma unroll
+    for (int j = 0; j < r; j++) {
+      const double keep = up ? acc[j + r] : acc[j], give = up ? acc[j] : acc[j + r];
+      acc[j] = keep + __shfl_xor_sync(kFull, give, d);
+    }
+  }
+#pragma unroll
+  for (; d > 0; d >>= 1) acc[0] += __shfl_xor_sync(kFull, acc[0], d);
+  return acc[0];
+}
+
+// R multi-leaf rows (lane j < R: row v's first slot and leaf count nl, 0: no
+// row) summed by the warp, kPair rows and kLeaves leaves in flight, and
+// finished together
+template <int R, int kPair, int kLeaves>
+__device__ __forceinline__ void bc_rows(const BfsArgs &a, const BcArgs &b, uint32_t v,
+                                        uint64_t base, uint32_t nl, int lvl, bool down,
+                                        const double *val) {
+  const int lane = threadIdx.x & 31;
+  double acc[R];
+#pragma unroll
+  for (int r = 0; r < R; r += kPair) {
+    const uint32_t *p[kPair];
+    uint32_t n[kPair], most = 0;
+#pragma unroll
+    for (int q = 0; q < kPair; q++) {
+      p[q] = a.g.slots + __shfl_sync(kFull, base, r + q) + lane;
+      n[q] = __shfl_sync(kFull, nl, r + q);
+      most = max(most, n[q]);
+      acc[r + q] = 0.0;
+    }
+    for (uint32_t l = 0; l < most; l += kLeaves) {
+      uint32_t x[kPair][kLeaves];
+#pragma unroll
+      for (int q = 0; q < kPair; q++)
+#pragma unroll
+        for (int k = 0; k < kLeaves; k++)
+          x[q][k] = l + k < n[q] ? ld_id(p[q] + ((uint64_t)(l + k) << kLeafLog)) : kEmpty;
+      double y[kPair][kLeaves];
+#pragma unroll
+      for (int q = 0; q < kPair; q++)
+#pragma unroll
+        for (int k = 0; k < kLeaves; k++) y[q][k] = x[q][k] != kEmpty ? val[x[q][k]] : 0.0;
+#pragma unroll
+      for (int q = 0; q < kPair; q++)
+#pragma unroll
+        for (int k = 0; k < kLeaves; k++)
+          if (l + k < n[q]) acc[r + q] += y[q][k];  // the same for the warp
+    }
+  }
+  const double sum = bc_reduce<R>(acc);
+  const int j = lane / (32 / R);
+  const uint32_t vj = __shfl_sync(kFull, v, j), nj = __shfl_sync(kFull, nl, j);
+  if (lane % (32 / R) == 0 && nj) bc_finish(a, b, vj, lvl, down, sum);
+}
+
+// The rows of level lvl: sigma from the level above (down), or dependencies
+// from the level below.  The level is in the queue ([r0, r1) and [b0, b1)), or
+// else, a level that a pull left, every list is searched for it: such levels
+// hold a fair share of the graph, so there are few of them.
+__device__ __forceinline__ void bc_level(const BfsArgs &a, const BcArgs &b, int lvl, bool down,
+                                         bool queued, uint32_t r0, uint32_t r1, uint32_t b0,
+                                         uint32_t b1) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nw = (gridDim.x * kCoopThreads) >> 5;
+  const uint32_t w0 = (blockIdx.x * kCoopThreads + threadIdx.x) >> 5;
+  const double *val = (down ? b.sigma : b.ratio) + (lvl & 1 ? 0 : (uint64_t)a.g.n);
+  // hubs: a warp a chunk, over all the hubs' chunks; the warp that sums a hub's
+  // last chunk adds the chunks up, in their order
+  const uint32_t nitems = __ldcg(&b.bc->items);
+  for (uint32_t i = w0; i < nitems; i += nw) {
+    const uint2 it = b.hub_item[i], hb = b.hub[it.x];
+    const uint32_t v = hb.x;
+    if (__shfl_sync(kFull, __ldcg(a.depth + v), 0) != lvl) continue;
+    const uint32_t nl = a.g.cap[v] >> kLeafLog, l0 = it.y * kBcLeaves;
+    const uint32_t nc = (nl + kBcLeaves - 1) / kBcLeaves;
+    const double s = bc_sum_leaves(a, a.g.base[v], l0, min(l0 + kBcLeaves, nl), val);
+    uint32_t done = 0;
+    if (lane == 0) {
+      __stcg(b.hub_part + i, s);
+      __threadfence();
+      done = atomicAdd(b.hub_done + it.x, 1u) + 1;
+      __threadfence();
+    }
+    if (__shfl_sync(kFull, done, 0) != nc) continue;
+    double t = 0.0;
+    for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
+      const double part = c0 + lane < nc ? __ldcg(b.hub_part + hb.y + c0 + lane) : 0.0;
+      for (uint32_t c = c0; c < min(c0 + 32, nc); c++) t += __shfl_sync(kFull, part, c - c0);
+    }
+    if (lane == 0) {
+      b.hub_done[it.x] = 0;
+      bc_finish(a, b, v, lvl, down, t);
+    }
+  }
+  // The other multi-leaf rows.  The list has the long ones first, and a warp
+  // takes the fewer the longer they are, so that the warps end together (in id
+  // order an RMAT graph's long rows sit side by side, and a warp with eight of
+  // them held the level up for 75 us); a queue is in no order.
+  const uint64_t nbig = queued ? b1 - b0 : b.nbig - __ldcg(&b.bc->count[0]);
+  uint64_t end[3] = {0, 0, nbig};  // rows of over 16 leaves, of 8 and 16, all
+  if (!queued) {
+    end[0] = __ldcg(&b.bc->count[1]);
+    end[1] = end[0] + __ldcg(&b.bc->count[2]) + __ldcg(&b.bc->count[3]);
+  }
+  for (int part = 0; part < 3; part++) {
+    const uint64_t first = part ? end[part - 1] : 0, n = end[part] - first;
+    const uint64_t share = (n + nw - 1) / nw;
+    const uint64_t most = part == 0 ? 2 : part == 1 ? 4 : 8;
+    const uint32_t per = (uint32_t)(share > most ? most : share);
+    for (uint64_t i0 = (uint64_t)w0 * per; i0 < n; i0 += (uint64_t)nw * per) {
+      const uint64_t i = first + i0 + lane;
+      const bool in = (uint32_t)lane < per && i0 + lane < n;
+      const uint32_t v = !in ? 0u : queued ? a.queue[a.g.n - 1 - (b0 + i)] : b.order[i];
+      const uint32_t cap = in ? a.g.cap[v] : 0u;
+      const uint64_t base = in ? a.g.base[v] : 0ull;
+      const bool on = in && cap <= kHubCap && (queued || a.depth[v] == lvl);
+      if (!__any_sync(kFull, on)) continue;
+      const uint32_t nl = on ? cap >> kLeafLog : 0u;
+      if (part == 0)
+        bc_rows<2, 1, 8>(a, b, v, base, nl, lvl, down, val);
+      else if (part == 1)
+        bc_rows<4, 1, 8>(a, b, v, base, nl, lvl, down, val);
+      else
+        bc_rows<8, 2, 4>(a, b, v, base, nl, lvl, down, val);
+    }
+  }
+  const uint64_t nrow = queued ? r1 - r0 : a.nsmall;
+  {  // one-leaf rows: a lane a row
+    const uint64_t share = (nrow + nw - 1) / nw;
+    const uint32_t per = share > 32 ? 32u : (uint32_t)share;
+    for (uint64_t i = (uint64_t)w0 * per + lane; i - lane < nrow; i += (uint64_t)nw * per) {
+      const bool in = (uint32_t)lane < per && i < nrow;
+      const uint32_t v = !in ? 0u : queued ? a.queue[r0 + i] : a.small[i];
+      const unsigned long long dsc = in && !queued ? a.sdesc[i] : 0ull;
+      const bool on = in && (queued || a.depth[v] == lvl);
+      if (!__any_sync(kFull, on)) continue;
+      const uint64_t base = !on ? 0ull : queued ? a.g.base[v] : dsc >> 6;
+      const uint32_t deg = !on ? 0u : queued ? a.g.deg[v] : (uint32_t)(dsc & 63);
+      const double s = bc_sum_rows(a, base, deg, val);
+      if (on) bc_finish(a, b, v, lvl, down, s);
+    }
+  }
+}
+
+// The multi-leaf rows by capacity class, in two passes with a barrier between
+// them: the classes' sizes, then their rows (in any order within a class) and
+// the hubs' chunks.  A block counts in shared memory and reserves once a class.
+__device__ __forceinline__ void bc_count_classes(const BfsArgs &a, const BcArgs &b) {
+  __shared__ uint32_t s_cnt[kBcClasses];
+  if (threadIdx.x < kBcClasses) s_cnt[threadIdx.x] = 0;
+  __syncthreads();
+  const uint64_t nt = (uint64_t)gridDim.x * kCoopThreads;
+  for (uint64_t i = (uint64_t)blockIdx.x * kCoopThreads + threadIdx.x; i < b.nbig; i += nt)
+    atomicAdd(&s_cnt[bc_class(a.g.cap[b.big[i]])], 1u);
+  __syncthreads();
+  if (threadIdx.x < kBcClasses && s_cnt[threadIdx.x])
+    atomicAdd(&b.bc->count[threadIdx.x], s_cnt[threadIdx.x]);
+}
+
+__device__ __forceinline__ void bc_list_classes(const BfsArgs &a, const BcArgs &b) {
+  __shared__ uint32_t s_cnt[kBcClasses], s_at[kBcClasses];
+  const uint64_t nt = (uint64_t)gridDim.x * kCoopThreads;
+  const uint64_t t0 = (uint64_t)blockIdx.x * kCoopThreads + threadIdx.x;
+  for (uint64_t i0 = t0 - threadIdx.x; i0 < b.nbig; i0 += nt) {  // the same for the block
+    if (threadIdx.x < kBcClasses) s_cnt[threadIdx.x] = 0;
+    __syncthreads();
+    const uint64_t i = i0 + threadIdx.x;
+    const uint32_t v = i < b.nbig ? b.big[i] : 0u;
+    const uint32_t cap = i < b.nbig ? a.g.cap[v] : 0u;
+    const int cls = i < b.nbig ? bc_class(cap) : 0;
+    uint32_t r = 0;
+    if (i < b.nbig) r = atomicAdd(&s_cnt[cls], 1u);
+    __syncthreads();
+    if (threadIdx.x < kBcClasses) {
+      uint32_t at = 0;  // hubs have a list of their own
+      for (int c = 1; c < (int)threadIdx.x; c++) at += __ldcg(&b.bc->count[c]);
+      if (s_cnt[threadIdx.x]) at += atomicAdd(&b.bc->at[threadIdx.x], s_cnt[threadIdx.x]);
+      s_at[threadIdx.x] = at;
+    }
+    __syncthreads();
+    if (i < b.nbig) {
+      r += s_at[cls];
+      if (cls) {
+        if (r < b.nbig) b.order[r] = v;
+      } else {
+        const uint32_t k = ((cap >> kLeafLog) + kBcLeaves - 1) / kBcLeaves;
+        const uint32_t at = atomicAdd(&b.bc->items, k);
+        if ((uint64_t)at + k > b.max_hub || r >= b.max_hub) {
+          a.ctl->err = 2;
+        } else {
+          b.hub[r] = make_uint2(v, at);
+          b.hub_done[r] = 0;
+          for (uint32_t j = 0; j < k; j++) b.hub_item[at + j] = make_uint2(r, j);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Every level of the search; with kBc also the rows' sigma, each level's beside
+// the search for the next one.  Returns the number of levels, -1 on an error.
+template <bool kBc>
+__device__ __forceinline__ int bfs_levels(const BfsArgs &a, const BcArgs &b, GridBarrier &bar) {
   BfsCtl *ctl = a.ctl;
-  GridBarrier bar{&ctl->bar, &ctl->err, 0};
   const uint32_t t0 = blockIdx.x * kCoopThreads + threadIdx.x;
   const uint32_t nt = gridDim.x * kCoopThreads;
   for (uint64_t v = t0; v < a.g.n; v += nt) {
     a.depth[v] = v == a.src ? 0 : -1;
     if (a.parent) a.parent[v] = v == a.src ? (int32_t)a.src : -1;
+  }
+  if (kBc) {
+    for (uint64_t v = t0; v < a.g.n; v += nt) {
+      const uint64_t w = v + a.g.n;
+      b.sigma[v] = v == a.src ? 1.0 : 0.0;
+      b.sigma[w] = b.ratio[v] = b.ratio[w] = b.dep[v] = 0.0;
+    }
+    bc_count_classes(a, b);
   }
   if (t0 < 32) {  // the source's row is level 0
     const uint32_t cap = a.g.cap[a.src];
@@ -581,7 +932,7 @@ __device__ __forceinline__ void bfs_levels(const BfsArgs &a) {
       ctl->cnt[0] = BfsCount{1, sum.degrees, 1u - sum.bigs, sum.bigs, sum.items};
     }
   }
-  if (!bar.wait()) return;
+  if (!bar.wait()) return -1;
   uint32_t rows = 0, bigs = 0, items = 0;  // queue entries of the levels before
   bool queued = true;                      // this level is in the queue
   for (int lvl = 0; (uint32_t)lvl <= a.g.n; lvl++) {
@@ -589,7 +940,7 @@ __device__ __forceinline__ void bfs_levels(const BfsArgs &a) {
     // barrier, and cleared two levels on
     const BfsCount *c = &ctl->cnt[lvl % 3];
     const unsigned long long fv = __ldcg(&c->vertices), fd = __ldcg(&c->degrees);
-    if (fv == 0) return;
+    if (fv == 0) return lvl;
     const uint32_t r1 = rows + __ldcg(&c->rows), b1 = bigs + __ldcg(&c->bigs);
     const uint32_t ni = __ldcg(&c->items);
     if (t0 == 0) ctl->cnt[(lvl + 2) % 3] = BfsCount{};
@@ -597,21 +948,30 @@ __device__ __forceinline__ void bfs_levels(const BfsArgs &a) {
     const bool pull = (fv + fd) * a.alpha > a.m;
     if (pull) {
       bfs_level_bits(a, lvl);
-      if (!bar.wait()) return;
+      if (!bar.wait()) return -1;
       bfs_pull_chunks(a, lvl, sum);
       bfs_pull_small(a, lvl, sum);
     } else {
       if (!queued) {  // the level was reached by a pull
         bfs_queue_level(a, lvl);
-        if (!bar.wait()) return;
+        if (!bar.wait()) return -1;
       }
       if (b1 > bigs) {
         bfs_list_items(a, bigs, b1);
-        if (!bar.wait()) return;
+        if (!bar.wait()) return -1;
         bfs_push_items(a, items, items + ni, lvl, sum);
         items += ni;
       }
       bfs_push_rows(a, rows, r1, lvl, sum);
+    }
+    if (kBc) {
+      const bool listed = queued || !pull;
+      if (lvl)
+        bc_level(a, b, lvl, true, listed, rows, r1, bigs, b1);
+      else
+        bc_list_classes(a, b);  // from level 1 on
+      if (t0 == 0)
+        b.level[lvl] = listed ? make_uint2(r1, b1) : make_uint2(rows, bigs | kNotQueued);
     }
     if (queued || !pull) {
       rows = r1;
@@ -619,22 +979,42 @@ __device__ __forceinline__ void bfs_levels(const BfsArgs &a) {
     }
     queued = !pull;  // what a push reaches is queued
     bfs_count(&ctl->cnt[(lvl + 1) % 3], sum);
-    if (!bar.wait()) return;
+    if (!bar.wait()) return -1;
   }
   if (t0 == 0) ctl->err = 3;  // more than n levels
+  return -1;
 }
 
-__global__ void __launch_bounds__(kCoopThreads, kCoopPerSm) k_bfs_levels(BfsArgs a) {
-  bfs_levels(a);
+// the last block to leave reports the error and leaves the state zero again
+__device__ __forceinline__ void bfs_leave(const BfsArgs &a, BcCtl *bc) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    if (atomicAdd(&a.ctl->left, 1u) == gridDim.x - 1) {  // the last block
+    if (atomicAdd(&a.ctl->left, 1u) == gridDim.x - 1) {
       __threadfence();
       *a.result = *(volatile unsigned int *)&a.ctl->err;
       *a.ctl = BfsCtl{};
+      if (bc) *bc = BcCtl{};
     }
   }
+}
+
+__global__ void __launch_bounds__(kCoopThreads, kCoopPerSm) k_bfs_levels(BfsArgs a) {
+  GridBarrier bar{&a.ctl->bar, &a.ctl->err, 0};
+  bfs_levels<false>(a, BcArgs{}, bar);
+  bfs_leave(a, nullptr);
+}
+
+__global__ void __launch_bounds__(kCoopThreads, kCoopPerSm) k_bc_levels(BfsArgs a, BcArgs b) {
+  GridBarrier bar{&a.ctl->bar, &a.ctl->err, 0};
+  const int levels = bfs_levels<true>(a, b, bar);
+  for (int lvl = levels - 1; lvl >= 0; lvl--) {
+    const uint2 e = b.level[lvl], e0 = lvl ? b.level[lvl - 1] : make_uint2(0u, 0u);
+    bc_level(a, b, lvl, false, !(e.y & kNotQueued), e0.x, e.x, e0.y & ~kNotQueued,
+             e.y & ~kNotQueued);
+    if (lvl && !bar.wait()) break;
+  }
+  bfs_leave(a, b.bc);
 }
 
 }  // namespace

@@ -89,7 +89,8 @@ struct TravState {
   DevBuf<int32_t> depth_tmp, parent_tmp;
   // bc
   DevBuf<double> sigma, ratio;
-  DevBuf<uint32_t> lvl_list, lvl_cnt;
+  DevBuf<uint2> levels, hub;
+  DevBuf<uint32_t> hub_done;
   // cc
   DevBuf<uint32_t> par;
   // tc
@@ -112,7 +113,7 @@ struct TravState {
   int64_t pr_kernels = 0;      // kernels in the captured graph
   uint64_t *h_small = nullptr;  // pinned readback slots
   unsigned long long *d_small = nullptr;
-  void *d_bfs = nullptr;  // BfsCtl, zero between searches
+  void *d_bfs = nullptr;  // BfsCtl and BcCtl, zero between searches
 };
 
 // frees every buffer and the captured PageRank graph; the tuning stays, and
@@ -144,8 +145,9 @@ static void trav_buffers_release(TravState *t) {
   t->parent_tmp.release();
   t->sigma.release();
   t->ratio.release();
-  t->lvl_list.release();
-  t->lvl_cnt.release();
+  t->levels.release();
+  t->hub.release();
+  t->hub_done.release();
   t->par.release();
   t->toff.release();
   t->tlpre.release();
@@ -201,8 +203,8 @@ uint64_t trav_device_bytes(const sst_graph *g) {
   add(t->cb.cap, 8); add(t->partial.cap, 8); add(t->qa.cap, 4); add(t->qb.cap, 4);
   add(t->fbits.cap, 4); add(t->qitems.cap, 8); add(t->icnt.cap, 4); add(t->ioff.cap, 4); add(t->iv.cap, 4);
   add(t->il0.cap, 4); add(t->depth_tmp.cap, 4); add(t->parent_tmp.cap, 4);
-  add(t->sigma.cap, 8); add(t->ratio.cap, 8); add(t->lvl_list.cap, 4);
-  add(t->lvl_cnt.cap, 4); add(t->par.cap, 4); add(t->toff.cap, 8); add(t->tlpre.cap, 8);
+  add(t->sigma.cap, 8); add(t->ratio.cap, 8); add(t->levels.cap, 8);
+  add(t->hub.cap, 8); add(t->hub_done.cap, 4); add(t->par.cap, 4); add(t->toff.cap, 8); add(t->tlpre.cap, 8);
   add(t->tlcnt.cap, 8); add(t->tadj.cap, 4); add(t->titems.cap, 8); add(t->tmask.cap, 4);
   add(t->mvis.cap, 8); add(t->mfr.cap, 8);
   add(t->mfr2.cap, 8); add(t->mnx.cap, 8); add(t->msrc.cap, 8); add(t->mdepth.cap, 4);
@@ -551,40 +553,12 @@ __global__ void k_fill_d(double *__restrict__ p, uint32_t n, double x) {
   if (v < n) p[v] = x;
 }
 
-// ------------------------------------------------------------- bfs
-__global__ void k_bfs_init(int32_t *__restrict__ depth, int32_t *__restrict__ parent,
-                           uint32_t n, uint32_t src) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  depth[v] = v == src ? 0 : -1;
-  parent[v] = v == src ? (int32_t)src : -1;
-}
-
-// warp-aggregated append of `mine` to the next queue
-// counters: [0] queue length, [1] degree sum, [2] work items of the queue
-__device__ __forceinline__ void enqueue(bool mine, uint32_t w, uint32_t wdeg,
-                                        uint32_t witems, uint32_t *q,
-                                        unsigned long long *qlen_deg) {
-  const int lane = threadIdx.x & 31;
-  uint32_t m = __ballot_sync(0xffffffffu, mine);
-  if (!m) return;
-  uint32_t dsum = __reduce_add_sync(0xffffffffu, mine ? wdeg : 0u);
-  uint32_t isum = __reduce_add_sync(0xffffffffu, mine ? witems : 0u);
-  int leader = __ffs(m) - 1;
-  unsigned long long base = 0;
-  if (lane == leader) {
-    base = atomicAdd(&qlen_deg[0], (unsigned long long)__popc(m));
-    atomicAdd(&qlen_deg[1], (unsigned long long)dsum);
-    atomicAdd(&qlen_deg[2], (unsigned long long)isum);
-  }
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (mine) q[base + __popc(m & ((1u << lane) - 1u))] = w;
-}
-
-// Block-aggregated form of enqueue for kernels in which every thread of the
+// ------------------------------------------------------- frontier queues
+// Append of `mine` to the next queue, for kernels in which every thread of the
 // block calls it once: one atomic per counter per block (the three queue
 // counters are single addresses, so per-warp atomics from a whole grid
-// serialise on them).
+// serialise on them).  Counters: [0] queue length, [1] degree sum, [2] work
+// items of the queue.
 __device__ __forceinline__ void enqueue_block(bool mine, uint32_t w, uint32_t wdeg,
                                               uint32_t witems, uint32_t *q,
                                               unsigned long long *qlen_deg) {
@@ -647,210 +621,6 @@ __global__ void k_front_expand(const uint32_t *__restrict__ q, uint32_t qn,
     iv[o + j] = v;
     il0[o + j] = j * kPushLeaves;
   }
-}
-
-// push: warp per work item (a frontier vertex's leaf chunk), lane = slot;
-// four leaves' slots, depths and claims are in flight at once, their newly
-// reached vertices take queue positions with one atomic per warp and batch,
-// and the warp adds its degree and work-item sums once
-__global__ void __launch_bounds__(kTB, 8)
-k_bfs_push(DGraph g, const uint32_t *__restrict__ iv,
-           const uint32_t *__restrict__ il0, uint32_t nitems,
-           int32_t *__restrict__ depth, int32_t *__restrict__ parent,
-           uint32_t *__restrict__ nq, unsigned long long *__restrict__ cnt,
-           int lvl) {
-  constexpr int kBatch = 4;  // leaves whose slots are in flight at once
-  const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (i >= nitems) return;
-  const uint32_t u = iv[i];
-  const uint64_t base = g.base[u];
-  const uint32_t cap = g.cap[u], deg = g.deg[u];
-  const uint32_t nl = cap ? nleaves_of(cap) : 0;
-  const uint32_t l0 = il0[i], l1 = min(l0 + kPushLeaves, nl);
-  // a one-leaf segment holds deg ids; a multi-leaf segment's leaves hold
-  // their ids packed left with EMPTY after them, so no leaf counts are read
-  const uint32_t lim = cap <= kLeaf ? deg : kLeaf;
-  const uint32_t below = (1u << lane) - 1u;
-  unsigned long long dsum = 0, isum = 0;
-  for (uint32_t l = l0; l < l1; l += kBatch) {
-    uint32_t w[kBatch];
-#pragma unroll
-    for (int k = 0; k < kBatch; k++)
-      w[k] = (l + k < l1 && (uint32_t)lane < lim)
-                 ? g.slots[base + ((uint64_t)(l + k) << kLeafLog) + lane]
-                 : kEmpty;
-    int32_t dd[kBatch];
-#pragma unroll
-    for (int k = 0; k < kBatch; k++) dd[k] = w[k] != kEmpty ? depth[w[k]] : 0;
-    uint32_t mine = 0;  // bit k: this lane claimed w[k]
-#pragma unroll
-    for (int k = 0; k < kBatch; k++)
-      if (dd[k] < 0 && atomicCAS(&depth[w[k]], -1, lvl + 1) == -1)
-        mine |= 1u << k;
-    // one queue reservation per batch, in (leaf, lane) order; leaves past
-    // the chunk's end (warp-uniform) take no ballot
-    uint32_t mm[kBatch], total = 0;
-#pragma unroll
-    for (int k = 0; k < kBatch; k++) {
-      mm[k] = l + k < l1 ? __ballot_sync(0xffffffffu, (mine >> k) & 1u) : 0u;
-      total += __popc(mm[k]);
-    }
-    if (total == 0) continue;
-    unsigned long long at = 0;
-    if (lane == 0) at = atomicAdd(&cnt[0], (unsigned long long)total);
-    at = __shfl_sync(0xffffffffu, at, 0);
-#pragma unroll
-    for (int k = 0; k < kBatch; k++) {
-      if ((mine >> k) & 1u) {
-        nq[at + __popc(mm[k] & below)] = w[k];
-        parent[w[k]] = (int32_t)u;
-        dsum += g.deg[w[k]];
-        isum += items_of(g.cap[w[k]]);
-      }
-      at += __popc(mm[k]);
-    }
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    dsum += __shfl_xor_sync(0xffffffffu, dsum, d);
-    isum += __shfl_xor_sync(0xffffffffu, isum, d);
-  }
-  if (lane == 0 && (dsum || isum)) {
-    atomicAdd(&cnt[1], dsum);
-    atomicAdd(&cnt[2], isum);
-  }
-}
-
-__global__ void k_q2bits(const uint32_t *__restrict__ q, uint32_t qn,
-                         uint32_t *__restrict__ bits) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= qn) return;
-  uint32_t u = q[i];
-  atomicOr(&bits[u >> 5], 1u << (u & 31));
-}
-
-__device__ __forceinline__ bool in_front(const uint32_t *bits, uint32_t u) {
-  return (bits[u >> 5] >> (u & 31)) & 1u;
-}
-
-// pull, one-leaf vertices (the one-leaf list): a group of 8 lanes per
-// vertex, 4 slots per lane, four vertices per group in flight; the parent is
-// the smallest frontier neighbour
-__global__ void k_bfs_pull_small8(DGraph g, const unsigned long long *__restrict__ sdesc,
-                                  const uint32_t *__restrict__ small, uint64_t nsmall,
-                                  const uint32_t *__restrict__ fbits,
-                                  int32_t *__restrict__ depth,
-                                  int32_t *__restrict__ parent,
-                                  uint32_t *__restrict__ nq,
-                                  unsigned long long *__restrict__ cnt, int lvl) {
-  const uint64_t grp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-  const uint32_t sub = threadIdx.x & 7;
-  const uint64_t i0 = grp * 4;
-  // each stage's loads for the group's four vertices go out together: the
-  // list entries, then their depths, then the open ones' slots, then the
-  // frontier bits of those neighbours
-  uint32_t v[4], d[4];
-  unsigned long long dsc[4];
-#pragma unroll
-  for (int u = 0; u < 4; u++) {
-    const bool in = i0 + u < nsmall;
-    v[u] = in ? small[i0 + u] : 0u;
-    dsc[u] = in ? sdesc[i0 + u] : 0ull;
-    d[u] = (uint32_t)(dsc[u] & 63);
-  }
-  bool open[4];
-#pragma unroll
-  for (int u = 0; u < 4; u++) open[u] = i0 + u < nsmall && depth[v[u]] < 0;
-  uint32_t w[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; u++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const uint32_t j = sub + 8 * q;
-      w[u][q] = (open[u] && j < d[u]) ? g.slots[(dsc[u] >> 6) + j] : kEmpty;
-    }
-  uint32_t fb[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; u++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) fb[u][q] = w[u][q] != kEmpty ? fbits[w[u][q] >> 5] : 0u;
-  bool mine = false;
-  uint32_t myv = 0, mydeg = 0;
-#pragma unroll
-  for (int u = 0; u < 4; u++) {
-    uint32_t best = kEmpty;
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (((fb[u][q] >> (w[u][q] & 31)) & 1u) && w[u][q] < best) best = w[u][q];
-    // smallest frontier neighbour over the group's 8 lanes
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (sub == (uint32_t)u && open[u] && best != kEmpty) {
-      depth[v[u]] = lvl + 1;
-      parent[v[u]] = (int32_t)best;
-      mine = true;
-      myv = v[u];
-      mydeg = d[u];
-    }
-  }
-  enqueue_block(mine, myv, mydeg, 1u, nq, cnt);
-}
-
-// pull, multi-leaf vertices: warp per chunk of the work lists (lane = slot,
-// eight leaves in flight), stops at the first frontier neighbour or once
-// another chunk has claimed the vertex; the claim is a compare-and-swap on
-// its depth, so one chunk records it
-__global__ void k_bfs_pull_chunks(DGraph g, const unsigned long long *__restrict__ cdesc,
-                                  const uint32_t *__restrict__ cv, uint64_t nchunks,
-                                  const uint32_t *__restrict__ fbits,
-                                  int32_t *__restrict__ depth,
-                                  int32_t *__restrict__ parent,
-                                  uint32_t *__restrict__ nq,
-                                  unsigned long long *__restrict__ cnt, int lvl) {
-  const uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  bool mine = false;
-  uint32_t v = 0;
-  if (c < nchunks) {
-    v = cv[c];
-    // the chunk's descriptor and leaf counts load beside the depth check
-    const unsigned long long dsc = cdesc[c];
-    const uint64_t leaf0 = dsc >> 8;
-    const uint32_t l1 = (uint32_t)(dsc & 63);
-    const uint32_t mycnt = (uint32_t)lane < l1 ? g.lcnt[leaf0 + lane] : 0u;
-    // another chunk may claim v at any time: every lane follows lane 0's
-    // reading, so the warp stays converged for its shuffles
-    if (__shfl_sync(0xffffffffu, __ldcg(depth + v), 0) < 0) {
-      const uint32_t *sl = g.slots + (leaf0 << kLeafLog) + lane;
-      uint32_t found = kEmpty;
-      for (uint32_t l = 0; l < l1 && found == kEmpty; l += 8) {
-        uint32_t x[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-          uint32_t cq = __shfl_sync(0xffffffffu, mycnt, (l + q) & 31);
-          if (l + q >= l1) cq = 0;
-          x[q] = (uint32_t)lane < cq ? sl[(uint64_t)(l + q) << kLeafLog] : kEmpty;
-        }
-        // the eight frontier words load together, then the smallest hit
-        uint32_t fw[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) fw[q] = x[q] != kEmpty ? fbits[x[q] >> 5] : 0u;
-        uint32_t best = kEmpty;
-#pragma unroll
-        for (int q = 0; q < 8; q++)
-          if (((fw[q] >> (x[q] & 31)) & 1u) && x[q] < best) best = x[q];
-        found = __reduce_min_sync(0xffffffffu, best);
-        if (found == kEmpty && __shfl_sync(0xffffffffu, __ldcg(depth + v), 0) >= 0)
-          break;  // claimed by another chunk
-      }
-      if (found != kEmpty && lane == 0 && atomicCAS(&depth[v], -1, lvl + 1) == -1) {
-        parent[v] = (int32_t)found;
-        mine = true;
-      }
-    }
-  }
-  enqueue_block(mine, v, mine ? g.deg[v] : 0u, mine ? items_of(g.cap[v]) : 0u, nq, cnt);
 }
 
 // ------------------------------------------------------------- cc
@@ -988,47 +758,8 @@ __device__ __forceinline__ void block_max_to(int32_t d, unsigned long long *out)
   if (threadIdx.x == 0 && s_max >= 0) atomicMax(out, (unsigned long long)s_max);
 }
 
-__global__ void k_bc_init(double *__restrict__ sigma, double *__restrict__ ratio,
-                          double *__restrict__ dep, uint32_t n, uint32_t src) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  sigma[v] = v == src ? 1.0 : 0.0;
-  ratio[v] = 0.0;
-  dep[v] = 0.0;
-}
-
 // neighbours (or leaves) whose loads the BC kernels keep in flight together
 constexpr int kBcAhead = 8;
-
-// sigma(v) = sum of sigma over neighbours one level up (thread per vertex)
-__global__ void k_sigma_small(DGraph g, const uint32_t *__restrict__ list,
-                              uint32_t cnt, const int32_t *__restrict__ depth,
-                              double *__restrict__ sigma, int32_t d) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cnt) return;
-  uint32_t v = list[i];
-  if (g.cap[v] > kLeaf) return;
-  const uint32_t *p = g.slots + g.base[v];
-  uint32_t dg = g.deg[v];
-  double s = 0.0;
-  // kBcAhead neighbours at a time, each load stage issued for all of them
-  // before any is used; the sum keeps neighbour order
-  for (uint32_t k0 = 0; k0 < dg; k0 += kBcAhead) {
-    uint32_t u[kBcAhead];
-    bool on[kBcAhead];
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++) u[q] = k0 + q < dg ? p[k0 + q] : 0u;
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++) on[q] = k0 + q < dg && depth[u[q]] == d - 1;
-    double x[kBcAhead];
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++) x[q] = on[q] ? sigma[u[q]] : 0.0;
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++)
-      if (on[q]) s += x[q];
-  }
-  sigma[v] = s;
-}
 
 // items (big vertices of the level list, one per leaf chunk)
 __global__ void k_bc_item_counts(const uint32_t *__restrict__ list, uint32_t nl,
@@ -1057,103 +788,6 @@ __global__ void k_gather_bounds(const uint32_t *__restrict__ off,
                                 uint32_t *__restrict__ out) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < k) out[i] = off[pos[i]];
-}
-
-// warp per chunk: partial sum of val[u] over the chunk's neighbours u at
-// depth want (sigma pass: want = d-1 over sigma; dependency pass: want =
-// d+1 over ratio)
-__global__ void k_bc_chunks(DGraph g, const uint32_t *__restrict__ iv,
-                            const uint32_t *__restrict__ il0, uint32_t i0,
-                            uint32_t ni, const int32_t *__restrict__ depth,
-                            const double *__restrict__ val, int32_t want,
-                            double *__restrict__ partial) {
-  uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (i >= ni) return;
-  i += i0;
-  uint32_t v = iv[i];
-  uint32_t nl = g.cap[v] >> kLeafLog;
-  uint32_t l0 = il0[i], l1 = min(l0 + kChunkLeaves, nl);
-  uint64_t base = g.base[v];
-  const uint8_t *lc = g.lcnt + (base >> kLeafLog);
-  double acc = 0.0;
-  // kBcAhead leaves at a time, each load stage issued for all of them before
-  // any is used; the sum keeps leaf order
-  for (uint32_t l = l0; l < l1; l += kBcAhead) {
-    uint32_t u[kBcAhead];
-    bool on[kBcAhead];
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++) on[q] = l + q < l1 && (uint32_t)lane < lc[l + q];
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++)
-      u[q] = on[q] ? g.slots[base + ((uint64_t)(l + q) << kLeafLog) + lane] : 0u;
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++) on[q] = on[q] && depth[u[q]] == want;
-    double x[kBcAhead];
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++) x[q] = on[q] ? val[u[q]] : 0.0;
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++)
-      if (on[q]) acc += x[q];
-  }
-  double s = warp_sum_d(acc);
-  if (lane == 0) partial[i] = s;
-}
-
-// thread per big vertex of the level: combine its chunk partials in order
-__global__ void k_bc_fix(const uint32_t *__restrict__ list, uint32_t p0,
-                         uint32_t np, const uint32_t *__restrict__ cnt,
-                         const uint32_t *__restrict__ off,
-                         const double *__restrict__ partial, bool sigma_pass,
-                         double *__restrict__ sigma, double *__restrict__ ratio,
-                         double *__restrict__ dep) {
-  uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= np) return;
-  p += p0;
-  uint32_t k = cnt[p];
-  if (k == 0) return;
-  double s = 0.0;
-  for (uint32_t j = 0; j < k; j++) s += partial[off[p] + j];
-  uint32_t v = list[p];
-  if (sigma_pass) {
-    sigma[v] = s;
-  } else {
-    double dv = sigma[v] * s;
-    dep[v] = dv;
-    ratio[v] = (1.0 + dv) / sigma[v];
-  }
-}
-
-// dep(v) = sigma(v) * sum over neighbours one level down of (1+dep(w))/sigma(w)
-__global__ void k_delta_small(DGraph g, const uint32_t *__restrict__ list,
-                              uint32_t cnt, const int32_t *__restrict__ depth,
-                              const double *__restrict__ sigma,
-                              double *__restrict__ ratio,
-                              double *__restrict__ dep, int32_t d) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cnt) return;
-  uint32_t v = list[i];
-  if (g.cap[v] > kLeaf) return;
-  const uint32_t *p = g.slots + g.base[v];
-  uint32_t dg = g.deg[v];
-  double s = 0.0;
-  for (uint32_t k0 = 0; k0 < dg; k0 += kBcAhead) {  // as in k_sigma_small
-    uint32_t w[kBcAhead];
-    bool on[kBcAhead];
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++) w[q] = k0 + q < dg ? p[k0 + q] : 0u;
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++) on[q] = k0 + q < dg && depth[w[q]] == d + 1;
-    double x[kBcAhead];
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++) x[q] = on[q] ? ratio[w[q]] : 0.0;
-#pragma unroll
-    for (int q = 0; q < kBcAhead; q++)
-      if (on[q]) s += x[q];
-  }
-  double dv = sigma[v] * s;
-  dep[v] = dv;
-  ratio[v] = (1.0 + dv) / sigma[v];
 }
 
 // ------------------------------------------------------------- tc
@@ -1350,8 +984,8 @@ static TravState *state(sst_graph *g) {
     g->trav = new TravState();
     cudaMallocHost(&g->trav->h_small, 64 * sizeof(uint64_t));
     cudaMalloc(&g->trav->d_small, 64 * sizeof(unsigned long long));
-    cudaMalloc(&g->trav->d_bfs, sizeof(BfsCtl));
-    cudaMemsetAsync(g->trav->d_bfs, 0, sizeof(BfsCtl), g->stream);
+    cudaMalloc(&g->trav->d_bfs, sizeof(BfsCtl) + sizeof(BcCtl));
+    cudaMemsetAsync(g->trav->d_bfs, 0, sizeof(BfsCtl) + sizeof(BcCtl), g->stream);
   }
   return g->trav;
 }
@@ -1568,100 +1202,6 @@ sst_status pagerank(sst_graph *g, uint32_t iters, double damping, double *d_rank
   return SST_OK;
 }
 
-// BFS from src; with d_levels (n entries, device) it also lists the vertices
-// level by level, as the level queues come (each level's new queue is
-// copied after the level), their counts in *level_counts.
-static sst_status bfs_run(sst_graph *g, uint32_t src, int32_t *d_parents, int32_t *d_depths,
-                          uint32_t *d_levels, std::vector<uint32_t> *level_counts) {
-  sst_status st = ensure_lists(g);
-  if (st != SST_OK) return st;
-  TravState *t = g->trav;
-  cudaStream_t s = g->stream;
-  uint32_t n = g->n;
-  SST_CUDA_TRY(t->qa.ensure(n + 1));
-  SST_CUDA_TRY(t->qb.ensure(n + 1));
-  SST_CUDA_TRY(t->fbits.ensure(n / 32 + 2));
-  int32_t *depth = d_depths, *parent = d_parents;
-  if (!depth) {
-    SST_CUDA_TRY(t->depth_tmp.ensure(n));
-    depth = t->depth_tmp.p;
-  }
-  if (!parent) {
-    SST_CUDA_TRY(t->parent_tmp.ensure(n));
-    parent = t->parent_tmp.p;
-  }
-  DGraph dg = g->view();
-  SST_LAUNCH(k_bfs_init, blocks_for(n), kTB, 0, s, depth, parent, n, src);
-  SST_CUDA_TRY(cudaMemcpyAsync(t->qa.p, &src, 4, cudaMemcpyHostToDevice, s));
-  uint32_t sinfo[2] = {0, 0};
-  SST_CUDA_TRY(cudaMemcpyAsync(&sinfo[0], g->d_deg + src, 4, cudaMemcpyDeviceToHost, s));
-  SST_CUDA_TRY(cudaMemcpyAsync(&sinfo[1], g->d_cap + src, 4, cudaMemcpyDeviceToHost, s));
-  SST_CUDA_TRY(cudaStreamSynchronize(s));
-  uint64_t qn = 1, qdeg = sinfo[0];
-  uint64_t qitems = sinfo[1] > kLeaf ? ((sinfo[1] >> kLeafLog) + kPushLeaves - 1) / kPushLeaves : 1;
-  uint32_t *q = t->qa.p, *nq = t->qb.p;
-  unsigned long long *cnt = t->d_small;
-  const uint64_t m = g->m;
-  uint64_t listed = 0;  // vertices listed in d_levels so far
-  if (d_levels) {
-    level_counts->assign(1, 1u);  // level 0: the source
-    SST_CUDA_TRY(cudaMemcpyAsync(d_levels, &src, 4, cudaMemcpyHostToDevice, s));
-    listed = 1;
-  }
-  SST_CUDA_TRY(t->icnt.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->ioff.ensure((uint64_t)n + 1));
-  g->arena.reset();
-  SST_CUDA_TRY(g->arena.reserve(scan_scratch_bytes((uint64_t)n + 1, 4) + 4096));
-  for (int lvl = 0; qn > 0; lvl++) {
-    if ((uint64_t)lvl > n) {
-      set_error_message("BFS exceeded n levels");
-      return SST_ETIMEDOUT;
-    }
-    SST_CUDA_TRY(cudaMemsetAsync(cnt, 0, 24, s));
-    if ((qn + qdeg) * t->bfs_alpha > m) {
-      SST_CUDA_TRY(cudaMemsetAsync(t->fbits.p, 0, ((uint64_t)n / 32 + 1) * 4, s));
-      SST_LAUNCH(k_q2bits, blocks_for(qn), kTB, 0, s, q, (uint32_t)qn, t->fbits.p);
-      if (t->nsmall)
-        SST_LAUNCH(k_bfs_pull_small8, blocks_for((t->nsmall + 3) / 4 * 8), kTB, 0,
-                   s, dg, t->sdesc.p, t->small.p, t->nsmall, t->fbits.p, depth,
-                   parent, nq, cnt, lvl);
-      if (t->nchunks)
-        SST_LAUNCH(k_bfs_pull_chunks, warp_blocks(t->nchunks), kTB, 0, s, dg,
-                   t->cdesc.p, t->cv.p, t->nchunks, t->fbits.p, depth, parent,
-                   nq, cnt, lvl);
-    } else {
-      SST_CUDA_TRY(t->iv.ensure(qitems + 1));
-      SST_CUDA_TRY(t->il0.ensure(qitems + 1));
-      SST_LAUNCH(k_front_items, blocks_for(qn), kTB, 0, s, q, (uint32_t)qn,
-                 g->d_cap, t->icnt.p);
-      g->arena.reset();
-      SST_CUDA_TRY((scan<uint32_t, OpAdd>(t->icnt.p, t->ioff.p, qn, 0u, OpAdd{},
-                                          true, false, nullptr, g->arena, s)));
-      SST_LAUNCH(k_front_expand, blocks_for(qn), kTB, 0, s, q, (uint32_t)qn,
-                 g->d_cap, t->ioff.p, t->iv.p, t->il0.p);
-      SST_LAUNCH(k_bfs_push, warp_blocks(qitems), kTB, 0, s, dg, t->iv.p, t->il0.p,
-                 (uint32_t)qitems, depth, parent, nq, cnt, lvl);
-    }
-    SST_CUDA_TRY(cudaMemcpyAsync(t->h_small, cnt, 24, cudaMemcpyDeviceToHost, s));
-    SST_CUDA_TRY(cudaStreamSynchronize(s));
-    qn = t->h_small[0];
-    qdeg = t->h_small[1];
-    qitems = t->h_small[2];
-    if (d_levels && qn) {
-      if (listed + qn > n) {
-        set_error_message("BFS listed more than n vertices");
-        return SST_EDEVICE;
-      }
-      SST_CUDA_TRY(cudaMemcpyAsync(d_levels + listed, nq, qn * 4, cudaMemcpyDeviceToDevice, s));
-      level_counts->push_back((uint32_t)qn);
-      listed += qn;
-    }
-    std::swap(q, nq);
-  }
-  SST_CUDA_TRY(cudaGetLastError());
-  return SST_OK;
-}
-
 // blocks of a cooperative grid for `threads` threads of work: no more than the
 // work fills (see bfslevels.cuh), no more than fit at once
 static sst_status coop_grid(const sst_graph *g, const void *kernel, uint64_t threads,
@@ -1677,11 +1217,13 @@ static sst_status coop_grid(const sst_graph *g, const void *kernel, uint64_t thr
   return SST_OK;
 }
 
-sst_status bfs(sst_graph *g, uint32_t src, int32_t *d_parents, int32_t *d_depths) {
+// A search's arguments over the graph's work lists, and its grid (see
+// bfslevels.cuh).  d_depths may be null (a temporary), d_parents too (none).
+static sst_status bfs_setup(sst_graph *g, uint32_t src, int32_t *d_parents, int32_t *d_depths,
+                            const void *kernel, BfsArgs *a, unsigned *grid) {
   sst_status st = ensure_lists(g);
   if (st != SST_OK) return st;
   TravState *t = g->trav;
-  cudaStream_t s = g->stream;
   const uint32_t n = g->n;
   // a row's push items are at most 32 / kBfsLeaves for each of its chunks in
   // the lists (chunks of up to 32 leaves)
@@ -1693,25 +1235,34 @@ sst_status bfs(sst_graph *g, uint32_t src, int32_t *d_parents, int32_t *d_depths
     SST_CUDA_TRY(t->depth_tmp.ensure(n));
     d_depths = t->depth_tmp.p;
   }
-  BfsCtl *ctl = reinterpret_cast<BfsCtl *>(t->d_bfs);
-  const BfsArgs a{g->view(), g->m,        src,        t->bfs_alpha, t->small.p,
-                  t->sdesc.p, t->nsmall,  t->cv.p,    t->cdesc.p,   t->nchunks,
-                  d_depths,  d_parents,   t->fbits.p, t->qa.p,      t->qitems.p,
-                  max_items, ctl, reinterpret_cast<unsigned long long *>(t->h_small)};
+  *a = BfsArgs{g->view(),   g->m,       src,         t->bfs_alpha, t->small.p,
+               t->sdesc.p,  t->nsmall,  t->cv.p,     t->cdesc.p,   t->nchunks,
+               d_depths,    d_parents,  t->fbits.p,  t->qa.p,      t->qitems.p,
+               max_items,   reinterpret_cast<BfsCtl *>(t->d_bfs),
+               reinterpret_cast<unsigned long long *>(t->h_small)};
+  return coop_grid(g, kernel, std::max(t->nsmall, 32 * t->nchunks), grid);
+}
+
+// waits for a search and reports its error
+static sst_status bfs_finish(sst_graph *g, const char *what) {
+  SST_CUDA_TRY(cudaStreamSynchronize(g->stream));
+  const uint64_t err = *(volatile uint64_t *)g->trav->h_small;
+  if (!err) return SST_OK;
+  set_error_message(err == 1   ? "%s: a grid barrier timed out"
+                    : err == 2 ? "%s: a level queue overflowed"
+                               : "%s exceeded n levels",
+                    what);
+  return err == 2 ? SST_EDEVICE : SST_ETIMEDOUT;
+}
+
+sst_status bfs(sst_graph *g, uint32_t src, int32_t *d_parents, int32_t *d_depths) {
+  BfsArgs a;
   unsigned grid = 1;
-  st = coop_grid(g, reinterpret_cast<const void *>(k_bfs_levels),
-                 std::max(t->nsmall, 32 * t->nchunks), &grid);
+  sst_status st = bfs_setup(g, src, d_parents, d_depths,
+                            reinterpret_cast<const void *>(k_bfs_levels), &a, &grid);
   if (st != SST_OK) return st;
-  SST_CUDA_TRY(launch_coop("k_bfs_levels", k_bfs_levels, grid, kCoopThreads, s, a));
-  SST_CUDA_TRY(cudaStreamSynchronize(s));
-  const uint64_t err = *(volatile uint64_t *)t->h_small;
-  if (err) {
-    set_error_message(err == 1   ? "BFS: a grid barrier timed out"
-                      : err == 2 ? "BFS: a level queue overflowed"
-                                 : "BFS exceeded n levels");
-    return err == 2 ? SST_EDEVICE : SST_ETIMEDOUT;
-  }
-  return SST_OK;
+  SST_CUDA_TRY(launch_coop("k_bfs_levels", k_bfs_levels, grid, kCoopThreads, g->stream, a));
+  return bfs_finish(g, "BFS");
 }
 
 sst_status cc(sst_graph *g, uint32_t *d_labels) {
@@ -1759,80 +1310,28 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
 }
 
 sst_status bc(sst_graph *g, uint32_t src, double *d_dep) {
-  TravState *t = state(g);
-  uint32_t n = g->n;
-  SST_CUDA_TRY(t->depth_tmp.ensure(n));
-  SST_CUDA_TRY(t->lvl_list.ensure(n + 1));
-  // the BFS lists the vertices level by level as its queues come (their
-  // order within a level does not enter any per-vertex sum below)
-  std::vector<uint32_t> hc;
-  sst_status st = bfs_run(g, src, nullptr, t->depth_tmp.p, t->lvl_list.p, &hc);
+  BfsArgs a;
+  unsigned grid = 1;
+  sst_status st = bfs_setup(g, src, nullptr, nullptr,
+                            reinterpret_cast<const void *>(k_bc_levels), &a, &grid);
   if (st != SST_OK) return st;
-  cudaStream_t s = g->stream;
-  const int32_t *depth = t->depth_tmp.p;
-  const uint32_t D = (uint32_t)hc.size() - 1;  // deepest level
-  hc.resize(D + 2, 0u);
-  SST_CUDA_TRY(t->lvl_cnt.ensure(2 * ((uint64_t)D + 2)));
-  SST_CUDA_TRY(t->sigma.ensure(n));
-  SST_CUDA_TRY(t->ratio.ensure(n));
-  uint32_t *off = t->lvl_cnt.p, *ibound = off + D + 2;
-  std::vector<uint32_t> ho(D + 2), hib(D + 2);
-  uint32_t acc = 0;
-  for (uint32_t d = 0; d <= D; d++) {
-    ho[d] = acc;
-    acc += hc[d];
-  }
-  ho[D + 1] = acc;
-  const uint32_t R = acc;  // reached vertices
-  SST_CUDA_TRY(cudaMemcpyAsync(off, ho.data(), (D + 2) * 4, cudaMemcpyHostToDevice, s));
-  // chunk items of the big vertices, in level-list order
-  SST_CUDA_TRY(t->icnt.ensure((uint64_t)R + 1));
-  SST_CUDA_TRY(t->ioff.ensure((uint64_t)R + 1));
-  const uint32_t *list = t->lvl_list.p;
-  SST_LAUNCH(k_bc_item_counts, blocks_for(R), kTB, 0, s, list, R, g->d_cap, t->icnt.p);
-  g->arena.reset();
-  SST_CUDA_TRY(g->arena.reserve(scan_scratch_bytes((uint64_t)R + 1, 4) + 4096));
-  SST_CUDA_TRY((scan<uint32_t, OpAdd>(t->icnt.p, t->ioff.p, R, 0u, OpAdd{}, true,
-                                      false, t->ioff.p + R, g->arena, s)));
-  SST_LAUNCH(k_gather_bounds, blocks_for(D + 2), kTB, 0, s, t->ioff.p, off,
-             D + 2, ibound);
-  SST_CUDA_TRY(cudaMemcpyAsync(hib.data(), ibound, (D + 2) * 4, cudaMemcpyDeviceToHost, s));
-  SST_CUDA_TRY(cudaStreamSynchronize(s));
-  uint32_t items = hib[D + 1];
-  SST_CUDA_TRY(t->iv.ensure((uint64_t)items + 1));
-  SST_CUDA_TRY(t->il0.ensure((uint64_t)items + 1));
-  SST_CUDA_TRY(t->partial.ensure((uint64_t)items + 1));
-  if (items)
-    SST_LAUNCH(k_bc_expand, blocks_for(R), kTB, 0, s, list, R, t->icnt.p,
-               t->ioff.p, t->iv.p, t->il0.p);
-  SST_LAUNCH(k_bc_init, blocks_for(n), kTB, 0, s, t->sigma.p, t->ratio.p, d_dep, n, src);
-  DGraph dg = g->view();
-  double *part = t->partial.p;
-  for (uint32_t d = 1; d <= D; d++) {
-    uint32_t c = hc[d], ni = hib[d + 1] - hib[d];
-    const uint32_t *lst = list + ho[d];
-    SST_LAUNCH(k_sigma_small, blocks_for(c), kTB, 0, s, dg, lst, c, depth, t->sigma.p, (int32_t)d);
-    if (ni) {
-      SST_LAUNCH(k_bc_chunks, warp_blocks(ni), kTB, 0, s, dg, t->iv.p, t->il0.p,
-                 hib[d], ni, depth, t->sigma.p, (int32_t)d - 1, part);
-      SST_LAUNCH(k_bc_fix, blocks_for(c), kTB, 0, s, list, ho[d], c, t->icnt.p,
-                 t->ioff.p, part, true, t->sigma.p, t->ratio.p, d_dep);
-    }
-  }
-  for (int32_t d = (int32_t)D; d >= 0; d--) {
-    uint32_t c = hc[d], ni = hib[d + 1] - hib[d];
-    const uint32_t *lst = list + ho[d];
-    SST_LAUNCH(k_delta_small, blocks_for(c), kTB, 0, s, dg, lst, c, depth,
-               t->sigma.p, t->ratio.p, d_dep, d);
-    if (ni) {
-      SST_LAUNCH(k_bc_chunks, warp_blocks(ni), kTB, 0, s, dg, t->iv.p, t->il0.p,
-                 hib[d], ni, depth, t->ratio.p, d + 1, part);
-      SST_LAUNCH(k_bc_fix, blocks_for(c), kTB, 0, s, list, ho[d], c, t->icnt.p,
-                 t->ioff.p, part, false, t->sigma.p, t->ratio.p, d_dep);
-    }
-  }
-  SST_CUDA_TRY(cudaGetLastError());
-  return SST_OK;
+  TravState *t = g->trav;
+  const uint64_t n = g->n;
+  SST_CUDA_TRY(t->sigma.ensure(2 * n));
+  SST_CUDA_TRY(t->ratio.ensure(2 * n));
+  SST_CUDA_TRY(t->levels.ensure(n + 1));
+  SST_CUDA_TRY(t->qb.ensure(n + 1));
+  // a hub's chunks of kBcLeaves leaves are at most its chunks in the lists
+  const uint64_t hubs = t->nchunks + 1;
+  SST_CUDA_TRY(t->hub.ensure(2 * hubs));
+  SST_CUDA_TRY(t->hub_done.ensure(hubs));
+  SST_CUDA_TRY(t->partial.ensure(hubs));
+  const BcArgs b{t->sigma.p,    t->ratio.p,        d_dep,        t->big.p,
+                 t->nbig,       hubs,              t->hub.p,     t->hub.p + hubs,
+                 t->partial.p,  t->hub_done.p,     t->qb.p,
+                 reinterpret_cast<BcCtl *>(a.ctl + 1), t->levels.p};
+  SST_CUDA_TRY(launch_coop("k_bc_levels", k_bc_levels, grid, kCoopThreads, g->stream, a, b));
+  return bfs_finish(g, "BC");
 }
 
 sst_status tc(sst_graph *g, uint64_t *total, uint64_t *d_pv) {
