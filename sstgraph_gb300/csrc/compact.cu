@@ -1231,7 +1231,7 @@ sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) 
   uint64_t *off = nullptr, *doff = nullptr;
   uint32_t *cols = nullptr, *keep = nullptr, *pos = nullptr, *adj = nullptr;
   uint32_t *icnt = nullptr, *ioff = nullptr;
-  uint64_t *items = nullptr;
+  uint64_t *items = nullptr, *desc = nullptr;
   cudaError_t e = cudaMalloc(&off, ((uint64_t)n + 1) * 8);
   if (e == cudaSuccess) e = cudaMalloc(&doff, ((uint64_t)n + 1) * 8);
   if (e == cudaSuccess) e = cudaMalloc(&cols, m * 4);
@@ -1240,8 +1240,10 @@ sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) 
   if (e == cudaSuccess) e = cudaMalloc(&adj, m * 4);
   if (e == cudaSuccess) e = cudaMalloc(&icnt, ((uint64_t)n + 1) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&ioff, ((uint64_t)n + 1) * 4);
-  // m bounds the oriented entries
-  if (e == cudaSuccess) e = cudaMalloc(&items, tc_items_bound(n, m) * 8);
+  // an item per started batch of 32 of a row
+  const uint64_t max_items = m / kTcBatch + n;
+  if (e == cudaSuccess) e = cudaMalloc(&items, max_items * 8);
+  if (e == cudaSuccess) e = cudaMalloc(&desc, (uint64_t)n * 8);
   if (e == cudaSuccess) {
     st = compact_to_csr(c, off, cols);
     if (st == SST_OK) {
@@ -1258,9 +1260,16 @@ sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) 
           SST_LAUNCH(k_ctc_off, blocks_for((uint64_t)n + 1), kTB, 0, s, off, pos, n, m, doff);
           e = cudaMemsetAsync(c->d_cnt, 0, 16, s);  // count, work cursor
           A.reset();
-          if (e == cudaSuccess)
-            e = tc_count_launch(doff, adj, n, m, TcScratch{icnt, ioff, items}, A, c->d_cnt,
+          if (e == cudaSuccess) {
+            SST_LAUNCH(k_tc_desc, blocks_for(n), kTB, 0, s, doff, n, desc);
+            SST_LAUNCH(k_tc_items_count, blocks_for(n), kTB, 0, s, off, desc, n, icnt);
+            e = scan<uint32_t, OpAdd>(icnt, ioff, n, 0u, OpAdd{}, true, false, ioff + n, A, s);
+          }
+          if (e == cudaSuccess) {
+            SST_LAUNCH(k_tc_items_fill, blocks_for(n), kTB, 0, s, icnt, ioff, n, items);
+            e = tc_count_launch(TcRows{off, cols, items, ioff + n}, desc, adj, c->d_cnt,
                                 reinterpret_cast<unsigned long long *>(d_pv), sms, s);
+          }
           if (e == cudaSuccess)
             e = cudaMemcpyAsync(c->h_cnt, c->d_cnt, 8, cudaMemcpyDeviceToHost, s);
           if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1270,7 +1279,7 @@ sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) 
     }
   }
   for (void *p : {(void *)off, (void *)doff, (void *)cols, (void *)keep, (void *)pos,
-                  (void *)adj, (void *)icnt, (void *)ioff, (void *)items})
+                  (void *)adj, (void *)icnt, (void *)ioff, (void *)items, (void *)desc})
     if (p) cudaFree(p);
   if (st != SST_OK) return st;
   SST_CUDA_TRY(e);

@@ -40,23 +40,29 @@ __device__ __forceinline__ bool sorted_has(const uint32_t *a, uint64_t n,
   return lo < n && a[lo] == x;
 }
 
-// The count runs over work items (u, j): the j-th batch of 32 entries of
-// N+(u), for every u with |N+(u)| >= 2 (a triangle needs two neighbours
-// above u).  A warp takes kTcGrab consecutive items at a time from a
-// global cursor, so the serial work a warp can be left with at the end is a
-// few items', whatever the degree distribution.  For an item the warp puts
-// N+(u) into a hash set in its shared memory (kept while the next item has
-// the same u), then reads the lists N+(v) of the item's 32 v as one
-// flattened stream: lane i holds v_i's list bounds and the warp's inclusive
-// prefix P of their lengths; stream item k lies in the first list i with
-// P_i > k, which each lane tracks with a cursor that only moves forward
-// (every lane's k grows by 32 a step); each lane issues kTcAhead loads
-// before it probes the set, so a warp keeps kTcAhead * 32 list entries in
-// flight.  A list N+(u) too long for the set is probed by binary search in
-// global memory instead.
+// A triangle is a common entry of the lists N+(x) and N+(y) of the ends of one
+// of its edges (the end w above both), so the count is the sum, over edges, of
+// |N+(x) n N+(y)|: one list goes into a hash set, the other is streamed past
+// it.  The set is the longer list (its vertex x), the stream the shorter one:
+// on an RMAT graph of 2^18 vertices that streams 96e6 entries where hashing
+// the lower-ranked end's list streamed 204e6 (k_tc_count 678 -> TC_COUNT_US).
+// A list too long for the set is streamed past the other end's set if that one
+// fits (tc_key), else probed by binary search.
+//
+// The count runs over work items: up to 32 neighbours y of one x.  A warp takes
+// kTcGrab consecutive items at a time from a global cursor, so the serial work
+// a warp can be left with at the end is a few items', whatever the degree
+// distribution.  For an item the warp puts N+(x) into a hash set in its shared
+// memory (kept while the next item has the same x), then reads the lists N+(y)
+// of the item's edges that x counts as one flattened stream: lane i holds
+// y_i's list bounds and the warp's inclusive prefix P of their lengths; stream
+// item k lies in the first list i with P_i > k, which each lane tracks with a
+// cursor that only moves forward (every lane's k grows by 32 a step); each
+// lane issues kTcAhead loads before it probes the set, so a warp keeps
+// kTcAhead * 32 list entries in flight.
 constexpr uint32_t kTcSlots = 2048;  // set slots per warp (8 KiB)
 constexpr int kTcBucketBits = 9;     // up to 2^9 buckets of 4 slots
-constexpr uint32_t kTcBatch = 32;    // v per work item
+constexpr uint32_t kTcBatch = 32;    // neighbours per work item
 constexpr int kTcWarps = 8;          // warps per block
 constexpr int kTcAhead = 4;          // stream items per lane in flight
 
@@ -104,16 +110,72 @@ __device__ __forceinline__ bool tc_set_has_warp(const uint4 *tab, uint32_t w, in
   return hit;
 }
 
-// per u: its number of work items
-__global__ void k_tc_items_count(const uint64_t *__restrict__ off, uint32_t n,
+// A vertex's oriented list as one word: (first entry << kTcLenBits) | length.
+// |N+(v)| ids have at least v's degree, so |N+(v)|^2 <= m: 24 bits hold it up
+// to 2^48 edges, and 40 bits the start.
+constexpr int kTcLenBits = 24;
+__device__ __forceinline__ uint32_t tc_len(uint64_t d) {
+  return (uint32_t)d & ((1u << kTcLenBits) - 1);
+}
+__global__ void k_tc_desc(const uint64_t *__restrict__ off, uint32_t n,
+                          uint64_t *__restrict__ desc) {
+  const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < n) desc[v] = (off[v] << kTcLenBits) | (off[v + 1] - off[v]);
+}
+
+// Which end of an edge takes the set: the one with the larger (key, id); a
+// list that does not fit a set comes last.
+__device__ __forceinline__ uint32_t tc_key(uint32_t len) {
+  return len <= kTcSlots / 2 ? len : 0u;
+}
+
+// Work items over the leaves of a graph's leaf directory: an item is a leaf.
+struct TcLeaves {
+  const uint32_t *slots, *owner, *cnt;
+  const uint64_t *slot;
+  uint64_t n;
+  struct Item {
+    uint32_t x, cnt;
+    uint64_t at;
+  };
+  __device__ __forceinline__ uint64_t count() const { return n; }
+  __device__ __forceinline__ Item item(uint64_t k) const {
+    return Item{owner[k], cnt[k], slot[k]};
+  }
+  __device__ __forceinline__ uint32_t id(uint64_t at) const { return slots[at]; }
+};
+
+// Work items over the rows of a CSR: an item is a batch of a row, listed as
+// (batch << 32) | row; rows without an oriented list have none.
+struct TcRows {
+  const uint64_t *off;
+  const uint32_t *cols;
+  const uint64_t *items;
+  const uint32_t *nitems;
+  struct Item {
+    uint32_t x, cnt;
+    uint64_t at;
+  };
+  __device__ __forceinline__ uint64_t count() const { return *nitems; }
+  __device__ __forceinline__ Item item(uint64_t k) const {
+    const uint64_t it = items[k];
+    const uint32_t x = (uint32_t)it;
+    const uint64_t at = off[x] + (it >> 32) * kTcBatch, left = off[x + 1] - at;
+    return Item{x, left < kTcBatch ? (uint32_t)left : kTcBatch, at};
+  }
+  __device__ __forceinline__ uint32_t id(uint64_t at) const { return cols[at]; }
+};
+
+// per row: its number of work items
+__global__ void k_tc_items_count(const uint64_t *__restrict__ off,
+                                 const uint64_t *__restrict__ desc, uint32_t n,
                                  uint32_t *__restrict__ cnt) {
   const uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n) return;
-  const uint64_t na = off[u + 1] - off[u];
-  cnt[u] = na < 2 ? 0u : (uint32_t)((na + kTcBatch - 1) / kTcBatch);
+  cnt[u] = tc_len(desc[u]) ? (uint32_t)((off[u + 1] - off[u] + kTcBatch - 1) / kTcBatch) : 0u;
 }
 
-// per u: its items (j << 32 | u) at its exclusive prefix ioff[u]
+// per row: its items at its exclusive prefix ioff[u]
 __global__ void k_tc_items_fill(const uint32_t *__restrict__ cnt,
                                 const uint32_t *__restrict__ ioff, uint32_t n,
                                 uint64_t *__restrict__ items) {
@@ -127,69 +189,90 @@ __global__ void k_tc_items_fill(const uint32_t *__restrict__ cnt,
 // parallel, one per lane
 constexpr int kTcGrab = 8;
 
+// position of the set bit of m with i set bits below it (32 if there is none)
+__device__ __forceinline__ int tc_nth_bit(uint32_t m, int i) {
+  int p = 0;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const int c = __popc(m & (((1u << d) - 1u) << p));
+    if (i >= c) {
+      i -= c;
+      p += d;
+    }
+  }
+  return (m >> p) & 1u && i == 0 ? p : 32;
+}
+
 // PV: also count, per vertex, the triangles it is in
-template <bool PV>
+template <bool PV, class Items>
 __global__ void __launch_bounds__(kTcWarps * 32, 3)
-k_tc_count(const uint64_t *__restrict__ off, const uint32_t *__restrict__ adj,
-           const uint64_t *__restrict__ items, const uint32_t *__restrict__ nitems,
+k_tc_count(Items src, const uint64_t *__restrict__ desc, const uint32_t *__restrict__ adj,
            unsigned long long *__restrict__ total, unsigned long long *__restrict__ pv) {
   extern __shared__ uint4 tc_sh[];
   const int lane = threadIdx.x & 31;
   const uint32_t full = 0xffffffffu;
   uint4 *tab = tc_sh + (threadIdx.x >> 5) * (kTcSlots / 4);
-  const uint32_t Q = *nitems;
+  const uint64_t Q = src.count();
   unsigned long long local = 0;
-  uint32_t set_u = kEmpty;  // the u whose N+ the set holds
+  uint32_t set_u = kEmpty;  // the x whose N+ the set holds
   for (;;) {
     unsigned long long q0 = 0;
     if (lane == 0) q0 = atomicAdd(total + 1, (unsigned long long)kTcGrab);
     q0 = __shfl_sync(full, q0, 0);
     if (q0 >= Q) break;
-    // lane g < kTcGrab: item q0 + g and its u's list bounds
-    uint64_t my_it = 0, my_a0 = 0, my_na = 0;
+    // lane g < kTcGrab: item q0 + g and its x's list
+    typename Items::Item my{0, 0, 0};
+    uint64_t my_d = 0;
     if (lane < kTcGrab && q0 + lane < Q) {
-      my_it = items[q0 + lane];
-      const uint32_t uu = (uint32_t)my_it;
-      my_a0 = off[uu];
-      my_na = off[uu + 1] - my_a0;
+      my = src.item(q0 + lane);
+      my_d = desc[my.x];
     }
     const int ng = (int)((Q - q0) < (unsigned long long)kTcGrab ? (Q - q0) : kTcGrab);
-    // The item's v (stage 1) and its list bounds (stage 2) load ahead: v two
-    // items before the item's turn, the bounds one item before (they need
-    // v), so a small item's three dependent loads overlap earlier items.
-    auto load_v = [&](int g, bool &okv) -> uint32_t {
-      const uint64_t itg = __shfl_sync(full, my_it, g & 31);
-      const uint64_t a0g = __shfl_sync(full, my_a0, g & 31);
-      const uint64_t nag = __shfl_sync(full, my_na, g & 31);
-      const uint64_t e = (itg >> 32) * kTcBatch + lane;
-      okv = g < ng && e < nag;
-      return okv ? adj[a0g + e] : 0u;
+    // The item's y (stage 1) and their lists (stage 2) load ahead: y two items
+    // before the item's turn, the lists one item before (they need y), so a
+    // small item's three dependent loads overlap earlier items.  An x without
+    // a list has nothing to load.
+    auto load_y = [&](int g, bool &ok) -> uint32_t {
+      const uint64_t at = __shfl_sync(full, my.at, g & 31);
+      const uint32_t c = __shfl_sync(full, my.cnt, g & 31);
+      const uint64_t d = __shfl_sync(full, my_d, g & 31);
+      ok = g < ng && (uint32_t)lane < c && tc_len(d);
+      return ok ? src.id(at + lane) : 0u;
     };
     bool ok_n1 = false, ok_n2 = false;
-    uint32_t v_n1 = load_v(0, ok_n1);  // item gi's v
-    uint32_t v_n2 = load_v(1, ok_n2);  // item gi + 1's v
-    uint64_t b_n1 = ok_n1 ? off[v_n1] : 0, e_n1 = ok_n1 ? off[v_n1 + 1] : 0;
+    uint32_t v_n1 = load_y(0, ok_n1);  // item gi's y
+    uint32_t v_n2 = load_y(1, ok_n2);  // item gi + 1's y
+    uint64_t d_n1 = ok_n1 ? desc[v_n1] : 0;
     for (int gi = 0; gi < ng; gi++) {
-      const uint64_t it = __shfl_sync(full, my_it, gi);
-      const uint64_t a0 = __shfl_sync(full, my_a0, gi);
-      const uint64_t na = __shfl_sync(full, my_na, gi);
-      const uint32_t u = (uint32_t)it;
-      const uint32_t *A = adj + a0;
-      // this lane's v and the bounds of N+(v), loaded ahead
-      const bool okv = ok_n1;
-      const uint32_t v = okv ? v_n1 : 0u;
-      const uint64_t b0 = okv ? b_n1 : 0;
-      const uint64_t l = okv ? e_n1 - b_n1 : 0;
-      const uint32_t len = l > 0xffffffffull ? 0xffffffffu : (uint32_t)l;
+      const uint32_t u = __shfl_sync(full, my.x, gi);
+      const uint64_t ud = __shfl_sync(full, my_d, gi);
+      const uint32_t na = tc_len(ud);
+      const uint32_t *A = adj + (ud >> kTcLenBits);
+      // this lane's y and its list, loaded ahead; x counts the edge if its own
+      // list is the set's
+      uint32_t v = v_n1;
+      uint64_t b0 = d_n1 >> kTcLenBits;
+      uint32_t len = ok_n1 ? tc_len(d_n1) : 0u;
+      const uint32_t kx = tc_key(na), ky = tc_key(len);
+      if (ky > kx || (ky == kx && v > u)) len = 0;
       // the next items' loads go out before this item's work
       bool ok_n3 = false;
-      const uint32_t v_n3 = load_v(gi + 2, ok_n3);
+      const uint32_t v_n3 = load_y(gi + 2, ok_n3);
       ok_n1 = ok_n2;
       v_n1 = v_n2;
-      b_n1 = ok_n2 ? off[v_n2] : 0;
-      e_n1 = ok_n2 ? off[v_n2 + 1] : 0;
+      d_n1 = ok_n2 ? desc[v_n2] : 0;
       ok_n2 = ok_n3;
       v_n2 = v_n3;
+      const uint32_t act = __ballot_sync(full, len != 0);
+      if (!act) continue;
+      {  // the edges that x counts to the front: the stream's cursor steps over
+         // no empty list
+        const int from = tc_nth_bit(act, lane);
+        v = __shfl_sync(full, v, from & 31);
+        b0 = __shfl_sync(full, b0, from & 31);
+        len = __shfl_sync(full, len, from & 31);
+        if (lane >= __popc(act)) len = 0;
+      }
       const bool hashed = na <= kTcSlots / 2;
       int bits = 3;
       while (bits < kTcBucketBits && (1ull << bits) < 2 * na) bits++;
@@ -202,9 +285,7 @@ k_tc_count(const uint64_t *__restrict__ off, const uint32_t *__restrict__ adj,
         __syncwarp();
         set_u = u;
       }
-      // inclusive prefix of the lengths.  It fits 32 bits: every w in N+(v)
-      // has degree >= deg(v) >= |N+(v)|, so |N+(v)|^2 <= m and 32 lists
-      // reach 2^32 items only past 2^54 edges
+      // inclusive prefix of the lengths: 32 of kTcLenBits bits
       uint32_t P = len;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -271,49 +352,28 @@ k_tc_count(const uint64_t *__restrict__ off, const uint32_t *__restrict__ adj,
   if (lane == 0 && local) atomicAdd(total, local);
 }
 
-// Scratch of a count over n vertices and madj oriented entries: cnt and
-// ioff n + 1 entries each, items tc_items_bound(n, madj) entries, and
-// scan_scratch_bytes(n + 1, 4) of arena.
-struct TcScratch {
-  uint32_t *cnt, *ioff;
-  uint64_t *items;
-};
-// an item per started batch of 32: sum ceil(na/32) <= madj/32 + n, and,
-// counting only na >= 2, <= madj/2
-inline uint64_t tc_items_bound(uint32_t n, uint64_t madj) {
-  return std::min<uint64_t>(madj / 32 + n, madj / 2) + 1;
-}
-
-// Counts the triangles of off[n + 1] / adj (device, madj entries).  total
-// (device) holds two counters the caller zeroes: total[0] gets the count,
-// total[1] is the work cursor.  pv (device, zeroed, may be null) gets
+// Counts the triangles of the oriented lists desc[n] / adj over the items of
+// src.  total (device) holds two counters the caller zeroes: total[0] gets the
+// count, total[1] is the work cursor.  pv (device, zeroed, may be null) gets
 // per-vertex counts.  One persistent grid of as many blocks as fit.
-inline cudaError_t tc_count_launch(const uint64_t *off, const uint32_t *adj, uint32_t n,
-                                   uint64_t madj, const TcScratch &sc, Arena &arena,
+template <class Items>
+inline cudaError_t tc_count_launch(const Items &src, const uint64_t *desc, const uint32_t *adj,
                                    unsigned long long *total, unsigned long long *pv,
                                    int sms, cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  if (tc_items_bound(n, madj) >= (1ull << 32)) return cudaErrorInvalidValue;
-  const unsigned vblocks = (unsigned)(((uint64_t)n + 255) / 256);
-  SST_LAUNCH(k_tc_items_count, vblocks, 256, 0, s, off, n, sc.cnt);
-  cudaError_t e = scan<uint32_t, OpAdd>(sc.cnt, sc.ioff, n, 0u, OpAdd{}, true, false,
-                                        sc.ioff + n, arena, s);
-  if (e != cudaSuccess) return e;
-  SST_LAUNCH(k_tc_items_fill, vblocks, 256, 0, s, sc.cnt, sc.ioff, n, sc.items);
   const size_t shm = (size_t)kTcWarps * kTcSlots * 4;
-  auto kern = pv ? k_tc_count<true> : k_tc_count<false>;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+  auto kern = pv ? k_tc_count<true, Items> : k_tc_count<false, Items>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTcWarps * 32, shm);
   if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)(std::max(per_sm, 1) * sms);
   if (pv)
-    SST_LAUNCH(k_tc_count<true>, grid, kTcWarps * 32, shm, s, off, adj, sc.items,
-               sc.ioff + n, total, pv);
+    SST_LAUNCH_NB("k_tc_count<true>", 0, (k_tc_count<true, Items>), grid, kTcWarps * 32, shm, s,
+                  src, desc, adj, total, pv);
   else
-    SST_LAUNCH(k_tc_count<false>, grid, kTcWarps * 32, shm, s, off, adj, sc.items,
-               sc.ioff + n, total, pv);
+    SST_LAUNCH_NB("k_tc_count<false>", 0, (k_tc_count<false, Items>), grid, kTcWarps * 32, shm, s,
+                  src, desc, adj, total, pv);
   return cudaGetLastError();
 }
 

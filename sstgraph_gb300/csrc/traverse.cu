@@ -94,7 +94,7 @@ struct TravState {
   // cc
   DevBuf<uint32_t> par;
   // tc
-  DevBuf<uint64_t> toff, tlpre, tlcnt, titems;
+  DevBuf<uint64_t> toff, tlpre, tlcnt;
   DevBuf<uint32_t> tadj, tmask;
   // multi-source bfs: per-vertex source masks (visited, frontier, next)
   DevBuf<unsigned long long> mvis, mfr, mfr2, mnx, msrc;
@@ -153,7 +153,6 @@ static void trav_buffers_release(TravState *t) {
   t->tlpre.release();
   t->tlcnt.release();
   t->tadj.release();
-  t->titems.release();
   t->tmask.release();
   t->mvis.release();
   t->mfr.release();
@@ -205,7 +204,7 @@ uint64_t trav_device_bytes(const sst_graph *g) {
   add(t->il0.cap, 4); add(t->depth_tmp.cap, 4); add(t->parent_tmp.cap, 4);
   add(t->sigma.cap, 8); add(t->ratio.cap, 8); add(t->levels.cap, 8);
   add(t->hub.cap, 8); add(t->hub_done.cap, 4); add(t->par.cap, 4); add(t->toff.cap, 8); add(t->tlpre.cap, 8);
-  add(t->tlcnt.cap, 8); add(t->tadj.cap, 4); add(t->titems.cap, 8); add(t->tmask.cap, 4);
+  add(t->tlcnt.cap, 8); add(t->tadj.cap, 4); add(t->tmask.cap, 4);
   add(t->mvis.cap, 8); add(t->mfr.cap, 8);
   add(t->mfr2.cap, 8); add(t->mnx.cap, 8); add(t->msrc.cap, 8); add(t->mdepth.cap, 4);
   add(t->msig.cap, 8); add(t->mrat.cap, 8); add(t->mpart.cap, 8); add(t->mlist.cap, 4);
@@ -864,11 +863,14 @@ __global__ void k_tc_fill(const uint32_t *__restrict__ slots,
     if ((m[j] >> lane) & 1u) adj[at[j] + __popc(m[j] & ((1u << lane) - 1u))] = x[j];
 }
 
-__global__ void k_tc_off(const uint64_t *__restrict__ vleaf,
-                         const uint64_t *__restrict__ lpre, uint32_t n,
-                         uint64_t *__restrict__ off) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v <= n) off[v] = lpre[vleaf[v]];
+// per vertex: its oriented list as one word (tcshared.cuh)
+__global__ void k_tc_lists(const uint64_t *__restrict__ vleaf,
+                           const uint64_t *__restrict__ lpre, uint32_t n,
+                           uint64_t *__restrict__ desc) {
+  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= n) return;
+  const uint64_t b = lpre[vleaf[v]], e = lpre[vleaf[v + 1]];
+  desc[v] = (b << kTcLenBits) | (e - b);
 }
 
 // ------------------------------------------------------------- pairs
@@ -1358,22 +1360,15 @@ sst_status tc(sst_graph *g, uint64_t *total, uint64_t *d_pv) {
   SST_CUDA_TRY(cudaMemcpyAsync(&madj, t->tlpre.p + nl, 8, cudaMemcpyDeviceToHost, s));
   SST_CUDA_TRY(cudaStreamSynchronize(s));
   SST_CUDA_TRY(t->tadj.ensure(madj + 1));
-  SST_CUDA_TRY(t->icnt.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->ioff.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->titems.ensure(tc_items_bound(n, madj)));
-  g->arena.reset();
-  SST_CUDA_TRY(g->arena.reserve(scan_scratch_bytes((uint64_t)n + 1, 4) + 4096));
   if (nl)
     SST_LAUNCH(k_tc_fill, warp_blocks(tc_warps), kTB, 0, s, g->d_slots, D.slot, nl,
                t->tmask.p, t->tlpre.p, t->tadj.p);
-  SST_LAUNCH(k_tc_off, blocks_for((uint64_t)n + 1), kTB, 0, s, D.vleaf,
-             t->tlpre.p, n, t->toff.p);
+  if (n) SST_LAUNCH(k_tc_lists, blocks_for(n), kTB, 0, s, D.vleaf, t->tlpre.p, n, t->toff.p);
   SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, 16, s));  // count, work cursor
   if (d_pv) SST_CUDA_TRY(cudaMemsetAsync(d_pv, 0, (uint64_t)n * 8, s));
-  if (n)
-    SST_CUDA_TRY(tc_count_launch(t->toff.p, t->tadj.p, n, madj,
-                                 TcScratch{t->icnt.p, t->ioff.p, t->titems.p}, g->arena,
-                                 t->d_small,
+  if (nl)
+    SST_CUDA_TRY(tc_count_launch(TcLeaves{g->d_slots, D.owner, D.cnt, D.slot, nl}, t->toff.p,
+                                 t->tadj.p, t->d_small,
                                  reinterpret_cast<unsigned long long *>(d_pv), g->sms, s));
   SST_CUDA_TRY(cudaMemcpyAsync(t->h_small, t->d_small, 8, cudaMemcpyDeviceToHost, s));
   SST_CUDA_TRY(cudaStreamSynchronize(s));
