@@ -45,7 +45,7 @@ __device__ __forceinline__ bool sorted_has(const uint32_t *a, uint64_t n,
 // |N+(x) n N+(y)|: one list goes into a hash set, the other is streamed past
 // it.  The set is the longer list (its vertex x), the stream the shorter one:
 // on an RMAT graph of 2^18 vertices that streams 96e6 entries where hashing
-// the lower-ranked end's list streamed 204e6 (k_tc_count 678 -> TC_COUNT_US).
+// the lower-ranked end's list streamed 204e6 (k_tc_count 678 -> 399 us).
 // A list too long for the set is streamed past the other end's set if that one
 // fits (tc_key), else probed by binary search.
 //
