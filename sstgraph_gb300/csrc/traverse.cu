@@ -74,13 +74,12 @@ struct TravState {
   // chunk list of multi-leaf vertices
   uint64_t nchunks = 0, nmulti = 0, nbig = 0, nsmall = 0;
   uint64_t inv_version = ~0ull;
-  DevBuf<uint64_t> choff;   // per vertex: first chunk (n+1)
-  DevBuf<uint32_t> cv, cl0; // per chunk: vertex, first leaf
+  DevBuf<uint32_t> cv;      // per chunk: vertex
   DevBuf<unsigned long long> cdesc, sdesc;  // packed chunk / one-leaf items
-  DevBuf<uint32_t> multi;   // vertices with more than one chunk
+  DevBuf<uint2> multi;      // vertices with more than one chunk: vertex, first chunk
   DevBuf<uint32_t> big;     // vertices with a multi-leaf segment
   DevBuf<uint32_t> small;   // vertices with a one-leaf segment (deg >= 1)
-  DevBuf<uint32_t> flag, pos;
+  DevBuf<uint32_t> lsum;    // per block of the list build: its list entries
   // pagerank
   DevBuf<double> inv_deg, ca, cb, partial;
   // bfs
@@ -119,16 +118,13 @@ struct TravState {
 // frees every buffer and the captured PageRank graph; the tuning stays, and
 // the work lists are rebuilt by the next traversal
 static void trav_buffers_release(TravState *t) {
-  t->choff.release();
   t->cv.release();
-  t->cl0.release();
   t->cdesc.release();
   t->sdesc.release();
   t->multi.release();
   t->big.release();
   t->small.release();
-  t->flag.release();
-  t->pos.release();
+  t->lsum.release();
   t->inv_deg.release();
   t->ca.release();
   t->cb.release();
@@ -196,9 +192,9 @@ uint64_t trav_device_bytes(const sst_graph *g) {
   if (!t) return 0;
   uint64_t b = 0;
   auto add = [&](uint64_t cap, size_t elem) { b += cap * elem; };
-  add(t->choff.cap, 8); add(t->cv.cap, 4); add(t->cl0.cap, 4); add(t->cdesc.cap, 8);
-  add(t->sdesc.cap, 8); add(t->multi.cap, 4); add(t->big.cap, 4); add(t->small.cap, 4);
-  add(t->flag.cap, 4); add(t->pos.cap, 4); add(t->inv_deg.cap, 8); add(t->ca.cap, 8);
+  add(t->cv.cap, 4); add(t->cdesc.cap, 8);
+  add(t->sdesc.cap, 8); add(t->multi.cap, 8); add(t->big.cap, 4); add(t->small.cap, 4);
+  add(t->lsum.cap, 4); add(t->inv_deg.cap, 8); add(t->ca.cap, 8);
   add(t->cb.cap, 8); add(t->partial.cap, 8); add(t->qa.cap, 4); add(t->qb.cap, 4);
   add(t->fbits.cap, 4); add(t->qitems.cap, 8); add(t->icnt.cap, 4); add(t->ioff.cap, 4); add(t->iv.cap, 4);
   add(t->il0.cap, 4); add(t->depth_tmp.cap, 4); add(t->parent_tmp.cap, 4);
@@ -216,57 +212,126 @@ uint64_t trav_device_bytes(const sst_graph *g) {
 namespace {
 
 // ------------------------------------------------------------- work lists
-__global__ void k_chunk_counts(const uint32_t *__restrict__ cap, uint32_t n,
-                               uint64_t *__restrict__ nch,
-                               uint32_t *__restrict__ bigf,
-                               uint32_t *__restrict__ multif,
-                               uint32_t *__restrict__ smallf, uint32_t cl) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  uint32_t c = cap[v];
-  uint64_t k = c > kLeaf ? ((c >> kLeafLog) + cl - 1) / cl : 0;
-  nch[v] = k;
-  bigf[v] = c > kLeaf;
-  multif[v] = k > 1;
-  smallf[v] = c > 0 && c <= kLeaf;
+// The four lists (one-leaf vertices, multi-leaf vertices, those of several
+// chunks, all chunks) in three launches: entries a block of vertices, their
+// prefix over the blocks, and the entries.  A thread takes kListPer
+// consecutive vertices.  Scanning a flag a vertex and list took eleven launches
+// and 24 bytes a vertex of scratch, and two readbacks.
+constexpr int kListPer = 8;
+constexpr uint32_t kListBlock = kScanThreads * kListPer;
+
+__device__ __forceinline__ uint32_t chunks_of(uint32_t cap, uint32_t cl) {
+  return cap > kLeaf ? ((cap >> kLeafLog) + cl - 1) / cl : 0u;
 }
 
-__global__ void k_chunk_fill(const uint32_t *__restrict__ cap,
-                             const uint64_t *__restrict__ base, uint32_t n,
-                             const uint64_t *__restrict__ choff,
-                             uint32_t *__restrict__ cv,
-                             uint32_t *__restrict__ cl0,
-                             unsigned long long *__restrict__ cdesc,
-                             uint32_t cl) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  uint64_t c0 = choff[v], c1 = choff[v + 1];
-  uint32_t nl = cap[v] >> kLeafLog;
-  uint64_t leaf = base[v] >> kLeafLog;
-  unsigned long long single = (c1 - c0) == 1 ? 128ull : 0ull;
-  for (uint64_t c = c0; c < c1; c++) {
-    uint32_t l0 = (uint32_t)((c - c0) * cl);
-    cv[c] = v;
-    cl0[c] = l0;
-    cdesc[c] = ((leaf + l0) << 8) | single | (unsigned long long)min(cl, nl - l0);
+// list entries of a thread's vertices: one-leaf, multi-leaf and multi-chunk
+// vertices (21 bits each, a block has 2048), and chunks
+struct ListCount {
+  unsigned long long rows = 0;
+  uint32_t chunks = 0;
+  __device__ __forceinline__ void add(uint32_t cap, uint32_t cl) {
+    const uint32_t k = chunks_of(cap, cl);
+    rows += (unsigned long long)(cap > 0 && cap <= kLeaf) |
+            (unsigned long long)(k > 0) << 21 | (unsigned long long)(k > 1) << 42;
+    chunks += k;
+  }
+};
+__device__ __forceinline__ void load_caps(const uint32_t *cap, uint64_t v0, uint32_t n,
+                                          uint32_t (&c)[kListPer]) {
+  if (v0 + kListPer <= n) {  // the table is a whole allocation: 16-byte aligned
+    const uint4 a = *reinterpret_cast<const uint4 *>(cap + v0);
+    const uint4 b = *reinterpret_cast<const uint4 *>(cap + v0 + 4);
+    c[0] = a.x, c[1] = a.y, c[2] = a.z, c[3] = a.w;
+    c[4] = b.x, c[5] = b.y, c[6] = b.z, c[7] = b.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < kListPer; k++) c[k] = v0 + k < n ? cap[v0 + k] : 0u;
   }
 }
 
-__global__ void k_small_desc(const uint32_t *__restrict__ small, uint64_t nsmall,
-                             const uint64_t *__restrict__ base,
-                             const uint32_t *__restrict__ deg,
-                             unsigned long long *__restrict__ sdesc) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsmall) return;
-  uint32_t v = small[i];
-  sdesc[i] = ((unsigned long long)base[v] << 6) | deg[v];
+__global__ void __launch_bounds__(kScanThreads)
+k_list_count(const uint32_t *__restrict__ cap, uint32_t n, uint32_t cl,
+             uint4 *__restrict__ sums) {
+  pdl_wait();
+  const uint64_t v0 = ((uint64_t)blockIdx.x * kScanThreads + threadIdx.x) * kListPer;
+  uint32_t c[kListPer];
+  load_caps(cap, v0, n, c);
+  ListCount e;
+#pragma unroll
+  for (int k = 0; k < kListPer; k++) e.add(c[k], cl);
+  unsigned long long rows;
+  uint32_t chunks;
+  block_exclusive(e.rows, 0ull, OpAdd{}, &rows);
+  block_exclusive(e.chunks, 0u, OpAdd{}, &chunks);
+  if (threadIdx.x == 0)
+    sums[blockIdx.x] = make_uint4((uint32_t)rows & 0x1FFFFF, (uint32_t)(rows >> 21) & 0x1FFFFF,
+                                  (uint32_t)(rows >> 42), chunks);
 }
 
-__global__ void k_compact_ids(const uint32_t *__restrict__ flag,
-                              const uint32_t *__restrict__ pos, uint32_t n,
-                              uint32_t *__restrict__ out) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < n && flag[v]) out[pos[v]] = v;
+// one block: exclusive prefixes in place, the totals to the host's pinned word
+__global__ void __launch_bounds__(kScanThreads)
+k_list_prefix(uint4 *__restrict__ sums, uint32_t nb, uint4 *__restrict__ totals) {
+  pdl_wait();
+  uint4 run = make_uint4(0, 0, 0, 0);
+  for (uint32_t i0 = 0; i0 < nb; i0 += kScanThreads) {
+    const uint32_t i = i0 + threadIdx.x;
+    const uint4 x = i < nb ? sums[i] : make_uint4(0, 0, 0, 0);
+    // two counters a word: each total is below 2^32
+    unsigned long long t0, t1;
+    const unsigned long long p0 =
+        block_exclusive((unsigned long long)x.y << 32 | x.x, 0ull, OpAdd{}, &t0);
+    const unsigned long long p1 =
+        block_exclusive((unsigned long long)x.w << 32 | x.z, 0ull, OpAdd{}, &t1);
+    if (i < nb)
+      sums[i] = make_uint4(run.x + (uint32_t)p0, run.y + (uint32_t)(p0 >> 32),
+                           run.z + (uint32_t)p1, run.w + (uint32_t)(p1 >> 32));
+    run.x += (uint32_t)t0;
+    run.y += (uint32_t)(t0 >> 32);
+    run.z += (uint32_t)t1;
+    run.w += (uint32_t)(t1 >> 32);
+  }
+  if (threadIdx.x == 0) *totals = run;
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+k_list_fill(DGraph g, uint32_t cl, const uint4 *__restrict__ sums, uint32_t *__restrict__ small,
+            unsigned long long *__restrict__ sdesc, uint32_t *__restrict__ big,
+            uint2 *__restrict__ multi, uint32_t *__restrict__ cv,
+            unsigned long long *__restrict__ cdesc) {
+  pdl_wait();
+  const uint64_t v0 = ((uint64_t)blockIdx.x * kScanThreads + threadIdx.x) * kListPer;
+  uint32_t c[kListPer];
+  load_caps(g.cap, v0, g.n, c);
+  ListCount e;
+#pragma unroll
+  for (int k = 0; k < kListPer; k++) e.add(c[k], cl);
+  unsigned long long rows;
+  uint32_t chunks;
+  const unsigned long long r = block_exclusive(e.rows, 0ull, OpAdd{}, &rows);
+  const uint32_t h = block_exclusive(e.chunks, 0u, OpAdd{}, &chunks);
+  const uint4 at = sums[blockIdx.x];
+  uint32_t is = at.x + ((uint32_t)r & 0x1FFFFF), ib = at.y + ((uint32_t)(r >> 21) & 0x1FFFFF);
+  uint32_t im = at.z + (uint32_t)(r >> 42), ic = at.w + h;
+#pragma unroll
+  for (int k = 0; k < kListPer; k++) {
+    if (!c[k]) continue;
+    const uint32_t v = (uint32_t)(v0 + k);
+    const uint64_t base = g.base[v];
+    if (c[k] <= kLeaf) {
+      small[is] = v;
+      sdesc[is++] = ((unsigned long long)base << 6) | g.deg[v];
+      continue;
+    }
+    big[ib++] = v;
+    const uint32_t nl = c[k] >> kLeafLog, nc = chunks_of(c[k], cl);
+    if (nc > 1) multi[im++] = make_uint2(v, ic);
+    const unsigned long long single = nc == 1 ? 128ull : 0ull;
+    for (uint32_t j = 0; j < nc; j++, ic++) {
+      cv[ic] = v;
+      cdesc[ic] = (((base >> kLeafLog) + (uint64_t)j * cl) << 8) | single |
+                  (unsigned long long)min(cl, nl - j * cl);
+    }
+  }
 }
 
 // ------------------------------------------------------------- pagerank
@@ -532,19 +597,17 @@ __global__ void __launch_bounds__(T, T == 1024 ? 1 : 2) k_pr_chunks_hot(DGraph g
   }
 }
 
-__global__ void k_pr_fix(DGraph g, const uint32_t *__restrict__ multi,
-                         uint64_t nmulti, const uint64_t *__restrict__ choff,
-                         const unsigned long long *__restrict__ partial,
-                         unsigned long long *__restrict__ cout,
-                         double *__restrict__ rank,
-                         const unsigned long long *__restrict__ rdeg, PrConst k,
-                         bool last) {
+__global__ void k_pr_fix(DGraph g, const uint2 *__restrict__ multi, uint64_t nmulti,
+                         uint32_t cl, const unsigned long long *__restrict__ partial,
+                         unsigned long long *__restrict__ cout, double *__restrict__ rank,
+                         const unsigned long long *__restrict__ rdeg, PrConst k, bool last) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nmulti) return;
-  uint32_t v = multi[i];
+  const uint2 e = multi[i];
+  const uint32_t nc = chunks_of(g.cap[e.x], cl);
   unsigned long long s = 0;
-  for (uint64_t c = choff[v]; c < choff[v + 1]; c++) s += partial[c];
-  pr_finish(v, s, k, g.deg[v], rdeg, cout, rank, last);
+  for (uint32_t c = 0; c < nc; c++) s += partial[e.y + c];
+  pr_finish(e.x, s, k, g.deg[e.x], rdeg, cout, rank, last);
 }
 
 __global__ void k_fill_d(double *__restrict__ p, uint32_t n, double x) {
@@ -996,56 +1059,31 @@ static sst_status ensure_lists(sst_graph *g) {
   TravState *t = state(g);
   if (t->version == g->version && t->lists_cl == t->chunk_leaves) return SST_OK;
   cudaStream_t s = g->stream;
-  uint32_t n = g->n;
-  SST_CUDA_TRY(t->choff.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->flag.ensure((uint64_t)n * 3 + 3));
-  SST_CUDA_TRY(t->pos.ensure((uint64_t)n * 3 + 3));
-  uint32_t *bigf = t->flag.p, *multif = t->flag.p + n + 1, *smallf = t->flag.p + 2 * (n + 1);
-  uint32_t *bigp = t->pos.p, *multip = t->pos.p + n + 1, *smallp = t->pos.p + 2 * (n + 1);
-  g->arena.reset();
-  SST_CUDA_TRY(g->arena.reserve(4 * scan_scratch_bytes((uint64_t)n + 1, 8) + 4096));
-  uint64_t *tot = g->arena.take<uint64_t>(1);
-  uint32_t *tot32 = g->arena.take<uint32_t>(3);
-  const uint32_t cl = t->chunk_leaves;
-  if (n) SST_LAUNCH(k_chunk_counts, blocks_for(n), kTB, 0, s, g->d_cap, n,
-                    t->choff.p, bigf, multif, smallf, cl);
-  SST_CUDA_TRY((scan<uint64_t, OpAdd>(t->choff.p, t->choff.p, n, 0ull, OpAdd{},
-                                      true, false, tot, g->arena, s)));
-  SST_CUDA_TRY((scan<uint32_t, OpAdd>(bigf, bigp, n, 0u, OpAdd{}, true, false,
-                                      tot32, g->arena, s)));
-  SST_CUDA_TRY((scan<uint32_t, OpAdd>(multif, multip, n, 0u, OpAdd{}, true,
-                                      false, tot32 + 1, g->arena, s)));
-  SST_CUDA_TRY((scan<uint32_t, OpAdd>(smallf, smallp, n, 0u, OpAdd{}, true,
-                                      false, tot32 + 2, g->arena, s)));
-  uint64_t h[2];
-  uint32_t h32[3];
-  SST_CUDA_TRY(cudaMemcpyAsync(h, tot, 8, cudaMemcpyDeviceToHost, s));
-  SST_CUDA_TRY(cudaMemcpyAsync(h32, tot32, 12, cudaMemcpyDeviceToHost, s));
-  SST_CUDA_TRY(cudaStreamSynchronize(s));
-  t->nchunks = h[0];
-  t->nbig = h32[0];
-  t->nmulti = h32[1];
-  t->nsmall = h32[2];
-  SST_CUDA_TRY(cudaMemcpyAsync(t->choff.p + n, &t->nchunks, 8, cudaMemcpyHostToDevice, s));
-  SST_CUDA_TRY(t->cv.ensure(t->nchunks + 1));
-  SST_CUDA_TRY(t->cl0.ensure(t->nchunks + 1));
-  SST_CUDA_TRY(t->big.ensure(t->nbig + 1));
-  SST_CUDA_TRY(t->multi.ensure(t->nmulti + 1));
-  SST_CUDA_TRY(t->small.ensure(t->nsmall + 1));
-  SST_CUDA_TRY(t->cdesc.ensure(t->nchunks + 1));
-  SST_CUDA_TRY(t->sdesc.ensure(t->nsmall + 1));
-  if (n) {
-    SST_LAUNCH(k_chunk_fill, blocks_for(n), kTB, 0, s, g->d_cap, g->d_base, n,
-               t->choff.p, t->cv.p, t->cl0.p, t->cdesc.p, cl);
-    SST_LAUNCH(k_compact_ids, blocks_for(n), kTB, 0, s, bigf, bigp, n, t->big.p);
-    SST_LAUNCH(k_compact_ids, blocks_for(n), kTB, 0, s, multif, multip, n, t->multi.p);
-    SST_LAUNCH(k_compact_ids, blocks_for(n), kTB, 0, s, smallf, smallp, n, t->small.p);
-    if (t->nsmall)
-      SST_LAUNCH(k_small_desc, blocks_for(t->nsmall), kTB, 0, s, t->small.p,
-                 t->nsmall, g->d_base, g->d_deg, t->sdesc.p);
-  }
+  const uint32_t n = g->n, cl = t->chunk_leaves;
+  // sized by what the slab can hold, so nothing waits for the counts and an
+  // update that moves no slab grows no list
+  const uint64_t most_big = std::min<uint64_t>(n, g->nslots / (2 * kLeaf));
+  const uint64_t most_chunks = most_big + g->nslots / ((uint64_t)kLeaf * cl);
+  const unsigned nb = blocks_for(n, kListBlock);
+  SST_CUDA_TRY(t->lsum.ensure(4 * (uint64_t)nb));
+  SST_CUDA_TRY(t->small.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->sdesc.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->big.ensure(most_big + 1));
+  SST_CUDA_TRY(t->multi.ensure(most_big + 1));
+  SST_CUDA_TRY(t->cv.ensure(most_chunks + 1));
+  SST_CUDA_TRY(t->cdesc.ensure(most_chunks + 1));
+  uint4 *sums = reinterpret_cast<uint4 *>(t->lsum.p);
+  uint4 *totals = reinterpret_cast<uint4 *>(t->h_small + 8);
+  SST_LAUNCH_PDL(k_list_count, nb, kScanThreads, 0, s, g->d_cap, n, cl, sums);
+  SST_LAUNCH_PDL(k_list_prefix, 1, kScanThreads, 0, s, sums, nb, totals);
+  SST_LAUNCH_PDL(k_list_fill, nb, kScanThreads, 0, s, g->view(), cl, sums, t->small.p, t->sdesc.p,
+                 t->big.p, t->multi.p, t->cv.p, t->cdesc.p);
   SST_CUDA_TRY(cudaStreamSynchronize(s));
   SST_CUDA_TRY(cudaGetLastError());
+  t->nsmall = totals->x;
+  t->nbig = totals->y;
+  t->nmulti = totals->z;
+  t->nchunks = totals->w;
   t->version = g->version;
   t->lists_cl = cl;
   t->lists_stamp++;
@@ -1159,8 +1197,8 @@ sst_status pagerank(sst_graph *g, uint32_t iters, double damping, double *d_rank
         SST_LAUNCH(k_pr_chunks, warp_blocks(t->nchunks), kTB, 0, s, dg, t->cdesc.p,
                    t->cv.p, t->nchunks, ci, co, d_rank, rdeg, part, K, last);
       if (t->nmulti)
-        SST_LAUNCH(k_pr_fix, blocks_for(t->nmulti), kTB, 0, s, dg, t->multi.p,
-                   t->nmulti, t->choff.p, part, co, d_rank, rdeg, K, last);
+        SST_LAUNCH(k_pr_fix, blocks_for(t->nmulti), kTB, 0, s, dg, t->multi.p, t->nmulti,
+                   t->lists_cl, part, co, d_rank, rdeg, K, last);
       std::swap(ci, co);
     }
   };
