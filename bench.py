@@ -476,7 +476,7 @@ def main():
                     "roofline": {"bound": "hbm", "achieved": pr_gbs, "peak": hbm_peak,
                                  "unit": "GB/s", "frac": pr_gbs / hbm_peak,
                                  "peak_kind": peak_kind, "traffic": None,
-                                 "kernels": "one iteration = k_pr_small + k_pr_chunks + k_pr_fix"},
+                                 "kernels": "one iteration = k_pr_iter + k_pr_fix"},
                     "kernels": pr_prof}
         return pagerank
 
