@@ -13,9 +13,11 @@
 // 270 MB of lists, depths and row sectors.
 //
 // The grid is one that fits at once (cooperative), and no larger than the
-// graph has work for: blocks beyond that only make the barrier wider.  It
-// leaves half of every SM's threads to the kernels of other streams (a served
-// graph is updated while it is queried).
+// graph has work for: blocks beyond that only make the barrier wider.  Two
+// blocks hold all of an SM's registers, so the largest grid leaves kCoopFree
+// block places to the kernels of other streams: a served graph is updated while
+// it is searched, and an update's small kernels would otherwise wait for the
+// search to end.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -28,6 +30,7 @@ namespace {
 
 constexpr int kCoopThreads = 512;
 constexpr int kCoopPerSm = 2;  // blocks of an SM
+constexpr int kCoopFree = 16;  // block places left free
 constexpr uint32_t kFull = 0xffffffffu;
 
 // ------------------------------------------------------------ grid barrier

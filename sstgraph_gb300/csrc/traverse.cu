@@ -1284,7 +1284,7 @@ static sst_status coop_grid(const sst_graph *g, const void *kernel, uint64_t thr
     set_error_message("a traversal kernel does not fit the device");
     return SST_EDEVICE;
   }
-  const uint64_t most = (uint64_t)std::min(per_sm, kCoopPerSm) * g->sms;
+  const uint64_t most = (uint64_t)std::max(std::min(per_sm, kCoopPerSm) * g->sms - kCoopFree, 1);
   *grid = (unsigned)std::min<uint64_t>(most, (threads + kCoopThreads - 1) / kCoopThreads + 1);
   return SST_OK;
 }
