@@ -28,6 +28,7 @@
 // PMA.hpp:612-702 (redistribute / double_list / half_list),
 // PMA.hpp:1185-1222 (take: lower-bound climb).
 #include <algorithm>
+#include <cooperative_groups.h>
 #include <cstddef>
 #include <cstdarg>
 #include <cstring>
@@ -295,6 +296,44 @@ __global__ void k_locate(const uint64_t *__restrict__ keys, uint64_t b,
 // in with one coalesced load.  Same outputs as k_locate (the heads of a
 // segment's leaves ascend, so the leaves whose head is <= x are a prefix).
 constexpr uint64_t kLocateWarpKeys = 16384;
+
+struct Located {
+  uint64_t S;        // the leaf's first slot
+  uint32_t leaf, cw; // its index in the row, its count word
+  uint32_t pos;      // ids of the leaf below x
+  bool present;
+};
+__device__ __forceinline__ Located locate_by_warp(const DGraph &g, uint32_t u, uint32_t x) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t base = g.base[u];
+  const uint32_t cap = g.cap[u], deg = g.deg[u];
+  Located r{0, 0, 0, 0, false};
+  if (cap == 0) return r;
+  if (cap > kLeaf) {
+    // the answer lies in leaves [lo, lo + n); lane j probes leaf lo + j*step
+    uint32_t lo = 0, n = cap >> kLeafLog;
+    for (;;) {
+      const uint32_t step = n > 32 ? (n + 31) / 32 : 1u;
+      const uint32_t j = (uint32_t)lane * step;
+      const bool le = lane > 0 && j < n && g.slots[base + ((uint64_t)(lo + j) << kLeafLog)] <= x;
+      const uint32_t m = __ballot_sync(0xffffffffu, le);
+      const uint32_t jj = m ? 31u - __clz(m) : 0u;
+      lo += jj * step;
+      if (step == 1) break;
+      n = n - jj * step < step ? n - jj * step : step;
+    }
+    r.leaf = lo;
+  }
+  const uint32_t c = leaf_count(g, base, cap, deg, r.leaf);
+  r.S = base + ((uint64_t)r.leaf << kLeafLog);
+  const uint32_t a = (uint32_t)lane < c ? g.slots[r.S + lane] : kEmpty;
+  r.pos = __popc(__ballot_sync(0xffffffffu, a < x));
+  const uint32_t at = __shfl_sync(0xffffffffu, a, r.pos & 31);
+  r.present = r.pos < c && at == x;
+  r.cw = c | (cap > kLeaf ? kMultiLeaf : cap << kCapShift);
+  return r;
+}
+
 __global__ void k_locate_warp(const uint64_t *__restrict__ keys, uint64_t b,
                               int dbits, DGraph g, bool insert,
                               uint32_t *__restrict__ flag,
@@ -316,44 +355,14 @@ __global__ void k_locate_warp(const uint64_t *__restrict__ keys, uint64_t b,
     }
     return;
   }
-  const uint32_t u = (uint32_t)(k >> dbits);
-  const uint32_t x = (uint32_t)(k & ((1ull << dbits) - 1));
-  const uint64_t base = g.base[u];
-  const uint32_t cap = g.cap[u], deg = g.deg[u];
-  bool present = false;
-  uint32_t l = 0, c = 0, pos = 0;
-  uint64_t S = 0;
-  uint32_t cw = 0;
-  if (cap > 0) {
-    if (cap > kLeaf) {
-      // the answer lies in leaves [lo, lo + n); lane j probes leaf lo + j*step
-      uint32_t lo = 0, n = cap >> kLeafLog;
-      for (;;) {
-        const uint32_t step = n > 32 ? (n + 31) / 32 : 1u;
-        const uint32_t j = (uint32_t)lane * step;
-        const bool le = lane > 0 && j < n && g.slots[base + ((uint64_t)(lo + j) << kLeafLog)] <= x;
-        const uint32_t m = __ballot_sync(0xffffffffu, le);
-        const uint32_t jj = m ? 31u - __clz(m) : 0u;
-        lo += jj * step;
-        if (step == 1) break;
-        n = n - jj * step < step ? n - jj * step : step;
-      }
-      l = lo;
-    }
-    c = leaf_count(g, base, cap, deg, l);
-    S = base + ((uint64_t)l << kLeafLog);
-    const uint32_t a = (uint32_t)lane < c ? g.slots[S + lane] : kEmpty;
-    pos = __popc(__ballot_sync(0xffffffffu, a < x));
-    const uint32_t at = __shfl_sync(0xffffffffu, a, pos & 31);
-    present = pos < c && at == x;
-    cw = c | (cap > kLeaf ? kMultiLeaf : cap << kCapShift);
-  }
+  const Located r = locate_by_warp(g, (uint32_t)(k >> dbits),
+                                   (uint32_t)(k & ((1ull << dbits) - 1)));
   if (lane == 0) {
-    if (present && insert && wv && g.vals) g.vals[S + pos] = wv[i];
-    flag[i] = insert ? !present : present;
-    leaf_out[i] = l;
-    lS[i] = S;
-    lc[i] = cw;
+    if (r.present && insert && wv && g.vals) g.vals[r.S + r.pos] = wv[i];
+    flag[i] = insert ? !r.present : r.present;
+    leaf_out[i] = r.leaf;
+    lS[i] = r.S;
+    lc[i] = r.cw;
   }
 }
 
@@ -420,6 +429,37 @@ struct GroupStartEpi {
 // one-leaf row, the row's capacity, as k_locate read them; nothing has
 // changed either since) decides, so no vertex record or leaf count is read
 // again.
+__device__ __forceinline__ void classify_insert(uint32_t gid, const uint64_t *__restrict__ p_ul,
+                                                const uint32_t *__restrict__ p_c,
+                                                const uint32_t *__restrict__ g_start,
+                                                uint8_t *__restrict__ gtype,
+                                                uint8_t *__restrict__ glev,
+                                                uint32_t *__restrict__ gw0,
+                                                uint32_t *__restrict__ gw1,
+                                                uint32_t *__restrict__ climb,
+                                                uint32_t *__restrict__ nclimb) {
+  const uint32_t j0 = g_start[gid], k = g_start[gid + 1] - j0;
+  const uint32_t leaf = (uint32_t)p_ul[j0];
+  const uint32_t cw = p_c[j0], c = cw & 0xff;
+  uint8_t type = kMerge;
+  uint32_t lev = 0, w0 = leaf, w1 = leaf + 1;
+  if (!(cw & kMultiLeaf)) {
+    if (c + k > one_leaf_cap(cw)) {  // a one-leaf row's count is its degree
+      type = kResize;
+      lev = 31;
+      w0 = 0;
+      w1 = 1;
+    }
+  } else if (c + k > kLeaf) {
+    type = kNone;  // decided by the climb
+    climb[atomicAdd(nclimb, 1u)] = gid;
+  }
+  gtype[gid] = type;
+  glev[gid] = (uint8_t)lev;
+  gw0[gid] = w0;
+  gw1[gid] = w1;
+}
+
 __global__ void k_classify_insert(const uint64_t *__restrict__ p_ul,
                                   const uint32_t *__restrict__ p_c,
                                   const uint32_t *__restrict__ g_start,
@@ -432,28 +472,8 @@ __global__ void k_classify_insert(const uint64_t *__restrict__ p_ul,
                                   uint32_t *__restrict__ nclimb) {
   pdl_wait();
   const uint32_t ng = *d_ngroups;
-  GRID_STRIDE(gid, ng) {
-    const uint32_t j0 = g_start[gid], k = g_start[gid + 1] - j0;
-    const uint32_t leaf = (uint32_t)p_ul[j0];
-    const uint32_t cw = p_c[j0], c = cw & 0xff;
-    uint8_t type = kMerge;
-    uint32_t lev = 0, w0 = leaf, w1 = leaf + 1;
-    if (!(cw & kMultiLeaf)) {
-      if (c + k > one_leaf_cap(cw)) {  // a one-leaf row's count is its degree
-        type = kResize;
-        lev = 31;
-        w0 = 0;
-        w1 = 1;
-      }
-    } else if (c + k > kLeaf) {
-      type = kNone;  // decided by the climb
-      climb[atomicAdd(nclimb, 1u)] = (uint32_t)gid;
-    }
-    gtype[gid] = type;
-    glev[gid] = (uint8_t)lev;
-    gw0[gid] = w0;
-    gw1[gid] = w1;
-  }
+  GRID_STRIDE(gid, ng)
+    classify_insert((uint32_t)gid, p_ul, p_c, g_start, gtype, glev, gw0, gw1, climb, nclimb);
 }
 
 constexpr int kGroupsPerWarp = 4;
@@ -519,6 +539,123 @@ __device__ __forceinline__ uint32_t list_groups(uint8_t *list, bool ok, bool one
 // lines loaded together, one dependent load per batch; the bookkeeping
 // (leaf count, degree, classification) runs once for all 32 groups, lane l
 // for group l.
+__device__ __forceinline__ void leaf_delete_chunk(
+    const DGraph &g, uint64_t w, uint32_t ng, uint8_t *list, uint32_t lo_leaf,
+    const uint64_t *__restrict__ p_ul, const uint32_t *__restrict__ p_x,
+    const uint64_t *__restrict__ p_S, const uint32_t *__restrict__ p_c,
+    const uint32_t *__restrict__ g_start, uint8_t *__restrict__ gtype,
+    uint8_t *__restrict__ glev, uint32_t *__restrict__ gw0, uint32_t *__restrict__ gw1,
+    uint32_t *__restrict__ climb, uint32_t *__restrict__ nclimb) {
+  const int lane = threadIdx.x & 31, sub = lane & 7;
+  constexpr int Q = kGroupsPerWarp;
+  const uint64_t gl = w * 32 + lane;
+  const bool okl = gl < ng;
+  const uint32_t j0l = okl ? g_start[gl] : 0;
+  const uint32_t kl = okl ? g_start[gl + 1] - j0l : 0;
+  const uint64_t Sl = okl ? p_S[j0l] : 0;
+  const uint32_t cwl = okl ? p_c[j0l] : 0;
+  const uint64_t keyl = okl ? p_ul[j0l] : 0;
+  const uint32_t ul = (uint32_t)(keyl >> 32), leafl = (uint32_t)keyl;
+  // a one-leaf row's capacity is in its count word; a multi-leaf row
+  // only needs to be told apart
+  const uint32_t capl = (cwl & kMultiLeaf) ? kLeaf + 1 : one_leaf_cap(cwl);
+  const uint32_t cnt = ng - w * 32 < 32 ? (uint32_t)(ng - w * 32) : 32u;
+  // one-item groups: the slots from the deleted id's place on take their
+  // right neighbour (kEmpty past the count)
+  const uint32_t n1 = list_groups(list, okl, kl == 1 && !g.vals, lane);
+  for (uint32_t f0 = 0; f0 < n1; f0 += 4) {
+    const uint32_t f = f0 + (lane >> 3);
+    const bool on = f < n1;
+    const int src = list[on ? f : 0];
+    const uint32_t j0 = __shfl_sync(0xffffffffu, j0l, src);
+    const uint64_t S = __shfl_sync(0xffffffffu, Sl, src);
+    const uint32_t cw = __shfl_sync(0xffffffffu, cwl, src);
+    const uint32_t c = on ? (cw & 0xff) : 0u;
+    const uint32_t d = on ? p_x[j0] : kEmpty;
+    uint32_t a[4];
+    load_quarter(g.slots, S, c, sub, a);
+    const uint32_t pos = below_in_octet(a, d);
+    const uint32_t nxt = __shfl_down_sync(0xffffffffu, a[0], 1, 8);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const uint32_t p = 4 * sub + r;
+      if (p >= pos && p < c) g.slots[S + p] = r < 3 ? a[r + 1] : (sub == 7 ? kEmpty : nxt);
+    }
+  }
+  // the other groups: a warp each, kGroupsPerWarp at a time
+  const uint32_t nrest = cnt - n1;
+  for (uint32_t q0 = 0; q0 < nrest; q0 += Q) {
+    uint32_t j0[Q], k[Q], d[Q], linev[Q], cw[Q];
+    uint64_t S[Q];
+    bool ok[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      ok[q] = q0 + q < nrest;
+      const int src = list[n1 + (ok[q] ? q0 + q : 0)];
+      j0[q] = __shfl_sync(0xffffffffu, j0l, src);
+      k[q] = ok[q] ? __shfl_sync(0xffffffffu, kl, src) : 0;
+      S[q] = __shfl_sync(0xffffffffu, Sl, src);
+      cw[q] = __shfl_sync(0xffffffffu, cwl, src);
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      d[q] = (uint32_t)lane < k[q] ? p_x[j0[q] + lane] : kEmpty;
+      linev[q] = ok[q] ? g.slots[(S[q] & ~uint64_t(kLeaf - 1)) + lane] : kEmpty;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      if (!ok[q]) break;
+      const uint32_t c = cw[q] & 0xff;
+      const uint32_t a = leaf_slot(linev[q], S[q], c, lane);
+      bool del = false;
+      for (uint32_t j = 0; j < k[q]; j++) del |= (__shfl_sync(0xffffffffu, d[q], j) == a);
+      const bool keep = (uint32_t)lane < c && !del;
+      const uint32_t mask = __ballot_sync(0xffffffffu, keep);
+      const uint32_t pos = __popc(mask & ((1u << lane) - 1u));
+      if (g.vals) {
+        const uint32_t av = (uint32_t)lane < c ? g.vals[S[q] + lane] : 0u;
+        __syncwarp();  // every value read before any is moved
+        if (keep) g.vals[S[q] + pos] = av;
+      }
+      // the ids come from registers: no lane reads the line again
+      if (keep) g.slots[S[q] + pos] = a;
+      if ((uint32_t)lane >= c - k[q] && (uint32_t)lane < c) g.slots[S[q] + lane] = kEmpty;
+    }
+  }
+  // the chunk's bookkeeping, lane l for group l
+  const uint32_t gid = (uint32_t)(w * 32) + lane;
+  bool to_climb = false;
+  if (okl) {
+    const uint32_t nc = (cwl & 0xff) - kl;  // every item of a group is present
+    if (cwl & kMultiLeaf) g.lcnt[Sl >> kLeafLog] = (uint8_t)nc;
+    atomicSub(&g.deg[ul], kl);
+    uint8_t type = kNone;
+    uint32_t lev = 0, w0 = leafl, w1 = leafl + 1;
+    if (capl <= kLeaf) {
+      if (nc == 0 || (capl > 1 && 4 * nc <= capl)) {
+        type = kResize;
+        lev = 31;
+        w0 = 0;
+        w1 = 1;
+      }
+    } else if (nc < lo_leaf) {
+      to_climb = true;
+    }
+    gtype[gid] = type;
+    glev[gid] = (uint8_t)lev;
+    gw0[gid] = w0;
+    gw1[gid] = w1;
+  }
+  // one reservation in the climb list for the warp's climbing groups
+  const uint32_t cm = __ballot_sync(0xffffffffu, to_climb);
+  if (cm) {
+    uint32_t at = 0;
+    if (lane == __ffs(cm) - 1) at = atomicAdd(nclimb, (uint32_t)__popc(cm));
+    at = __shfl_sync(0xffffffffu, at, __ffs(cm) - 1);
+    if (to_climb) climb[at + __popc(cm & ((1u << lane) - 1u))] = gid;
+  }
+}
+
 __global__ void __launch_bounds__(256, 4)
 k_leaf_delete(DGraph g, uint32_t lo_leaf, const uint64_t *__restrict__ p_ul,
               const uint32_t *__restrict__ p_x,
@@ -530,120 +667,12 @@ k_leaf_delete(DGraph g, uint32_t lo_leaf, const uint64_t *__restrict__ p_ul,
               uint32_t *__restrict__ climb, uint32_t *__restrict__ nclimb) {
   pdl_wait();
   __shared__ uint8_t glist[kLeafWarps][32];
-  const int lane = threadIdx.x & 31, sub = lane & 7;
-  uint8_t *list = glist[threadIdx.x >> 5];
-  constexpr int Q = kGroupsPerWarp;
   const uint32_t ng = *d_ngroups;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-       w * 32 < ng; w += nw) {
-    const uint64_t gl = w * 32 + lane;
-    const bool okl = gl < ng;
-    const uint32_t j0l = okl ? g_start[gl] : 0;
-    const uint32_t kl = okl ? g_start[gl + 1] - j0l : 0;
-    const uint64_t Sl = okl ? p_S[j0l] : 0;
-    const uint32_t cwl = okl ? p_c[j0l] : 0;
-    const uint64_t keyl = okl ? p_ul[j0l] : 0;
-    const uint32_t ul = (uint32_t)(keyl >> 32), leafl = (uint32_t)keyl;
-    // a one-leaf row's capacity is in its count word; a multi-leaf row
-    // only needs to be told apart
-    const uint32_t capl = (cwl & kMultiLeaf) ? kLeaf + 1 : one_leaf_cap(cwl);
-    const uint32_t cnt = ng - w * 32 < 32 ? (uint32_t)(ng - w * 32) : 32u;
-    // one-item groups: the slots from the deleted id's place on take their
-    // right neighbour (kEmpty past the count)
-    const uint32_t n1 = list_groups(list, okl, kl == 1 && !g.vals, lane);
-    for (uint32_t f0 = 0; f0 < n1; f0 += 4) {
-      const uint32_t f = f0 + (lane >> 3);
-      const bool on = f < n1;
-      const int src = list[on ? f : 0];
-      const uint32_t j0 = __shfl_sync(0xffffffffu, j0l, src);
-      const uint64_t S = __shfl_sync(0xffffffffu, Sl, src);
-      const uint32_t cw = __shfl_sync(0xffffffffu, cwl, src);
-      const uint32_t c = on ? (cw & 0xff) : 0u;
-      const uint32_t d = on ? p_x[j0] : kEmpty;
-      uint32_t a[4];
-      load_quarter(g.slots, S, c, sub, a);
-      const uint32_t pos = below_in_octet(a, d);
-      const uint32_t nxt = __shfl_down_sync(0xffffffffu, a[0], 1, 8);
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const uint32_t p = 4 * sub + r;
-        if (p >= pos && p < c) g.slots[S + p] = r < 3 ? a[r + 1] : (sub == 7 ? kEmpty : nxt);
-      }
-    }
-    // the other groups: a warp each, kGroupsPerWarp at a time
-    const uint32_t nrest = cnt - n1;
-    for (uint32_t q0 = 0; q0 < nrest; q0 += Q) {
-      uint32_t j0[Q], k[Q], d[Q], linev[Q], cw[Q];
-      uint64_t S[Q];
-      bool ok[Q];
-#pragma unroll
-      for (int q = 0; q < Q; q++) {
-        ok[q] = q0 + q < nrest;
-        const int src = list[n1 + (ok[q] ? q0 + q : 0)];
-        j0[q] = __shfl_sync(0xffffffffu, j0l, src);
-        k[q] = ok[q] ? __shfl_sync(0xffffffffu, kl, src) : 0;
-        S[q] = __shfl_sync(0xffffffffu, Sl, src);
-        cw[q] = __shfl_sync(0xffffffffu, cwl, src);
-      }
-#pragma unroll
-      for (int q = 0; q < Q; q++) {
-        d[q] = (uint32_t)lane < k[q] ? p_x[j0[q] + lane] : kEmpty;
-        linev[q] = ok[q] ? g.slots[(S[q] & ~uint64_t(kLeaf - 1)) + lane] : kEmpty;
-      }
-#pragma unroll
-      for (int q = 0; q < Q; q++) {
-        if (!ok[q]) break;
-        const uint32_t c = cw[q] & 0xff;
-        const uint32_t a = leaf_slot(linev[q], S[q], c, lane);
-        bool del = false;
-        for (uint32_t j = 0; j < k[q]; j++) del |= (__shfl_sync(0xffffffffu, d[q], j) == a);
-        const bool keep = (uint32_t)lane < c && !del;
-        const uint32_t mask = __ballot_sync(0xffffffffu, keep);
-        const uint32_t pos = __popc(mask & ((1u << lane) - 1u));
-        if (g.vals) {
-          const uint32_t av = (uint32_t)lane < c ? g.vals[S[q] + lane] : 0u;
-          __syncwarp();  // every value read before any is moved
-          if (keep) g.vals[S[q] + pos] = av;
-        }
-        // the ids come from registers: no lane reads the line again
-        if (keep) g.slots[S[q] + pos] = a;
-        if ((uint32_t)lane >= c - k[q] && (uint32_t)lane < c) g.slots[S[q] + lane] = kEmpty;
-      }
-    }
-    // the chunk's bookkeeping, lane l for group l
-    const uint32_t gid = (uint32_t)(w * 32) + lane;
-    bool to_climb = false;
-    if (okl) {
-      const uint32_t nc = (cwl & 0xff) - kl;  // every item of a group is present
-      if (cwl & kMultiLeaf) g.lcnt[Sl >> kLeafLog] = (uint8_t)nc;
-      atomicSub(&g.deg[ul], kl);
-      uint8_t type = kNone;
-      uint32_t lev = 0, w0 = leafl, w1 = leafl + 1;
-      if (capl <= kLeaf) {
-        if (nc == 0 || (capl > 1 && 4 * nc <= capl)) {
-          type = kResize;
-          lev = 31;
-          w0 = 0;
-          w1 = 1;
-        }
-      } else if (nc < lo_leaf) {
-        to_climb = true;
-      }
-      gtype[gid] = type;
-      glev[gid] = (uint8_t)lev;
-      gw0[gid] = w0;
-      gw1[gid] = w1;
-    }
-    // one reservation in the climb list for the warp's climbing groups
-    const uint32_t cm = __ballot_sync(0xffffffffu, to_climb);
-    if (cm) {
-      uint32_t at = 0;
-      if (lane == __ffs(cm) - 1) at = atomicAdd(nclimb, (uint32_t)__popc(cm));
-      at = __shfl_sync(0xffffffffu, at, __ffs(cm) - 1);
-      if (to_climb) climb[at + __popc(cm & ((1u << lane) - 1u))] = gid;
-    }
-  }
+       w * 32 < ng; w += nw)
+    leaf_delete_chunk(g, w, ng, glist[threadIdx.x >> 5], lo_leaf, p_ul, p_x, p_S, p_c, g_start,
+                      gtype, glev, gw0, gw1, climb, nclimb);
 }
 
 // window density bounds by segment height H (2^H leaves, H < kBoundsH: a
@@ -655,6 +684,70 @@ constexpr uint32_t kBoundsH = 32;
 // warp per climbing group: the smallest aligned window of 2^t leaves that
 // meets the density bound (insert: upper bound with the batch's new ids in
 // the window counted; remove: lower bound), else a resize of the segment
+__device__ __forceinline__ void climb_group(const DGraph &g, const uint64_t *__restrict__ bound,
+                                            bool insert, const uint64_t *__restrict__ p_ul,
+                                            const uint32_t *__restrict__ g_start,
+                                            uint32_t nitems, uint32_t gid,
+                                            uint8_t *__restrict__ gtype,
+                                            uint8_t *__restrict__ glev,
+                                            uint32_t *__restrict__ gw0,
+                                            uint32_t *__restrict__ gw1) {
+  const int lane = threadIdx.x & 31;
+  uint32_t j0 = g_start[gid];
+  uint64_t key = p_ul[j0];
+  uint32_t u = (uint32_t)(key >> 32), leaf = (uint32_t)key;
+  uint32_t cap = g.cap[u];
+  uint64_t lbase = g.base[u] >> kLeafLog;
+  uint32_t H = log2_floor(cap >> kLeafLog);
+  uint64_t cur = g.lcnt[lbase + leaf];
+  uint32_t w0 = leaf, size = 1, w1 = leaf + 1, lev = 31;
+  uint8_t type = kResize;
+  const uint64_t kk = (uint64_t)u << 32;
+  // new items of the growing window: bounds inside the row's items, the
+  // lower one only moving left and the upper one only right
+  uint32_t rb = 0, re = 0, ib = 0, ie = 0;
+  if (insert) {
+    rb = warp_lb_u64(p_ul, 0, j0 + 1, kk);
+    re = warp_lb_u64(p_ul, j0, nitems, kk + (1ull << 32));
+    ib = j0;
+    ie = j0;
+  }
+  for (uint32_t t = 1; t <= H; t++) {
+    uint32_t nw0 = (leaf >> t) << t;
+    if (nw0 == w0)
+      cur += warp_sum_lcnt(g.lcnt, lbase + w0 + size, lbase + w0 + 2 * size);
+    else
+      cur += warp_sum_lcnt(g.lcnt, lbase + nw0, lbase + w0);
+    w0 = nw0;
+    size <<= 1;
+    w1 = w0 + size;
+    bool ok;
+    if (insert) {
+      ib = warp_lb_u64(p_ul, rb, ib + 1 < re ? ib + 1 : re, kk | w0);
+      ie = warp_lb_u64(p_ul, ie, re, kk | w1);
+      ok = cur + (ie - ib) <= bound[H * kBoundsH + t];
+    } else {
+      ok = cur >= bound[H * kBoundsH + t];
+    }
+    if (ok) {
+      type = kWindow;
+      lev = t;
+      break;
+    }
+  }
+  if (type == kResize) {
+    w0 = 0;
+    w1 = cap >> kLeafLog;
+  }
+  if (lane == 0) {
+    gtype[gid] = type;
+    glev[gid] = (uint8_t)lev;
+    gw0[gid] = w0;
+    gw1[gid] = w1;
+  }
+  __syncwarp();
+}
+
 __global__ void k_climb(DGraph g, const uint64_t *__restrict__ bound, bool insert,
                         const uint64_t *__restrict__ p_ul,
                         const uint32_t *__restrict__ g_start,
@@ -664,69 +757,25 @@ __global__ void k_climb(DGraph g, const uint64_t *__restrict__ bound, bool inser
                         uint8_t *__restrict__ gtype, uint8_t *__restrict__ glev,
                         uint32_t *__restrict__ gw0, uint32_t *__restrict__ gw1) {
   pdl_wait();
-  const int lane = threadIdx.x & 31;
   const uint32_t nc = *nclimb, nitems = *d_nitems;
   for (uint64_t ci = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-       ci < nc; ci += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
-    uint32_t gid = climb[ci];
-    uint32_t j0 = g_start[gid];
-    uint64_t key = p_ul[j0];
-    uint32_t u = (uint32_t)(key >> 32), leaf = (uint32_t)key;
-    uint32_t cap = g.cap[u];
-    uint64_t lbase = g.base[u] >> kLeafLog;
-    uint32_t H = log2_floor(cap >> kLeafLog);
-    uint64_t cur = g.lcnt[lbase + leaf];
-    uint32_t w0 = leaf, size = 1, w1 = leaf + 1, lev = 31;
-    uint8_t type = kResize;
-    const uint64_t kk = (uint64_t)u << 32;
-    // new items of the growing window: bounds inside the row's items, the
-    // lower one only moving left and the upper one only right
-    uint32_t rb = 0, re = 0, ib = 0, ie = 0;
-    if (insert) {
-      rb = warp_lb_u64(p_ul, 0, j0 + 1, kk);
-      re = warp_lb_u64(p_ul, j0, nitems, kk + (1ull << 32));
-      ib = j0;
-      ie = j0;
-    }
-    for (uint32_t t = 1; t <= H; t++) {
-      uint32_t nw0 = (leaf >> t) << t;
-      if (nw0 == w0)
-        cur += warp_sum_lcnt(g.lcnt, lbase + w0 + size, lbase + w0 + 2 * size);
-      else
-        cur += warp_sum_lcnt(g.lcnt, lbase + nw0, lbase + w0);
-      w0 = nw0;
-      size <<= 1;
-      w1 = w0 + size;
-      bool ok;
-      if (insert) {
-        ib = warp_lb_u64(p_ul, rb, ib + 1 < re ? ib + 1 : re, kk | w0);
-        ie = warp_lb_u64(p_ul, ie, re, kk | w1);
-        ok = cur + (ie - ib) <= bound[H * kBoundsH + t];
-      } else {
-        ok = cur >= bound[H * kBoundsH + t];
-      }
-      if (ok) {
-        type = kWindow;
-        lev = t;
-        break;
-      }
-    }
-    if (type == kResize) {
-      w0 = 0;
-      w1 = cap >> kLeafLog;
-    }
-    if (lane == 0) {
-      gtype[gid] = type;
-      glev[gid] = (uint8_t)lev;
-      gw0[gid] = w0;
-      gw1[gid] = w1;
-    }
-    __syncwarp();
-  }
+       ci < nc; ci += ((uint64_t)gridDim.x * blockDim.x) >> 5)
+    climb_group(g, bound, insert, p_ul, g_start, nitems, climb[ci], gtype, glev, gw0, gw1);
 }
 
 // ---------------------------------------------------------------- step 7
 constexpr uint64_t kWinMask = (1ull << 27) - 1;
+
+// a group's window as the two scans' keys (0 and ~0: no window)
+__device__ __forceinline__ void dom_keys(uint64_t u, uint8_t type, uint64_t lev, uint64_t w0,
+                                         uint64_t w1, uint64_t *f, uint64_t *bk) {
+  *f = 0;
+  *bk = ~0ull;
+  if (type >= kWindow) {
+    *f = (u << 32) | (w1 << 5) | lev;
+    *bk = (u << 32) | (w0 << 5) | (31 - lev);
+  }
+}
 
 __global__ void k_dom_keys(const uint64_t *__restrict__ p_ul,
                            const uint32_t *__restrict__ g_start,
@@ -741,12 +790,8 @@ __global__ void k_dom_keys(const uint64_t *__restrict__ p_ul,
   uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= gmax) return;
   uint64_t f = 0, bk = ~0ull;
-  if (gid < *d_ngroups && gtype[gid] >= kWindow) {
-    uint64_t u = p_ul[g_start[gid]] >> 32;
-    uint64_t lev = glev[gid];
-    f = (u << 32) | ((uint64_t)gw1[gid] << 5) | lev;
-    bk = (u << 32) | ((uint64_t)gw0[gid] << 5) | (31 - lev);
-  }
+  if (gid < *d_ngroups && gtype[gid] >= kWindow)
+    dom_keys(p_ul[g_start[gid]] >> 32, gtype[gid], glev[gid], gw0[gid], gw1[gid], &f, &bk);
   fkey[gid] = f;
   bkey[gid] = bk;
 }
@@ -754,6 +799,21 @@ __global__ void k_dom_keys(const uint64_t *__restrict__ p_ul,
 // fscan[g] = max of fkey over groups before g, bscan[g] = min of bkey over
 // groups after g.  A group is covered when a window of the same row from
 // either side contains its leaf and is larger (or equal and earlier).
+// The group's flags: merge in the low word, task in the high word (one scan of
+// the packed words gives both positions: the counts stay below 2^32).
+__device__ __forceinline__ uint64_t dom_flags(uint64_t key, uint8_t type, uint32_t lev, uint64_t L,
+                                              uint64_t R) {
+  if (type == kNone) return 0;
+  const uint64_t u = key >> 32;
+  const uint32_t leaf = (uint32_t)key;
+  const bool lcov = L != 0 && (L >> 32) == u && ((L >> 5) & kWinMask) > leaf;
+  const bool rcov = R != ~0ull && (R >> 32) == u && ((R >> 5) & kWinMask) <= leaf;
+  if (type == kMerge) return !(lcov || rcov);
+  const uint32_t lt = (uint32_t)(L & 31), rt = 31u - (uint32_t)(R & 31);
+  const bool dom = (lcov && lt >= lev) || (rcov && rt > lev);
+  return (uint64_t)!dom << 32;
+}
+
 __global__ void k_dom_classify(const uint64_t *__restrict__ p_ul,
                                const uint32_t *__restrict__ g_start,
                                const uint8_t *__restrict__ gtype,
@@ -765,26 +825,9 @@ __global__ void k_dom_classify(const uint64_t *__restrict__ p_ul,
   pdl_wait();
   uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= gmax) return;
-  uint32_t mf = 0, tf = 0;
-  if (gid < *d_ngroups && gtype[gid] != kNone) {
-    uint64_t key = p_ul[g_start[gid]];
-    uint64_t u = key >> 32;
-    uint32_t leaf = (uint32_t)key;
-    uint64_t L = fscan[gid], R = bscan[gid];
-    bool lcov = L != 0 && (L >> 32) == u && ((L >> 5) & kWinMask) > leaf;
-    bool rcov = R != ~0ull && (R >> 32) == u && ((R >> 5) & kWinMask) <= leaf;
-    uint32_t lt = (uint32_t)(L & 31), rt = 31u - (uint32_t)(R & 31);
-    if (gtype[gid] == kMerge) {
-      mf = !(lcov || rcov);
-    } else {
-      uint32_t lev = glev[gid];
-      bool dom = (lcov && lt >= lev) || (rcov && rt > lev);
-      tf = !dom;
-    }
-  }
-  // merge flag in the low word, task flag in the high word: one scan of
-  // the packed words gives both positions (the counts stay below 2^32)
-  mt[gid] = ((uint64_t)tf << 32) | mf;
+  mt[gid] = gid < *d_ngroups ? dom_flags(p_ul[g_start[gid]], gtype[gid], glev[gid], fscan[gid],
+                                         bscan[gid])
+                             : 0ull;
 }
 
 
@@ -930,6 +973,51 @@ __global__ void k_emit(const uint64_t *__restrict__ mt, const uint64_t *__restri
   emit_group(a, gid, in ? mt[gid] : 0, in ? mtpos[gid] : 0);
 }
 
+__device__ __forceinline__ void task_setup_hard(const DGraph &g, uint64_t inv_fill, bool insert,
+                                                const uint64_t *__restrict__ p_ul,
+                                                const uint32_t *__restrict__ g_start,
+                                                const uint8_t *__restrict__ gtype,
+                                                const uint32_t *__restrict__ gw0,
+                                                const uint32_t *__restrict__ gw1,
+                                                const uint32_t *__restrict__ task_group,
+                                                uint32_t tid, uint32_t nitems, Tasks &t,
+                                                uint32_t *__restrict__ class_cnt) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t gid = task_group[tid];
+  const uint32_t j0 = g_start[gid];
+  const uint32_t u = (uint32_t)(p_ul[j0] >> 32);
+  const uint8_t type = gtype[gid];
+  const uint64_t base = g.base[u];
+  const uint32_t cap = g.cap[u];
+  const uint64_t kk = (uint64_t)u << 32;
+  uint32_t w0, b = 0, e = 0, rank = 0;
+  uint64_t nsrc, ndst, old, capn = 0;
+  if (type == kWindow) {
+    w0 = gw0[gid];
+    const uint32_t w1 = gw1[gid];
+    nsrc = w1 - w0;
+    old = warp_sum_lcnt(g.lcnt, (base >> kLeafLog) + w0, (base >> kLeafLog) + w1);
+    if (insert) {  // the group's first item lies between the two bounds
+      b = warp_lb_u64(p_ul, 0, j0 + 1, kk | w0);
+      e = warp_lb_u64(p_ul, j0, nitems, kk | w1);
+    }
+    ndst = nsrc;
+  } else {
+    w0 = 0;
+    nsrc = cap == 0 ? 0 : nleaves_of(cap);
+    old = g.deg[u];
+    if (insert) {
+      b = warp_lb_u64(p_ul, 0, j0 + 1, kk);
+      e = warp_lb_u64(p_ul, j0, nitems, kk + (1ull << 32));
+    }
+    capn = cap_for(old + (e - b), inv_fill);
+    ndst = capn == 0 ? 0 : nleaves_of((uint32_t)capn);
+    if (lane == 0 && capn > 0) rank = atomicAdd(&class_cnt[log2_floor(capn)], 1u);
+  }
+  if (lane == 0) task_store(t, tid, u, w0, nsrc, ndst, b, e, old, capn, rank, type);
+  __syncwarp();
+}
+
 __global__ void k_task_setup_hard(DGraph g, uint64_t inv_fill, bool insert,
                                   const uint64_t *__restrict__ p_ul,
                                   const uint32_t *__restrict__ g_start,
@@ -942,45 +1030,11 @@ __global__ void k_task_setup_hard(DGraph g, uint64_t inv_fill, bool insert,
                                   const uint32_t *__restrict__ d_nitems, Tasks t,
                                   uint32_t *__restrict__ class_cnt) {
   pdl_wait();
-  const int lane = threadIdx.x & 31;
   const uint32_t nh = *nhard, nitems = *d_nitems;
   for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nh;
-       i += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
-    const uint32_t tid = hard[i];
-    const uint32_t gid = task_group[tid];
-    const uint32_t j0 = g_start[gid];
-    const uint32_t u = (uint32_t)(p_ul[j0] >> 32);
-    const uint8_t type = gtype[gid];
-    const uint64_t base = g.base[u];
-    const uint32_t cap = g.cap[u];
-    const uint64_t kk = (uint64_t)u << 32;
-    uint32_t w0, b = 0, e = 0, rank = 0;
-    uint64_t nsrc, ndst, old, capn = 0;
-    if (type == kWindow) {
-      w0 = gw0[gid];
-      const uint32_t w1 = gw1[gid];
-      nsrc = w1 - w0;
-      old = warp_sum_lcnt(g.lcnt, (base >> kLeafLog) + w0, (base >> kLeafLog) + w1);
-      if (insert) {  // the group's first item lies between the two bounds
-        b = warp_lb_u64(p_ul, 0, j0 + 1, kk | w0);
-        e = warp_lb_u64(p_ul, j0, nitems, kk | w1);
-      }
-      ndst = nsrc;
-    } else {
-      w0 = 0;
-      nsrc = cap == 0 ? 0 : nleaves_of(cap);
-      old = g.deg[u];
-      if (insert) {
-        b = warp_lb_u64(p_ul, 0, j0 + 1, kk);
-        e = warp_lb_u64(p_ul, j0, nitems, kk + (1ull << 32));
-      }
-      capn = cap_for(old + (e - b), inv_fill);
-      ndst = capn == 0 ? 0 : nleaves_of((uint32_t)capn);
-      if (lane == 0 && capn > 0) rank = atomicAdd(&class_cnt[log2_floor(capn)], 1u);
-    }
-    if (lane == 0) task_store(t, tid, u, w0, nsrc, ndst, b, e, old, capn, rank, type);
-    __syncwarp();
-  }
+       i += ((uint64_t)gridDim.x * blockDim.x) >> 5)
+    task_setup_hard(g, inv_fill, insert, p_ul, g_start, gtype, gw0, gw1, task_group, hard[i],
+                    nitems, t, class_cnt);
 }
 
 // The plan summary to the host, written by one block straight into the
@@ -1012,6 +1066,100 @@ __global__ void k_err_out(const unsigned long long *__restrict__ err,
 // first item's leaf start and count word (two dependent loads for all 32
 // groups at once), then the groups go kGroupsPerWarp at a time with their
 // items and leaf lines loaded together, one dependent load per batch.
+__device__ __forceinline__ void leaf_merge_chunk(
+    const DGraph &g, uint64_t w, uint32_t nmerge, uint8_t *list,
+    const uint64_t *__restrict__ p_ul, const uint32_t *__restrict__ p_x,
+    const uint64_t *__restrict__ p_S, const uint32_t *__restrict__ p_c,
+    const uint64_t *__restrict__ merge_jk, const uint32_t *__restrict__ p_w) {
+  const int lane = threadIdx.x & 31, sub = lane & 7;
+  constexpr int Q = kGroupsPerWarp;
+  const uint64_t gl = w * 32 + lane;
+  const bool okl = gl < nmerge;
+  const uint64_t jkl = okl ? merge_jk[gl] : 0;
+  const uint32_t j0l = (uint32_t)(jkl >> 32), kl = (uint32_t)jkl;
+  const uint64_t Sl = okl ? p_S[j0l] : 0;
+  const uint32_t cwl = okl ? p_c[j0l] : 0;
+  const uint32_t ul = okl ? (uint32_t)(p_ul[j0l] >> 32) : 0u;
+  const uint32_t cnt = nmerge - w * 32 < 32 ? (uint32_t)(nmerge - w * 32) : 32u;
+  // one-item groups: the new id goes to the count of the slots below it,
+  // the slots from there up move one place right
+  const uint32_t n1 = list_groups(list, okl, kl == 1 && !g.vals, lane);
+  for (uint32_t f0 = 0; f0 < n1; f0 += 4) {
+    const uint32_t f = f0 + (lane >> 3);
+    const bool on = f < n1;
+    const int src = list[on ? f : 0];
+    const uint32_t j0 = __shfl_sync(0xffffffffu, j0l, src);
+    const uint64_t S = __shfl_sync(0xffffffffu, Sl, src);
+    const uint32_t cw = __shfl_sync(0xffffffffu, cwl, src);
+    const uint32_t c = on ? (cw & 0xff) : 0u;
+    const uint32_t x = on ? p_x[j0] : kEmpty;
+    uint32_t a[4];
+    load_quarter(g.slots, S, c, sub, a);
+    const uint32_t pos = below_in_octet(a, x);
+    const uint32_t prev = __shfl_up_sync(0xffffffffu, a[3], 1, 8);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const uint32_t p = 4 * sub + r;
+      if (on && p >= pos && p <= c) g.slots[S + p] = p == pos ? x : (r ? a[r - 1] : prev);
+    }
+  }
+  // the other groups: a warp each, kGroupsPerWarp at a time
+  const uint32_t nrest = cnt - n1;
+  for (uint32_t q0 = 0; q0 < nrest; q0 += Q) {
+    uint32_t j0[Q], k[Q], x[Q], linev[Q], cw[Q];
+    uint64_t S[Q];
+    bool ok[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      ok[q] = q0 + q < nrest;
+      const int src = list[n1 + (ok[q] ? q0 + q : 0)];
+      j0[q] = __shfl_sync(0xffffffffu, j0l, src);
+      k[q] = ok[q] ? __shfl_sync(0xffffffffu, kl, src) : 0;
+      S[q] = __shfl_sync(0xffffffffu, Sl, src);
+      cw[q] = __shfl_sync(0xffffffffu, cwl, src);
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      x[q] = (uint32_t)lane < k[q] ? p_x[j0[q] + lane] : kEmpty;
+      linev[q] = ok[q] ? g.slots[(S[q] & ~uint64_t(kLeaf - 1)) + lane] : kEmpty;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      if (!ok[q]) break;
+      const uint32_t c = cw[q] & 0xff;
+      const uint32_t a = leaf_slot(linev[q], S[q], c, lane);
+      // merged ranks in O(k) steps (k new ids, usually one or two): an old
+      // id moves up by the new ids below it; new id j lands at j + the old
+      // ids below it (a ballot per new id)
+      uint32_t pa = lane, px = lane;
+      for (uint32_t j = 0; j < k[q]; j++) {
+        uint32_t xj = __shfl_sync(0xffffffffu, x[q], j);
+        pa += xj < a;
+        uint32_t below = __popc(__ballot_sync(0xffffffffu, (uint32_t)lane < c && a < xj));
+        if ((uint32_t)lane == j) px = j + below;
+      }
+      // values move with their ids (weighted graphs)
+      if (g.vals) {
+        const uint32_t av = (uint32_t)lane < c ? g.vals[S[q] + lane] : 0u;
+        const uint32_t xv = (uint32_t)lane < k[q] ? (p_w ? p_w[j0[q] + lane] : 1u) : 0u;
+        __syncwarp();  // every value read before any is moved
+        if ((uint32_t)lane < c) g.vals[S[q] + pa] = av;
+        if ((uint32_t)lane < k[q]) g.vals[S[q] + px] = xv;
+      }
+      // the ids come from registers: no lane reads the line again
+      if ((uint32_t)lane < c) g.slots[S[q] + pa] = a;
+      if ((uint32_t)lane < k[q]) g.slots[S[q] + px] = x[q];
+    }
+  }
+  // the chunk's leaf counts and degrees, lane l for group l.  No task
+  // reads these rows' degrees: a one-leaf row is one group (a merge or a
+  // resize), and a row with a resize task has no merge group.
+  if (okl) {
+    if (cwl & kMultiLeaf) g.lcnt[Sl >> kLeafLog] = (uint8_t)((cwl & 0xff) + kl);
+    atomicAdd(&g.deg[ul], kl);
+  }
+}
+
 __global__ void __launch_bounds__(256, 4)
 k_leaf_merge(DGraph g, const uint64_t *__restrict__ p_ul, const uint32_t *__restrict__ p_x,
              const uint64_t *__restrict__ p_S, const uint32_t *__restrict__ p_c,
@@ -1019,99 +1167,11 @@ k_leaf_merge(DGraph g, const uint64_t *__restrict__ p_ul, const uint32_t *__rest
              const uint32_t *__restrict__ p_w) {
   pdl_wait();
   __shared__ uint8_t glist[kLeafWarps][32];
-  const int lane = threadIdx.x & 31, sub = lane & 7;
-  uint8_t *list = glist[threadIdx.x >> 5];
-  constexpr int Q = kGroupsPerWarp;
   const uint32_t nmerge = *d_nmerge;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-       w * 32 < nmerge; w += nw) {
-    const uint64_t gl = w * 32 + lane;
-    const bool okl = gl < nmerge;
-    const uint64_t jkl = okl ? merge_jk[gl] : 0;
-    const uint32_t j0l = (uint32_t)(jkl >> 32), kl = (uint32_t)jkl;
-    const uint64_t Sl = okl ? p_S[j0l] : 0;
-    const uint32_t cwl = okl ? p_c[j0l] : 0;
-    const uint32_t ul = okl ? (uint32_t)(p_ul[j0l] >> 32) : 0u;
-    const uint32_t cnt = nmerge - w * 32 < 32 ? (uint32_t)(nmerge - w * 32) : 32u;
-    // one-item groups: the new id goes to the count of the slots below it,
-    // the slots from there up move one place right
-    const uint32_t n1 = list_groups(list, okl, kl == 1 && !g.vals, lane);
-    for (uint32_t f0 = 0; f0 < n1; f0 += 4) {
-      const uint32_t f = f0 + (lane >> 3);
-      const bool on = f < n1;
-      const int src = list[on ? f : 0];
-      const uint32_t j0 = __shfl_sync(0xffffffffu, j0l, src);
-      const uint64_t S = __shfl_sync(0xffffffffu, Sl, src);
-      const uint32_t cw = __shfl_sync(0xffffffffu, cwl, src);
-      const uint32_t c = on ? (cw & 0xff) : 0u;
-      const uint32_t x = on ? p_x[j0] : kEmpty;
-      uint32_t a[4];
-      load_quarter(g.slots, S, c, sub, a);
-      const uint32_t pos = below_in_octet(a, x);
-      const uint32_t prev = __shfl_up_sync(0xffffffffu, a[3], 1, 8);
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const uint32_t p = 4 * sub + r;
-        if (on && p >= pos && p <= c) g.slots[S + p] = p == pos ? x : (r ? a[r - 1] : prev);
-      }
-    }
-    // the other groups: a warp each, kGroupsPerWarp at a time
-    const uint32_t nrest = cnt - n1;
-    for (uint32_t q0 = 0; q0 < nrest; q0 += Q) {
-      uint32_t j0[Q], k[Q], x[Q], linev[Q], cw[Q];
-      uint64_t S[Q];
-      bool ok[Q];
-#pragma unroll
-      for (int q = 0; q < Q; q++) {
-        ok[q] = q0 + q < nrest;
-        const int src = list[n1 + (ok[q] ? q0 + q : 0)];
-        j0[q] = __shfl_sync(0xffffffffu, j0l, src);
-        k[q] = ok[q] ? __shfl_sync(0xffffffffu, kl, src) : 0;
-        S[q] = __shfl_sync(0xffffffffu, Sl, src);
-        cw[q] = __shfl_sync(0xffffffffu, cwl, src);
-      }
-#pragma unroll
-      for (int q = 0; q < Q; q++) {
-        x[q] = (uint32_t)lane < k[q] ? p_x[j0[q] + lane] : kEmpty;
-        linev[q] = ok[q] ? g.slots[(S[q] & ~uint64_t(kLeaf - 1)) + lane] : kEmpty;
-      }
-#pragma unroll
-      for (int q = 0; q < Q; q++) {
-        if (!ok[q]) break;
-        const uint32_t c = cw[q] & 0xff;
-        const uint32_t a = leaf_slot(linev[q], S[q], c, lane);
-        // merged ranks in O(k) steps (k new ids, usually one or two): an old
-        // id moves up by the new ids below it; new id j lands at j + the old
-        // ids below it (a ballot per new id)
-        uint32_t pa = lane, px = lane;
-        for (uint32_t j = 0; j < k[q]; j++) {
-          uint32_t xj = __shfl_sync(0xffffffffu, x[q], j);
-          pa += xj < a;
-          uint32_t below = __popc(__ballot_sync(0xffffffffu, (uint32_t)lane < c && a < xj));
-          if ((uint32_t)lane == j) px = j + below;
-        }
-        // values move with their ids (weighted graphs)
-        if (g.vals) {
-          const uint32_t av = (uint32_t)lane < c ? g.vals[S[q] + lane] : 0u;
-          const uint32_t xv = (uint32_t)lane < k[q] ? (p_w ? p_w[j0[q] + lane] : 1u) : 0u;
-          __syncwarp();  // every value read before any is moved
-          if ((uint32_t)lane < c) g.vals[S[q] + pa] = av;
-          if ((uint32_t)lane < k[q]) g.vals[S[q] + px] = xv;
-        }
-        // the ids come from registers: no lane reads the line again
-        if ((uint32_t)lane < c) g.slots[S[q] + pa] = a;
-        if ((uint32_t)lane < k[q]) g.slots[S[q] + px] = x[q];
-      }
-    }
-    // the chunk's leaf counts and degrees, lane l for group l.  No task
-    // reads these rows' degrees: a one-leaf row is one group (a merge or a
-    // resize), and a row with a resize task has no merge group.
-    if (okl) {
-      if (cwl & kMultiLeaf) g.lcnt[Sl >> kLeafLog] = (uint8_t)((cwl & 0xff) + kl);
-      atomicAdd(&g.deg[ul], kl);
-    }
-  }
+       w * 32 < nmerge; w += nw)
+    leaf_merge_chunk(g, w, nmerge, glist[threadIdx.x >> 5], p_ul, p_x, p_S, p_c, merge_jk, p_w);
 }
 
 // the task of every source and destination leaf of the window / resize
@@ -1147,15 +1207,12 @@ __global__ void k_task_index(DGraph g, Tasks t, uint32_t ntasks, uint32_t *__res
 // `sub` taking slots sub, sub + 8, sub + 16, sub + 24, four leaves a warp
 // (the chain of dependent loads -- task, row, count, ids, rank among the
 // task's new ids -- is paid once per four leaves, not once per leaf)
-__global__ void k_gather_old(DGraph g, Tasks t, uint32_t ntasks,
+__device__ __forceinline__ void gather_old(const uint64_t s, const uint32_t sub, DGraph g, Tasks t, uint32_t ntasks,
                              uint64_t nsrc_total,
-                             const uint64_t *__restrict__ spre,
-                             const uint32_t *__restrict__ p_x,
-                             uint32_t *__restrict__ stage,
-                             const uint32_t *__restrict__ stask) {
-  pdl_wait();
-  const uint64_t s = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-  const uint32_t sub = threadIdx.x & 7;
+                             const uint64_t *spre,
+                             const uint32_t *p_x,
+                             uint32_t *stage,
+                             const uint32_t *stask) {
   if (s >= nsrc_total) return;
   const uint64_t tau = stask[s];
   const uint32_t u = t.u[tau];
@@ -1184,15 +1241,25 @@ __global__ void k_gather_old(DGraph g, Tasks t, uint32_t ntasks,
   }
 }
 
-// thread per packed item owned by a task: new elements to their merged rank
-__global__ void k_gather_new(DGraph g, Tasks t, uint32_t ntasks,
+__global__ void k_gather_old(DGraph g, Tasks t, uint32_t ntasks,
+                             uint64_t nsrc_total,
                              const uint64_t *__restrict__ spre,
-                             const uint64_t *__restrict__ p_ul,
-                             const uint32_t *__restrict__ p_x, uint32_t nitems,
+                             const uint32_t *__restrict__ p_x,
                              uint32_t *__restrict__ stage,
-                             const uint32_t *__restrict__ itask) {
+                             const uint32_t *__restrict__ stask) {
   pdl_wait();
-  uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t s = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const uint32_t sub = threadIdx.x & 7;
+  gather_old(s, sub, g, t, ntasks, nsrc_total, spre, p_x, stage, stask);
+}
+
+// thread per packed item owned by a task: new elements to their merged rank
+__device__ __forceinline__ void gather_new(const uint64_t j, DGraph g, Tasks t, uint32_t ntasks,
+                             const uint64_t *spre,
+                             const uint64_t *p_ul,
+                             const uint32_t *p_x, uint32_t nitems,
+                             uint32_t *stage,
+                             const uint32_t *itask) {
   if (j >= nitems || ntasks == 0) return;
   const uint32_t tau = itask[j];
   if (tau >= ntasks) return;  // a leaf merge takes this item (kEmpty)
@@ -1227,6 +1294,17 @@ __global__ void k_gather_new(DGraph g, Tasks t, uint32_t ntasks,
   if (t.stage_v) t.stage_v[t.out[tau] + rank] = t.p_w ? t.p_w[j] : 1u;
 }
 
+__global__ void k_gather_new(DGraph g, Tasks t, uint32_t ntasks,
+                             const uint64_t *__restrict__ spre,
+                             const uint64_t *__restrict__ p_ul,
+                             const uint32_t *__restrict__ p_x, uint32_t nitems,
+                             uint32_t *__restrict__ stage,
+                             const uint32_t *__restrict__ itask) {
+  pdl_wait();
+  uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  gather_new(j, g, t, ntasks, spre, p_ul, p_x, nitems, stage, itask);
+}
+
 // first slab slot of each capacity class's new segments (largest class
 // first), passed by value: the apply kernels need no copy of it on the device
 struct ClassStarts {
@@ -1245,14 +1323,11 @@ __device__ __forceinline__ uint64_t task_new_base(const Tasks &t, uint64_t tau,
 // lane finds the leaf's task and its share of the task's elements itself
 // (the loads are the same address across the eight; 32-bit arithmetic: a
 // task holds fewer than 2^32 elements).
-__global__ void k_task_scatter(DGraph g, Tasks t, uint32_t ntasks,
+__device__ __forceinline__ void task_scatter(const uint64_t d, const uint32_t sub, DGraph g, Tasks t, uint32_t ntasks,
                                uint64_t ndst_total,
                                const ClassStarts class_start,
-                               const uint32_t *__restrict__ stage,
-                               const uint32_t *__restrict__ dtask) {
-  pdl_wait();
-  const uint64_t d = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-  const uint32_t sub = threadIdx.x & 7;
+                               const uint32_t *stage,
+                               const uint32_t *dtask) {
   if (d >= ndst_total) return;
   const uint64_t tau = dtask[d];
   const uint32_t i = (uint32_t)(d - t.doff[tau]);
@@ -1282,13 +1357,22 @@ __global__ void k_task_scatter(DGraph g, Tasks t, uint32_t ntasks,
   if (sub == 0 && multi) g.lcnt[S >> kLeafLog] = (uint8_t)cnt;
 }
 
+__global__ void k_task_scatter(DGraph g, Tasks t, uint32_t ntasks,
+                               uint64_t ndst_total,
+                               const ClassStarts class_start,
+                               const uint32_t *__restrict__ stage,
+                               const uint32_t *__restrict__ dtask) {
+  pdl_wait();
+  const uint64_t d = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const uint32_t sub = threadIdx.x & 7;
+  task_scatter(d, sub, g, t, ntasks, ndst_total, class_start, stage, dtask);
+}
+
 // resized rows get their new segment; every task's row gets the new items
 // the task took (an insert's items are each taken by one merge group or one
 // task, and the merge kernel counts its own)
-__global__ void k_finalize(DGraph g, Tasks t, uint32_t ntasks,
+__device__ __forceinline__ void task_finalize(const uint64_t tau, DGraph g, Tasks t, uint32_t ntasks,
                            const ClassStarts class_start) {
-  pdl_wait();
-  uint64_t tau = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tau >= ntasks) return;
   uint32_t u = t.u[tau];
   const uint32_t added = t.newend[tau] - t.newbeg[tau];
@@ -1297,6 +1381,376 @@ __global__ void k_finalize(DGraph g, Tasks t, uint32_t ntasks,
   uint64_t capn = t.capn[tau];
   g.base[u] = capn ? task_new_base(t, tau, class_start) : 0;
   g.cap[u] = (uint32_t)capn;
+}
+
+__global__ void k_finalize(DGraph g, Tasks t, uint32_t ntasks,
+                           const ClassStarts class_start) {
+  pdl_wait();
+  uint64_t tau = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  task_finalize(tau, g, t, ntasks, class_start);
+}
+
+// ------------------------------------------------------ small batches
+// A batch of up to kSmallBatch pairs in three launches, where the general
+// sequence takes about 26: each of those is one block that runs for 2 to 4 us,
+// nearly all of it launch and first loads.  (1) a warp a pair locates it,
+// unsorted; (2) one block sorts the pairs that change the graph and plans the
+// batch, its steps a block barrier apart; (3) one cluster applies the plan, its
+// steps a cluster barrier apart.  An insert and a remove at RMAT scale 20, with
+// a degree copy and a lookup: 1 pair 115 -> 54 us, 300 136 -> 74, 1000 150 -> 92.
+// The plan's block has 512 threads, half of what an SM holds: one of 1024 would
+// wait for an idle SM where other streams' kernels run (a served graph).  Above
+// kSmallBatch its shared arrays outgrow the block, and its serial share (20 us
+// a batch at 1000 pairs, where the general sequence is flat) the launches.
+constexpr uint32_t kSmallBatch = 1024;
+constexpr int kSmallThreads = 512;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallPer = kSmallBatch / kSmallThreads;
+static_assert(kSmallPer == 2, "two items a thread");
+
+// what the plan makes of a pair
+enum : uint32_t { kPairDropped = 0, kPairKept = 1, kPairInvalid = 2 };
+
+__global__ void k_small_locate(const uint32_t *__restrict__ pairs, uint32_t b, DGraph g, int dbits,
+                               bool insert, bool drop_loops, uint64_t *__restrict__ keys,
+                               uint32_t *__restrict__ state, uint32_t *__restrict__ leaf,
+                               uint64_t *__restrict__ lS, uint32_t *__restrict__ lc) {
+  pdl_wait();
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (i >= b) return;  // whole warps
+  const uint32_t r = pairs[2 * (uint64_t)i], c = pairs[2 * (uint64_t)i + 1];
+  const bool ok = r < g.n && c < g.width && c != kEmpty;
+  if (!ok || (drop_loops && r == c)) {
+    if (lane == 0) state[i] = ok ? kPairDropped : kPairInvalid;
+    return;
+  }
+  const Located p = locate_by_warp(g, r, c);
+  if (lane == 0) {
+    state[i] = p.present != insert ? kPairKept : kPairDropped;
+    keys[i] = ((uint64_t)r << dbits) | c;
+    leaf[i] = p.leaf;
+    lS[i] = p.S;
+    lc[i] = p.cw;
+  }
+}
+
+// exclusive scan of a value a thread over the plan's block; sm holds one value
+// a warp and is free again afterwards
+template <typename T, typename Op>
+__device__ __forceinline__ T small_scan(T v, T identity, Op op, T *total, T *sm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const T inc = warp_inclusive(v, op);
+  if (lane == 31) sm[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    const T w = lane < kSmallWarps ? sm[lane] : identity;
+    const T wi = warp_inclusive(w, op);
+    if (lane < kSmallWarps) sm[lane] = wi;
+  }
+  __syncthreads();
+  T ex = __shfl_up_sync(0xffffffffu, inc, 1);
+  if (lane == 0) ex = identity;
+  if (warp) ex = op(sm[warp - 1], ex);
+  *total = sm[kSmallWarps - 1];
+  __syncthreads();
+  return ex;
+}
+
+// Sort of n <= kSmallBatch keys in shared memory with their places i: warps
+// sort runs of 32 in registers (a bitonic network of shuffles), then each key
+// finds its place in its run's neighbour by binary search, run lengths doubling.
+// Returns which of the two buffers holds the result.  Equal keys may change
+// places.
+__device__ __forceinline__ int small_sort(uint64_t (&key)[2][kSmallBatch],
+                                          uint16_t (&at)[2][kSmallBatch], uint32_t n) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t N = 32;
+  while (N < n) N <<= 1;
+  for (uint32_t r = warp; r * 32 < N; r += kSmallWarps) {
+    const uint32_t e = r * 32 + lane;
+    uint64_t x = e < n ? key[0][e] : ~0ull;
+    uint32_t i = e < n ? at[0][e] : 0u;
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        const uint64_t y = __shfl_xor_sync(0xffffffffu, x, j);
+        const uint32_t o = __shfl_xor_sync(0xffffffffu, i, j);
+        const bool low = !(lane & j), up = !(lane & k);
+        if (x != y && (y < x) == (low == up)) {
+          x = y;
+          i = o;
+        }
+      }
+    key[0][e] = x;
+    at[0][e] = (uint16_t)i;
+  }
+  __syncthreads();
+  int cur = 0;
+  for (uint32_t len = 32; len < N; len <<= 1, cur ^= 1) {
+    for (uint32_t e = threadIdx.x; e < N; e += kSmallThreads) {
+      const bool second = e & len;
+      const uint32_t other = (e & ~(2 * len - 1)) + (second ? 0 : len);
+      const uint64_t x = key[cur][e];
+      uint32_t lo = 0, cnt = len;  // keys of the other run before x
+      while (cnt) {
+        const uint32_t half = cnt >> 1;
+        const uint64_t y = key[cur][other + lo + half];
+        if (y < x || (second && y == x)) {
+          lo += half + 1;
+          cnt -= half + 1;
+        } else {
+          cnt = half;
+        }
+      }
+      const uint32_t to = (e & ~(2 * len - 1)) + (e & (len - 1)) + lo;
+      key[cur ^ 1][to] = x;
+      at[cur ^ 1][to] = at[cur][e];
+    }
+    __syncthreads();
+  }
+  return cur;
+}
+
+struct SmallPlan {
+  DGraph g;
+  uint32_t b;      // pairs
+  int dbits;
+  bool insert;
+  uint32_t lo_leaf;
+  const uint64_t *bounds;
+  const uint64_t *keys;  // per pair, from k_small_locate
+  const uint32_t *state, *leaf, *lc;
+  const uint64_t *lS;
+  uint64_t *p_ul, *p_S;  // per item, sorted
+  uint32_t *p_x, *p_c;
+  uint32_t *g_start, *gw0, *gw1, *climb, *hard;  // per group
+  uint8_t *gtype, *glev;
+  EmitArgs emit;         // its class counts and hard count are the block's own
+  const unsigned long long *err;
+  PlanSummary *host;
+};
+
+__global__ void __launch_bounds__(kSmallThreads) k_small_plan(SmallPlan a) {
+  pdl_wait();
+  __shared__ uint64_t s_key[2][kSmallBatch];
+  __shared__ uint16_t s_at[2][kSmallBatch];
+  __shared__ uint64_t s_w64[kSmallWarps];
+  __shared__ uint32_t s_w32[kSmallWarps];
+  __shared__ uint64_t s_mirror[kSmallThreads];
+  __shared__ uint8_t s_list[kSmallWarps][32];
+  __shared__ uint32_t s_class[kNumClasses], s_nclimb, s_nhard;
+  const uint32_t t = threadIdx.x;
+  const int warp = t >> 5;
+  if (t < kNumClasses) s_class[t] = 0;
+  if (t == 0) s_nclimb = s_nhard = 0;
+  // the pairs that change the graph, to the front
+  uint32_t st[kSmallPer], own = 0;
+#pragma unroll
+  for (int k = 0; k < kSmallPer; k++) {
+    const uint32_t i = t + k * kSmallThreads;
+    st[k] = i < a.b ? a.state[i] : (uint32_t)kPairDropped;
+    own += st[k] == kPairKept ? 1u : st[k] == kPairInvalid ? 1u << 16 : 0u;
+  }
+  uint32_t tot;
+  uint32_t at = small_scan(own, 0u, OpAdd{}, &tot, s_w32) & 0xffff;
+  const uint32_t n = tot & 0xffff, invalid = tot >> 16;
+#pragma unroll
+  for (int k = 0; k < kSmallPer; k++)
+    if (st[k] == kPairKept) {
+      const uint32_t i = t + k * kSmallThreads;
+      s_key[0][at] = a.keys[i];
+      s_at[0][at++] = (uint16_t)i;
+    }
+  __syncthreads();
+  const int cur = small_sort(s_key, s_at, n);
+  // items (the first of equal pairs) and groups (one leaf of one row each)
+  uint64_t *s_ul = s_key[cur ^ 1];
+  uint64_t ul[kSmallPer];
+  uint32_t src[kSmallPer];
+#pragma unroll
+  for (int k = 0; k < kSmallPer; k++) {
+    const uint32_t j = kSmallPer * t + k;
+    src[k] = j < n ? s_at[cur][j] : 0u;
+    ul[k] = j < n ? (s_key[cur][j] >> a.dbits) << 32 | a.leaf[src[k]] : ~0ull;
+    s_ul[j] = ul[k];
+  }
+  __syncthreads();
+  bool keep[kSmallPer], head[kSmallPer];
+  uint32_t cnt = 0;
+#pragma unroll
+  for (int k = 0; k < kSmallPer; k++) {
+    const uint32_t j = kSmallPer * t + k;
+    keep[k] = j < n && (j == 0 || s_key[cur][j] != s_key[cur][j - 1]);
+    head[k] = keep[k] && (j == 0 || s_ul[j] != s_ul[j - 1]);
+    cnt += (keep[k] ? 1u : 0u) + (head[k] ? 1u << 16 : 0u);
+  }
+  at = small_scan(cnt, 0u, OpAdd{}, &tot, s_w32);
+  const uint32_t ni = tot & 0xffff, ng = tot >> 16;
+#pragma unroll
+  for (int k = 0; k < kSmallPer; k++) {
+    const uint32_t j = kSmallPer * t + k, item = at & 0xffff, grp = at >> 16;
+    if (head[k]) a.g_start[grp] = item;
+    if (keep[k]) {
+      a.p_ul[item] = ul[k];
+      a.p_x[item] = (uint32_t)(s_key[cur][j] & ((1ull << a.dbits) - 1));
+      a.p_S[item] = a.lS[src[k]];
+      a.p_c[item] = a.lc[src[k]];
+    }
+    at += (keep[k] ? 1u : 0u) + (head[k] ? 1u << 16 : 0u);
+  }
+  if (t == 0) a.g_start[ng] = ni;
+  __syncthreads();
+  // classify (a remove also deletes), then the climbs
+  if (a.insert) {
+    for (uint32_t gid = t; gid < ng; gid += kSmallThreads)
+      classify_insert(gid, a.p_ul, a.p_c, a.g_start, a.gtype, a.glev, a.gw0, a.gw1, a.climb,
+                      &s_nclimb);
+  } else {
+    for (uint32_t w = warp; w * 32 < ng; w += kSmallWarps)
+      leaf_delete_chunk(a.g, w, ng, s_list[warp], a.lo_leaf, a.p_ul, a.p_x, a.p_S, a.p_c,
+                        a.g_start, a.gtype, a.glev, a.gw0, a.gw1, a.climb, &s_nclimb);
+  }
+  __syncthreads();
+  for (uint32_t c = warp; c < s_nclimb; c += kSmallWarps)
+    climb_group(a.g, a.bounds, a.insert, a.p_ul, a.g_start, ni, a.climb[c], a.gtype, a.glev,
+                a.gw0, a.gw1);
+  __syncthreads();
+  // dominance: the largest window from either side
+  uint64_t key[kSmallPer], f[kSmallPer], r[kSmallPer], flags[kSmallPer];
+  uint8_t type[kSmallPer], lev[kSmallPer];
+#pragma unroll
+  for (int k = 0; k < kSmallPer; k++) {
+    const uint32_t gid = kSmallPer * t + k;
+    const bool in = gid < ng;
+    key[k] = in ? a.p_ul[a.g_start[gid]] : 0ull;
+    type[k] = in ? a.gtype[gid] : (uint8_t)kNone;
+    lev[k] = in ? a.glev[gid] : (uint8_t)0;
+    dom_keys(key[k] >> 32, type[k], lev[k], in ? a.gw0[gid] : 0u, in ? a.gw1[gid] : 0u, &f[k],
+             &r[k]);
+  }
+  uint64_t tot64;
+  const uint64_t fx = small_scan(f[0] > f[1] ? f[0] : f[1], (uint64_t)0, OpMax{}, &tot64, s_w64);
+  s_mirror[kSmallThreads - 1 - t] = r[0] < r[1] ? r[0] : r[1];
+  __syncthreads();
+  const uint64_t rm = small_scan(s_mirror[t], ~(uint64_t)0, OpMin{}, &tot64, s_w64);
+  s_mirror[kSmallThreads - 1 - t] = rm;
+  __syncthreads();
+  const uint64_t rx = s_mirror[t];
+  flags[0] = dom_flags(key[0], type[0], lev[0], fx, r[1] < rx ? r[1] : rx);
+  flags[1] = dom_flags(key[1], type[1], lev[1], f[0] > fx ? f[0] : fx, rx);
+  const uint64_t px = small_scan(flags[0] + flags[1], (uint64_t)0, OpAdd{}, &tot64, s_w64);
+  const uint32_t nmerge = (uint32_t)tot64, ntasks = (uint32_t)(tot64 >> 32);
+  EmitArgs e = a.emit;
+  e.class_cnt = s_class;
+  e.nhard = &s_nhard;
+  emit_group(e, kSmallPer * t, flags[0], px);
+  emit_group(e, kSmallPer * t + 1, flags[1], px + flags[0]);
+  __syncthreads();
+  for (uint32_t i = warp; i < s_nhard; i += kSmallWarps)
+    task_setup_hard(a.g, e.inv_fill, a.insert, a.p_ul, a.g_start, a.gtype, a.gw0, a.gw1,
+                    e.task_group, a.hard[i], ni, e.t, s_class);
+  __syncthreads();
+  // the tasks' places in the staging and among the leaves read and written
+  uint64_t el[kSmallPer], lf[kSmallPer], totl;
+#pragma unroll
+  for (int k = 0; k < kSmallPer; k++) {
+    const uint32_t i = kSmallPer * t + k;
+    el[k] = i < ntasks ? e.t.total[i] : 0;
+    lf[k] = i < ntasks ? e.t.ndst[i] << 32 | e.t.nsrc[i] : 0;
+  }
+  const uint64_t ex = small_scan(el[0] + el[1], (uint64_t)0, OpAdd{}, &tot64, s_w64);
+  const uint64_t lx = small_scan(lf[0] + lf[1], (uint64_t)0, OpAdd{}, &totl, s_w64);
+#pragma unroll
+  for (int k = 0; k < kSmallPer; k++) {
+    const uint32_t i = kSmallPer * t + k;
+    if (i >= ntasks) continue;
+    const uint64_t l = lx + (k ? lf[0] : 0);
+    e.t.out[i] = ex + (k ? el[0] : 0);
+    e.t.soff[i] = l & 0xffffffffu;
+    e.t.doff[i] = l >> 32;
+  }
+  if (t < kNumClasses) a.host->class_cnt[t] = s_class[t];
+  if (t == 0) {
+    a.host->n_items = ni;
+    a.host->n_groups = ng;
+    a.host->n_merge = nmerge;
+    a.host->n_tasks = ntasks;
+    a.host->n_climb = s_nclimb;
+    a.host->task_elems = tot64;
+    a.host->src_leaves = totl & 0xffffffffu;
+    a.host->dst_leaves = totl >> 32;
+    a.host->invalid = invalid;
+    a.host->apply_err = *a.err;
+    a.host->n_keys = n;
+    a.host->n_hard = s_nhard;
+  }
+}
+
+constexpr int kApplyCtas = 8;
+
+// The merges and the tasks of a small batch by one cluster (see k_leaf_merge,
+// k_task_index, k_gather_*, k_task_scatter and k_finalize).  A task's source
+// leaves are prefixed by its own eight lanes.
+__global__ void __cluster_dims__(kApplyCtas, 1, 1) __launch_bounds__(kSmallThreads)
+k_small_apply(DGraph g, Tasks t, const ClassStarts class_start, uint32_t nmerge, uint32_t ntasks,
+              uint32_t nitems, uint32_t nsrc, uint32_t ndst, const uint64_t *__restrict__ p_ul,
+              const uint32_t *__restrict__ p_x, const uint64_t *__restrict__ p_S,
+              const uint32_t *__restrict__ p_c, const uint64_t *__restrict__ merge_jk,
+              uint32_t *stage, uint64_t *spre, uint32_t *stask, uint32_t *dtask,
+              uint32_t *itask) {
+  pdl_wait();
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ uint8_t s_list[kSmallWarps][32];
+  constexpr uint32_t kAll = kApplyCtas * kSmallThreads;
+  const uint32_t tid = cl.block_rank() * kSmallThreads + threadIdx.x;
+  const uint32_t sub = threadIdx.x & 7;
+  for (uint64_t w = tid >> 5; w * 32 < nmerge; w += kAll / 32)
+    leaf_merge_chunk(g, w, nmerge, s_list[threadIdx.x >> 5], p_ul, p_x, p_S, p_c, merge_jk,
+                     nullptr);
+  if (ntasks == 0) return;
+  const uint32_t octet = 0xffu << (threadIdx.x & 24);
+  for (uint32_t w = tid >> 3; w < ntasks; w += kAll / 8) {
+    const uint64_t s0 = t.soff[w], ns = t.nsrc[w], d0 = t.doff[w], nd = t.ndst[w];
+    if (ns) {
+      const uint32_t u = t.u[w], l0 = t.w0[w];
+      const uint64_t base = g.base[u];
+      const uint32_t cap = g.cap[u], deg = g.deg[u];
+      uint64_t run = 0;
+      for (uint64_t j0 = 0; j0 < ns; j0 += 8) {
+        const uint64_t j = j0 + sub;
+        const uint32_t c = j < ns ? leaf_count(g, base, cap, deg, l0 + (uint32_t)j) : 0u;
+        uint32_t inc = c;
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) {
+          const uint32_t y = __shfl_up_sync(octet, inc, d, 8);
+          if (sub >= (uint32_t)d) inc += y;
+        }
+        if (j < ns) {
+          stask[s0 + j] = w;
+          spre[s0 + j] = run + inc - c;
+        }
+        run += __shfl_sync(octet, inc, 7, 8);
+      }
+    }
+    for (uint64_t j = sub; j < nd; j += 8) dtask[d0 + j] = w;
+    if (itask)
+      for (uint32_t j = t.newbeg[w] + sub; j < t.newend[w]; j += 8) itask[j] = w;
+  }
+  cl.sync();
+  if (itask)
+    for (uint32_t j = tid; j < nitems; j += kAll)
+      gather_new(j, g, t, ntasks, spre, p_ul, p_x, nitems, stage, itask);
+  for (uint32_t s = tid >> 3; s < nsrc; s += kAll / 8)
+    gather_old(s, sub, g, t, ntasks, nsrc, spre, p_x, stage, stask);
+  cl.sync();
+  for (uint32_t d = tid >> 3; d < ndst; d += kAll / 8)
+    task_scatter(d, sub, g, t, ntasks, ndst, class_start, stage, dtask);
+  // the scatter reads no row that a resize moves here
+  for (uint32_t tau = tid; tau < ntasks; tau += kAll)
+    task_finalize(tau, g, t, ntasks, class_start);
 }
 
 // ---------------------------------------------------------------- repack
@@ -1773,6 +2227,136 @@ sst_status update_batch(sst_graph *g, const uint32_t *d_pairs, uint64_t b,
   return run_pipeline(g, d_pairs, nullptr, b, insert, n_invalid, d_w);
 }
 
+static Tasks take_tasks(const sst_graph *g, Arena &A, uint64_t b) {
+  Tasks T;
+  T.u = A.take<uint32_t>(b);
+  T.w0 = A.take<uint32_t>(b);
+  T.key = A.take<uint64_t>(b);
+  T.nsrc = A.take<uint64_t>(b);
+  T.ndst = A.take<uint64_t>(b);
+  T.newbeg = A.take<uint32_t>(b);
+  T.newend = A.take<uint32_t>(b);
+  T.total = A.take<uint64_t>(b);
+  T.capn = A.take<uint64_t>(b);
+  T.rank = A.take<uint32_t>(b);
+  T.type = A.take<uint8_t>(b);
+  T.out = A.take<uint64_t>(b);
+  T.soff = A.take<uint64_t>(b);
+  T.doff = A.take<uint64_t>(b);
+  T.err = g->d_err;
+  T.stage_v = nullptr;  // weighted graphs set these
+  T.p_w = nullptr;
+  return T;
+}
+
+// slab slots of a plan's resized segments, and each capacity class's first one
+// (largest class first, so each segment is aligned to min(cap, 32))
+static uint64_t plan_growth(const PlanSummary &ps) {
+  uint64_t grow = 0;
+  for (int c = 0; c < kNumClasses; c++) grow += (uint64_t)ps.class_cnt[c] << c;
+  return grow;
+}
+static ClassStarts plan_class_starts(sst_graph *g, const PlanSummary &ps) {
+  ClassStarts cs;
+  uint64_t off = (g->bump + kLeaf - 1) & ~uint64_t(kLeaf - 1);
+  for (int c = kNumClasses - 1; c >= 0; c--) {
+    cs.s[c] = off;
+    off += (uint64_t)ps.class_cnt[c] << c;
+  }
+  if (plan_growth(ps)) g->bump = off;
+  return cs;
+}
+
+// One pass of up to kSmallBatch raw pairs on an unweighted graph, in three
+// launches (see k_small_locate); same result as run_pipeline.
+static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, bool insert,
+                            uint64_t *n_invalid) {
+  cudaStream_t s = g->stream;
+  const size_t need = update_scratch_bytes(kSmallBatch);
+  if (need > g->arena.cap) {
+    sst_status st = budget_check(g, need - g->arena.cap);
+    if (st != SST_OK) return st;
+  }
+  SST_CUDA_TRY(g->arena.reserve(need));
+  Arena &A = g->arena;
+  A.reset();
+  constexpr uint32_t B = kSmallBatch;
+  uint64_t *keys = A.take<uint64_t>(B), *lS = A.take<uint64_t>(B);
+  uint32_t *state = A.take<uint32_t>(B), *leaf = A.take<uint32_t>(B), *lc = A.take<uint32_t>(B);
+  uint64_t *p_ul = A.take<uint64_t>(B), *p_S = A.take<uint64_t>(B);
+  uint32_t *p_x = A.take<uint32_t>(B), *p_c = A.take<uint32_t>(B);
+  uint32_t *g_start = A.take<uint32_t>(B + 1);
+  uint32_t *gw0 = A.take<uint32_t>(B), *gw1 = A.take<uint32_t>(B);
+  uint8_t *gtype = A.take<uint8_t>(B), *glev = A.take<uint8_t>(B);
+  uint32_t *climb = A.take<uint32_t>(B), *hard = A.take<uint32_t>(B);
+  uint64_t *merge_jk = A.take<uint64_t>(B);
+  uint32_t *task_group = A.take<uint32_t>(B), *itask = A.take<uint32_t>(B);
+  Tasks T = take_tasks(g, A, B);
+  if (!T.doff) {
+    set_error_message("update scratch sizing error");
+    return SST_ENOMEM;
+  }
+  const DGraph dg = g->view();
+  SST_LAUNCH_PDL(k_small_locate, warp_blocks(b), kTB, 0, s, d_pairs, b, dg, g->dbits, insert,
+                 insert && !g->keep_loops, keys, state, leaf, lS, lc);
+  const EmitArgs ea{b,    g_start, merge_jk, task_group, fill_inv_q24(g->params.grow_fill),
+                    insert, p_ul,  p_c,      gtype,      T,
+                    nullptr, hard, nullptr,  insert ? itask : nullptr};
+  const SmallPlan sp{dg,    b,     g->dbits, insert, (uint32_t)window_lower(g->params, 0, 1),
+                     g->d_bounds + (insert ? 0 : kBoundsH * kBoundsH),
+                     keys,  state, leaf,     lc,     lS,
+                     p_ul,  p_S,   p_x,      p_c,    g_start,
+                     gw0,   gw1,   climb,    hard,   gtype,
+                     glev,  ea,    g->d_err, g->h_plan_dev};
+  SST_LAUNCH_PDL(k_small_plan, 1, kSmallThreads, 0, s, sp);
+  if (!g->plan_ready)
+    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->plan_ready, cudaEventDisableTiming));
+  SST_CUDA_TRY(cudaEventRecord(g->plan_ready, s));
+  SST_CUDA_TRY(cudaEventSynchronize(g->plan_ready));
+  SST_CUDA_TRY(cudaGetLastError());
+  const PlanSummary ps = *g->h_plan;
+  if (ps.apply_err) {
+    set_error_message("internal error: %llu failed device checks (staging rank out of range)",
+                      (unsigned long long)ps.apply_err);
+    return SST_EDEVICE;
+  }
+  if (n_invalid) *n_invalid = ps.invalid;
+  const size_t wneed = ps.task_elems * 4 + ps.src_leaves * 12 + ps.dst_leaves * 4 + 4096;
+  if (wneed > g->work.cap) {
+    sst_status st = budget_check(g, wneed - g->work.cap);
+    if (st != SST_OK) return st;
+  }
+  SST_CUDA_TRY(g->work.reserve(wneed));
+  g->work.reset();
+  uint32_t *stage = g->work.take<uint32_t>(ps.task_elems);
+  uint64_t *spre = g->work.take<uint64_t>(ps.src_leaves);
+  uint32_t *stask = g->work.take<uint32_t>(ps.src_leaves);
+  uint32_t *dtask = g->work.take<uint32_t>(ps.dst_leaves);
+  auto apply = [&](uint32_t nmerge, uint32_t ntasks, const ClassStarts &cs) {
+    SST_LAUNCH_PDL(k_small_apply, kApplyCtas, kSmallThreads, 0, s, g->view(), T, cs, nmerge,
+                   ntasks, ps.n_items, (uint32_t)ps.src_leaves, (uint32_t)ps.dst_leaves, p_ul,
+                   p_x, p_S, p_c, merge_jk, stage, spre, stask, dtask, insert ? itask : nullptr);
+  };
+  uint32_t nmerge = insert ? ps.n_merge : 0;
+  const uint64_t grow = plan_growth(ps);
+  if (grow && ((g->bump + kLeaf - 1) & ~uint64_t(kLeaf - 1)) + grow > g->nslots) {
+    // the merges' leaf starts point into the slab that the repack leaves
+    if (nmerge) apply(nmerge, 0, ClassStarts{});
+    nmerge = 0;
+    sst_status st = repack(g, grow);
+    if (st != SST_OK) return st;
+  }
+  const ClassStarts cs = plan_class_starts(g, ps);
+  if (nmerge || ps.n_tasks) apply(nmerge, ps.n_tasks, cs);
+  SST_CUDA_TRY(cudaGetLastError());
+  if (insert)
+    g->m += ps.n_items;
+  else
+    g->m -= ps.n_items;
+  if (ps.n_items) g->version++;
+  return SST_OK;
+}
+
 // d_w: the pairs' values on a weighted graph (null: value 1)
 static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
                                const uint64_t *presorted, uint64_t b,
@@ -1784,6 +2368,8 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
     set_error_message("batch of %llu pairs exceeds 2^32", (unsigned long long)b);
     return SST_EINVAL;
   }
+  if (!presorted && !g->weighted && b <= kSmallBatch)
+    return run_small(g, d_pairs, (uint32_t)b, insert, n_invalid);
   // Small batches are bound by the host's launch rate, so their planning
   // sequence (sort to plan readback) is captured once per size class and
   // graph layout and replayed as one graph launch.  Every launch after the
@@ -1826,22 +2412,7 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
   uint32_t *lc = A.take<uint32_t>(b), *p_c = A.take<uint32_t>(b);
   uint32_t *climb = A.take<uint32_t>(b);
   uint32_t *itask = A.take<uint32_t>(b);  // inserts: each item's task, or none
-  Tasks T;
-  T.u = A.take<uint32_t>(b);
-  T.w0 = A.take<uint32_t>(b);
-  T.key = A.take<uint64_t>(b);
-  T.nsrc = A.take<uint64_t>(b);
-  T.ndst = A.take<uint64_t>(b);
-  T.newbeg = A.take<uint32_t>(b);
-  T.newend = A.take<uint32_t>(b);
-  T.total = A.take<uint64_t>(b);
-  T.capn = A.take<uint64_t>(b);
-  T.rank = A.take<uint32_t>(b);
-  T.type = A.take<uint8_t>(b);
-  T.out = A.take<uint64_t>(b);
-  T.soff = A.take<uint64_t>(b);
-  T.doff = A.take<uint64_t>(b);
-  T.err = g->d_err;
+  Tasks T = take_tasks(g, A, b);
   // weighted graphs: values beside the keys (sorted with them) and the packed
   // items
   uint32_t *wv = wt ? A.take<uint32_t>(b) : nullptr;
@@ -2061,27 +2632,16 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
   }
   if (n_invalid) *n_invalid = ps.invalid;
 
-  // slab space for resized segments, laid out largest class first so each
-  // segment is aligned to min(cap, 32)
-  uint64_t grow = 0;
-  for (int c = 0; c < kNumClasses; c++) grow += (uint64_t)ps.class_cnt[c] << c;
-  uint64_t start = (g->bump + kLeaf - 1) & ~uint64_t(kLeaf - 1);
-  if (grow > 0 && start + grow > g->nslots) {
+  const uint64_t grow = plan_growth(ps);
+  if (grow > 0 && ((g->bump + kLeaf - 1) & ~uint64_t(kLeaf - 1)) + grow > g->nslots) {
     join.wait();  // the merges write the slab the repack copies and frees
     sst_status st = repack(g, grow);
     if (st != SST_OK) return st;
     dg = g->view();
-    start = (g->bump + kLeaf - 1) & ~uint64_t(kLeaf - 1);
     // the items' leaf starts (p_S) point into the old slab now, but the leaf
     // merges and deletes that read them have run already
   }
-  ClassStarts cstart;
-  uint64_t off = start;
-  for (int c = kNumClasses - 1; c >= 0; c--) {
-    cstart.s[c] = off;
-    off += (uint64_t)ps.class_cnt[c] << c;
-  }
-  if (grow > 0) g->bump = off;
+  const ClassStarts cstart = plan_class_starts(g, ps);
 
   // staging for window / resize tasks
   size_t wneed = ps.task_elems * (g->weighted ? 8 : 4) + ps.src_leaves * 20 +
