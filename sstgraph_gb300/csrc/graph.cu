@@ -1753,6 +1753,168 @@ k_small_apply(DGraph g, Tasks t, const ClassStarts class_start, uint32_t nmerge,
     task_finalize(tau, g, t, ntasks, class_start);
 }
 
+// ------------------------------------------------------------- first load
+// Pairs loaded into a graph that holds no segment: no row has anything to be
+// located, merged or moved, so the sorted keys alone give each row's size and
+// each id's place: three reads of the keys and two of the rows' ranges, where the
+// general sequence makes about twenty passes over them, with 311 B of scratch a pair.
+// Bound by the key sort (250 of 374 us; 27 MB of slab and 38 MB of pairs take 10).
+// 4.8M pairs of 300,000 rows: kernels 890 -> 374 us, and with the scratch's and the
+// graph's allocation and freeing 3.00 -> 1.08 ms.
+
+// Ranks of the kept keys (the first of each run of equal ones) among a tile of
+// sorted keys: a warp takes kLoadRows runs of 32 neighbouring keys, a vote gives
+// each key its rank in its run, and the block adds up the runs before it.
+// Computed twice (k_load_bounds, k_load_place) rather than stored: a key is read
+// in 8 bytes, and a stored flag and rank would cost 16 more.
+constexpr int kLoadTB = 256, kLoadRows = 8;
+constexpr int kLoadTile = kLoadTB * kLoadRows;
+struct LoadTile {
+  uint64_t key[kLoadRows];
+  uint64_t prev[kLoadRows];  // the key before (~0 before the first)
+  uint32_t rank[kLoadRows];  // within the tile
+  uint32_t kept;             // bit k: key[k] is kept
+  uint32_t total;            // kept keys of the tile
+  __device__ __forceinline__ static uint64_t index(int k) {
+    return (uint64_t)blockIdx.x * kLoadTile + (threadIdx.x >> 5) * (32 * kLoadRows) + 32 * k +
+           (threadIdx.x & 31);
+  }
+  __device__ __forceinline__ void load(const uint64_t *__restrict__ keys, uint64_t nk,
+                                       uint32_t *s_warp) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < kLoadRows; k++) {
+      const uint64_t i = index(k);
+      key[k] = i < nk ? keys[i] : ~0ull;
+      prev[k] = i && i < nk && lane == 0 ? keys[i - 1] : ~0ull;
+    }
+    uint32_t run = 0;
+    kept = 0;
+#pragma unroll
+    for (int k = 0; k < kLoadRows; k++) {
+      const uint64_t up = __shfl_up_sync(0xffffffffu, key[k], 1);
+      if (lane) prev[k] = up;
+      const bool f = index(k) < nk && prev[k] != key[k];  // no key is ~0
+      const uint32_t v = __ballot_sync(0xffffffffu, f);
+      rank[k] = run + __popc(v & ((1u << lane) - 1u));
+      run += __popc(v);
+      kept |= (uint32_t)f << k;
+    }
+    if (lane == 0) s_warp[warp] = run;
+    __syncthreads();
+    uint32_t before = 0;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < kLoadTB / 32; w++) {
+      if (w < warp) before += s_warp[w];
+      total += s_warp[w];
+    }
+#pragma unroll
+    for (int k = 0; k < kLoadRows; k++) rank[k] += before;
+  }
+};
+
+__global__ void __launch_bounds__(kLoadTB)
+k_load_count(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ nkeys,
+             uint32_t *__restrict__ tiles) {
+  pdl_wait();
+  __shared__ uint32_t s_warp[kLoadTB / 32];
+  LoadTile t;
+  t.load(keys, *nkeys, s_warp);
+  if (threadIdx.x == 0) tiles[blockIdx.x] = t.total;
+}
+
+// Each row's range of ranks (rows without a key keep the 0 they were cleared to).
+__global__ void __launch_bounds__(kLoadTB)
+k_load_bounds(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ nkeys, int dbits,
+              const uint32_t *__restrict__ tiles, uint32_t *__restrict__ beg,
+              uint32_t *__restrict__ end) {
+  pdl_wait();
+  __shared__ uint32_t s_warp[kLoadTB / 32];
+  LoadTile t;
+  const uint64_t nk = *nkeys;
+  t.load(keys, nk, s_warp);
+  const uint32_t at = tiles[blockIdx.x];
+#pragma unroll
+  for (int k = 0; k < kLoadRows; k++) {
+    // a row's first key is always kept, and it ends the row before
+    const uint64_t i = LoadTile::index(k), u = t.key[k] >> dbits;
+    if (i >= nk) break;
+    if (i == 0 || (t.prev[k] >> dbits) != u) {
+      beg[u] = at + t.rank[k];
+      if (i) end[t.prev[k] >> dbits] = at + t.rank[k];
+    }
+    if (i + 1 == nk) end[u] = at + t.rank[k] + ((t.kept >> k) & 1u);
+  }
+}
+
+// Each row's rank in its capacity class.  A block takes one range of rows,
+// counts its classes in shared memory and reserves each class once: atomics on
+// one address take about 25 ns each, so one a warp would be 230 us for 300,000
+// rows of one class.
+constexpr int kLoadThreads = 1024;
+__global__ void __launch_bounds__(kLoadThreads)
+k_load_rows(const uint32_t *__restrict__ beg, const uint32_t *__restrict__ end, uint32_t n,
+            uint64_t inv_fill, uint32_t *__restrict__ rank, uint32_t *__restrict__ class_cnt) {
+  pdl_wait();
+  __shared__ uint32_t s_cnt[kNumClasses];
+  for (int c = threadIdx.x; c < kNumClasses; c += kLoadThreads) s_cnt[c] = 0;
+  __syncthreads();
+  const uint64_t r0 = (uint64_t)n * blockIdx.x / gridDim.x;
+  const uint64_t r1 = (uint64_t)n * (blockIdx.x + 1) / gridDim.x;
+  for (uint64_t u = r0 + threadIdx.x; u < r1; u += kLoadThreads) {
+    const uint64_t c = cap_for(end[u] - beg[u], inv_fill);
+    if (c) atomicAdd(&s_cnt[log2_floor(c)], 1u);
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < kNumClasses; c += kLoadThreads)
+    if (s_cnt[c]) s_cnt[c] = atomicAdd(&class_cnt[c], s_cnt[c]);
+  __syncthreads();
+  for (uint64_t u = r0 + threadIdx.x; u < r1; u += kLoadThreads) {
+    const uint64_t c = cap_for(end[u] - beg[u], inv_fill);
+    if (c) rank[u] = atomicAdd(&s_cnt[log2_floor(c)], 1u);
+  }
+}
+
+// Each kept key's id to its slot, rows spread over their leaves as task_scatter
+// spreads them (the segments' slots hold kEmpty and their leaf counts 0).  The
+// thread of a row's first key writes the row's record, and that of a leaf's
+// first key its count.
+__global__ void __launch_bounds__(kLoadTB)
+k_load_place(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ nkeys, int dbits,
+             const uint32_t *__restrict__ tiles, const uint32_t *__restrict__ beg,
+             const uint32_t *__restrict__ end, const uint32_t *__restrict__ rank,
+             uint64_t inv_fill, const ClassStarts cs, DGraph g) {
+  pdl_wait();
+  __shared__ uint32_t s_warp[kLoadTB / 32];
+  LoadTile t;
+  t.load(keys, *nkeys, s_warp);
+  const uint32_t tile = tiles[blockIdx.x];
+#pragma unroll
+  for (int k = 0; k < kLoadRows; k++) {
+    if (!((t.kept >> k) & 1u)) continue;
+    const uint32_t u = (uint32_t)(t.key[k] >> dbits);
+    const uint32_t b0 = beg[u], deg = end[u] - b0, r = tile + t.rank[k] - b0;
+    const uint64_t cap = cap_for(deg, inv_fill);
+    const uint64_t base = cs.s[log2_floor(cap)] + (uint64_t)rank[u] * cap;
+    if (r == 0) {
+      g.base[u] = base;
+      g.cap[u] = (uint32_t)cap;
+      g.deg[u] = deg;
+    }
+    uint64_t at = base + r;
+    if (cap > kLeaf) {
+      const uint32_t nl = nleaves_of((uint32_t)cap), per = deg / nl, ext = deg - per * nl;
+      const uint32_t cut = ext * (per + 1);  // ids of the leaves that take one more
+      const uint32_t l = r < cut ? r / (per + 1) : ext + (r - cut) / per;
+      const uint32_t o = r < cut ? r - l * (per + 1) : r - cut - (l - ext) * per;
+      at = base + ((uint64_t)l << kLeafLog) + o;
+      if (o == 0) g.lcnt[at >> kLeafLog] = (uint8_t)(per + (l < ext));
+    }
+    g.slots[at] = (uint32_t)(t.key[k] & ((1ull << dbits) - 1));
+  }
+}
+
 // ---------------------------------------------------------------- repack
 __global__ void k_class_count(const uint32_t *__restrict__ cap, uint32_t n,
                               uint32_t *__restrict__ cnt) {
@@ -2267,6 +2429,38 @@ static ClassStarts plan_class_starts(sst_graph *g, const PlanSummary &ps) {
   return cs;
 }
 
+static void launch_packed_keys(const sst_graph *g, const uint32_t *d_pairs, uint64_t npairs,
+                               bool drop_loops, uint64_t *keys, const SortDigits &sdig,
+                               cudaStream_t s) {
+  PlanSummary *P = g->d_plan;
+  auto launch = [&](auto *kernel) {
+    SST_LAUNCH_PDL_NB("k_make_keys_packed", 16 * npairs, kernel,
+                      blocks_for(npairs, kTB * kPackItems), kTB, 0, s, d_pairs, npairs, g->n,
+                      g->width, g->dbits, drop_loops, keys,
+                      reinterpret_cast<unsigned long long *>(&P->invalid), &P->n_keys, sdig);
+  };
+  if ((reinterpret_cast<uintptr_t>(d_pairs) & 7) == 0)
+    launch(k_make_keys_packed<true>);
+  else
+    launch(k_make_keys_packed<false>);
+}
+
+// the plan that the kernels before it left in the mapped host copy
+static sst_status read_plan(sst_graph *g, PlanSummary *ps) {
+  if (!g->plan_ready)
+    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->plan_ready, cudaEventDisableTiming));
+  SST_CUDA_TRY(cudaEventRecord(g->plan_ready, g->stream));
+  SST_CUDA_TRY(cudaEventSynchronize(g->plan_ready));
+  SST_CUDA_TRY(cudaGetLastError());
+  *ps = *g->h_plan;
+  if (ps->apply_err) {
+    set_error_message("internal error: %llu failed device checks (staging rank out of range)",
+                      (unsigned long long)ps->apply_err);
+    return SST_EDEVICE;
+  }
+  return SST_OK;
+}
+
 // One pass of up to kSmallBatch raw pairs on an unweighted graph, in three
 // launches (see k_small_locate); same result as run_pipeline.
 static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, bool insert,
@@ -2309,17 +2503,9 @@ static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, b
                      gw0,   gw1,   climb,    hard,   gtype,
                      glev,  ea,    g->d_err, g->h_plan_dev};
   SST_LAUNCH_PDL(k_small_plan, 1, kSmallThreads, 0, s, sp);
-  if (!g->plan_ready)
-    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->plan_ready, cudaEventDisableTiming));
-  SST_CUDA_TRY(cudaEventRecord(g->plan_ready, s));
-  SST_CUDA_TRY(cudaEventSynchronize(g->plan_ready));
-  SST_CUDA_TRY(cudaGetLastError());
-  const PlanSummary ps = *g->h_plan;
-  if (ps.apply_err) {
-    set_error_message("internal error: %llu failed device checks (staging rank out of range)",
-                      (unsigned long long)ps.apply_err);
-    return SST_EDEVICE;
-  }
+  PlanSummary ps;
+  sst_status rst = read_plan(g, &ps);
+  if (rst != SST_OK) return rst;
   if (n_invalid) *n_invalid = ps.invalid;
   const size_t wneed = ps.task_elems * 4 + ps.src_leaves * 12 + ps.dst_leaves * 4 + 4096;
   if (wneed > g->work.cap) {
@@ -2357,6 +2543,95 @@ static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, b
   return SST_OK;
 }
 
+// From one pair more than the one-block sort takes.  A graph made, loaded and
+// freed, by the general sequence and so: 2,200 pairs of 300 rows 0.93 -> 0.66 ms,
+// 18,000 of 2,000 rows 0.96 -> 0.67, 18,000 of 300,000 rows 1.20 -> 0.94, 600,000
+// (RMAT) of 32,768 rows 1.29 -> 0.84.  Smaller loads take the launches that later
+// batches of their size replay.
+constexpr uint64_t kLoadPairs = 2049;
+
+// Pairs into a graph without segments (see k_load_flags); same result as
+// run_pipeline.  The slab holds nothing, so one that is too small is replaced,
+// not repacked.
+static sst_status run_load(sst_graph *g, const uint32_t *d_pairs, uint64_t b,
+                           uint64_t *n_invalid) {
+  cudaStream_t s = g->stream;
+  const uint64_t n = g->n;
+  const uint64_t ntiles = (b + kLoadTile - 1) / kLoadTile;
+  // with room for later updates of a twelfth of the load: about what the load
+  // itself takes, so that the first of them allocate nothing
+  const size_t need = std::max<size_t>(b * 16 + n * 12 + ntiles * 8 + radix_sort_scratch_bytes(b) +
+                                           scan_scratch_bytes(ntiles, 4) + (1 << 14),
+                                       update_scratch_bytes(b / 12));
+  if (need > g->arena.cap) {
+    sst_status st = budget_check(g, need - g->arena.cap);
+    if (st != SST_OK) return st;
+  }
+  SST_CUDA_TRY(g->arena.reserve(need));
+  Arena &A = g->arena;
+  A.reset();
+  PlanSummary *P = g->d_plan;
+  SST_CUDA_TRY(cudaMemsetAsync(P, 0, sizeof(PlanSummary), s));
+  uint64_t *keys = A.take<uint64_t>(b), *ktmp = A.take<uint64_t>(b);
+  uint32_t *tcnt = A.take<uint32_t>(ntiles), *tiles = A.take<uint32_t>(ntiles);
+  uint32_t *beg = A.take<uint32_t>(2 * n), *end = beg + n, *rank = A.take<uint32_t>(n);
+  if (!rank) {
+    set_error_message("update scratch sizing error");
+    return SST_ENOMEM;
+  }
+  const int dbits = g->dbits, bits = bits_for(n - 1) + dbits;
+  SortDigits sdig;
+  if (radix_sort_digits(b, bits, A, &sdig))
+    SST_CUDA_TRY(cudaMemsetAsync(sdig.totals, 0, (size_t)sdig.passes * 256 * 4, s));
+  else
+    sdig = SortDigits{};
+  SST_CUDA_TRY(cudaMemsetAsync(beg, 0, n * 8, s));
+  launch_packed_keys(g, d_pairs, b, !g->keep_loops, keys, sdig, s);
+  uint64_t *sorted = keys;
+  SST_CUDA_TRY(radix_sort_u64(keys, ktmp, b, bits, A, s, &sorted, &P->n_keys,
+                              sdig.passes ? &sdig : nullptr));
+  SST_LAUNCH_PDL_B(8 * b, k_load_count, (unsigned)ntiles, kLoadTB, 0, s, sorted, &P->n_keys, tcnt);
+  SST_CUDA_TRY((scan<uint32_t, OpAdd>(tcnt, tiles, ntiles, 0u, OpAdd{}, true, false, &P->n_items,
+                                      A, s)));
+  SST_LAUNCH_PDL_B(8 * b, k_load_bounds, (unsigned)ntiles, kLoadTB, 0, s, sorted, &P->n_keys,
+                   dbits, tiles, beg, end);
+  const uint64_t inv_fill = fill_inv_q24(g->params.grow_fill);
+  SST_LAUNCH_PDL(k_load_rows, std::min(blocks_for(n, kLoadThreads), 2u * g->sms), kLoadThreads,
+                 0, s, beg, end, (uint32_t)n, inv_fill, rank, P->class_cnt);
+  SST_LAUNCH_PDL(k_plan_out, 1, 64, 0, s, P, g->d_err, g->h_plan_dev);
+  PlanSummary ps;
+  sst_status st = read_plan(g, &ps);
+  if (st != SST_OK) return st;
+  if (n_invalid) *n_invalid = ps.invalid;
+  const uint64_t grow = plan_growth(ps);
+  if (grow == 0) return SST_OK;
+  if (grow > g->nslots) {
+    // as large as repack would make it
+    uint64_t nsl = std::max<uint64_t>(2 * (grow + kLeaf), 1ull << 20);
+    nsl = (nsl + kLeaf - 1) & ~uint64_t(kLeaf - 1);
+    st = budget_check(g, nsl * 4 + nsl / kLeaf);
+    if (st != SST_OK) return st;
+    uint32_t *slots, *vals;
+    uint8_t *lcnt;
+    st = alloc_slab(g, nsl, &slots, &lcnt, &vals);
+    if (st != SST_OK) return st;
+    cudaFree(g->d_slots);
+    cudaFree(g->d_lcnt);
+    g->d_slots = slots;
+    g->d_lcnt = lcnt;
+    g->nslots = nsl;
+  }
+  const ClassStarts cs = plan_class_starts(g, ps);
+  SST_CUDA_TRY(cudaMemsetAsync(g->d_slots, 0xFF, g->bump * 4, s));
+  SST_CUDA_TRY(cudaMemsetAsync(g->d_lcnt, 0, g->bump / kLeaf, s));
+  SST_LAUNCH_PDL_B(12 * b, k_load_place, (unsigned)ntiles, kLoadTB, 0, s, sorted, &P->n_keys,
+                   dbits, tiles, beg, end, rank, inv_fill, cs, g->view());
+  SST_CUDA_TRY(cudaGetLastError());
+  g->m += ps.n_items;
+  g->version++;
+  return SST_OK;
+}
+
 // d_w: the pairs' values on a weighted graph (null: value 1)
 static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
                                const uint64_t *presorted, uint64_t b,
@@ -2370,6 +2645,8 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
   }
   if (!presorted && !g->weighted && b <= kSmallBatch)
     return run_small(g, d_pairs, (uint32_t)b, insert, n_invalid);
+  if (!presorted && !g->weighted && insert && g->bump == 0 && b >= kLoadPairs && g->n)
+    return run_load(g, d_pairs, b, n_invalid);
   // Small batches are bound by the host's launch rate, so their planning
   // sequence (sort to plan readback) is captured once per size class and
   // graph layout and replayed as one graph launch.  Every launch after the
@@ -2443,16 +2720,7 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
       } else {
         sdig = SortDigits{};
       }
-      if ((reinterpret_cast<uintptr_t>(d_pairs) & 7) == 0)
-        SST_LAUNCH_PDL_NB("k_make_keys_packed", 16 * npairs, k_make_keys_packed<true>,
-                     blocks_for(npairs, kTB * kPackItems), kTB, 0, s, d_pairs, npairs, g->n,
-                     g->width, dbits, insert && !g->keep_loops, keys,
-                     reinterpret_cast<unsigned long long *>(&P->invalid), nkeys, sdig);
-      else
-        SST_LAUNCH_PDL_NB("k_make_keys_packed", 16 * npairs, k_make_keys_packed<false>,
-                     blocks_for(npairs, kTB * kPackItems), kTB, 0, s, d_pairs, npairs, g->n,
-                     g->width, dbits, insert && !g->keep_loops, keys,
-                     reinterpret_cast<unsigned long long *>(&P->invalid), nkeys, sdig);
+      launch_packed_keys(g, d_pairs, npairs, insert && !g->keep_loops, keys, sdig, s);
     }
   }
   MergeJoin join{s, nullptr};
@@ -2619,17 +2887,9 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
     sst_status st = plan(s, true);
     if (st != SST_OK) return st;
   }
-  if (!g->plan_ready)
-    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->plan_ready, cudaEventDisableTiming));
-  SST_CUDA_TRY(cudaEventRecord(g->plan_ready, s));
-  SST_CUDA_TRY(cudaEventSynchronize(g->plan_ready));
-  SST_CUDA_TRY(cudaGetLastError());
-  PlanSummary ps = *g->h_plan;
-  if (ps.apply_err) {
-    set_error_message("internal error: %llu failed device checks (staging rank out of range)",
-                      (unsigned long long)ps.apply_err);
-    return SST_EDEVICE;
-  }
+  PlanSummary ps;
+  sst_status rst = read_plan(g, &ps);
+  if (rst != SST_OK) return rst;
   if (n_invalid) *n_invalid = ps.invalid;
 
   const uint64_t grow = plan_growth(ps);
