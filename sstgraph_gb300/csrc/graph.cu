@@ -31,7 +31,9 @@
 #include <cooperative_groups.h>
 #include <cstddef>
 #include <cstdarg>
+#include <cstdlib>
 #include <cstring>
+#include <unistd.h>
 #include <vector>
 
 #include "graph.cuh"
@@ -2042,30 +2044,50 @@ static sst_status budget_check(sst_graph *g, uint64_t extra) {
   return SST_OK;
 }
 
-static sst_status alloc_slab(sst_graph *g, uint64_t nslots, uint32_t **slots,
-                             uint8_t **lcnt, uint32_t **vals) {
-  if (cudaMalloc(slots, nslots * 4) != cudaSuccess) {
+// A slab of nslots slots, a value each on a weighted graph, and the leaf counts,
+// in one allocation (its address is *slots): cudaMalloc and cudaFree take 30 us
+// each, whatever the size up to some 20 MB.
+sst_status alloc_slab(const sst_graph *g, uint64_t nslots, uint32_t **slots, uint8_t **lcnt,
+                      uint32_t **vals) {
+  const uint64_t words = nslots * (g->weighted ? 2 : 1);
+  if (cudaMalloc(slots, words * 4 + nslots / kLeaf + 1) != cudaSuccess) {
     cudaGetLastError();
+    *slots = nullptr;
     set_error_message("cannot allocate a slab of %llu slots",
                       (unsigned long long)nslots);
     return SST_ENOMEM;
   }
-  if (cudaMalloc(lcnt, nslots / kLeaf + 1) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(*slots);
-    set_error_message("cannot allocate leaf counts");
-    return SST_ENOMEM;
-  }
-  *vals = nullptr;
-  if (g->weighted && cudaMalloc(vals, nslots * 4) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(*slots);
-    cudaFree(*lcnt);
-    set_error_message("cannot allocate a value slab of %llu slots",
-                      (unsigned long long)nslots);
-    return SST_ENOMEM;
-  }
+  *vals = g->weighted ? *slots + nslots : nullptr;
+  *lcnt = reinterpret_cast<uint8_t *>(*slots + words);
   return SST_OK;
+}
+
+// The host copy of the plan, in a page of its own that kernels write: a page
+// registered and unregistered takes 7 and 12 us, where a pinned allocation and its
+// freeing took 105 and 149.  Kernels write both alike.
+static sst_status plan_host_alloc(sst_graph *g) {
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  void *p = aligned_alloc(page, page);
+  if (p && cudaHostRegister(p, page, cudaHostRegisterMapped) == cudaSuccess) {
+    g->h_plan_registered = true;
+  } else {
+    cudaGetLastError();
+    free(p);
+    SST_CUDA_TRY(cudaMallocHost(&p, sizeof(PlanSummary)));
+  }
+  g->h_plan = static_cast<PlanSummary *>(p);
+  SST_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&g->h_plan_dev), p, 0));
+  return SST_OK;
+}
+static void plan_host_free(sst_graph *g) {
+  if (!g->h_plan) return;
+  if (g->h_plan_registered) {
+    cudaHostUnregister(g->h_plan);
+    free(g->h_plan);
+  } else {
+    cudaFreeHost(g->h_plan);
+  }
+  g->h_plan = nullptr;
 }
 
 sst_status graph_init(sst_graph *g, uint32_t height, uint32_t width,
@@ -2088,12 +2110,21 @@ sst_status graph_init(sst_graph *g, uint32_t height, uint32_t width,
   SST_CUDA_TRY(cudaStreamCreateWithFlags(&g->own_stream, cudaStreamNonBlocking));
   g->stream = g->own_stream;
   uint64_t n = std::max<uint64_t>(height, 1);
-  SST_CUDA_TRY(cudaMalloc(&g->d_base, n * 8));
-  SST_CUDA_TRY(cudaMalloc(&g->d_cap, n * 4));
-  SST_CUDA_TRY(cudaMalloc(&g->d_deg, n * 4));
-  SST_CUDA_TRY(cudaMemsetAsync(g->d_base, 0, n * 8, g->stream));
-  SST_CUDA_TRY(cudaMemsetAsync(g->d_cap, 0, n * 4, g->stream));
-  SST_CUDA_TRY(cudaMemsetAsync(g->d_deg, 0, n * 4, g->stream));
+  // the vertex records and the small per-graph words in one allocation
+  constexpr uint64_t kBoundsBytes = 2 * kBoundsH * kBoundsH * 8;
+  auto line = [](uint64_t bytes) { return (bytes + 255) & ~uint64_t(255); };
+  const uint64_t cap = line(n * 8), deg = cap + line(n * 4), bounds = deg + line(n * 4);
+  const uint64_t plan = bounds + kBoundsBytes, total = plan + sizeof(PlanSummary) + 16;
+  char *blk = nullptr;
+  SST_CUDA_TRY(cudaMalloc(&blk, total));
+  g->d_base = reinterpret_cast<uint64_t *>(blk);
+  g->d_cap = reinterpret_cast<uint32_t *>(blk + cap);
+  g->d_deg = reinterpret_cast<uint32_t *>(blk + deg);
+  g->d_bounds = reinterpret_cast<uint64_t *>(blk + bounds);
+  g->d_plan = reinterpret_cast<PlanSummary *>(blk + plan);
+  g->d_err = reinterpret_cast<unsigned long long *>(blk + plan + sizeof(PlanSummary));
+  g->d_scan_epoch = g->d_err + 1;
+  SST_CUDA_TRY(cudaMemsetAsync(blk, 0, total, g->stream));
   uint64_t slots = cfg && cfg->initial_slots ? cfg->initial_slots : (1ull << 20);
   slots = (slots + kLeaf - 1) & ~uint64_t(kLeaf - 1);
   sst_status st = budget_check(g, slots * 4 + slots / kLeaf);
@@ -2102,13 +2133,8 @@ sst_status graph_init(sst_graph *g, uint32_t height, uint32_t width,
   if (st != SST_OK) return st;
   g->nslots = slots;
   g->bump = 0;
-  SST_CUDA_TRY(cudaMallocHost(&g->h_plan, sizeof(PlanSummary)));
-  SST_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&g->h_plan_dev), g->h_plan, 0));
-  SST_CUDA_TRY(cudaMalloc(&g->d_plan, sizeof(PlanSummary)));
-  SST_CUDA_TRY(cudaMalloc(&g->d_err, sizeof(unsigned long long)));
-  SST_CUDA_TRY(cudaMemsetAsync(g->d_err, 0, sizeof(unsigned long long), g->stream));
-  SST_CUDA_TRY(cudaMalloc(&g->d_scan_epoch, sizeof(unsigned long long)));
-  SST_CUDA_TRY(cudaMemsetAsync(g->d_scan_epoch, 0, sizeof(unsigned long long), g->stream));
+  sst_status hst = plan_host_alloc(g);
+  if (hst != SST_OK) return hst;
   // the climb's density bounds per (segment height, window level), computed
   // once here with the graph's parameters: no FP64 on the device
   std::vector<uint64_t> wb(2 * kBoundsH * kBoundsH, 0);
@@ -2117,8 +2143,8 @@ sst_status graph_init(sst_graph *g, uint32_t height, uint32_t width,
       wb[H * kBoundsH + t] = window_upper(g->params, t, H);
       wb[kBoundsH * kBoundsH + H * kBoundsH + t] = window_lower(g->params, t, H);
     }
-  SST_CUDA_TRY(cudaMalloc(&g->d_bounds, wb.size() * 8));
-  SST_CUDA_TRY(cudaMemcpy(g->d_bounds, wb.data(), wb.size() * 8, cudaMemcpyHostToDevice));
+  SST_CUDA_TRY(cudaMemcpyAsync(g->d_bounds, wb.data(), kBoundsBytes, cudaMemcpyHostToDevice,
+                               g->stream));
   SST_CUDA_TRY(cudaStreamSynchronize(g->stream));
   return SST_OK;
 }
@@ -2126,17 +2152,9 @@ sst_status graph_init(sst_graph *g, uint32_t height, uint32_t width,
 void graph_release(sst_graph *g) {
   cudaSetDevice(g->device);
   if (g->stream) cudaStreamSynchronize(g->stream);
-  cudaFree(g->d_base);
-  cudaFree(g->d_cap);
-  cudaFree(g->d_deg);
-  cudaFree(g->d_slots);
-  cudaFree(g->d_vals);
-  cudaFree(g->d_lcnt);
-  cudaFree(g->d_plan);
-  cudaFree(g->d_err);
-  cudaFree(g->d_bounds);
-  cudaFree(g->d_scan_epoch);
-  if (g->h_plan) cudaFreeHost(g->h_plan);
+  cudaFree(g->d_base);   // and the vertex records' other words, see graph_init
+  cudaFree(g->d_slots);  // and the slab's values and counts
+  plan_host_free(g);
   if (g->h_pinned) cudaFreeHost(g->h_pinned);
   g->arena.release();
   g->work.release();
@@ -2243,8 +2261,6 @@ sst_status repack(sst_graph *g, uint64_t extra) {
   SST_CUDA_TRY(cudaStreamSynchronize(s));
   SST_CUDA_TRY(cudaGetLastError());
   cudaFree(g->d_slots);
-  cudaFree(g->d_lcnt);
-  cudaFree(g->d_vals);
   g->d_slots = nslots_;
   g->d_lcnt = nlcnt;
   g->d_vals = nvals;
@@ -2616,7 +2632,6 @@ static sst_status run_load(sst_graph *g, const uint32_t *d_pairs, uint64_t b,
     st = alloc_slab(g, nsl, &slots, &lcnt, &vals);
     if (st != SST_OK) return st;
     cudaFree(g->d_slots);
-    cudaFree(g->d_lcnt);
     g->d_slots = slots;
     g->d_lcnt = lcnt;
     g->nslots = nsl;

@@ -87,7 +87,8 @@ struct sst_graph {
   sst::Arena arena;  // per-operation scratch
   sst::Arena work;   // window / resize staging
   sst::Arena io;     // device copies of host-pointer arguments
-  sst::PlanSummary *h_plan = nullptr;  // pinned
+  sst::PlanSummary *h_plan = nullptr;  // page-locked
+  bool h_plan_registered = false;      // a registered page, else a pinned allocation
   sst::PlanSummary *h_plan_dev = nullptr;  // h_plan's address for kernels (mapped)
   sst::PlanSummary *d_plan = nullptr;
   unsigned long long *d_err = nullptr;  // staging-rank check, read lazily
@@ -105,6 +106,8 @@ struct sst_graph {
 
 namespace sst {
 
+sst_status alloc_slab(const sst_graph *g, uint64_t nslots, uint32_t **slots, uint8_t **lcnt,
+                      uint32_t **vals);
 sst_status graph_init(sst_graph *g, uint32_t height, uint32_t width,
                       const sst_config *cfg);
 void graph_release(sst_graph *g);

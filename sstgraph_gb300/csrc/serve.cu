@@ -40,16 +40,14 @@ sst_status graph_copy_into(sst_graph *dst, sst_graph *src) {
   if (dst->nslots < used) {
     cudaStreamSynchronize(dst->stream);
     cudaFree(dst->d_slots);
-    cudaFree(dst->d_lcnt);
-    cudaFree(dst->d_vals);
     dst->d_slots = nullptr;
     dst->d_lcnt = nullptr;
     dst->d_vals = nullptr;
+    dst->nslots = 0;
     uint64_t want = std::max(used + used / 4, src->nslots);
     want = (want + kLeaf - 1) & ~uint64_t(kLeaf - 1);
-    SST_CUDA_TRY(cudaMalloc(&dst->d_slots, want * 4));
-    SST_CUDA_TRY(cudaMalloc(&dst->d_lcnt, want / kLeaf + 1));
-    if (dst->weighted) SST_CUDA_TRY(cudaMalloc(&dst->d_vals, want * 4));
+    sst_status st = alloc_slab(dst, want, &dst->d_slots, &dst->d_lcnt, &dst->d_vals);
+    if (st != SST_OK) return st;
     dst->nslots = want;
   }
   uint64_t n = std::max<uint64_t>(src->n, 1);
