@@ -12,6 +12,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "primitives.cuh"
@@ -171,17 +172,19 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kItems = 16;
 constexpr int kTile = kThreads * kItems;  // 4096
-// Sorts of at most kSmallTileKeys keys (without values) use tiles of
-// kSmallItems items per thread: four times the blocks, each ranking a
-// quarter of the keys, so a pass's dependent chain is shorter.
+// Shorter sorts use smaller tiles: more blocks, each ranking fewer keys, so a
+// pass's dependent chain is shorter, until the blocks no longer fit the GPU at
+// once.  Five passes, by items a thread (us; keys alone, then with values):
+//   keys        4             8             16
+//   60,000     26.7    -     36.1  36.3     35.0  48.8
+//   260,000    33.5    -     35.1  38.4     45     50
+//   800,000    81      -     50.3  56.7     57.6  65.6
+//   1,200,000   -      -     69.6  77.2     59.3  67.4
+//   4,800,000   -      -      195   240      169   224
 constexpr int kSmallItems = 4;
-constexpr uint64_t kSmallTileKeys = 256ull * kThreads * kSmallItems;  // 2^18
-// (1024-key tiles for larger one-sweep sorts were measured too: at 1e6 keys
-// 977 tiles made a pass 29 us against 19 us for 245 tiles of 4096 -- the
-// longer look-back walks cost more than the extra resident warps gain; and
-// 2048-key tiles, three blocks an SM, made a 1e6-pair insert 567 us against
-// 553 us; measured again with the match-word ranking: 21.3 against 17.8 us a
-// pass)
+constexpr uint64_t kSmallTileKeys = 256ull * kThreads * kSmallItems;  // 2^18, no values
+constexpr int kMidItems = 8;
+constexpr uint64_t kMidTileKeys = 448ull * kThreads * kMidItems;  // 7 * 2^17
 constexpr int kRadix = 256;
 constexpr uint32_t kNoDigit = 0xffffffffu;  // an item past the end
 // Sorts of at most this many tiles run one launch per pass: every block
@@ -222,11 +225,10 @@ __device__ __forceinline__ void warp_rank(const uint32_t (&dg)[ITEMS],
     if (valid) atomicOr(&wm[d], 1u << lane);
     __syncwarp();
     const uint32_t peers = valid ? wm[d] : 0u;
-    const uint32_t c = valid ? wc[d] : 0u;
-    lr[it] = c + __popc(peers & below);
+    lr[it] = (valid ? wc[d] : 0u) + __popc(peers & below);
     __syncwarp();
-    if (valid && (peers & below) == 0) {
-      wc[d] = c + __popc(peers);
+    if (valid && (peers & below) == 0) {  // the lowest: its rank is the counter
+      wc[d] = lr[it] + __popc(peers);
       wm[d] = 0;
     }
     __syncwarp();
@@ -430,16 +432,39 @@ k_scatter(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
 // ---- one-sweep passes (after Adinets and Merrill, "Onesweep", 2022).
 // k_hist_all reads the keys once and counts every pass's digits (global
 // totals, no per-tile tables) and clears the passes' tile status words.
-// Each pass is then one launch: a block ranks its tile as k_scatter does,
-// publishes its per-digit count, and thread d finds the count of digit d in
-// all tiles before its own by looking back over their status words (an
-// inclusive prefix ends the walk, an aggregate is added and the walk goes
-// on).  A status word is (state << 30) | count, state 1 = this tile's
-// count, 2 = the count of this and every earlier tile; 0 = not yet
-// published.  Every wait is bounded: a tile that has not published in time
-// is counted from its keys instead, and the walk goes on.
-constexpr uint32_t kOsAgg = 1u << 30, kOsIncl = 2u << 30, kOsMask = kOsAgg - 1;
+// Each pass is then one launch: a block ranks its tile as k_scatter does and
+// publishes its per-digit counts, and thread d finds the count of digit d in
+// all tiles before its own.  Those are not walked tile by tile to the nearest
+// inclusive prefix, which moves on by some 32 tiles a step of 0.7 us: every tile
+// also adds its counts to the sums of its group of 8 tiles, of 64, and so on, and
+// reads the words of the up to 7 tiles, 7 groups of 8, ... that make up the tiles
+// before it.  They are read together, and depend on no other tile's look-back.
+// A tile's word is kOsAgg | count (0 = not yet published); a group's is (tiles
+// published << 32) | count, complete when it holds all its tiles.  Every wait is
+// bounded: a word that is not complete in time is made up from its tiles' words
+// or keys instead.
+constexpr uint32_t kOsAgg = 1u << 30, kOsMask = kOsAgg - 1;
 constexpr int kOsPolls = 1 << 14;
+constexpr int kOsLog = 3, kOsGroup = 1 << kOsLog;
+// levels of groups above nt tiles (fewer than 2^18): the last has at most
+// kOsGroup words
+__host__ __device__ inline int os_levels(uint32_t nt) {
+  int l = 0;
+  while (nt > kOsGroup) {
+    nt = (nt + kOsGroup - 1) >> kOsLog;
+    l++;
+  }
+  return l;
+}
+// status words (32-bit) of a pass over nt tiles: the tiles', then each level's
+inline uint64_t os_status_words(uint32_t nt) {
+  uint64_t w = (uint64_t)nt * kRadix;
+  while (nt > kOsGroup) {
+    nt = (nt + kOsGroup - 1) >> kOsLog;
+    w += 2 * (uint64_t)nt * kRadix;
+  }
+  return w;
+}
 
 template <int IT>
 __global__ void __launch_bounds__(kThreads)
@@ -479,8 +504,15 @@ __device__ __forceinline__ uint32_t os_count_tile(const uint64_t *in, uint64_t n
   return c;
 }
 
+// resident blocks an SM that the registers are held to: as many as fit without
+// spilling what the ranking holds (4.8M keys in 16 items a thread, 2 / 3 / 4 / 5
+// blocks: 207, 174, 169, 220 us; with values 3 / 4: 224, 280)
 template <bool KV, int IT>
-__global__ void __launch_bounds__(kThreads, IT == kSmallItems ? 3 : 2)
+constexpr int os_blocks() {
+  return IT == kSmallItems ? 6 : IT == kMidItems ? (KV ? 4 : 5) : (KV ? 3 : 4);
+}
+template <bool KV, int IT>
+__global__ void __launch_bounds__(kThreads, os_blocks<KV, IT>())
 k_scatter_os(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
              uint64_t n, int shift, const uint32_t *__restrict__ totals,
              uint32_t *__restrict__ status, const uint32_t *__restrict__ vin,
@@ -499,8 +531,8 @@ k_scatter_os(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
   const uint32_t d = threadIdx.x;  // this thread's digit in the bookkeeping
 #pragma unroll
   for (int w = 0; w < kWarps; w++) wcnt[w][d] = 0;
-  const uint64_t tile = blockIdx.x;
-  const uint64_t t0 = tile * TILE;
+  const uint32_t tile = blockIdx.x;
+  const uint64_t t0 = (uint64_t)tile * TILE;
   uint64_t kk[IT];
   uint32_t vv[KV ? IT : 1];
   uint32_t dg[IT];
@@ -514,54 +546,30 @@ k_scatter_os(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
   // the match words sit in the staging area, free until the reorder
   uint32_t *wm = reinterpret_cast<uint32_t *>(smem) + warp * kRadix;
   clear_match_words(wm);
-  __syncthreads();
+  // all keys of smaller digits (while the keys are on their way)
+  const uint32_t smaller = block_excl_scan(totals[d], wsum);
   uint32_t lr[IT];
   warp_rank<IT>(dg, lr, wcnt[warp], wm);
   __syncthreads();
   uint32_t tcount = 0;
 #pragma unroll
   for (int w = 0; w < kWarps; w++) tcount += wcnt[w][d];
-  // publish this tile's count of digit d, then find the earlier tiles'
-  uint32_t *mine = status + tile * kRadix + d;
-  uint32_t before = 0;
-  if (tile == 0) {
-    atomicExch(mine, kOsIncl | tcount);
-  } else {
-    atomicExch(mine, kOsAgg | tcount);
-    // the walk loads kOsAhead earlier tiles' words at once, then takes them
-    // in order (a word not yet published is polled again on its own)
-    constexpr int kOsAhead = 16;
-    bool done = false;
-    for (int64_t t0 = (int64_t)tile - 1; t0 >= 0 && !done; t0 -= kOsAhead) {
-      uint32_t w[kOsAhead];
-#pragma unroll
-      for (int q = 0; q < kOsAhead; q++)
-        w[q] = t0 - q >= 0 ? *(const volatile uint32_t *)(status + (uint64_t)(t0 - q) * kRadix + d)
-                           : kOsIncl;
-#pragma unroll
-      for (int q = 0; q < kOsAhead; q++) {
-        const int64_t t = t0 - q;
-        if (done || t < 0) break;
-        uint32_t v = w[q];
-        const volatile uint32_t *sp = status + (uint64_t)t * kRadix + d;
-        for (int p = 0; (v & ~kOsMask) == 0 && p < kOsPolls; p++) {
-          __nanosleep(p < 32 ? 20 : 200);
-          v = *sp;
-        }
-        if ((v & ~kOsMask) == 0) {  // never published: count its keys
-          before += os_count_tile(in, n, (uint64_t)t, TILE, shift, d);
-          continue;
-        }
-        before += v & kOsMask;
-        if ((v & ~kOsMask) == kOsIncl) done = true;
-      }
+  // publish this tile's count of digit d
+  const int levels = os_levels(gridDim.x);
+  atomicExch(status + (uint64_t)tile * kRadix + d, kOsAgg | tcount);
+  unsigned long long *const group =
+      reinterpret_cast<unsigned long long *>(status + (uint64_t)gridDim.x * kRadix) + d;
+  {
+    unsigned long long *at = group;
+    uint32_t nt = gridDim.x, i = tile;
+    for (int l = 0; l < levels; l++) {
+      nt = (nt + kOsGroup - 1) >> kOsLog;
+      i >>= kOsLog;
+      atomicAdd(at + (uint64_t)i * kRadix, (1ull << 32) | tcount);
+      at += (uint64_t)nt * kRadix;
     }
-    atomicExch(mine, kOsIncl | (before + tcount));
   }
-  // global start of digit d: all keys of smaller digits, then the earlier
-  // tiles' keys of digit d
-  const uint32_t gbase = block_excl_scan(totals[d], wsum) + before;
-  __syncthreads();  // wsum is read by every thread before it is reused
+  // the tile in order, while the earlier tiles publish theirs
   const uint32_t tstart = block_excl_scan(tcount, wsum);
   uint32_t sacc = tstart;
 #pragma unroll
@@ -570,15 +578,63 @@ k_scatter_os(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
     wcnt[w][d] = sacc;
     sacc += c;
   }
-  adj[d] = gbase - tstart;
   __syncthreads();
 #pragma unroll
   for (int it = 0; it < IT; it++) {
-    if (dg[it] == kNoDigit) continue;
-    const uint32_t lp = wcnt[warp][dg[it]] + lr[it];
+    if (t0 + tile_offset<IT>(it) >= n) continue;
+    const uint32_t lp = wcnt[warp][(kk[it] >> shift) & 0xff] + lr[it];
     skeys[lp] = kk[it];
     if (KV) svals[lp] = vv[it];
   }
+  // the earlier tiles' keys of digit d
+  uint32_t before = 0;
+  bool whole = true;
+  {
+    const uint32_t n0 = tile & (kOsGroup - 1);
+    const volatile uint32_t *p = status + (uint64_t)(tile - n0) * kRadix + d;
+    uint32_t w[kOsGroup - 1];
+#pragma unroll
+    for (int q = 0; q < kOsGroup - 1; q++) w[q] = q < n0 ? p[q * kRadix] : kOsAgg;
+    const unsigned long long *at = group;
+    uint32_t nt = gridDim.x, i = tile;
+    for (int l = 0; l < levels; l++) {
+      nt = (nt + kOsGroup - 1) >> kOsLog;
+      i >>= kOsLog;
+      const uint32_t nl = i & (kOsGroup - 1);
+      const unsigned long long full = 1ull << (kOsLog * (l + 1));
+      const volatile unsigned long long *gp = at + (uint64_t)(i - nl) * kRadix;
+      unsigned long long v[kOsGroup - 1];
+#pragma unroll
+      for (int q = 0; q < kOsGroup - 1; q++) v[q] = q < nl ? gp[q * kRadix] : full << 32;
+#pragma unroll
+      for (int q = 0; q < kOsGroup - 1; q++) {
+        for (int t = 0; (v[q] >> 32) != full && t < kOsPolls; t++) {
+          __nanosleep(t < 32 ? 20 : 200);
+          v[q] = gp[q * kRadix];
+        }
+        whole &= (v[q] >> 32) == full;
+        before += (uint32_t)v[q];
+      }
+      at += (uint64_t)nt * kRadix;
+    }
+#pragma unroll
+    for (int q = 0; q < kOsGroup - 1; q++) {
+      for (int t = 0; w[q] == 0 && t < kOsPolls; t++) {
+        __nanosleep(t < 32 ? 20 : 200);
+        w[q] = p[q * kRadix];
+      }
+      whole &= w[q] != 0;
+      before += w[q] & kOsMask;
+    }
+  }
+  if (!whole) {  // a tile never published: the words that are there, else the keys
+    before = 0;
+    for (uint32_t t = 0; t < tile; t++) {
+      const uint32_t v = *(const volatile uint32_t *)(status + (uint64_t)t * kRadix + d);
+      before += v ? v & kOsMask : os_count_tile(in, n, t, TILE, shift, d);
+    }
+  }
+  adj[d] = smaller + before - tstart;
   __syncthreads();
   const uint32_t tn = t0 >= n ? 0u : (uint32_t)(n - t0 < (uint64_t)TILE ? n - t0 : TILE);
   for (uint32_t j = threadIdx.x; j < tn; j += kThreads) {
@@ -713,12 +769,14 @@ k_sort_bitonic(uint64_t *__restrict__ keys, uint64_t n, const uint32_t *__restri
 }  // namespace
 
 size_t radix_sort_scratch_bytes(uint64_t n) {
-  const uint64_t tile = n <= kSmallTileKeys ? (uint64_t)kThreads * kSmallItems : kTile;
+  const uint64_t tile = n <= kSmallTileKeys ? (uint64_t)kThreads * kSmallItems
+                        : n <= kMidTileKeys ? (uint64_t)kThreads * kMidItems
+                                            : kTile;
   uint64_t nblocks = (n + tile - 1) / tile;
   uint64_t hn = nblocks * kRadix;
   // the one-sweep form: digit totals and up to eight passes' tile status;
   // the counting forms: three count tables or counts and their scan
-  const size_t os = 8 * kRadix * 4 + 8 * ((hn * 4 + 255) & ~size_t(255)) + 512;
+  const size_t os = 8 * kRadix * 4 + 8 * os_status_words((uint32_t)nblocks) * 4 + 512;
   const size_t cnt = 3 * ((hn * 4 + 255) & ~size_t(255)) + scan_scratch_bytes(hn, 4) + 512;
   return os > cnt ? os : cnt;
 }
@@ -728,6 +786,8 @@ template <bool KV, int IT>
 constexpr const char *scatter_name() {
   if constexpr (IT == kSmallItems)
     return KV ? "(k_scatter<true, 4>)" : "(k_scatter<false, 4>)";
+  else if constexpr (IT == kMidItems)
+    return KV ? "(k_scatter<true, 8>)" : "(k_scatter<false, 8>)";
   else
     return KV ? "(k_scatter<true, 16>)" : "(k_scatter<false, 16>)";
 }
@@ -736,6 +796,8 @@ template <bool KV, int IT>
 constexpr const char *scatter_os_name() {
   if constexpr (IT == kSmallItems)
     return KV ? "(k_scatter_os<true, 4>)" : "(k_scatter_os<false, 4>)";
+  else if constexpr (IT == kMidItems)
+    return KV ? "(k_scatter_os<true, 8>)" : "(k_scatter_os<false, 8>)";
   else
     return KV ? "(k_scatter_os<true, 16>)" : "(k_scatter_os<false, 16>)";
 }
@@ -764,30 +826,31 @@ static cudaError_t radix_sort_tiles(uint64_t *keys, uint64_t *tmp, uint32_t *val
     // one sweep: all passes' digit totals in one read, then one launch a
     // pass whose tiles find their offsets by looking back
     uint32_t *totals, *status;
+    const uint64_t sw = os_status_words(nblocks);
     if (pre) {  // counted by the caller, status words cleared
-      if (pre->passes != passes || pre->status_words != (uint64_t)passes * hn)
+      if (pre->passes != passes || pre->status_words != (uint64_t)passes * sw)
         return cudaErrorInvalidValue;
       totals = pre->totals;
       status = pre->status;
     } else {
       totals = arena.take<uint32_t>(8 * kRadix);
-      status = arena.take<uint32_t>((uint64_t)passes * hn);
+      status = arena.take<uint32_t>((uint64_t)passes * sw);
       if (!totals || !status) return cudaErrorMemoryAllocation;
       cudaError_t e = cudaMemsetAsync(totals, 0, (size_t)passes * kRadix * 4, s);
       if (e != cudaSuccess) return e;
       SST_LAUNCH_PDL_NB("(k_hist_all)", 8 * n, k_hist_all<IT>, nblocks, kThreads, 0, s, src, n,
-                    passes, totals, status, (uint64_t)passes * hn, d_n);
+                    passes, totals, status, (uint64_t)passes * sw, d_n);
     }
     for (int p = 0; p < passes; p++) {
       const uint64_t sb = (vals ? 24 : 16) * n + 8 * (uint64_t)kRadix * nblocks;
       if (vals)
         SST_LAUNCH_PDL_NB((scatter_os_name<true, IT>()), sb, (k_scatter_os<true, IT>), nblocks,
                       kThreads, (scatter_smem_bytes<true, IT>()), s, src, dst, n, 8 * p,
-                      totals + p * kRadix, status + (uint64_t)p * hn, vsrc, vdst, d_n);
+                      totals + p * kRadix, status + (uint64_t)p * sw, vsrc, vdst, d_n);
       else
         SST_LAUNCH_PDL_NB((scatter_os_name<false, IT>()), sb, (k_scatter_os<false, IT>), nblocks,
                       kThreads, (scatter_smem_bytes<false, IT>()), s, src, dst, n, 8 * p,
-                      totals + p * kRadix, status + (uint64_t)p * hn, vsrc, vdst, d_n);
+                      totals + p * kRadix, status + (uint64_t)p * sw, vsrc, vdst, d_n);
       std::swap(src, dst);
       std::swap(vsrc, vdst);
     }
@@ -850,25 +913,28 @@ static cudaError_t radix_sort_tiles(uint64_t *keys, uint64_t *tmp, uint32_t *val
   return cudaGetLastError();
 }
 
-// the form radix_sort_impl takes: 0 none (n < 2), 1 one CTA, 2 tiles of
-// kSmallItems a thread, 3 tiles of kItems
+// items a thread of the multi-tile form
+static int sort_items(uint64_t n, bool vals) {
+  if (!vals && n <= kSmallTileKeys) return kSmallItems;
+  return n <= kMidTileKeys ? kMidItems : kItems;
+}
+// the form radix_sort_impl takes: 0 none (n < 2), 1 one CTA, 2 tiles
 static int sort_form(uint64_t n, int bits, bool vals) {
   if (n < 2 || bits <= 0) return 0;
   if (!vals && n <= (uint64_t)kSmallSort) return 1;
   if (vals && n <= (uint64_t)kSmallSortKV) return 1;
-  if (!vals && n <= kSmallTileKeys) return 2;
-  return 3;
+  return 2;
 }
 
 bool radix_sort_digits(uint64_t n, int bits, Arena &arena, SortDigits *d) {
   const int form = sort_form(n, bits, false);
   const int passes = (bits + 7) / 8;
   if (form < 2 || n >= (1ull << 30) || passes > 8) return false;
-  const uint64_t tile = (uint64_t)kThreads * (form == 2 ? kSmallItems : kItems);
-  const uint64_t hn = (n + tile - 1) / tile * kRadix;
+  const uint64_t tile = (uint64_t)kThreads * sort_items(n, false);
+  const uint64_t sw = os_status_words((uint32_t)((n + tile - 1) / tile));
   d->totals = arena.take<uint32_t>(8 * kRadix);
-  d->status = arena.take<uint32_t>((uint64_t)passes * hn);
-  d->status_words = (uint64_t)passes * hn;
+  d->status = arena.take<uint32_t>((uint64_t)passes * sw);
+  d->status_words = (uint64_t)passes * sw;
   d->passes = passes;
   return d->totals && d->status;
 }
@@ -896,11 +962,15 @@ static cudaError_t radix_sort_impl(uint64_t *keys, uint64_t *tmp,
                n, bits, d_n);
     return cudaGetLastError();
   }
-  if (!vals && n <= kSmallTileKeys)
-    return radix_sort_tiles<kSmallItems>(keys, tmp, vals, vtmp, n, bits, arena, s, result,
-                                         vresult, d_n, pre);
-  return radix_sort_tiles<kItems>(keys, tmp, vals, vtmp, n, bits, arena, s, result, vresult,
-                                  d_n, pre);
+  auto tiles = [&](auto items) {
+    return radix_sort_tiles<decltype(items)::value>(keys, tmp, vals, vtmp, n, bits, arena, s,
+                                                    result, vresult, d_n, pre);
+  };
+  switch (sort_items(n, vals != nullptr)) {
+    case kSmallItems: return tiles(std::integral_constant<int, kSmallItems>{});
+    case kMidItems: return tiles(std::integral_constant<int, kMidItems>{});
+    default: return tiles(std::integral_constant<int, kItems>{});
+  }
 }
 
 cudaError_t radix_sort_u64(uint64_t *keys, uint64_t *tmp, uint64_t n, int bits,

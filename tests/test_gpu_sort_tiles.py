@@ -1,0 +1,61 @@
+"""The key sort at the edges of its tile sizes (1024, 2048 and 4096 keys) and
+of the groups of 8, 64 and 512 tiles whose digit counts a pass adds up, through
+the bulk insert (keys) and the batched form (keys with operations)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def sg():
+    import __graft_entry__ as ge
+    ge.build()
+    import sstgraph_gb300
+    return sstgraph_gb300
+
+
+def pairs(n, b, seed):
+    rng = np.random.default_rng(seed)
+    e = rng.integers(0, n, (b, 2)).astype(np.uint32)
+    e[: b // 3, 0] = 7           # one digit for a third of the keys
+    return e
+
+
+def edges(n, *es):
+    k = np.concatenate([e[:, 0].astype(np.uint64) * n + e[:, 1] for e in es])
+    k = np.unique(k)
+    return k[k // n != k % n]
+
+
+def of(g):
+    off, cols = g.csr()
+    rows = np.repeat(np.arange(g.rows, dtype=np.uint64), np.diff(off.astype(np.int64)))
+    return rows * g.rows + cols
+
+
+@pytest.mark.parametrize("b", [7 * 1024 + 1, 8 * 1024, 8 * 1024 + 1, 64 * 1024, 64 * 1024 + 1,
+                               1 << 18, (1 << 18) + 1, 448 * 2048, 448 * 2048 + 1,
+                               512 * 4096, 512 * 4096 + 1, 1100 * 4096 + 77])
+@pytest.mark.parametrize("n", [60000, 1 << 20])
+def test_keys(sg, b, n):
+    e, f = pairs(n, b, b), pairs(n, b // 2, b + 1)
+    g = sg.SparseMatrixV(n)
+    g.insert_batch(e)                    # a load
+    assert np.array_equal(of(g), edges(n, e))
+    g.insert_batch(f)                    # an update
+    assert np.array_equal(of(g), edges(n, e, f))
+    g.close()
+
+
+@pytest.mark.parametrize("b", [1025, 8 * 2048, 8 * 2048 + 1, 64 * 2048 + 1, 448 * 2048,
+                               448 * 2048 + 1, 512 * 4096 + 1])
+def test_keys_with_values(sg, b):
+    n = 50000
+    e = pairs(n, b, b)
+    a, r, c = e[: b // 2], e[b // 4: b // 4 * 3], e[b // 2:]
+    g = sg.SparseMatrixV(n)
+    g.update_batches([a, r, c], [1, 0, 1])   # b + b / 2 pairs, the last operation wins
+    want = np.setdiff1d(edges(n, a), edges(n, r))
+    assert np.array_equal(of(g), np.union1d(want, edges(n, c)))
+    g.close()
