@@ -2559,8 +2559,7 @@ static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, b
   return SST_OK;
 }
 
-// From one pair more than the one-block sort takes.  A graph made, loaded and
-// freed, by the general sequence and so: 2,200 pairs of 300 rows 0.93 -> 0.66 ms,
+// A graph made, loaded and freed, by the general sequence and so: 2,200 pairs of 300 rows 0.93 -> 0.66 ms,
 // 18,000 of 2,000 rows 0.96 -> 0.67, 18,000 of 300,000 rows 1.20 -> 0.94, 600,000
 // (RMAT) of 32,768 rows 1.29 -> 0.84.  Smaller loads take the launches that later
 // batches of their size replay.

@@ -663,10 +663,10 @@ cudaError_t scatter_smem_optin() {
   return e;
 }
 
-// Whole sort in one CTA for n <= TILE: keys (and payloads) staged in shared
+// Whole sort of keys with values in one CTA for n <= TILE, both staged in shared
 // memory; each pass ranks warp-contiguous items as k_scatter does, the digit
 // offsets coming from a block scan of the warps' counts.
-template <bool KV, int TILE>
+template <int TILE>
 __global__ void __launch_bounds__(kThreads)
 k_sort_small(uint64_t *__restrict__ keys, uint32_t *__restrict__ vals,
              uint64_t n, int bits, const uint32_t *__restrict__ d_n) {
@@ -674,7 +674,7 @@ k_sort_small(uint64_t *__restrict__ keys, uint32_t *__restrict__ vals,
   if (d_n && *d_n < n) n = *d_n;
   constexpr int IT = TILE / kThreads;
   __shared__ uint64_t buf[2][TILE];
-  __shared__ uint32_t vbuf[KV ? 2 : 1][KV ? TILE : 1];
+  __shared__ uint32_t vbuf[2][TILE];
   __shared__ uint32_t wcnt[kWarps][kRadix];
   __shared__ uint32_t wmatch[kWarps][kRadix];
   __shared__ uint32_t wsum[kWarps];
@@ -682,7 +682,7 @@ k_sort_small(uint64_t *__restrict__ keys, uint32_t *__restrict__ vals,
   clear_match_words(wmatch[warp]);  // warp_rank leaves them clear again
   for (uint64_t i = threadIdx.x; i < n; i += kThreads) {
     buf[0][i] = keys[i];
-    if (KV) vbuf[0][i] = vals[i];
+    vbuf[0][i] = vals[i];
   }
   int cur = 0;
   for (int shift = 0; shift < bits; shift += 8) {
@@ -715,55 +715,136 @@ k_sort_small(uint64_t *__restrict__ keys, uint32_t *__restrict__ vals,
       if (dg[it] == kNoDigit) continue;
       const uint32_t pos = wcnt[warp][dg[it]] + lr[it];
       buf[cur ^ 1][pos] = kk[it];
-      if (KV) vbuf[cur ^ 1][pos] = vbuf[cur][tile_offset<IT>(it)];
+      vbuf[cur ^ 1][pos] = vbuf[cur][tile_offset<IT>(it)];
     }
     __syncthreads();  // all reads of the counters done before the next pass
     cur ^= 1;
   }
   for (uint64_t i = threadIdx.x; i < n; i += kThreads) {
     keys[i] = buf[cur][i];
-    if (KV) vals[i] = vbuf[cur][i];
+    vals[i] = vbuf[cur][i];
   }
 }
 
 constexpr int kSmallSortKV = 1024;
 
-// Keys alone (no payload: equal keys are indistinguishable, so the order
-// need not be stable) of 1025 .. kSmallSort: a bitonic sort in one CTA of
-// kBitonicThreads, each thread taking the compare-exchanges of its pairs
-// at every stage (66 stages for 2048 keys).  Up to 1024 keys the one-CTA
-// radix form (k_sort_small, whose ranking by shared-memory match words is
-// cheap) is faster: 10.5 against 12.9 us at 1e3 keys (serialised); its
-// buffers for 2048 keys would pass the 48 KB of static shared memory.
-// (Holding two keys a thread in registers, with warp shuffles for the
-// stages within a warp and the shared array only for the rest, measured
-// slower than this bitonic form: 15.7 against 13.0 us at 1e3 keys.)
-constexpr int kBitonicThreads = 1024;
-static_assert(kSmallSort <= 2 * kBitonicThreads, "one pair per thread and stage");
-__global__ void __launch_bounds__(kBitonicThreads)
-k_sort_bitonic(uint64_t *__restrict__ keys, uint64_t n, const uint32_t *__restrict__ d_n) {
+// Keys alone, up to kSmallSort, in one CTA of kBlockThreads holding IT keys a
+// thread in registers: radix passes whose counts, offsets and exchange stay in
+// shared memory, where a pass over several CTAs is a launch of its own (about
+// 5 us).  A pass is bound by its warps' chains of match-word rankings, IT of
+// them, and seven block barriers.  Five passes against the forms before (one CTA
+// of 256 threads, a bitonic network, tiles of 1024; us with the launch): 1000
+// keys 10.1 and 10.5, 2048 14.0 and 20.7, 3000 16.5 and 24.0, 4096 18.2 and 24.0;
+// with 1024 threads 12.9, 15.1, 18.7, 20.5, and 8192 keys 30.7 where tiles take
+// 23.9.
+constexpr int kBlockThreads = 512;
+constexpr int kBlockWarps = kBlockThreads / 32;
+template <int IT>
+constexpr size_t block_sort_smem() {
+  return (size_t)kBlockThreads * IT * 8 + 2 * (size_t)kBlockWarps * kRadix * 4 +
+         (size_t)kBlockThreads * 4 + kBlockWarps * 4;
+}
+template <int IT>
+__global__ void __launch_bounds__(kBlockThreads)
+k_sort_block(uint64_t *__restrict__ keys, uint64_t n, int bits,
+             const uint32_t *__restrict__ d_n) {
   pdl_wait();
-  __shared__ uint64_t sk[kSmallSort];
   if (d_n && *d_n < n) n = *d_n;
-  uint32_t N = 2;
-  while (N < n) N <<= 1;
-  const uint32_t t = threadIdx.x;
-  for (uint32_t i = t; i < N; i += kBitonicThreads) sk[i] = i < n ? keys[i] : ~0ull;
-  __syncthreads();
-  for (uint32_t k = 2; k <= N; k <<= 1)
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      // thread t takes the pair (i, i ^ j) whose lower index i is its t-th
-      const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1));
-      if (i + j < N) {
-        const uint64_t a = sk[i], b = sk[i + j];
-        if ((a > b) == ((i & k) == 0)) {
-          sk[i] = b;
-          sk[i + j] = a;
-        }
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint64_t *buf = reinterpret_cast<uint64_t *>(smem);
+  uint32_t *wcnt = reinterpret_cast<uint32_t *>(buf + kBlockThreads * IT);  // [warp][digit]
+  uint32_t *wmatch = wcnt + kBlockWarps * kRadix;
+  uint32_t *part = wmatch + kBlockWarps * kRadix;  // [quarter of the warps][digit]
+  uint32_t *wsum = part + kBlockThreads;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t t = threadIdx.x, d = t & (kRadix - 1), q = t / kRadix;
+  constexpr int kQuarters = kBlockThreads / kRadix, kShare = kBlockWarps / kQuarters;
+  uint32_t *wc = wcnt + warp * kRadix, *wm = wmatch + warp * kRadix;
+  clear_match_words(wm);  // warp_rank leaves them clear again
+  uint64_t kk[IT];
+#pragma unroll
+  for (int it = 0; it < IT; it++) {
+    const uint32_t o = tile_offset<IT>(it);
+    kk[it] = o < n ? keys[o] : 0;
+  }
+  for (int shift = 0; shift < bits; shift += 8) {
+    clear_match_words(wc);
+    uint32_t dg[IT], lr[IT];
+#pragma unroll
+    for (int it = 0; it < IT; it++)
+      dg[it] = tile_offset<IT>(it) < n ? (uint32_t)(kk[it] >> shift) & 0xff : kNoDigit;
+    warp_rank<IT>(dg, lr, wc, wm);
+    __syncthreads();
+    uint32_t sum = 0;
+#pragma unroll
+    for (int w = 0; w < kShare; w++) sum += wcnt[(q * kShare + w) * kRadix + d];
+    part[t] = sum;
+    __syncthreads();
+    uint32_t tot = 0, inc = 0;
+    if (t < kRadix) {
+#pragma unroll
+      for (int r = 0; r < kQuarters; r++) tot += part[r * kRadix + t];
+      inc = tot;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += x;
       }
-      __syncthreads();
+      if (lane == 31) wsum[warp] = inc;
     }
-  for (uint32_t i = t; i < n; i += kBitonicThreads) keys[i] = sk[i];
+    __syncthreads();
+    if (t < kRadix) {
+      uint32_t run = inc - tot;
+      for (int w = 0; w < warp; w++) run += wsum[w];
+#pragma unroll
+      for (int r = 0; r < kQuarters; r++) {
+        const uint32_t c = part[r * kRadix + t];
+        part[r * kRadix + t] = run;
+        run += c;
+      }
+    }
+    __syncthreads();
+    uint32_t run = part[t];
+#pragma unroll
+    for (int w = 0; w < kShare; w++) {
+      uint32_t *c = wcnt + (q * kShare + w) * kRadix + d;
+      const uint32_t x = *c;
+      *c = run;
+      run += x;
+    }
+    __syncthreads();
+    const bool last = shift + 8 >= bits;
+#pragma unroll
+    for (int it = 0; it < IT; it++) {
+      if (dg[it] == kNoDigit) continue;
+      (last ? keys : buf)[wc[dg[it]] + lr[it]] = kk[it];
+    }
+    if (last) break;
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < IT; it++) {
+      const uint32_t o = tile_offset<IT>(it);
+      if (o < n) kk[it] = buf[o];
+    }
+  }
+}
+
+template <int IT>
+cudaError_t sort_block(uint64_t *keys, uint64_t n, int bits, const uint32_t *d_n,
+                       cudaStream_t s) {
+  static std::atomic<uint64_t> done{0};  // one bit per device below 64
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 64 || !((done.load(std::memory_order_relaxed) >> dev) & 1)) {
+    e = cudaFuncSetAttribute(k_sort_block<IT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)block_sort_smem<IT>());
+    if (e != cudaSuccess) return e;
+    if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_relaxed);
+  }
+  SST_LAUNCH_PDL_NB("k_sort_block", 16 * n, k_sort_block<IT>, 1, kBlockThreads,
+                    (block_sort_smem<IT>()), s, keys, n, bits, d_n);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -948,17 +1029,14 @@ static cudaError_t radix_sort_impl(uint64_t *keys, uint64_t *tmp,
   if (vresult) *vresult = vals;
   if (n < 2 || bits <= 0) return cudaSuccess;
   if (pre && (vals || sort_form(n, bits, false) < 2)) return cudaErrorInvalidValue;
-  if (!vals && n <= (uint64_t)kSmallSortKV) {
-    SST_LAUNCH_PDL_B(16 * n, (k_sort_small<false, kSmallSortKV>), 1, kThreads, 0, s, keys,
-                     (uint32_t *)nullptr, n, bits, d_n);
-    return cudaGetLastError();
-  }
   if (!vals && n <= (uint64_t)kSmallSort) {
-    SST_LAUNCH_PDL_B(16 * n, k_sort_bitonic, 1, kBitonicThreads, 0, s, keys, n, d_n);
-    return cudaGetLastError();
+    if (n <= kBlockThreads) return sort_block<1>(keys, n, bits, d_n, s);
+    if (n <= 2 * kBlockThreads) return sort_block<2>(keys, n, bits, d_n, s);
+    if (n <= 4 * kBlockThreads) return sort_block<4>(keys, n, bits, d_n, s);
+    return sort_block<8>(keys, n, bits, d_n, s);
   }
   if (vals && n <= (uint64_t)kSmallSortKV) {
-    SST_LAUNCH_PDL_B(24 * n, (k_sort_small<true, kSmallSortKV>), 1, kThreads, 0, s, keys, vals,
+    SST_LAUNCH_PDL_B(24 * n, k_sort_small<kSmallSortKV>, 1, kThreads, 0, s, keys, vals,
                n, bits, d_n);
     return cudaGetLastError();
   }

@@ -1,4 +1,5 @@
-"""The key sort at the edges of its tile sizes (1024, 2048 and 4096 keys) and
+"""The key sort at the edges of its one-block forms, of its tiles (1024, 2048 and
+4096 keys) and
 of the groups of 8, 64 and 512 tiles whose digit counts a pass adds up, through
 the bulk insert (keys) and the batched form (keys with operations)."""
 import numpy as np
@@ -34,7 +35,7 @@ def of(g):
     return rows * g.rows + cols
 
 
-@pytest.mark.parametrize("b", [7 * 1024 + 1, 8 * 1024, 8 * 1024 + 1, 64 * 1024, 64 * 1024 + 1,
+@pytest.mark.parametrize("b", [1025, 2048, 2049, 4095, 4096, 4097, 7 * 1024 + 1, 8 * 1024, 8 * 1024 + 1, 64 * 1024, 64 * 1024 + 1,
                                1 << 18, (1 << 18) + 1, 448 * 2048, 448 * 2048 + 1,
                                512 * 4096, 512 * 4096 + 1, 1100 * 4096 + 77])
 @pytest.mark.parametrize("n", [60000, 1 << 20])
