@@ -2985,52 +2985,139 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
 // insert pass over already sorted keys.  Self-loops are dropped from both
 // (an inserted self-loop is skipped, a removed one is absent).
 namespace {
-__global__ void k_make_keys_batched(const uint32_t *__restrict__ pairs,
-                                    uint64_t N, const uint64_t *__restrict__ boff,
-                                    uint32_t nb, const uint8_t *__restrict__ ops,
-                                    uint32_t n, uint32_t width, int dbits,
-                                    bool drop_loops, uint64_t *__restrict__ keys,
-                                    uint32_t *__restrict__ vals,
-                                    unsigned long long *__restrict__ invalid) {
+// The keys of a sequence of batches, edge ids with the batch's operation.  The
+// operation is the key's low bit, below the bits that the sort looks at, so that
+// no value is moved beside the key (16 bytes a pass and key, not 24); where an id
+// takes all 64 bits (lo = 0) it is a value.  Digits are counted as in
+// k_make_keys_packed.
+__global__ void __launch_bounds__(256)
+k_make_keys_batched(const uint32_t *__restrict__ pairs, uint64_t N,
+                    const uint64_t *__restrict__ boff, uint32_t nb,
+                    const uint8_t *__restrict__ ops, uint32_t n, uint32_t width, int dbits,
+                    int lo, bool drop_loops, uint64_t sent, uint64_t *__restrict__ keys,
+                    uint32_t *__restrict__ vals, unsigned long long *__restrict__ invalid,
+                    SortDigits sd) {
   pdl_wait();
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  uint32_t lo = 0, hi = nb;  // batch: last with boff[b] <= i
-  while (hi - lo > 1) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (boff[mid] <= i)
-      lo = mid;
-    else
-      hi = mid;
+  __shared__ uint32_t s_hist[8][256];
+  for (int p = 0; p < sd.passes; p++) s_hist[p][threadIdx.x] = 0;
+  __syncthreads();
+  uint32_t bad = 0;
+#pragma unroll
+  for (int k = 0; k < kPackItems; k++) {
+    const uint64_t i = (uint64_t)blockIdx.x * (256 * kPackItems) + k * 256 + threadIdx.x;
+    if (i >= N) break;
+    uint32_t first = 0, last = nb;  // batch: last with boff[b] <= i
+    while (last - first > 1) {
+      const uint32_t mid = (first + last) >> 1;
+      if (boff[mid] <= i)
+        first = mid;
+      else
+        last = mid;
+    }
+    const uint32_t r = pairs[2 * i], c = pairs[2 * i + 1];
+    const bool ok = r < n && c < width && c != kEmpty;
+    bad += !ok;
+    const uint64_t id = !ok || (drop_loops && r == c) ? sent : ((uint64_t)r << dbits) | c;
+    const uint32_t op = ops[first] ? 1u : 0u;
+    if (lo)
+      keys[i] = id << 1 | op;
+    else {
+      keys[i] = id;
+      vals[i] = op;
+    }
+    for (int p = 0; p < sd.passes; p++) atomicAdd(&s_hist[p][(id >> (8 * p)) & 0xff], 1u);
   }
-  uint32_t r = pairs[2 * i], c = pairs[2 * i + 1];
-  const uint64_t sent = (uint64_t)n << dbits;
-  bool ok = r < n && c < width && c != kEmpty;
-  if (!ok) atomicAdd(invalid, 1ull);
-  keys[i] = (!ok || (drop_loops && r == c)) ? sent : (((uint64_t)r << dbits) | c);
-  vals[i] = ops[lo] ? 1u : 0u;
+  if (bad) atomicAdd(invalid, (unsigned long long)bad);
+  if (!sd.passes) return;
+  for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < sd.status_words;
+       i += (uint64_t)gridDim.x * 256)
+    sd.status[i] = 0;
+  __syncthreads();
+  for (int p = 0; p < sd.passes; p++)
+    if (s_hist[p][threadIdx.x])
+      atomicAdd(&sd.totals[p * 256 + threadIdx.x], s_hist[p][threadIdx.x]);
 }
 
-__global__ void k_last_op(const uint64_t *__restrict__ keys,
-                          const uint32_t *__restrict__ vals, uint64_t N,
-                          uint64_t sent, uint32_t *__restrict__ fins,
-                          uint32_t *__restrict__ fdel) {
+// The net operations (the last of each run of equal ids) of a tile of sorted
+// keys, with their ranks among the tile's insertions and removals; as LoadTile,
+// computed twice rather than stored (two flags, two positions and their scans
+// took 56 us for 1.8M keys, this and the scan of the tiles' counts 23).
+struct NetTile {
+  uint64_t id[kLoadRows];
+  uint32_t rank[kLoadRows];  // in the tile, among the key's own operation
+  uint32_t ins, del;         // bit k: key k is a net insertion / removal
+  uint32_t nins, ndel;       // of the tile
+  __device__ __forceinline__ void load(const uint64_t *__restrict__ keys,
+                                       const uint32_t *__restrict__ vals, uint64_t N, int lo,
+                                       uint64_t sent, uint32_t *s_warp) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t below = (1u << lane) - 1u;
+    uint64_t key[kLoadRows], after[kLoadRows];
+#pragma unroll
+    for (int k = 0; k < kLoadRows; k++) {
+      const uint64_t i = LoadTile::index(k);
+      key[k] = i < N ? keys[i] : 0;
+      after[k] = lane == 31 && i + 1 < N ? keys[i + 1] : 0;
+    }
+    uint32_t run = 0;  // insertions | removals << 16
+    ins = del = 0;
+#pragma unroll
+    for (int k = 0; k < kLoadRows; k++) {
+      const uint64_t i = LoadTile::index(k);
+      const uint64_t down = __shfl_down_sync(0xffffffffu, key[k], 1);
+      if (lane < 31) after[k] = down;
+      id[k] = key[k] >> lo;
+      const bool net = i < N && id[k] != sent && (i + 1 >= N || after[k] >> lo != id[k]);
+      const bool op = lo ? key[k] & 1 : net && vals[i];
+      const uint32_t vi = __ballot_sync(0xffffffffu, net && op);
+      const uint32_t vd = __ballot_sync(0xffffffffu, net && !op);
+      rank[k] = op ? (run & 0xffff) + __popc(vi & below) : (run >> 16) + __popc(vd & below);
+      run += __popc(vi) | __popc(vd) << 16;
+      ins |= (uint32_t)(net && op) << k;
+      del |= (uint32_t)(net && !op) << k;
+    }
+    if (lane == 0) s_warp[warp] = run;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kLoadTB / 32; w++) {
+      if (w < warp) before += s_warp[w];
+      total += s_warp[w];
+    }
+#pragma unroll
+    for (int k = 0; k < kLoadRows; k++)
+      rank[k] += (ins >> k) & 1u ? before & 0xffff : before >> 16;
+    nins = total & 0xffff;
+    ndel = total >> 16;
+  }
+};
+static_assert(kLoadTile < 1 << 16, "a tile's counts share a word");
+
+// tiles: (removals << 32) | insertions of each tile
+__global__ void __launch_bounds__(kLoadTB)
+k_net_count(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ vals, uint64_t N,
+            int lo, uint64_t sent, uint64_t *__restrict__ tiles) {
   pdl_wait();
-  uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= N) return;
-  uint64_t k = keys[j];
-  bool last = k < sent && (j + 1 == N || keys[j + 1] != k);
-  fins[j] = last && vals[j];
-  fdel[j] = last && !vals[j];
+  __shared__ uint32_t s_warp[kLoadTB / 32];
+  NetTile t;
+  t.load(keys, vals, N, lo, sent, s_warp);
+  if (threadIdx.x == 0) tiles[blockIdx.x] = (uint64_t)t.ndel << 32 | t.nins;
 }
 
-__global__ void k_compact_keys(const uint64_t *__restrict__ keys,
-                               const uint32_t *__restrict__ f,
-                               const uint32_t *__restrict__ pos, uint64_t N,
-                               uint64_t *__restrict__ out) {
+__global__ void __launch_bounds__(kLoadTB)
+k_net_place(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ vals, uint64_t N,
+            int lo, uint64_t sent, const uint64_t *__restrict__ tiles,
+            uint64_t *__restrict__ ins, uint64_t *__restrict__ del) {
   pdl_wait();
-  uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < N && f[j]) out[pos[j]] = keys[j];
+  __shared__ uint32_t s_warp[kLoadTB / 32];
+  NetTile t;
+  t.load(keys, vals, N, lo, sent, s_warp);
+  const uint64_t at = tiles[blockIdx.x];
+#pragma unroll
+  for (int k = 0; k < kLoadRows; k++) {
+    if ((t.ins >> k) & 1u) ins[(uint32_t)at + t.rank[k]] = t.id[k];
+    if ((t.del >> k) & 1u) del[(uint32_t)(at >> 32) + t.rank[k]] = t.id[k];
+  }
 }
 }  // namespace
 
@@ -3044,8 +3131,15 @@ sst_status update_batches(sst_graph *g, const uint32_t *d_pairs,
     return SST_EINVAL;
   }
   cudaStream_t s = g->stream;
-  size_t need = N * (8 * 2 + 4 * 6 + 64) + radix_sort_scratch_bytes(N) +
-                4 * scan_scratch_bytes(N, 4) + (1 << 16);
+  const int dbits = g->dbits;
+  // A dropped pair's id: on a graph that keeps no self-loops that of (0, 0), else
+  // of a row n, which takes a bit more when n is a power of two.
+  const uint64_t sent = g->keep_loops ? (uint64_t)g->n << dbits : 0;
+  const int bits = (g->keep_loops ? g->rbits : bits_for(g->n ? g->n - 1 : 0)) + dbits;
+  const int lo = bits < 64 ? 1 : 0;  // the operation in the key, see k_make_keys_batched
+  const uint64_t ntiles = (N + kLoadTile - 1) / kLoadTile;
+  const size_t need = N * (lo ? 16 : 24) + ntiles * 16 + radix_sort_scratch_bytes(N) +
+                      scan_scratch_bytes(ntiles, 8) + (1 << 14);
   if (need > g->arena.cap) {
     sst_status st = budget_check(g, need - g->arena.cap);
     if (st != SST_OK) return st;
@@ -3056,38 +3150,45 @@ sst_status update_batches(sst_graph *g, const uint32_t *d_pairs,
   PlanSummary *P = g->d_plan;
   SST_CUDA_TRY(cudaMemsetAsync(P, 0, sizeof(PlanSummary), s));
   uint64_t *keys = A.take<uint64_t>(N), *ktmp = A.take<uint64_t>(N);
-  uint32_t *vals = A.take<uint32_t>(N), *vtmp = A.take<uint32_t>(N);
-  uint32_t *fins = A.take<uint32_t>(N), *fdel = A.take<uint32_t>(N);
-  uint32_t *pins = A.take<uint32_t>(N), *pdel = A.take<uint32_t>(N);
-  if (!pdel) {
+  uint32_t *vals = lo ? nullptr : A.take<uint32_t>(N), *vtmp = lo ? nullptr : A.take<uint32_t>(N);
+  uint64_t *tcnt = A.take<uint64_t>(ntiles), *tiles = A.take<uint64_t>(ntiles);
+  if (!tiles) {
     set_error_message("batched update scratch sizing error");
     return SST_ENOMEM;
   }
-  const int dbits = g->dbits;
-  const uint64_t sent = (uint64_t)g->n << dbits;
-  SST_LAUNCH_PDL(k_make_keys_batched, blocks_for(N), kTB, 0, s, d_pairs, N, d_boff,
-             nb, d_ops, g->n, g->width, dbits, !g->keep_loops, keys, vals,
-             reinterpret_cast<unsigned long long *>(&P->invalid));
+  SortDigits sdig;
+  if (lo && radix_sort_digits(N, bits, A, &sdig))
+    SST_CUDA_TRY(cudaMemsetAsync(sdig.totals, 0, (size_t)sdig.passes * 256 * 4, s));
+  else
+    sdig = SortDigits{};
+  SST_LAUNCH_PDL(k_make_keys_batched, blocks_for(N, kTB * kPackItems), kTB, 0, s, d_pairs, N,
+             d_boff, nb, d_ops, g->n, g->width, dbits, lo, !g->keep_loops, sent, keys, vals,
+             reinterpret_cast<unsigned long long *>(&P->invalid), sdig);
   uint64_t *sk = keys;
   uint32_t *sv = vals;
-  SST_CUDA_TRY(radix_sort_kv(keys, ktmp, vals, vtmp, N, g->rbits + dbits, A, s,
-                             &sk, &sv));
-  SST_LAUNCH_PDL(k_last_op, blocks_for(N), kTB, 0, s, sk, sv, N, sent, fins, fdel);
-  SST_CUDA_TRY((scan<uint32_t, OpAdd>(fins, pins, N, 0u, OpAdd{}, true, false,
-                                      &P->n_items, A, s)));
-  SST_CUDA_TRY((scan<uint32_t, OpAdd>(fdel, pdel, N, 0u, OpAdd{}, true, false,
-                                      &P->n_groups, A, s)));
-  SST_CUDA_TRY(cudaMemcpyAsync(g->h_plan, P, sizeof(PlanSummary),
-                               cudaMemcpyDeviceToHost, s));
-  SST_CUDA_TRY(cudaStreamSynchronize(s));
-  uint64_t n_ins = g->h_plan->n_items, n_del = g->h_plan->n_groups;
-  if (n_invalid) *n_invalid = g->h_plan->invalid;
+  if (lo)
+    SST_CUDA_TRY(radix_sort_u64(keys, ktmp, N, bits, A, s, &sk, nullptr,
+                                sdig.passes ? &sdig : nullptr, lo));
+  else
+    SST_CUDA_TRY(radix_sort_kv(keys, ktmp, vals, vtmp, N, bits, A, s, &sk, &sv));
+  SST_LAUNCH_PDL_B(8 * N, k_net_count, (unsigned)ntiles, kLoadTB, 0, s, sk, sv, N, lo, sent, tcnt);
+  static_assert(offsetof(PlanSummary, n_items) % 8 == 0 &&
+                    offsetof(PlanSummary, n_groups) == offsetof(PlanSummary, n_items) + 4,
+                "the net insertions and removals share one aligned 64-bit word");
+  SST_CUDA_TRY((scan<uint64_t, OpAdd>(tcnt, tiles, ntiles, 0ull, OpAdd{}, true, false,
+                                      reinterpret_cast<uint64_t *>(&P->n_items), A, s)));
+  SST_LAUNCH_PDL(k_plan_out, 1, 64, 0, s, P, g->d_err, g->h_plan_dev);
+  PlanSummary ps;
+  sst_status st = read_plan(g, &ps);
+  if (st != SST_OK) return st;
+  const uint64_t n_ins = ps.n_items, n_del = ps.n_groups;
+  if (n_invalid) *n_invalid = ps.invalid;
   if (n_ins + n_del == 0) return SST_OK;
   uint64_t *net = nullptr;
   SST_CUDA_TRY(cudaMallocAsync(&net, (n_ins + n_del) * 8, s));
-  SST_LAUNCH_PDL(k_compact_keys, blocks_for(N), kTB, 0, s, sk, fins, pins, N, net);
-  SST_LAUNCH_PDL(k_compact_keys, blocks_for(N), kTB, 0, s, sk, fdel, pdel, N, net + n_ins);
-  sst_status st = run_pipeline(g, nullptr, net + n_ins, n_del, false, nullptr, nullptr);
+  SST_LAUNCH_PDL_B(16 * N, k_net_place, (unsigned)ntiles, kLoadTB, 0, s, sk, sv, N, lo, sent,
+                   tiles, net, net + n_ins);
+  st = run_pipeline(g, nullptr, net + n_ins, n_del, false, nullptr, nullptr);
   if (st == SST_OK) st = run_pipeline(g, nullptr, net, n_ins, true, nullptr, nullptr);
   cudaFreeAsync(net, s);
   return st;

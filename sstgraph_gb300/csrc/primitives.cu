@@ -468,7 +468,7 @@ inline uint64_t os_status_words(uint32_t nt) {
 
 template <int IT>
 __global__ void __launch_bounds__(kThreads)
-k_hist_all(const uint64_t *__restrict__ keys, uint64_t n, int passes,
+k_hist_all(const uint64_t *__restrict__ keys, uint64_t n, int lo, int passes,
            uint32_t *__restrict__ totals, uint32_t *__restrict__ status,
            uint64_t status_words, const uint32_t *__restrict__ d_n) {
   pdl_wait();
@@ -482,7 +482,7 @@ k_hist_all(const uint64_t *__restrict__ keys, uint64_t n, int passes,
     const uint64_t i = t0 + (uint64_t)it * kThreads + threadIdx.x;
     if (i < n) {
       const uint64_t k = keys[i];
-      for (int p = 0; p < passes; p++) atomicAdd(&h[p][(k >> (8 * p)) & 0xff], 1u);
+      for (int p = 0; p < passes; p++) atomicAdd(&h[p][(k >> (lo + 8 * p)) & 0xff], 1u);
     }
   }
   __syncthreads();
@@ -746,7 +746,7 @@ constexpr size_t block_sort_smem() {
 }
 template <int IT>
 __global__ void __launch_bounds__(kBlockThreads)
-k_sort_block(uint64_t *__restrict__ keys, uint64_t n, int bits,
+k_sort_block(uint64_t *__restrict__ keys, uint64_t n, int lo, int bits,
              const uint32_t *__restrict__ d_n) {
   pdl_wait();
   if (d_n && *d_n < n) n = *d_n;
@@ -767,7 +767,7 @@ k_sort_block(uint64_t *__restrict__ keys, uint64_t n, int bits,
     const uint32_t o = tile_offset<IT>(it);
     kk[it] = o < n ? keys[o] : 0;
   }
-  for (int shift = 0; shift < bits; shift += 8) {
+  for (int shift = lo; shift < lo + bits; shift += 8) {
     clear_match_words(wc);
     uint32_t dg[IT], lr[IT];
 #pragma unroll
@@ -813,7 +813,7 @@ k_sort_block(uint64_t *__restrict__ keys, uint64_t n, int bits,
       run += x;
     }
     __syncthreads();
-    const bool last = shift + 8 >= bits;
+    const bool last = shift + 8 >= lo + bits;
 #pragma unroll
     for (int it = 0; it < IT; it++) {
       if (dg[it] == kNoDigit) continue;
@@ -830,7 +830,7 @@ k_sort_block(uint64_t *__restrict__ keys, uint64_t n, int bits,
 }
 
 template <int IT>
-cudaError_t sort_block(uint64_t *keys, uint64_t n, int bits, const uint32_t *d_n,
+cudaError_t sort_block(uint64_t *keys, uint64_t n, int lo, int bits, const uint32_t *d_n,
                        cudaStream_t s) {
   static std::atomic<uint64_t> done{0};  // one bit per device below 64
   int dev = 0;
@@ -843,7 +843,7 @@ cudaError_t sort_block(uint64_t *keys, uint64_t n, int bits, const uint32_t *d_n
     if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_relaxed);
   }
   SST_LAUNCH_PDL_NB("k_sort_block", 16 * n, k_sort_block<IT>, 1, kBlockThreads,
-                    (block_sort_smem<IT>()), s, keys, n, bits, d_n);
+                    (block_sort_smem<IT>()), s, keys, n, lo, bits, d_n);
   return cudaGetLastError();
 }
 
@@ -886,7 +886,7 @@ constexpr const char *scatter_os_name() {
 // The multi-tile sort with tiles of IT items per thread (see radix_sort_impl).
 template <int IT>
 static cudaError_t radix_sort_tiles(uint64_t *keys, uint64_t *tmp, uint32_t *vals,
-                                    uint32_t *vtmp, uint64_t n, int bits, Arena &arena,
+                                    uint32_t *vtmp, uint64_t n, int lo, int bits, Arena &arena,
                                     cudaStream_t s, uint64_t **result,
                                     uint32_t **vresult, const uint32_t *d_n,
                                     const SortDigits *pre) {
@@ -920,17 +920,17 @@ static cudaError_t radix_sort_tiles(uint64_t *keys, uint64_t *tmp, uint32_t *val
       cudaError_t e = cudaMemsetAsync(totals, 0, (size_t)passes * kRadix * 4, s);
       if (e != cudaSuccess) return e;
       SST_LAUNCH_PDL_NB("(k_hist_all)", 8 * n, k_hist_all<IT>, nblocks, kThreads, 0, s, src, n,
-                    passes, totals, status, (uint64_t)passes * sw, d_n);
+                    lo, passes, totals, status, (uint64_t)passes * sw, d_n);
     }
     for (int p = 0; p < passes; p++) {
       const uint64_t sb = (vals ? 24 : 16) * n + 8 * (uint64_t)kRadix * nblocks;
       if (vals)
         SST_LAUNCH_PDL_NB((scatter_os_name<true, IT>()), sb, (k_scatter_os<true, IT>), nblocks,
-                      kThreads, (scatter_smem_bytes<true, IT>()), s, src, dst, n, 8 * p,
+                      kThreads, (scatter_smem_bytes<true, IT>()), s, src, dst, n, lo + 8 * p,
                       totals + p * kRadix, status + (uint64_t)p * sw, vsrc, vdst, d_n);
       else
         SST_LAUNCH_PDL_NB((scatter_os_name<false, IT>()), sb, (k_scatter_os<false, IT>), nblocks,
-                      kThreads, (scatter_smem_bytes<false, IT>()), s, src, dst, n, 8 * p,
+                      kThreads, (scatter_smem_bytes<false, IT>()), s, src, dst, n, lo + 8 * p,
                       totals + p * kRadix, status + (uint64_t)p * sw, vsrc, vdst, d_n);
       std::swap(src, dst);
       std::swap(vsrc, vdst);
@@ -941,11 +941,11 @@ static cudaError_t radix_sort_tiles(uint64_t *keys, uint64_t *tmp, uint32_t *val
     uint32_t *h[3];
     for (auto &t : h)
       if (!(t = arena.take<uint32_t>(hn))) return cudaErrorMemoryAllocation;
-    SST_LAUNCH_PDL_B(hist_bytes, k_hist<IT>, nblocks, kThreads, 0, s, src, n, 0, h[0],
+    SST_LAUNCH_PDL_B(hist_bytes, k_hist<IT>, nblocks, kThreads, 0, s, src, n, lo, h[0],
                  1u, (uint32_t)kRadix, h[1], d_n);
     int p = 0;
-    for (int shift = 0; shift < bits; shift += 8, p++) {
-      const bool more = shift + 8 < bits;
+    for (int shift = lo; shift < lo + bits; shift += 8, p++) {
+      const bool more = shift + 8 < lo + bits;
       uint32_t *nx = more ? h[(p + 1) % 3] : nullptr;
       uint32_t *zr = more ? h[(p + 2) % 3] : nullptr;
       if (vals)
@@ -967,7 +967,7 @@ static cudaError_t radix_sort_tiles(uint64_t *keys, uint64_t *tmp, uint32_t *val
     uint32_t *cnts = arena.take<uint32_t>(hn);
     uint32_t *hist = arena.take<uint32_t>(hn);
     if (!cnts || !hist) return cudaErrorMemoryAllocation;
-    for (int shift = 0; shift < bits; shift += 8) {
+    for (int shift = lo; shift < lo + bits; shift += 8) {
       SST_LAUNCH_PDL_B(hist_bytes, k_hist<IT>, nblocks, kThreads, 0, s, src, n, shift,
                    cnts, nblocks, 1u, (uint32_t *)nullptr, d_n);
       size_t mark = arena.used;
@@ -1022,7 +1022,7 @@ bool radix_sort_digits(uint64_t n, int bits, Arena &arena, SortDigits *d) {
 
 static cudaError_t radix_sort_impl(uint64_t *keys, uint64_t *tmp,
                                    uint32_t *vals, uint32_t *vtmp, uint64_t n,
-                                   int bits, Arena &arena, cudaStream_t s,
+                                   int lo, int bits, Arena &arena, cudaStream_t s,
                                    uint64_t **result, uint32_t **vresult,
                                    const uint32_t *d_n, const SortDigits *pre = nullptr) {
   *result = keys;
@@ -1030,10 +1030,10 @@ static cudaError_t radix_sort_impl(uint64_t *keys, uint64_t *tmp,
   if (n < 2 || bits <= 0) return cudaSuccess;
   if (pre && (vals || sort_form(n, bits, false) < 2)) return cudaErrorInvalidValue;
   if (!vals && n <= (uint64_t)kSmallSort) {
-    if (n <= kBlockThreads) return sort_block<1>(keys, n, bits, d_n, s);
-    if (n <= 2 * kBlockThreads) return sort_block<2>(keys, n, bits, d_n, s);
-    if (n <= 4 * kBlockThreads) return sort_block<4>(keys, n, bits, d_n, s);
-    return sort_block<8>(keys, n, bits, d_n, s);
+    if (n <= kBlockThreads) return sort_block<1>(keys, n, lo, bits, d_n, s);
+    if (n <= 2 * kBlockThreads) return sort_block<2>(keys, n, lo, bits, d_n, s);
+    if (n <= 4 * kBlockThreads) return sort_block<4>(keys, n, lo, bits, d_n, s);
+    return sort_block<8>(keys, n, lo, bits, d_n, s);
   }
   if (vals && n <= (uint64_t)kSmallSortKV) {
     SST_LAUNCH_PDL_B(24 * n, k_sort_small<kSmallSortKV>, 1, kThreads, 0, s, keys, vals,
@@ -1041,7 +1041,7 @@ static cudaError_t radix_sort_impl(uint64_t *keys, uint64_t *tmp,
     return cudaGetLastError();
   }
   auto tiles = [&](auto items) {
-    return radix_sort_tiles<decltype(items)::value>(keys, tmp, vals, vtmp, n, bits, arena, s,
+    return radix_sort_tiles<decltype(items)::value>(keys, tmp, vals, vtmp, n, lo, bits, arena, s,
                                                     result, vresult, d_n, pre);
   };
   switch (sort_items(n, vals != nullptr)) {
@@ -1053,15 +1053,15 @@ static cudaError_t radix_sort_impl(uint64_t *keys, uint64_t *tmp,
 
 cudaError_t radix_sort_u64(uint64_t *keys, uint64_t *tmp, uint64_t n, int bits,
                            Arena &arena, cudaStream_t s, uint64_t **result,
-                           const uint32_t *d_n, const SortDigits *pre) {
-  return radix_sort_impl(keys, tmp, nullptr, nullptr, n, bits, arena, s, result,
+                           const uint32_t *d_n, const SortDigits *pre, int lo) {
+  return radix_sort_impl(keys, tmp, nullptr, nullptr, n, lo, bits, arena, s, result,
                          nullptr, d_n, pre);
 }
 
 cudaError_t radix_sort_kv(uint64_t *keys, uint64_t *tmp, uint32_t *vals,
                           uint32_t *vtmp, uint64_t n, int bits, Arena &arena,
                           cudaStream_t s, uint64_t **result, uint32_t **vresult) {
-  return radix_sort_impl(keys, tmp, vals, vtmp, n, bits, arena, s, result,
+  return radix_sort_impl(keys, tmp, vals, vtmp, n, 0, bits, arena, s, result,
                          vresult, nullptr);
 }
 

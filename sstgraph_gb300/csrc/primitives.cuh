@@ -662,6 +662,8 @@ constexpr int kSmallSort = 4096;
 cudaError_t radix_sort_kv(uint64_t *keys, uint64_t *tmp, uint32_t *vals,
                           uint32_t *vtmp, uint64_t n, int bits, Arena &arena,
                           cudaStream_t s, uint64_t **result, uint32_t **vresult);
+// radix_sort_u64's lo: the sort looks at bits lo .. lo + bits - 1 (the bits below
+// go along, and equal keys keep their order)
 // d_n (device, may be null): sort only the first min(n, *d_n) keys; n sizes
 // the launches, the rest of the arrays is left as it was
 // The digit counts of the one-sweep form (key-only sorts of more than
@@ -682,7 +684,7 @@ bool radix_sort_digits(uint64_t n, int bits, Arena &arena, SortDigits *d);
 cudaError_t radix_sort_u64(uint64_t *keys, uint64_t *tmp, uint64_t n, int bits,
                            Arena &arena, cudaStream_t s, uint64_t **result,
                            const uint32_t *d_n = nullptr,
-                           const SortDigits *pre = nullptr);
+                           const SortDigits *pre = nullptr, int lo = 0);
 size_t radix_sort_scratch_bytes(uint64_t n);
 
 }  // namespace sst

@@ -60,3 +60,49 @@ def test_keys_with_values(sg, b):
     want = np.setdiff1d(edges(n, a), edges(n, r))
     assert np.array_equal(of(g), np.union1d(want, edges(n, c)))
     g.close()
+
+
+@pytest.mark.parametrize("loops", [False, True])
+def test_batches_with_dropped_pairs(sg, loops):
+    """Self-loops (of row 0 too), ids out of range and edges given many times;
+    n a power of two, so a row n would take one more bit."""
+    n, b = 1 << 10, 20000
+    rng = np.random.default_rng(1)
+    es = [rng.integers(0, n, (b, 2)).astype(np.uint32) for _ in range(5)]
+    for e in es:
+        e[::9] = 0
+        e[1::9, 1] = e[1::9, 0]
+        e[2::9, 0] = n
+        e[3::9] = (0, 1)
+    ops = [1, 0, 1, 0, 1]
+    g = sg.SparseMatrixV(n, keep_self_loops=loops)
+    assert g.update_batches(es, ops) == sum(int((e.max(1) >= n).sum()) for e in es)
+    have = np.zeros(n * n, bool)
+    for e, op in zip(es, ops):
+        e = e[e.max(1) < n].astype(np.int64)
+        have[e[:, 0] * n + e[:, 1]] = op
+    if not loops:
+        have[np.arange(n) * n + np.arange(n)] = False
+    assert np.array_equal(of(g), np.flatnonzero(have).astype(np.uint64))
+    g.close()
+
+
+def test_batches_with_ids_of_64_bits(sg):
+    """Rows and columns of 32 bits: no bit of a key is free for its operation."""
+    torch = pytest.importorskip("torch")
+    if torch.cuda.mem_get_info()[0] < 120 << 30:
+        pytest.skip("the vertex records take 34 GB")
+    n, w = (1 << 31) + 5, 0xfffffff0
+    rng = np.random.default_rng(2)
+    a = np.stack([rng.integers(0, n, 5000), rng.integers(0, w, 5000)], 1).astype(np.uint32)
+    a[:3] = [(0, 0), (n - 1, w - 1), (n - 1, 0)]
+    r = a[1::2].copy()
+    g = sg.SparseMatrixV(n, w)
+    assert g.update_batches([a, r, a[3::4]], [1, 0, 1]) == 0
+    want = np.ones(5000, bool)
+    want[1::2] = False
+    want[3::4] = True
+    want[0] = False  # a self-loop
+    assert np.array_equal(np.asarray(g.has_batch(a)).astype(bool), want)
+    assert g.M() == int(want.sum())
+    g.close()
