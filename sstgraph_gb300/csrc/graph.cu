@@ -1045,15 +1045,19 @@ __global__ void k_task_setup_hard(DGraph g, uint64_t inv_fill, bool insert,
 // launch), where a copy-engine transfer would start only after they finish.
 static_assert(sizeof(PlanSummary) % 8 == 0 && offsetof(PlanSummary, apply_err) % 8 == 0,
               "the plan summary is copied as 8-byte words");
-__global__ void k_plan_out(const PlanSummary *__restrict__ P,
-                           const unsigned long long *__restrict__ err,
-                           PlanSummary *__restrict__ host) {
-  pdl_wait();
+__device__ __forceinline__ void plan_out(const PlanSummary *P, const unsigned long long *err,
+                                         PlanSummary *host) {
   constexpr int kWords = (int)(sizeof(PlanSummary) / 8);
   constexpr int kErrWord = (int)(offsetof(PlanSummary, apply_err) / 8);
   const unsigned long long *src = reinterpret_cast<const unsigned long long *>(P);
   unsigned long long *dst = reinterpret_cast<unsigned long long *>(host);
   for (int i = threadIdx.x; i < kWords; i += blockDim.x) dst[i] = i == kErrWord ? *err : src[i];
+}
+__global__ void k_plan_out(const PlanSummary *__restrict__ P,
+                           const unsigned long long *__restrict__ err,
+                           PlanSummary *__restrict__ host) {
+  pdl_wait();
+  plan_out(P, err, host);
 }
 // the staging-rank error count alone (the end of a host-pointer call)
 __global__ void k_err_out(const unsigned long long *__restrict__ err,
@@ -1439,22 +1443,22 @@ __global__ void k_small_locate(const uint32_t *__restrict__ pairs, uint32_t b, D
 
 // exclusive scan of a value a thread over the plan's block; sm holds one value
 // a warp and is free again afterwards
-template <typename T, typename Op>
+template <int WARPS = kSmallWarps, typename T, typename Op>
 __device__ __forceinline__ T small_scan(T v, T identity, Op op, T *total, T *sm) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const T inc = warp_inclusive(v, op);
   if (lane == 31) sm[warp] = inc;
   __syncthreads();
   if (warp == 0) {
-    const T w = lane < kSmallWarps ? sm[lane] : identity;
+    const T w = lane < WARPS ? sm[lane] : identity;
     const T wi = warp_inclusive(w, op);
-    if (lane < kSmallWarps) sm[lane] = wi;
+    if (lane < WARPS) sm[lane] = wi;
   }
   __syncthreads();
   T ex = __shfl_up_sync(0xffffffffu, inc, 1);
   if (lane == 0) ex = identity;
   if (warp) ex = op(sm[warp - 1], ex);
-  *total = sm[kSmallWarps - 1];
+  *total = sm[WARPS - 1];
   __syncthreads();
   return ex;
 }
@@ -1753,6 +1757,173 @@ k_small_apply(DGraph g, Tasks t, const ClassStarts class_start, uint32_t nmerge,
   // the scatter reads no row that a resize moves here
   for (uint32_t tau = tid; tau < ntasks; tau += kAll)
     task_finalize(tau, g, t, ntasks, class_start);
+}
+
+// ---------------------------------------------------- middling batches
+// Up to kMidBatch keys, steps 4 to 8 take one block where the general sequence
+// launches a grid a step: of 20 launches of 2 to 4 us, nearly all of it launch
+// and first loads, 7 remain.  The steps whose work a key is long (locate, the
+// removes' leaf deletes, climbs, the tasks that a warp sets up) keep their grids.
+// Bound by the chain of launches.  An insert and a remove at RMAT scale 20, with a
+// degree copy and a lookup: 1500 pairs 150 -> 132 us, 4000 170 -> 161; above, a
+// block's share grows and a grid's does not.
+constexpr uint32_t kMidBatch = 4096;
+constexpr int kMidThreads = 1024, kMidWarps = kMidThreads / 32;
+constexpr int kMidPer = kMidBatch / kMidThreads;
+
+// k_pack, k_group_flags, the scans of both flags and, for inserts,
+// k_classify_insert
+__global__ void __launch_bounds__(kMidThreads)
+k_mid_items(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ flag,
+            const uint32_t *__restrict__ leaf, const uint64_t *__restrict__ lS,
+            const uint32_t *__restrict__ lc, uint32_t b, int dbits, bool insert, uint64_t *p_ul,
+            uint32_t *__restrict__ p_x, uint64_t *__restrict__ p_S, uint32_t *p_c,
+            uint32_t *g_start, uint8_t *gtype, uint8_t *glev, uint32_t *gw0, uint32_t *gw1,
+            uint32_t *climb, PlanSummary *__restrict__ P) {
+  pdl_wait();
+  __shared__ uint64_t s_w64[kMidWarps];
+  __shared__ uint32_t s_w32[kMidWarps];
+  const uint32_t t = threadIdx.x;
+  uint64_t key[kMidPer], ul[kMidPer], last = 0;  // last: the thread's last item's ul, plus one
+  bool keep[kMidPer];
+#pragma unroll
+  for (int k = 0; k < kMidPer; k++) {
+    const uint32_t j = kMidPer * t + k;
+    keep[k] = j < b && flag[j];
+    key[k] = keep[k] ? keys[j] : 0;
+    ul[k] = keep[k] ? (key[k] >> dbits) << 32 | leaf[j] : 0;
+    if (keep[k]) last = ul[k] + 1;
+  }
+  // the item before opens another group if it lies in another leaf (ul ascends)
+  uint64_t tot64;
+  uint64_t prev = small_scan<kMidWarps>(last, (uint64_t)0, OpMax{}, &tot64, s_w64);
+  uint32_t cnt = 0;  // items | groups << 16
+  bool head[kMidPer];
+#pragma unroll
+  for (int k = 0; k < kMidPer; k++) {
+    head[k] = keep[k] && prev != ul[k] + 1;
+    if (keep[k]) prev = ul[k] + 1;
+    cnt += (keep[k] ? 1u : 0u) + (head[k] ? 1u << 16 : 0u);
+  }
+  uint32_t tot;
+  uint32_t at = small_scan<kMidWarps>(cnt, 0u, OpAdd{}, &tot, s_w32);
+  const uint32_t ni = tot & 0xffff, ng = tot >> 16;
+#pragma unroll
+  for (int k = 0; k < kMidPer; k++) {
+    const uint32_t j = kMidPer * t + k, item = at & 0xffff;
+    if (head[k]) g_start[at >> 16] = item;
+    if (keep[k]) {
+      p_ul[item] = ul[k];
+      p_x[item] = (uint32_t)(key[k] & ((1ull << dbits) - 1));
+      p_S[item] = lS[j];
+      p_c[item] = lc[j];
+    }
+    at += (keep[k] ? 1u : 0u) + (head[k] ? 1u << 16 : 0u);
+  }
+  if (t == 0) {
+    g_start[ng] = ni;
+    P->n_items = ni;
+    P->n_groups = ng;
+  }
+  if (!insert) return;
+  __syncthreads();
+  for (uint32_t gid = t; gid < ng; gid += kMidThreads)
+    classify_insert(gid, p_ul, p_c, g_start, gtype, glev, gw0, gw1, climb, &P->n_climb);
+}
+
+// k_dom_keys, the scans from either side, k_dom_classify, the scan of the merge
+// and task flags, and k_emit
+__global__ void __launch_bounds__(kMidThreads)
+k_mid_emit(const uint64_t *__restrict__ p_ul, const uint32_t *__restrict__ g_start,
+           const uint8_t *__restrict__ gtype, const uint8_t *__restrict__ glev,
+           const uint32_t *__restrict__ gw0, const uint32_t *__restrict__ gw1, EmitArgs e,
+           PlanSummary *__restrict__ P) {
+  pdl_wait();
+  __shared__ uint64_t s_w64[kMidWarps];
+  __shared__ uint64_t s_mirror[kMidThreads];
+  const uint32_t t = threadIdx.x, ng = P->n_groups;
+  uint64_t key[kMidPer], f[kMidPer], r[kMidPer], flags[kMidPer];
+  uint8_t type[kMidPer], lev[kMidPer];
+  uint64_t fmax = 0, rmin = ~0ull;
+#pragma unroll
+  for (int k = 0; k < kMidPer; k++) {
+    const uint32_t gid = kMidPer * t + k;
+    const bool in = gid < ng;
+    key[k] = in ? p_ul[g_start[gid]] : 0ull;
+    type[k] = in ? gtype[gid] : (uint8_t)kNone;
+    lev[k] = in ? glev[gid] : (uint8_t)0;
+    dom_keys(key[k] >> 32, type[k], lev[k], in ? gw0[gid] : 0u, in ? gw1[gid] : 0u, &f[k], &r[k]);
+    fmax = f[k] > fmax ? f[k] : fmax;
+    rmin = r[k] < rmin ? r[k] : rmin;
+  }
+  uint64_t tot64;
+  uint64_t fx = small_scan<kMidWarps>(fmax, (uint64_t)0, OpMax{}, &tot64, s_w64);
+  s_mirror[kMidThreads - 1 - t] = rmin;
+  __syncthreads();
+  const uint64_t rm = small_scan<kMidWarps>(s_mirror[t], ~(uint64_t)0, OpMin{}, &tot64, s_w64);
+  s_mirror[kMidThreads - 1 - t] = rm;
+  __syncthreads();
+  uint64_t rx[kMidPer];
+  rx[kMidPer - 1] = s_mirror[t];
+#pragma unroll
+  for (int k = kMidPer - 1; k > 0; k--) rx[k - 1] = r[k] < rx[k] ? r[k] : rx[k];
+  uint64_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < kMidPer; k++) {
+    flags[k] = dom_flags(key[k], type[k], lev[k], fx, rx[k]);
+    fx = f[k] > fx ? f[k] : fx;
+    sum += flags[k];
+  }
+  uint64_t px = small_scan<kMidWarps>(sum, (uint64_t)0, OpAdd{}, &tot64, s_w64);
+  if (t == 0) {
+    P->n_merge = (uint32_t)tot64;
+    P->n_tasks = (uint32_t)(tot64 >> 32);
+  }
+#pragma unroll
+  for (int k = 0; k < kMidPer; k++) {
+    emit_group(e, kMidPer * t + k, flags[k], px);
+    px += flags[k];
+  }
+}
+
+// the tasks' places in the staging and among the leaves read and written, and
+// k_plan_out
+__global__ void __launch_bounds__(kMidThreads)
+k_mid_out(Tasks t, PlanSummary *P, const unsigned long long *__restrict__ err,
+          PlanSummary *__restrict__ host) {
+  pdl_wait();
+  __shared__ uint64_t s_w64[kMidWarps];
+  const uint32_t n = P->n_tasks;
+  uint64_t el[kMidPer], src[kMidPer], dst[kMidPer], e = 0, s = 0, d = 0;
+#pragma unroll
+  for (int k = 0; k < kMidPer; k++) {
+    const uint32_t i = kMidPer * threadIdx.x + k;
+    e += el[k] = i < n ? t.total[i] : 0;
+    s += src[k] = i < n ? t.nsrc[i] : 0;
+    d += dst[k] = i < n ? t.ndst[i] : 0;
+  }
+  uint64_t te, ts, td;
+  e = small_scan<kMidWarps>(e, (uint64_t)0, OpAdd{}, &te, s_w64);
+  s = small_scan<kMidWarps>(s, (uint64_t)0, OpAdd{}, &ts, s_w64);
+  d = small_scan<kMidWarps>(d, (uint64_t)0, OpAdd{}, &td, s_w64);
+#pragma unroll
+  for (int k = 0; k < kMidPer; k++) {
+    const uint32_t i = kMidPer * threadIdx.x + k;
+    if (i >= n) break;
+    t.out[i] = e;
+    t.soff[i] = s;
+    t.doff[i] = d;
+    e += el[k];
+    s += src[k];
+    d += dst[k];
+  }
+  if (threadIdx.x == 0) {
+    P->task_elems = te;
+    P->src_leaves = ts;
+    P->dst_leaves = td;
+  }
+  __syncthreads();
+  plan_out(P, err, host);
 }
 
 // ------------------------------------------------------------- first load
@@ -2788,7 +2959,8 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
   auto plan = [&](cudaStream_t s, bool fork) -> sst_status {
     // a replayed sequence tags its single-pass scans from the device
     DeviceScanTags tags(replay ? g->d_scan_epoch : nullptr);
-    if (replay) SST_CUDA_TRY(tags.bump(s));
+    const bool mid = b <= kMidBatch && !wt;  // one-block steps: no scans to tag
+    if (replay && !mid) SST_CUDA_TRY(tags.bump(s));
     if (!presorted) {
       uint64_t *out = keys;
       if (wt) {
@@ -2810,19 +2982,26 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
     else
       SST_LAUNCH_PDL_B(16 * b, k_locate, blocks_for(b), kTB, 0, s, sorted, b, dbits, dg,
                    insert, flag, leaf, wt ? wv : nullptr, lS, lc, nkeys);
-    SST_CUDA_TRY((scan<uint32_t, OpAdd>(flag, pos, b, 0u, OpAdd{}, true, false,
-                                        &P->n_items, A, s)));
-    SST_LAUNCH_PDL(k_pack, blocks_for(b), kTB, 0, s, sorted, flag, pos, leaf, b, dbits,
-                   p_ul, p_x, wv, p_w, lS, lc, p_S, p_c);
-    SST_LAUNCH_PDL(k_group_flags, blocks_for(b), kTB, 0, s, p_ul, &P->n_items, b, gflag);
-    SST_CUDA_TRY((scan_epi<uint32_t, OpAdd, GroupStartEpi>(
-        gflag, b, 0u, OpAdd{}, true, false, &P->n_groups, A, s, nullptr,
-        GroupStartEpi{gflag, &P->n_items, b, g_start}, false)));
+    if (mid) {
+      SST_LAUNCH_PDL(k_mid_items, 1, kMidThreads, 0, s, sorted, flag, leaf, lS, lc, (uint32_t)b,
+                     dbits, insert, p_ul, p_x, p_S, p_c, g_start, gtype, glev, gw0, gw1, climb, P);
+    } else {
+      SST_CUDA_TRY((scan<uint32_t, OpAdd>(flag, pos, b, 0u, OpAdd{}, true, false,
+                                          &P->n_items, A, s)));
+      SST_LAUNCH_PDL(k_pack, blocks_for(b), kTB, 0, s, sorted, flag, pos, leaf, b, dbits,
+                     p_ul, p_x, wv, p_w, lS, lc, p_S, p_c);
+      SST_LAUNCH_PDL(k_group_flags, blocks_for(b), kTB, 0, s, p_ul, &P->n_items, b, gflag);
+      SST_CUDA_TRY((scan_epi<uint32_t, OpAdd, GroupStartEpi>(
+          gflag, b, 0u, OpAdd{}, true, false, &P->n_groups, A, s, nullptr,
+          GroupStartEpi{gflag, &P->n_items, b, g_start}, false)));
+    }
     // 6: classify (grids capped: the kernels stride over the device count)
     const unsigned cap_blocks = (unsigned)g->sms * 8;
     const unsigned tgrid = std::min(blocks_for(b), cap_blocks);
     const unsigned wgrid = std::min(warp_blocks(b), cap_blocks);
-    if (insert) {
+    if (insert && mid) {
+      // classified by k_mid_items
+    } else if (insert) {
       SST_LAUNCH_PDL(k_classify_insert, tgrid, kTB, 0, s, p_ul, p_c, g_start,
                  &P->n_groups, gtype, glev, gw0, gw1, climb, &P->n_climb);
     } else {
@@ -2843,6 +3022,19 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
     static_assert(offsetof(PlanSummary, n_tasks) == offsetof(PlanSummary, n_merge) + 4 &&
                       offsetof(PlanSummary, n_merge) % 8 == 0,
                   "n_merge and n_tasks share one aligned 64-bit word");
+    if (mid) {
+      SST_LAUNCH_PDL(k_mid_emit, 1, kMidThreads, 0, s, p_ul, g_start, gtype, glev, gw0, gw1, ea,
+                     P);
+      if (fork && insert) {
+        sst_status st = fork_merges(s);
+        if (st != SST_OK) return st;
+      }
+      SST_LAUNCH_PDL(k_task_setup_hard, wgrid, kTB, 0, s, dg, ea.inv_fill, insert, p_ul, g_start,
+                     gtype, gw0, gw1, task_group, climb, &P->n_hard, &P->n_items, T,
+                     P->class_cnt);
+      SST_LAUNCH_PDL(k_mid_out, 1, kMidThreads, 0, s, T, P, g->d_err, g->h_plan_dev);
+      return SST_OK;
+    }
     SST_LAUNCH_PDL(k_dom_keys, blocks_for(b), kTB, 0, s, p_ul, g_start, gtype, glev,
                    gw0, gw1, &P->n_groups, b, fkey, bkey);
     // the scans run out of place into merge_jk and mtpos, which hold
