@@ -73,15 +73,28 @@ sst_status graph_copy_into(sst_graph *dst, sst_graph *src) {
 // Three passes over work items:
 //  1. leaf items (query, leaf of N(u)); each item and lane is a pair slot
 //     holding the neighbour w in that slot of the leaf (or nothing);
-//  2. each pair's cost: the shorter of N(u) and N(w), in chunks of 32
-//     leaves;
-//  3. a warp per chunk: lanes take the chunk's leaves of the shorter list one
+//  2. each pair's cost: the shorter of N(u) and N(w), in chunks of leaves;
+//  3. eight lanes per chunk: they take the chunk's leaves of the shorter list one
 //     at a time and probe each id in the longer list (binary search over its
 //     leaf heads, then within the leaf).
-// A pair of two long lists spreads over as many warps as the shorter one has
-// 32-leaf chunks, so no warp walks a long list alone.
+// A pair of two long lists spreads over as many lane groups as the shorter one
+// has chunks, so none walks a long list alone.
 namespace {
-constexpr uint32_t kTcvChunkLeaves = 32;
+// Leaves a chunk, by the pair slots of the call.  A few queries, whose chunks are
+// all in flight at once, end when the longest chunk does (2 to 3 us a leaf of
+// dependent probes); many have chunks to spare and pay for each one's search among
+// the pairs.  The sum of the chunks has to stay below 2^32: 2^22 slots would need
+// as many lists of 8192 leaves to pass it in chunks of 8, more than fits the
+// device, and beyond that the chunks are long.  Pass 3 at RMAT scale 18 (us, by
+// leaves a chunk; last, a warp a chunk of 32):
+//   vertices    1     2     4     8    32    warp
+//   100        17    23    34    51    81     42
+//   1,000      62    56    57    72   141     91
+//   10,000    650   526   483   508   668    699
+//   100,000  5255  4184  3722  3724  4653   5366
+inline uint32_t tcv_chunk_leaves(uint64_t nslots) {
+  return nslots <= 1 << 17 ? 2 : nslots <= 1 << 20 ? 4 : nslots <= 1 << 22 ? 8 : 32;
+}
 
 __device__ __forceinline__ uint32_t leaves_of(uint32_t cap) {
   return cap == 0 ? 0 : (cap <= kLeaf ? 1 : cap >> kLeafLog);
@@ -100,8 +113,8 @@ __global__ void k_tcv_leaves(DGraph g, const uint32_t *__restrict__ vs,
 // pass 2: warp per leaf item; lane = pair slot
 __global__ void k_tcv_pairs(DGraph g, const uint32_t *__restrict__ vs, uint64_t k,
                             const uint64_t *__restrict__ loff, uint64_t items,
-                            uint32_t *__restrict__ pq, uint32_t *__restrict__ pw,
-                            uint32_t *__restrict__ cost) {
+                            uint32_t chunk, uint32_t *__restrict__ pq,
+                            uint32_t *__restrict__ pw, uint32_t *__restrict__ cost) {
   const int lane = threadIdx.x & 31;
   const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t wi = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -122,7 +135,7 @@ __global__ void k_tcv_pairs(DGraph g, const uint32_t *__restrict__ vs, uint64_t 
     uint32_t chunks = 0;
     if (w != kEmpty) {
       const uint32_t s = deg <= g.deg[w] ? u : w;  // the shorter list
-      chunks = (leaves_of(g.cap[s]) + kTcvChunkLeaves - 1) / kTcvChunkLeaves;
+      chunks = (leaves_of(g.cap[s]) + chunk - 1) / chunk;
     }
     pw[wi * 32 + lane] = w;
     cost[wi * 32 + lane] = chunks;
@@ -130,40 +143,64 @@ __global__ void k_tcv_pairs(DGraph g, const uint32_t *__restrict__ vs, uint64_t 
   }
 }
 
-// pass 3: warp per chunk of a pair
-__global__ void k_tcv_count(DGraph g, const uint32_t *__restrict__ vs,
-                            const uint32_t *__restrict__ pq,
-                            const uint32_t *__restrict__ pw,
-                            const uint32_t *__restrict__ coff, uint64_t nslots,
-                            uint64_t nchunks, unsigned long long *__restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t ci = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-       ci < nchunks; ci += warps) {
+// pass 3: eight lanes a chunk of a pair.  Most leaves hold far fewer than 32 ids
+// and a chunk is a chain of dependent loads, so four chunks share a warp, and a
+// lane searches for its up to four ids of a leaf together (the longer list is the
+// same, so the searches take the same steps).
+__global__ void __launch_bounds__(256)
+k_tcv_count(DGraph g, const uint32_t *__restrict__ vs, const uint32_t *__restrict__ pq,
+            const uint32_t *__restrict__ pw, const uint32_t *__restrict__ coff, uint64_t nslots,
+            uint64_t nchunks, uint32_t chunk, unsigned long long *__restrict__ out) {
+  const uint32_t sub = threadIdx.x & 7;
+  const int shift = threadIdx.x & 24;
+  const uint32_t group = 0xffu << shift;
+  const uint64_t groups = ((uint64_t)gridDim.x * blockDim.x) >> 3;
+  for (uint64_t ci = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; ci < nchunks;
+       ci += groups) {
     // pair slot p: the last with coff[p] <= ci (slots of cost 0 share their
     // offset with the next slot, so the last one is the pair that owns ci)
+    // (the lanes probe eight offsets a step)
     uint64_t lo = 0, hi = nslots;
     while (hi - lo > 1) {
-      const uint64_t mid = (lo + hi) >> 1;
-      if (coff[mid] <= ci) lo = mid; else hi = mid;
+      const uint64_t step = (hi - lo + 7) >> 3, at = lo + step * sub;
+      const uint32_t le = __ballot_sync(group, at < hi && coff[at] <= ci) >> shift & 0xff;
+      lo += step * (31 - __clz(le));  // lane 0's offset is not above ci
+      hi = min(hi, lo + step);
     }
     const uint32_t q = pq[lo >> 5], w = pw[lo], u = vs[q];
     const uint32_t j = (uint32_t)(ci - coff[lo]);  // chunk of the pair
     const uint32_t s = g.deg[u] <= g.deg[w] ? u : w, o = s == u ? w : u;
-    const uint64_t sbase = g.base[s], obase = g.base[o];
-    const uint32_t scap = g.cap[s], sdeg = g.deg[s];
-    const uint32_t ocap = g.cap[o];
-    const uint32_t l0 = j * kTcvChunkLeaves;
-    const uint32_t l1 = min(l0 + kTcvChunkLeaves, leaves_of(scap));
+    const uint32_t *sl = g.slots + g.base[s], *ol = g.slots + g.base[o];
+    const uint32_t scap = g.cap[s], ocap = g.cap[o];
+    const uint32_t l1 = min((j + 1) * chunk, leaves_of(scap));
+    const uint32_t own = scap < kLeaf ? scap : kLeaf, other = ocap < kLeaf ? ocap : kLeaf;
     uint32_t hits = 0;
-    for (uint32_t l = l0; l < l1; l++) {
-      const uint32_t c = leaf_count(g, sbase, scap, sdeg, l);
-      if ((uint32_t)lane < c)
-        hits += seg_has(g.slots, obase, ocap, g.slots[sbase + ((uint64_t)l << kLeafLog) + lane]);
+    for (uint32_t l = j * chunk; l < l1; l++) {
+      uint32_t x[4];
+      uint64_t at[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const uint32_t p = sub + 8 * r;
+        x[r] = p < own ? sl[((uint64_t)l << kLeafLog) + p] : kEmpty;  // kEmpty past the ids
+        at[r] = 0;
+      }
+      // the last leaf whose head is not above x, then the last such slot of it
+      for (uint32_t n = leaves_of(ocap) >> 1; n; n >>= 1)
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const uint64_t to = at[r] + ((uint64_t)n << kLeafLog);
+          if (x[r] != kEmpty && ol[to] <= x[r]) at[r] = to;
+        }
+      for (uint32_t n = other >> 1; n; n >>= 1)
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          if (x[r] != kEmpty && ol[at[r] + n] <= x[r]) at[r] += n;
+#pragma unroll
+      for (int r = 0; r < 4; r++) hits += x[r] != kEmpty && ol[at[r]] == x[r];
     }
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, d);
-    if (lane == 0 && hits) atomicAdd(&out[q], (unsigned long long)hits);
+    for (int d = 4; d > 0; d >>= 1) hits += __shfl_xor_sync(group, hits, d);
+    if (sub == 0 && hits) atomicAdd(&out[q], (unsigned long long)hits);
   }
 }
 
@@ -199,6 +236,7 @@ sst_status tc_vertices(sst_graph *g, const uint32_t *d_vs, uint64_t k,
   // pass 2: pair slots and their chunk counts
   uint32_t *pq = nullptr, *pw = nullptr, *cost = nullptr, *coff = nullptr;
   const uint64_t nslots = items * 32;
+  const uint32_t chunk = tcv_chunk_leaves(nslots);
   uint32_t nchunks = 0;
   if (e == cudaSuccess && items) {
     e = cudaMallocAsync(&pq, items * 4, s);
@@ -213,7 +251,7 @@ sst_status tc_vertices(sst_graph *g, const uint32_t *d_vs, uint64_t k,
     if (e == cudaSuccess && !ctot) e = cudaErrorMemoryAllocation;
     if (e == cudaSuccess) {
       SST_LAUNCH(k_tcv_pairs, (unsigned)std::min<uint64_t>((items * 32 + tb - 1) / tb, cap_blocks),
-                 tb, 0, s, g->view(), d_vs, k, loff, items, pq, pw, cost);
+                 tb, 0, s, g->view(), d_vs, k, loff, items, chunk, pq, pw, cost);
       e = scan<uint32_t, OpAdd>(cost, coff, nslots, 0u, OpAdd{}, true, false, ctot,
                                 g->arena, s);
     }
@@ -222,8 +260,8 @@ sst_status tc_vertices(sst_graph *g, const uint32_t *d_vs, uint64_t k,
     // pass 3
     if (e == cudaSuccess && nchunks) {
       SST_LAUNCH(k_tcv_count,
-                 (unsigned)std::min<uint64_t>(((uint64_t)nchunks * 32 + tb - 1) / tb, cap_blocks),
-                 tb, 0, s, g->view(), d_vs, pq, pw, coff, nslots, nchunks, out);
+                 (unsigned)std::min<uint64_t>(((uint64_t)nchunks * 8 + tb - 1) / tb, cap_blocks),
+                 tb, 0, s, g->view(), d_vs, pq, pw, coff, nslots, nchunks, chunk, out);
       SST_LAUNCH(k_tcv_half, (unsigned)((k + tb - 1) / tb), tb, 0, s, out, k);
       e = cudaGetLastError();
     }
