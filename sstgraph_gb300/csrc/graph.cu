@@ -158,87 +158,62 @@ __global__ void k_make_keys(const uint32_t *__restrict__ pairs, uint64_t b,
                                             : (((uint64_t)r << dbits) | c);
 }
 
-// k_make_keys_packed: only the kept keys, packed to the front in any order
-// (*nkeys of them; one reservation per block of kPackItems x 256 pairs).
-// Equal keys are equal, so their order does not matter (unweighted
-// graphs), and the sort needs no bit for the sentinel row.  With V2 (the
-// pairs 8-byte aligned) a pair comes in with one 8-byte load: the warp's
+// k_make_keys_packed (unweighted graphs, where equal keys need no order): a
+// dropped pair takes the key `sent`, on a graph without self-loops that of (0, 0),
+// which no kept pair has, so the sort needs no bit for a row n.  (Packing only the
+// kept keys to the front cost an atomic on one counter for every 2048 pairs, one
+// after another: 39 us for 4.8M pairs, 30 now; 15.4 for 1M, 10.6.)  With V2
+// (the pairs 8-byte aligned) a pair comes in with one 8-byte load: the warp's
 // load covers 256 contiguous bytes once, where two 4-byte loads a pair read
 // each line twice (pinned host pairs are read across the host link).
 // With sd.passes > 0 it also counts every radix pass's 8-bit digits of the
-// keys it keeps into sd.totals (zero on entry) and clears the sort's tile
+// keys into sd.totals (zero on entry) and clears the sort's tile
 // status words (SortDigits): the sort then skips its own counting read.
 constexpr int kPackItems = 8;
 template <bool V2>
 __global__ void __launch_bounds__(256)
 k_make_keys_packed(const uint32_t *__restrict__ pairs, uint64_t b, uint32_t n,
-                   uint32_t width, int dbits, bool drop_loops,
+                   uint32_t width, int dbits, bool drop_loops, uint64_t sent,
                    uint64_t *__restrict__ keys,
                    unsigned long long *__restrict__ invalid,
                    uint32_t *__restrict__ nkeys, SortDigits sd) {
   pdl_wait();
-  __shared__ uint32_t s_warp[8];
-  __shared__ uint32_t s_base;
   __shared__ uint32_t s_hist[8][256];
   for (int p = 0; p < sd.passes; p++) s_hist[p][threadIdx.x] = 0;
-  const uint64_t t0 = (uint64_t)blockIdx.x * (256 * kPackItems);
-  uint64_t key[kPackItems];
-  uint32_t kept = 0, bad = 0;  // bit k: item k is kept
+  __syncthreads();
+  const uint64_t t0 = (uint64_t)blockIdx.x * (256 * kPackItems) + threadIdx.x;
+  uint32_t r[kPackItems], c[kPackItems], bad = 0;
 #pragma unroll
   for (int k = 0; k < kPackItems; k++) {
-    const uint64_t i = t0 + (uint64_t)k * 256 + threadIdx.x;
-    uint32_t r = 0, c = 0;
-    if (i < b) {
-      if (V2) {
-        const uint2 rc = reinterpret_cast<const uint2 *>(pairs)[i];
-        r = rc.x;
-        c = rc.y;
-      } else {
-        r = pairs[2 * i];
-        c = pairs[2 * i + 1];
-      }
+    const uint64_t i = t0 + k * 256;
+    r[k] = c[k] = 0;
+    if (i >= b) continue;
+    if (V2) {
+      const uint2 rc = reinterpret_cast<const uint2 *>(pairs)[i];
+      r[k] = rc.x;
+      c[k] = rc.y;
+    } else {
+      r[k] = pairs[2 * i];
+      c[k] = pairs[2 * i + 1];
     }
-    const bool ok = i < b && r < n && c < width && c != kEmpty;
-    bad += i < b && !ok;
-    if (ok && !(drop_loops && r == c)) kept |= 1u << k;
-    key[k] = ((uint64_t)r << dbits) | c;
   }
-  const uint32_t keep = __popc(kept);
+#pragma unroll
+  for (int k = 0; k < kPackItems; k++) {
+    if (t0 + k * 256 >= b) break;
+    const bool ok = r[k] < n && c[k] < width && c[k] != kEmpty;
+    bad += !ok;
+    const uint64_t key =
+        !ok || (drop_loops && r[k] == c[k]) ? sent : ((uint64_t)r[k] << dbits) | c[k];
+    keys[t0 + k * 256] = key;
+    for (int p = 0; p < sd.passes; p++) atomicAdd(&s_hist[p][(key >> (8 * p)) & 0xff], 1u);
+  }
   if (bad) atomicAdd(invalid, (unsigned long long)bad);
-  // block prefix of the kept counts, one reservation for the block
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t inc = keep;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t o = __shfl_up_sync(0xffffffffu, inc, d);
-    if (lane >= d) inc += o;
-  }
-  if (lane == 31) s_warp[warp] = inc;
+  if (t0 == 0) *nkeys = (uint32_t)b;
+  if (!sd.passes) return;
+  for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < sd.status_words;
+       i += (uint64_t)gridDim.x * 256)
+    sd.status[i] = 0;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t tot = 0;
-    for (int w = 0; w < 8; w++) {
-      const uint32_t c = s_warp[w];
-      s_warp[w] = tot;
-      tot += c;
-    }
-    s_base = tot ? atomicAdd(nkeys, tot) : 0u;
-  }
-  if (sd.passes) {
-#pragma unroll
-    for (int k = 0; k < kPackItems; k++)
-      if ((kept >> k) & 1u)
-        for (int p = 0; p < sd.passes; p++)
-          atomicAdd(&s_hist[p][(key[k] >> (8 * p)) & 0xff], 1u);
-    for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < sd.status_words;
-         i += (uint64_t)gridDim.x * 256)
-      sd.status[i] = 0;
-  }
-  __syncthreads();
-  const uint64_t at = (uint64_t)s_base + s_warp[warp] + inc - keep;
-#pragma unroll
-  for (int k = 0; k < kPackItems; k++)
-    if ((kept >> k) & 1u) keys[at + __popc(kept & ((1u << k) - 1u))] = key[k];
   for (int p = 0; p < sd.passes; p++)
     if (s_hist[p][threadIdx.x]) atomicAdd(&sd.totals[p * 256 + threadIdx.x], s_hist[p][threadIdx.x]);
 }
@@ -253,15 +228,14 @@ __global__ void k_locate(const uint64_t *__restrict__ keys, uint64_t b,
                          uint32_t *__restrict__ leaf_out,
                          const uint32_t *__restrict__ wv,
                          uint64_t *__restrict__ lS, uint32_t *__restrict__ lc,
-                         const uint32_t *__restrict__ nkeys) {
+                         uint64_t sent, const uint32_t *__restrict__ nkeys) {
   pdl_wait();
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= b) return;
-  const uint64_t sent = (uint64_t)g.n << dbits;
-  // a compacting key build leaves nkeys sorted keys and nothing after them
+  // a replayed sequence is sized by more keys than the batch has
   const uint64_t nk = nkeys ? *nkeys : b;
   uint64_t k = i < nk ? keys[i] : sent;
-  if (k >= sent || (i + 1 < nk && keys[i + 1] == k)) {
+  if (k == sent || (i + 1 < nk && keys[i + 1] == k)) {
     flag[i] = 0;
     leaf_out[i] = 0;
     return;
@@ -342,15 +316,14 @@ __global__ void k_locate_warp(const uint64_t *__restrict__ keys, uint64_t b,
                               uint32_t *__restrict__ leaf_out,
                               const uint32_t *__restrict__ wv,
                               uint64_t *__restrict__ lS, uint32_t *__restrict__ lc,
-                              const uint32_t *__restrict__ nkeys) {
+                              uint64_t sent, const uint32_t *__restrict__ nkeys) {
   pdl_wait();
   const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (i >= b) return;  // whole warps
-  const uint64_t sent = (uint64_t)g.n << dbits;
   const uint64_t nk = nkeys ? *nkeys : b;
   const uint64_t k = i < nk ? keys[i] : sent;
-  if (k >= sent || (i + 1 < nk && keys[i + 1] == k)) {
+  if (k == sent || (i + 1 < nk && keys[i + 1] == k)) {
     if (lane == 0) {
       flag[i] = 0;
       leaf_out[i] = 0;
@@ -1953,7 +1926,7 @@ struct LoadTile {
            (threadIdx.x & 31);
   }
   __device__ __forceinline__ void load(const uint64_t *__restrict__ keys, uint64_t nk,
-                                       uint32_t *s_warp) {
+                                       uint64_t sent, uint32_t *s_warp) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < kLoadRows; k++) {
@@ -1967,7 +1940,7 @@ struct LoadTile {
     for (int k = 0; k < kLoadRows; k++) {
       const uint64_t up = __shfl_up_sync(0xffffffffu, key[k], 1);
       if (lane) prev[k] = up;
-      const bool f = index(k) < nk && prev[k] != key[k];  // no key is ~0
+      const bool f = index(k) < nk && key[k] != sent && prev[k] != key[k];  // no key is ~0
       const uint32_t v = __ballot_sync(0xffffffffu, f);
       rank[k] = run + __popc(v & ((1u << lane) - 1u));
       run += __popc(v);
@@ -1989,35 +1962,35 @@ struct LoadTile {
 
 __global__ void __launch_bounds__(kLoadTB)
 k_load_count(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ nkeys,
-             uint32_t *__restrict__ tiles) {
+             uint64_t sent, uint32_t *__restrict__ tiles) {
   pdl_wait();
   __shared__ uint32_t s_warp[kLoadTB / 32];
   LoadTile t;
-  t.load(keys, *nkeys, s_warp);
+  t.load(keys, *nkeys, sent, s_warp);
   if (threadIdx.x == 0) tiles[blockIdx.x] = t.total;
 }
 
 // Each row's range of ranks (rows without a key keep the 0 they were cleared to).
 __global__ void __launch_bounds__(kLoadTB)
 k_load_bounds(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ nkeys, int dbits,
-              const uint32_t *__restrict__ tiles, uint32_t *__restrict__ beg,
+              uint64_t sent, uint32_t n, const uint32_t *__restrict__ tiles, uint32_t *__restrict__ beg,
               uint32_t *__restrict__ end) {
   pdl_wait();
   __shared__ uint32_t s_warp[kLoadTB / 32];
   LoadTile t;
   const uint64_t nk = *nkeys;
-  t.load(keys, nk, s_warp);
+  t.load(keys, nk, sent, s_warp);
   const uint32_t at = tiles[blockIdx.x];
 #pragma unroll
   for (int k = 0; k < kLoadRows; k++) {
-    // a row's first key is always kept, and it ends the row before
+    // a row's first key ends the row before (dropped pairs may form a row n)
     const uint64_t i = LoadTile::index(k), u = t.key[k] >> dbits;
     if (i >= nk) break;
     if (i == 0 || (t.prev[k] >> dbits) != u) {
-      beg[u] = at + t.rank[k];
+      if (u < n) beg[u] = at + t.rank[k];
       if (i) end[t.prev[k] >> dbits] = at + t.rank[k];
     }
-    if (i + 1 == nk) end[u] = at + t.rank[k] + ((t.kept >> k) & 1u);
+    if (i + 1 == nk && u < n) end[u] = at + t.rank[k] + ((t.kept >> k) & 1u);
   }
 }
 
@@ -2055,13 +2028,13 @@ k_load_rows(const uint32_t *__restrict__ beg, const uint32_t *__restrict__ end, 
 // first key its count.
 __global__ void __launch_bounds__(kLoadTB)
 k_load_place(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ nkeys, int dbits,
-             const uint32_t *__restrict__ tiles, const uint32_t *__restrict__ beg,
+             uint64_t sent, const uint32_t *__restrict__ tiles, const uint32_t *__restrict__ beg,
              const uint32_t *__restrict__ end, const uint32_t *__restrict__ rank,
              uint64_t inv_fill, const ClassStarts cs, DGraph g) {
   pdl_wait();
   __shared__ uint32_t s_warp[kLoadTB / 32];
   LoadTile t;
-  t.load(keys, *nkeys, s_warp);
+  t.load(keys, *nkeys, sent, s_warp);
   const uint32_t tile = tiles[blockIdx.x];
 #pragma unroll
   for (int k = 0; k < kLoadRows; k++) {
@@ -2616,14 +2589,31 @@ static ClassStarts plan_class_starts(sst_graph *g, const PlanSummary &ps) {
   return cs;
 }
 
+// The key of a dropped pair, one that no kept pair has: on a graph that keeps no
+// self-loops that of (0, 0), else of the highest column if that is out of range,
+// else of a row n (a bit more if the rows too are a power of two).
+static uint64_t free_column(const sst_graph *g) {
+  const uint64_t c = (1ull << g->dbits) - 1;
+  return c == kEmpty || g->width <= c ? c : 0;
+}
+static uint64_t dropped_key(const sst_graph *g) {
+  if (!g->keep_loops) return 0;
+  const uint64_t c = free_column(g);
+  return c ? c : (uint64_t)g->n << g->dbits;
+}
+static int key_bits(const sst_graph *g) {
+  const bool row = g->keep_loops && !free_column(g);
+  return (row ? g->rbits : bits_for(g->n ? g->n - 1 : 0)) + g->dbits;
+}
+
 static void launch_packed_keys(const sst_graph *g, const uint32_t *d_pairs, uint64_t npairs,
-                               bool drop_loops, uint64_t *keys, const SortDigits &sdig,
+                               bool insert, uint64_t *keys, const SortDigits &sdig,
                                cudaStream_t s) {
   PlanSummary *P = g->d_plan;
   auto launch = [&](auto *kernel) {
     SST_LAUNCH_PDL_NB("k_make_keys_packed", 16 * npairs, kernel,
                       blocks_for(npairs, kTB * kPackItems), kTB, 0, s, d_pairs, npairs, g->n,
-                      g->width, g->dbits, drop_loops, keys,
+                      g->width, g->dbits, insert && !g->keep_loops, dropped_key(g), keys,
                       reinterpret_cast<unsigned long long *>(&P->invalid), &P->n_keys, sdig);
   };
   if ((reinterpret_cast<uintptr_t>(d_pairs) & 7) == 0)
@@ -2765,22 +2755,24 @@ static sst_status run_load(sst_graph *g, const uint32_t *d_pairs, uint64_t b,
     set_error_message("update scratch sizing error");
     return SST_ENOMEM;
   }
-  const int dbits = g->dbits, bits = bits_for(n - 1) + dbits;
+  const int dbits = g->dbits, bits = key_bits(g);
+  const uint64_t sent = dropped_key(g);
   SortDigits sdig;
   if (radix_sort_digits(b, bits, A, &sdig))
     SST_CUDA_TRY(cudaMemsetAsync(sdig.totals, 0, (size_t)sdig.passes * 256 * 4, s));
   else
     sdig = SortDigits{};
   SST_CUDA_TRY(cudaMemsetAsync(beg, 0, n * 8, s));
-  launch_packed_keys(g, d_pairs, b, !g->keep_loops, keys, sdig, s);
+  launch_packed_keys(g, d_pairs, b, true, keys, sdig, s);
   uint64_t *sorted = keys;
   SST_CUDA_TRY(radix_sort_u64(keys, ktmp, b, bits, A, s, &sorted, &P->n_keys,
                               sdig.passes ? &sdig : nullptr));
-  SST_LAUNCH_PDL_B(8 * b, k_load_count, (unsigned)ntiles, kLoadTB, 0, s, sorted, &P->n_keys, tcnt);
+  SST_LAUNCH_PDL_B(8 * b, k_load_count, (unsigned)ntiles, kLoadTB, 0, s, sorted, &P->n_keys, sent,
+                   tcnt);
   SST_CUDA_TRY((scan<uint32_t, OpAdd>(tcnt, tiles, ntiles, 0u, OpAdd{}, true, false, &P->n_items,
                                       A, s)));
   SST_LAUNCH_PDL_B(8 * b, k_load_bounds, (unsigned)ntiles, kLoadTB, 0, s, sorted, &P->n_keys,
-                   dbits, tiles, beg, end);
+                   dbits, sent, (uint32_t)n, tiles, beg, end);
   const uint64_t inv_fill = fill_inv_q24(g->params.grow_fill);
   SST_LAUNCH_PDL(k_load_rows, std::min(blocks_for(n, kLoadThreads), 2u * g->sms), kLoadThreads,
                  0, s, beg, end, (uint32_t)n, inv_fill, rank, P->class_cnt);
@@ -2810,7 +2802,7 @@ static sst_status run_load(sst_graph *g, const uint32_t *d_pairs, uint64_t b,
   SST_CUDA_TRY(cudaMemsetAsync(g->d_slots, 0xFF, g->bump * 4, s));
   SST_CUDA_TRY(cudaMemsetAsync(g->d_lcnt, 0, g->bump / kLeaf, s));
   SST_LAUNCH_PDL_B(12 * b, k_load_place, (unsigned)ntiles, kLoadTB, 0, s, sorted, &P->n_keys,
-                   dbits, tiles, beg, end, rank, inv_fill, cs, g->view());
+                   dbits, sent, tiles, beg, end, rank, inv_fill, cs, g->view());
   SST_CUDA_TRY(cudaGetLastError());
   g->m += ps.n_items;
   g->version++;
@@ -2886,12 +2878,12 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
   // 1: keys
   const uint64_t *sorted = presorted;
   uint32_t *nkeys = nullptr;
-  const int sort_bits = bits_for(g->n ? g->n - 1 : 0) + dbits;  // unweighted keys
+  const int sort_bits = key_bits(g);  // unweighted keys
+  // the key of a dropped pair (none among presorted ones)
+  const uint64_t sent = presorted ? ~0ull : wt ? (uint64_t)g->n << dbits : dropped_key(g);
   SortDigits sdig;
   if (!presorted) {
     // pair in (8 B), key out (8 B)
-    // unweighted keys are compacted (see k_make_keys): their rows are below
-    // n, one bit fewer to sort when n is a power of two
     nkeys = wt ? nullptr : &P->n_keys;
     if (wt)
       SST_LAUNCH_PDL_B(16 * b, k_make_keys, blocks_for(b), kTB, 0, s, d_pairs, b, g->n,
@@ -2905,7 +2897,7 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
       } else {
         sdig = SortDigits{};
       }
-      launch_packed_keys(g, d_pairs, npairs, insert && !g->keep_loops, keys, sdig, s);
+      launch_packed_keys(g, d_pairs, npairs, insert, keys, sdig, s);
     }
   }
   MergeJoin join{s, nullptr};
@@ -2978,10 +2970,10 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
     // sorted key in (8 B), flag and leaf out (8 B)
     if (b <= kLocateWarpKeys)
       SST_LAUNCH_PDL_B(16 * b, k_locate_warp, warp_blocks(b), kTB, 0, s, sorted, b, dbits, dg,
-                   insert, flag, leaf, wt ? wv : nullptr, lS, lc, nkeys);
+                   insert, flag, leaf, wt ? wv : nullptr, lS, lc, sent, nkeys);
     else
       SST_LAUNCH_PDL_B(16 * b, k_locate, blocks_for(b), kTB, 0, s, sorted, b, dbits, dg,
-                   insert, flag, leaf, wt ? wv : nullptr, lS, lc, nkeys);
+                   insert, flag, leaf, wt ? wv : nullptr, lS, lc, sent, nkeys);
     if (mid) {
       SST_LAUNCH_PDL(k_mid_items, 1, kMidThreads, 0, s, sorted, flag, leaf, lS, lc, (uint32_t)b,
                      dbits, insert, p_ul, p_x, p_S, p_c, g_start, gtype, glev, gw0, gw1, climb, P);
@@ -3324,10 +3316,8 @@ sst_status update_batches(sst_graph *g, const uint32_t *d_pairs,
   }
   cudaStream_t s = g->stream;
   const int dbits = g->dbits;
-  // A dropped pair's id: on a graph that keeps no self-loops that of (0, 0), else
-  // of a row n, which takes a bit more when n is a power of two.
-  const uint64_t sent = g->keep_loops ? (uint64_t)g->n << dbits : 0;
-  const int bits = (g->keep_loops ? g->rbits : bits_for(g->n ? g->n - 1 : 0)) + dbits;
+  const uint64_t sent = dropped_key(g);
+  const int bits = key_bits(g);
   const int lo = bits < 64 ? 1 : 0;  // the operation in the key, see k_make_keys_batched
   const uint64_t ntiles = (N + kLoadTile - 1) / kLoadTile;
   const size_t need = N * (lo ? 16 : 24) + ntiles * 16 + radix_sort_scratch_bytes(N) +

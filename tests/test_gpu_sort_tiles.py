@@ -62,11 +62,13 @@ def test_keys_with_values(sg, b):
     g.close()
 
 
+@pytest.mark.parametrize("one_by_one", [False, True])
+@pytest.mark.parametrize("n", [1 << 10, 1000])
 @pytest.mark.parametrize("loops", [False, True])
-def test_batches_with_dropped_pairs(sg, loops):
-    """Self-loops (of row 0 too), ids out of range and edges given many times;
-    n a power of two, so a row n would take one more bit."""
-    n, b = 1 << 10, 20000
+def test_dropped_pairs(sg, loops, n, one_by_one):
+    """Self-loops (of row 0 too), ids out of range and edges given many times,
+    on rows and columns that fill their bits and that do not."""
+    b = 20000
     rng = np.random.default_rng(1)
     es = [rng.integers(0, n, (b, 2)).astype(np.uint32) for _ in range(5)]
     for e in es:
@@ -76,7 +78,12 @@ def test_batches_with_dropped_pairs(sg, loops):
         e[3::9] = (0, 1)
     ops = [1, 0, 1, 0, 1]
     g = sg.SparseMatrixV(n, keep_self_loops=loops)
-    assert g.update_batches(es, ops) == sum(int((e.max(1) >= n).sum()) for e in es)
+    bad = sum(int((e.max(1) >= n).sum()) for e in es)
+    if one_by_one:
+        assert sum((g.insert_batch if op else g.remove_batch)(e)
+                   for e, op in zip(es, ops)) == bad
+    else:
+        assert g.update_batches(es, ops) == bad
     have = np.zeros(n * n, bool)
     for e, op in zip(es, ops):
         e = e[e.max(1) < n].astype(np.int64)
