@@ -1913,7 +1913,7 @@ k_mid_out(Tasks t, PlanSummary *P, const unsigned long long *__restrict__ err,
 // each key its rank in its run, and the block adds up the runs before it.
 // Computed twice (k_load_bounds, k_load_place) rather than stored: a key is read
 // in 8 bytes, and a stored flag and rank would cost 16 more.
-constexpr int kLoadTB = 256, kLoadRows = 8;
+constexpr int kLoadTB = 256, kLoadRows = 4;
 constexpr int kLoadTile = kLoadTB * kLoadRows;
 struct LoadTile {
   uint64_t key[kLoadRows];
@@ -1985,7 +1985,7 @@ k_load_bounds(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ nk
   for (int k = 0; k < kLoadRows; k++) {
     // a row's first key ends the row before (dropped pairs may form a row n)
     const uint64_t i = LoadTile::index(k), u = t.key[k] >> dbits;
-    if (i >= nk) break;
+    if (i >= nk) continue;
     if (i == 0 || (t.prev[k] >> dbits) != u) {
       if (u < n) beg[u] = at + t.rank[k];
       if (i) end[t.prev[k] >> dbits] = at + t.rank[k];
