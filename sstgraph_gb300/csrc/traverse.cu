@@ -719,12 +719,13 @@ __global__ void k_front_expand(const uint32_t *__restrict__ q, uint32_t qn,
 // without a loop.  Linking every vertex to its first two neighbours by find
 // and compare-and-swap (the form before) had 2e6 threads chase and extend
 // chains of fresh roots: 385 us a neighbour on a uniform graph of 2e6 vertices
-// and 14e6 stored edges, where all of the rounds below take 175 us together.  They
+// and 14e6 stored edges, where a whole call takes 172 us now.  The rounds
 // are bound by scattered 32-byte sectors: a row's first ids (read once, here),
 // and two parents a vertex and round.
 // The start: every vertex below its smallest neighbour (rows ascend), if that
 // is smaller.  A parent is smaller than its child, so the links are a forest.
-// nb keeps the next two neighbours (kEmpty: none) for the rounds.
+// nb1 and nb2 keep what is left of its first two neighbours' edges for the rounds
+// (kEmpty: none): the second, and the smallest if it is larger than u.
 __global__ void k_cc_hook_first(DGraph g, uint32_t *__restrict__ par,
                                 uint32_t *__restrict__ nb1, uint32_t *__restrict__ nb2) {
   pdl_wait();
@@ -741,29 +742,29 @@ __global__ void k_cc_hook_first(DGraph g, uint32_t *__restrict__ par,
   }
   par[u] = min(u, x.x);
   nb1[u] = x.y;
-  nb2[u] = x.z;
+  nb2[u] = x.x > u ? x.x : kEmpty;
 }
 
 // A round, after a compression: of the roots of u and its two kept neighbours
 // the larger ones go below the smallest.  A root keeps the smallest that any
 // vertex offers it, and a parent that is read while it changes is an ancestor:
 // either way a tree only moves below a vertex of its own component with a
-// smaller id.  A hook that another one replaces is linked later: phase 3 takes
-// every edge of every vertex outside the largest component.
+// smaller id.  A hook that another one replaces is linked later, by
+// k_cc_link_kept.
 // The first round, of every vertex, leaves 5e3 trees on that uniform graph.
 // Their roots would get hundreds of offers each, and atomics on one address
 // wait for each other (25 ns apiece: a second round of every vertex takes 240
 // us, of every 8th 74 us).  So on a large graph the second round takes every
-// 32nd vertex, the third every 512th, which joins the two or three trees that
-// then hold most vertices, and the last every vertex: 0.1% are outside the
-// largest tree after it (4% at average degree 2.4).  Below kCcSampledN there
-// are too few vertices for that, and launches cost more than the atomics.
-// When the second round finds nothing to hook the later ones return at once.
+// 32nd vertex and the third every 512th, which joins the two or three trees that
+// then hold most vertices and leaves few edges to k_cc_link_kept.  Below
+// kCcSampledN there are too few vertices for that, and launches cost more than
+// the atomics.  When the second round finds nothing to hook the third returns at
+// once.
 // The parents come through L1: nearly all are one hot root, whose loads would
 // queue at one L2 slice, and a stale one is an ancestor too.
 constexpr uint32_t kCcSampledN = 1u << 17;
-constexpr int kCcMaxRounds = 4;
-constexpr uint32_t kCcStride[2][kCcMaxRounds] = {{1, 1, 0, 0}, {1, 32, 512, 1}};
+constexpr int kCcMaxRounds = 3;
+constexpr uint32_t kCcStride[2][kCcMaxRounds] = {{1, 0, 0}, {1, 32, 512}};
 __global__ void k_cc_hook(const uint32_t *__restrict__ nb1, const uint32_t *__restrict__ nb2,
                           uint32_t n, uint32_t stride, uint32_t *par,
                           const unsigned long long *__restrict__ before,
@@ -784,6 +785,25 @@ __global__ void k_cc_hook(const uint32_t *__restrict__ nb1, const uint32_t *__re
     if (c > m && ld_par(par, c) > m) hooked |= atomicMin(&par[c], m) > m;
   }
   if (__syncthreads_or(hooked) && threadIdx.x == 0) *(volatile unsigned long long *)hooks = 1;
+}
+
+// The kept edges that the rounds have not joined, by find and compare-and-swap:
+// afterwards the trees are the components of every vertex's first two edges, in
+// whatever order the hooks went.
+__global__ void k_cc_link_kept(const uint32_t *__restrict__ nb1, const uint32_t *__restrict__ nb2,
+                               uint32_t n, uint32_t *par, unsigned long long *__restrict__ hooks,
+                               unsigned long long *__restrict__ err) {
+  pdl_wait();
+  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
+  bool linked = false;
+  if (u < n) {
+    const uint32_t x = nb1[u], y = nb2[u], a = par[u];
+    const uint32_t b = x != kEmpty ? par[x] : a, c = y != kEmpty ? par[y] : a;
+    if (b != a) cc_link(par, u, x, err);
+    if (c != a) cc_link(par, u, y, err);
+    linked = b != a || c != a;
+  }
+  if (__syncthreads_or(linked) && threadIdx.x == 0) *(volatile unsigned long long *)hooks = 1;
 }
 
 // phase 3, one-leaf vertices: thread per vertex
@@ -1348,19 +1368,22 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
   unsigned long long *giant = t->d_small, *err = t->d_small + 1, *hooks = t->d_small + 2;
   SST_CUDA_TRY(t->qa.ensure((uint64_t)n + 1));
   SST_CUDA_TRY(t->qb.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, (2 + kCcMaxRounds) * 8, s));
+  SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, (3 + kCcMaxRounds) * 8, s));
   const DGraph dg = g->view();
   SST_LAUNCH_PDL(k_cc_hook_first, blocks_for(n), kTB, 0, s, dg, par, t->qa.p, t->qb.p);
   SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n,
                  static_cast<const unsigned long long *>(nullptr));
   const bool sampled = n >= kCcSampledN;
-  for (int r = 0; r < (sampled ? 4 : 2); r++) {
+  for (int r = 0; r < (sampled ? kCcMaxRounds : 1); r++) {
     const uint32_t stride = kCcStride[sampled][r];
     SST_LAUNCH_PDL(k_cc_hook, blocks_for((n + stride - 1) / stride), kTB, 0, s, t->qa.p,
                    t->qb.p, n, stride, par, r ? hooks + std::min(r - 1, 1) : nullptr,
                    hooks + r);
     SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, hooks + r);
   }
+  SST_LAUNCH_PDL(k_cc_link_kept, blocks_for(n), kTB, 0, s, t->qa.p, t->qb.p, n, par,
+                 hooks + kCcMaxRounds, err);
+  SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, hooks + kCcMaxRounds);
   SST_LAUNCH_PDL(k_cc_giant, 1, 1024, 0, s, par, n, giant);
   if (t->nsmall)
     SST_LAUNCH_PDL(k_cc_rest_small, blocks_for(t->nsmall), kTB, 0, s, dg, t->sdesc.p,

@@ -37,3 +37,19 @@ def test_components(sg, n, shape):
         g.insert_batch(e)
         o.insert_batch(e)
     assert np.array_equal(sg.CC(g), o.cc())
+
+
+@pytest.mark.parametrize("n,m", [(1000, 1500), (200000, 400000), (200000, 900000)])
+def test_one_way_edges(sg, n, m):
+    """Edges stored in one direction only: the same labels at every call, and
+    those of the byte-width snapshot, whose links are single ones."""
+    rng = np.random.default_rng(m)
+    g = sg.SparseMatrixV(n)
+    g.insert_batch(rng.integers(0, n, (m, 2)).astype(np.uint32))
+    want = np.asarray(sg.CC(g))
+    c = sg.CompactGraph(g)
+    assert np.array_equal(np.asarray(c.cc()), want)
+    for _ in range(3):
+        assert np.array_equal(np.asarray(sg.CC(g)), want)
+    c.close()
+    g.close()
