@@ -254,7 +254,7 @@ k_tc_count(Items src, const uint64_t *__restrict__ desc, const uint32_t *__restr
       uint64_t b0 = d_n1 >> kTcLenBits;
       uint32_t len = ok_n1 ? tc_len(d_n1) : 0u;
       const uint32_t kx = tc_key(na), ky = tc_key(len);
-      if (ky > kx || (ky == kx && v > u)) len = 0;
+      if (ky > kx || (ky == kx && v >= u)) len = 0;  // v == u: a stored self-loop
       // the next items' loads go out before this item's work
       bool ok_n3 = false;
       const uint32_t v_n3 = load_y(gi + 2, ok_n3);
