@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "gridbarrier.h"
 #include "primitives.cuh"
 
 namespace sst {
@@ -43,20 +44,20 @@ constexpr uint32_t kFull = 0xffffffffu;
 constexpr unsigned long long kBarrierWaitNs = 20ull * 1000 * 1000 * 1000;
 
 struct GridBarrier {
-  unsigned int *count;  // zero at launch
+  BarrierCount *count;  // zero at launch
   unsigned int *err;    // zero at launch
-  unsigned int target;  // arrivals that complete the next barrier
+  BarrierCount target;  // arrivals that complete the last barrier (0: none yet)
 
   // false: some block gave up, leave the kernel
   __device__ __forceinline__ bool wait() {
     __shared__ unsigned int s_err;
     __syncthreads();
-    target += gridDim.x;
+    target = barrier_next(target, gridDim.x);
     if (threadIdx.x == 0) {
       __threadfence();
-      atomicAdd(count, 1u);
+      atomicAdd(count, BarrierCount{1});
       unsigned long long t0 = 0;
-      for (uint32_t spin = 0; *(volatile unsigned int *)count < target; spin++) {
+      for (uint32_t spin = 0; !barrier_complete(*(volatile BarrierCount *)count, target); spin++) {
         if ((spin & 1023u) != 1023u) continue;
         if (*(volatile unsigned int *)err) break;  // a block may have left already
         unsigned long long t;
@@ -121,7 +122,8 @@ struct BfsCount {
 // device state of a search, zero at launch; the last block to leave zeroes it
 // again (no clearing launch before the next search)
 struct BfsCtl {
-  unsigned int bar, err;
+  BarrierCount bar;
+  unsigned int err;
   unsigned int rows, bigs, items;  // tails of the queues
   unsigned int left;               // blocks that have left
   BfsCount cnt[3];
