@@ -11,6 +11,7 @@
 //    are combined in chunk order, so sums are deterministic.
 #include <algorithm>
 #include <cooperative_groups.h>
+#include <new>
 #include <vector>
 
 #include "bfslevels.cuh"
@@ -18,6 +19,7 @@
 #include "prfixed.cuh"
 #include "tcshared.cuh"
 #include "traverse.cuh"
+#include "travwords.h"
 
 namespace sst {
 
@@ -61,7 +63,7 @@ template <typename T> struct DevBuf {
   }
 };
 
-struct TravState {
+struct TravState : TravWords {
   uint64_t version = ~0ull;
   // tuning (sst_autotune): leaves per work-list chunk (<= 32), lanes per
   // one-leaf vertex in PageRank, and the BFS switch to pull once
@@ -110,9 +112,6 @@ struct TravState {
   double pr_damping = 0.0;
   const void *pr_key[6] = {};  // output, stream and the buffers it reads
   int64_t pr_kernels = 0;      // kernels in the captured graph
-  uint64_t *h_small = nullptr;  // pinned readback slots
-  unsigned long long *d_small = nullptr;
-  void *d_bfs = nullptr;  // BfsCtl and BcCtl, zero between searches
 };
 
 // frees every buffer and the captured PageRank graph; the tuning stays, and
@@ -176,13 +175,21 @@ void trav_trim(sst_graph *g) {
   if (g->trav) trav_buffers_release(g->trav);
 }
 
+// the CUDA side of TravWords
+struct TravWordsRt {
+  cudaStream_t s;
+  bool pinned(void **p, size_t bytes) { return cudaMallocHost(p, bytes) == cudaSuccess; }
+  bool device(void **p, size_t bytes) { return cudaMalloc(p, bytes) == cudaSuccess; }
+  bool zero(void *p, size_t bytes) { return cudaMemsetAsync(p, 0, bytes, s) == cudaSuccess; }
+  void free_pinned(void *p) { cudaFreeHost(p); }
+  void free_device(void *p) { cudaFree(p); }
+};
+
 void trav_release(sst_graph *g) {
   TravState *t = g->trav;
   if (!t) return;
   trav_buffers_release(t);
-  if (t->h_small) cudaFreeHost(t->h_small);
-  if (t->d_small) cudaFree(t->d_small);
-  if (t->d_bfs) cudaFree(t->d_bfs);
+  trav_words_free(t, TravWordsRt{g->stream});
   delete t;
   g->trav = nullptr;
 }
@@ -1093,19 +1100,26 @@ k_common(DGraph g, const uint32_t *__restrict__ pairs, uint64_t n, uint32_t per_
 }  // namespace
 
 // ================================================================== host
-static TravState *state(sst_graph *g) {
+// the graph's traversal state, made by the first traversal
+static sst_status state(sst_graph *g, TravState **out) {
   if (!g->trav) {
-    g->trav = new TravState();
-    cudaMallocHost(&g->trav->h_small, 64 * sizeof(uint64_t));
-    cudaMalloc(&g->trav->d_small, 64 * sizeof(unsigned long long));
-    cudaMalloc(&g->trav->d_bfs, sizeof(BfsCtl) + sizeof(BcCtl));
-    cudaMemsetAsync(g->trav->d_bfs, 0, sizeof(BfsCtl) + sizeof(BcCtl), g->stream);
+    TravState *t = new (std::nothrow) TravState();
+    if (!t || !trav_words_init(t, sizeof(BfsCtl) + sizeof(BcCtl), TravWordsRt{g->stream})) {
+      cudaGetLastError();
+      delete t;
+      set_error_message("cannot allocate the traversal state");
+      return SST_ENOMEM;
+    }
+    g->trav = t;
   }
-  return g->trav;
+  *out = g->trav;
+  return SST_OK;
 }
 
 static sst_status ensure_lists(sst_graph *g) {
-  TravState *t = state(g);
+  TravState *t = nullptr;
+  sst_status st = state(g, &t);
+  if (st != SST_OK) return st;
   if (t->version == g->version && t->lists_cl == t->chunk_leaves) return SST_OK;
   cudaStream_t s = g->stream;
   const uint32_t n = g->n, cl = t->chunk_leaves;
@@ -1432,7 +1446,9 @@ sst_status bc(sst_graph *g, uint32_t src, double *d_dep) {
 sst_status tc(sst_graph *g, uint64_t *total, uint64_t *d_pv) {
   sst_status st = ensure_leaf_dir(g);
   if (st != SST_OK) return st;
-  TravState *t = state(g);
+  TravState *t = nullptr;
+  st = state(g, &t);
+  if (st != SST_OK) return st;
   cudaStream_t s = g->stream;
   uint32_t n = g->n;
   LeafDir &D = g->dir;
@@ -1931,10 +1947,12 @@ sst_status bfs_multi(sst_graph *g, const uint32_t *h_srcs, uint32_t k,
 sst_status bc_multi(sst_graph *g, const uint32_t *h_srcs, uint32_t k,
                     double *d_dep) {
   if (k == 0) return SST_OK;
-  TravState *t = state(g);
+  TravState *t = nullptr;
+  sst_status st = state(g, &t);
+  if (st != SST_OK) return st;
   const uint32_t n = g->n;
   SST_CUDA_TRY(t->mdepth.ensure((uint64_t)k * n));
-  sst_status st = bfs_multi(g, h_srcs, k, t->mdepth.p);
+  st = bfs_multi(g, h_srcs, k, t->mdepth.p);
   if (st != SST_OK) return st;
   cudaStream_t s = g->stream;
   const int32_t *depth = t->mdepth.p;
@@ -2057,7 +2075,9 @@ sst_status bc_multi(sst_graph *g, const uint32_t *h_srcs, uint32_t k,
 // shared-memory cache {0, 2048, 4096, 8192}, then BFS from three sources
 // over push/pull thresholds {5, 10, 20, 40, 80}.
 sst_status get_tuning(sst_graph *g, sst_tuning *out) {
-  TravState *t = state(g);
+  TravState *t = nullptr;
+  sst_status st = state(g, &t);
+  if (st != SST_OK) return st;
   out->chunk_leaves = t->chunk_leaves;
   out->pr_lanes = t->pr_lanes;
   out->bfs_alpha = t->bfs_alpha;
@@ -2075,7 +2095,9 @@ sst_status set_tuning(sst_graph *g, const sst_tuning *in) {
                       "bfs_alpha >= 1, pr_hot <= 24576)");
     return SST_EINVAL;
   }
-  TravState *t = state(g);
+  TravState *t = nullptr;
+  sst_status st = state(g, &t);
+  if (st != SST_OK) return st;
   t->chunk_leaves = in->chunk_leaves;
   t->pr_lanes = in->pr_lanes;
   t->bfs_alpha = in->bfs_alpha;
@@ -2084,9 +2106,11 @@ sst_status set_tuning(sst_graph *g, const sst_tuning *in) {
 }
 
 sst_status autotune(sst_graph *g, sst_tuning *out) {
-  TravState *t = state(g);
+  TravState *t = nullptr;
+  sst_status st = state(g, &t);
+  if (st != SST_OK) return st;
   const uint32_t n = g->n;
-  sst_status st = get_tuning(g, out);
+  st = get_tuning(g, out);
   if (st != SST_OK || n == 0 || g->m == 0) return st;
   cudaStream_t s = g->stream;
   double *rank = nullptr;
@@ -2307,7 +2331,9 @@ sst_status bellman_ford(sst_graph *g, uint32_t src, int32_t *d_out) {
     set_error_message("Bellman-Ford needs a weighted graph (sst_config.weighted)");
     return SST_ESTATE;
   }
-  TravState *t = state(g);
+  TravState *t = nullptr;
+  sst_status st = state(g, &t);
+  if (st != SST_OK) return st;
   cudaStream_t s = g->stream;
   const uint32_t n = g->n;
   if (n == 0) return SST_OK;

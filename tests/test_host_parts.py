@@ -1,0 +1,21 @@
+"""Parts of the CUDA sources that the host can check by itself.
+
+The search kernels' grid barrier: a search of more levels than 32 bits of
+arrivals count (15 million, a path) still waits at every barrier.  The words
+that every traversal uses: an allocation that fails leaves none of them."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.mark.parametrize("name,says", [("barrier_check", "barrier ok"),
+                                       ("travwords_check", "words ok")])
+def test_part(tmp_path, name, says):
+    out = os.path.join(str(tmp_path), name)
+    subprocess.run(["g++", "-std=c++17", "-O1", os.path.join(ROOT, "tests", "cpp", name + ".cpp"),
+                    "-o", out], check=True)
+    r = subprocess.run([out], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and says in r.stdout, (r.returncode, r.stdout)
