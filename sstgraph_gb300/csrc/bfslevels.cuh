@@ -619,7 +619,9 @@ constexpr uint32_t kNotQueued = 1u << 31;
 constexpr int kBcFlight = 8;  // neighbours (or leaves) in flight
 
 // Row ids are read once a pass and leave L1 to the gathered values; those
-// change between levels, so they are not read through the read-only path.
+// change between levels, so they are not read through the read-only path.  (The
+// ids do not change while the kernel runs, and it is no programmatic launch, so
+// nothing has to order these loads.)
 __device__ __forceinline__ uint32_t ld_id(const uint32_t *p) {
   uint32_t v;
   asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));

@@ -61,8 +61,12 @@ __device__ __forceinline__ void pr_finish(uint32_t v, unsigned long long sum,
   if (last) rank[v] = __ull2double_rn(r) * (1.0 / 9223372036854775808.0);
 }
 
-// row ids are read once per iteration: keep them out of L1 and first in
-// line for eviction from L2, so the contribution gathers keep both caches
+// Row ids are read once per iteration: keep them out of L1 and first in
+// line for eviction from L2, so the contribution gathers keep both caches.
+// The loads are volatile, as pdl_wait's griddepcontrol.wait is, so they stay
+// after it; a "memory" clobber would also hold back the plain loads around them.
+// Contributions come from the kernel before, which a programmatic launch may
+// overlap, so they do not take the read-only path.
 __device__ __forceinline__ unsigned long long l2_evict_first() {
   unsigned long long pol;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -71,14 +75,14 @@ __device__ __forceinline__ unsigned long long l2_evict_first() {
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p,
                                               unsigned long long pol) {
   uint32_t v;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.b32 %0, [%1], %2;"
-      : "=r"(v)
-      : "l"(p), "l"(pol));
+  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.b32 %0, [%1], %2;"
+               : "=r"(v)
+               : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ unsigned long long ld_keep(const unsigned long long *p) {
   unsigned long long v;
-  asm("ld.global.nc.L1::evict_last.b64 %0, [%1];" : "=l"(v) : "l"(p));
+  asm volatile("ld.global.L1::evict_last.b64 %0, [%1];" : "=l"(v) : "l"(p));
   return v;
 }
 

@@ -2,8 +2,11 @@
 
 The search kernels' grid barrier: a search of more levels than 32 bits of
 arrivals count (15 million, a path) still waits at every barrier.  The words
-that every traversal uses: an allocation that fails leaves none of them."""
+that every traversal uses: an allocation that fails leaves none of them.  The
+PageRank kernels' inline loads: volatile, or nothing keeps them after the wait
+for the kernel whose results they read."""
 import os
+import re
 import subprocess
 
 import pytest
@@ -19,3 +22,12 @@ def test_part(tmp_path, name, says):
                     "-o", out], check=True)
     r = subprocess.run([out], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and says in r.stdout, (r.returncode, r.stdout)
+
+
+def test_pagerank_loads_are_ordered():
+    src = open(os.path.join(ROOT, "sstgraph_gb300", "csrc", "prfixed.cuh")).read()
+    loads = re.findall(r"asm( volatile)?\s*\(\s*\"(ld\.[^ ]*)", src)
+    assert len(loads) >= 2
+    assert all(v for v, _ in loads), loads
+    # contributions: written by the kernel before
+    assert [op for _, op in loads if "evict_last" in op] == ["ld.global.L1::evict_last.b64"]
