@@ -2720,13 +2720,24 @@ static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, b
   return SST_OK;
 }
 
-// A graph made, loaded and freed, by the general sequence and so: 2,200 pairs of 300 rows 0.93 -> 0.66 ms,
-// 18,000 of 2,000 rows 0.96 -> 0.67, 18,000 of 300,000 rows 1.20 -> 0.94, 600,000
-// (RMAT) of 32,768 rows 1.29 -> 0.84.  Smaller loads take the launches that later
-// batches of their size replay.
+// Loads from here on take run_load.  A graph made, loaded and freed, by the general
+// sequence and so: 2,200 pairs of 300 rows 0.93 -> 0.66 ms, 18,000 of 2,000 rows
+// 0.96 -> 0.67, 18,000 of 300,000 rows 1.20 -> 0.94, 600,000 (RMAT) of 32,768 rows
+// 1.29 -> 0.84.  Smaller loads take the launches that later batches of their size
+// replay.
 constexpr uint64_t kLoadPairs = 2049;
 
-// Pairs into a graph without segments (see k_load_flags); same result as
+// Its scratch: 16 bytes a pair, and 12 a row.  It is taken only where that is no
+// more than the general sequence's (up to some 23 rows a pair), so that no load
+// needs more than it did: 3,000 pairs of 2^26 rows took 805 MB and 2.3 ms, where
+// the general sequence takes 1 MB and 1.8 ms.
+static size_t load_scratch_bytes(uint64_t b, uint64_t n) {
+  const uint64_t ntiles = (b + kLoadTile - 1) / kLoadTile;
+  return b * 16 + n * 12 + ntiles * 8 + radix_sort_scratch_bytes(b) +
+         scan_scratch_bytes(ntiles, 4) + (1 << 14);
+}
+
+// Pairs into a graph without segments (see LoadTile); same result as
 // run_pipeline.  The slab holds nothing, so one that is too small is replaced,
 // not repacked.
 static sst_status run_load(sst_graph *g, const uint32_t *d_pairs, uint64_t b,
@@ -2736,9 +2747,7 @@ static sst_status run_load(sst_graph *g, const uint32_t *d_pairs, uint64_t b,
   const uint64_t ntiles = (b + kLoadTile - 1) / kLoadTile;
   // with room for later updates of a twelfth of the load: about what the load
   // itself takes, so that the first of them allocate nothing
-  const size_t need = std::max<size_t>(b * 16 + n * 12 + ntiles * 8 + radix_sort_scratch_bytes(b) +
-                                           scan_scratch_bytes(ntiles, 4) + (1 << 14),
-                                       update_scratch_bytes(b / 12));
+  const size_t need = std::max(load_scratch_bytes(b, n), update_scratch_bytes(b / 12));
   if (need > g->arena.cap) {
     sst_status st = budget_check(g, need - g->arena.cap);
     if (st != SST_OK) return st;
@@ -2822,7 +2831,8 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
   }
   if (!presorted && !g->weighted && b <= kSmallBatch)
     return run_small(g, d_pairs, (uint32_t)b, insert, n_invalid);
-  if (!presorted && !g->weighted && insert && g->bump == 0 && b >= kLoadPairs && g->n)
+  if (!presorted && !g->weighted && insert && g->bump == 0 && b >= kLoadPairs && g->n &&
+      load_scratch_bytes(b, g->n) <= update_scratch_bytes(b))
     return run_load(g, d_pairs, b, n_invalid);
   // Small batches are bound by the host's launch rate, so their planning
   // sequence (sort to plan readback) is captured once per size class and

@@ -1,0 +1,39 @@
+"""Work that fits a memory budget: what an update may take beside the graph
+does not grow with the rows of the matrix or with the form that it takes."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def sg():
+    import __graft_entry__ as ge
+    ge.build()
+    import sstgraph_gb300
+    return sstgraph_gb300
+
+
+def device(e):
+    import torch
+    t = torch.from_numpy(np.ascontiguousarray(e).astype(np.int32)).cuda()
+    torch.cuda.synchronize()
+    return t
+
+
+# fewer pairs than rows: on the load's own path as many as its scratch allows
+@pytest.mark.parametrize("n,b", [(1 << 22, 3000), (1 << 20, 40000), (1 << 20, 50000), (5000, 3000)])
+def test_load_of_few_pairs(sg, n, b):
+    e = np.random.default_rng(b).integers(0, n, (b, 2))
+    e = e[e[:, 0] != e[:, 1]]
+    g = sg.SparseMatrixV(n)
+    empty = g.get_memory_size()
+    g.close()
+    # the general sequence's planning, rounded up and over, and its staging
+    g = sg.SparseMatrixV(n, hbm_budget_bytes=empty + 550 * b + (3 << 20))
+    g.insert_batch(device(e))
+    k = np.unique(e[:, 0] * n + e[:, 1])
+    assert g.M() == len(k)
+    off, cols = g.csr()
+    assert np.array_equal(np.repeat(np.arange(n), np.diff(off.astype(np.int64))) * n + cols, k)
+    g.close()
