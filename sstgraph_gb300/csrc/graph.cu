@@ -2530,7 +2530,7 @@ static sst_status plan_graph_launch(sst_graph *g, uint64_t b, bool insert,
 // bytes of arena scratch an update batch of b pairs takes
 static size_t update_scratch_bytes(uint64_t b) {
   size_t per = 8 * 2 + 4 * 5 + 8 + 4 + 4 * 3 + 1 * 2 + 4 * 2 + 8 * 4 + 4 * 6 +
-               8 * 8 + 4 * 4 + 1 + 64 + 4 * 3 /* values */ +
+               8 * 8 + 4 * 4 + 1 + 48 + 4 * 3 /* values */ +
                8 + 4 + 8 + 4 + 4 /* leaf starts and counts, merge ranges */;
   return b * per + radix_sort_scratch_bytes(b) + 8 * scan_scratch_bytes(b, 8) +
          (1 << 16);
@@ -2643,7 +2643,8 @@ static sst_status read_plan(sst_graph *g, PlanSummary *ps) {
 static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, bool insert,
                             uint64_t *n_invalid) {
   cudaStream_t s = g->stream;
-  const size_t need = update_scratch_bytes(kSmallBatch);
+  // as the general sequence's (see run_pipeline), which some batches also take
+  const size_t need = update_scratch_bytes(g->plan_graphs ? plan_size_class(b) : b);
   if (need > g->arena.cap) {
     sst_status st = budget_check(g, need - g->arena.cap);
     if (st != SST_OK) return st;
@@ -2651,7 +2652,7 @@ static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, b
   SST_CUDA_TRY(g->arena.reserve(need));
   Arena &A = g->arena;
   A.reset();
-  constexpr uint32_t B = kSmallBatch;
+  const uint32_t B = b;
   uint64_t *keys = A.take<uint64_t>(B), *lS = A.take<uint64_t>(B);
   uint32_t *state = A.take<uint32_t>(B), *leaf = A.take<uint32_t>(B), *lc = A.take<uint32_t>(B);
   uint64_t *p_ul = A.take<uint64_t>(B), *p_S = A.take<uint64_t>(B);

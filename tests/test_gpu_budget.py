@@ -37,3 +37,25 @@ def test_load_of_few_pairs(sg, n, b):
     off, cols = g.csr()
     assert np.array_equal(np.repeat(np.arange(n), np.diff(off.astype(np.int64))) * n + cols, k)
     g.close()
+
+
+# The least beside the graph that each was found to fit when one sequence of
+# launches took every batch and sort tiles held 4096 keys.
+@pytest.mark.parametrize("b,least", [(1, 1236928), (100, 1256384), (700, 1516224),
+                                     (20000, 9527808), (262145, 131383296),
+                                     (600000, 261840896), (1 << 20, 423149568)])
+@pytest.mark.parametrize("plan", [True, False])
+def test_batches_of_any_form(sg, b, least, plan):
+    n = 1 << 20
+    first = device([[5, 7], [7, 5]])
+    e = device(np.random.default_rng(2).integers(0, n, (b, 2)))
+    g = sg.SparseMatrixV(n)
+    empty = g.get_memory_size()
+    g.close()
+    g = sg.SparseMatrixV(n, hbm_budget_bytes=empty + least)
+    g.set_plan_graphs(plan)
+    g.insert_batch(first)  # no graph without segments: that is a load
+    g.release_scratch()
+    g.insert_batch(e)
+    assert g.M() > b // 2
+    g.close()
