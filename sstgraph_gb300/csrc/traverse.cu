@@ -48,12 +48,14 @@ template <typename T> struct DevBuf {
   uint64_t cap = 0;
   cudaError_t ensure(uint64_t n) {
     if (n <= cap) return cudaSuccess;
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
-    uint64_t want = n + n / 8 + 64;
-    cudaError_t e = cudaMalloc(&p, want * sizeof(T));
-    if (e == cudaSuccess) cap = want;
+    return exact(n + n / 8 + 64);
+  }
+  // without room to grow: for sizes that only the number of vertices sets
+  cudaError_t exact(uint64_t n) {
+    if (n <= cap) return cudaSuccess;
+    release();
+    cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+    if (e == cudaSuccess) cap = n;
     return e;
   }
   void release() {
@@ -1126,13 +1128,15 @@ static sst_status ensure_lists(sst_graph *g) {
   // sized by what the slab can hold, so nothing waits for the counts and an
   // update that moves no slab grows no list
   const uint64_t most_big = std::min<uint64_t>(n, g->nslots / (2 * kLeaf));
+  // (several chunks: more than cl leaves)
+  const uint64_t most_multi = std::min<uint64_t>(n, g->nslots / ((uint64_t)kLeaf * (cl + 1)));
   const uint64_t most_chunks = most_big + g->nslots / ((uint64_t)kLeaf * cl);
   const unsigned nb = blocks_for(n, kListBlock);
   SST_CUDA_TRY(t->lsum.ensure(4 * (uint64_t)nb));
-  SST_CUDA_TRY(t->small.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->sdesc.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->small.exact((uint64_t)n + 1));
+  SST_CUDA_TRY(t->sdesc.exact((uint64_t)n + 1));
   SST_CUDA_TRY(t->big.ensure(most_big + 1));
-  SST_CUDA_TRY(t->multi.ensure(most_big + 1));
+  SST_CUDA_TRY(t->multi.ensure(most_multi + 1));
   SST_CUDA_TRY(t->cv.ensure(most_chunks + 1));
   SST_CUDA_TRY(t->cdesc.ensure(most_chunks + 1));
   uint4 *sums = reinterpret_cast<uint4 *>(t->lsum.p);
@@ -1160,10 +1164,10 @@ sst_status pagerank(sst_graph *g, uint32_t iters, double damping, double *d_rank
   cudaStream_t s = g->stream;
   uint32_t n = g->n;
   if (n == 0) return SST_OK;
-  SST_CUDA_TRY(t->ca.ensure(n));
-  SST_CUDA_TRY(t->cb.ensure(n));
+  SST_CUDA_TRY(t->ca.exact(n));
+  SST_CUDA_TRY(t->cb.exact(n));
   SST_CUDA_TRY(t->partial.ensure(t->nchunks + 1));
-  SST_CUDA_TRY(t->inv_deg.ensure(n));
+  SST_CUDA_TRY(t->inv_deg.exact(n));
   unsigned long long *rdeg = reinterpret_cast<unsigned long long *>(t->inv_deg.p);
   static bool carveout = false;
   if (!carveout) {
@@ -1334,11 +1338,11 @@ static sst_status bfs_setup(sst_graph *g, uint32_t src, int32_t *d_parents, int3
   // a row's push items are at most 32 / kBfsLeaves for each of its chunks in
   // the lists (chunks of up to 32 leaves)
   const uint64_t max_items = t->nchunks * (32 / kBfsLeaves) + 1;
-  SST_CUDA_TRY(t->qa.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->qa.exact((uint64_t)n + 1));
   SST_CUDA_TRY(t->qitems.ensure(max_items));
   SST_CUDA_TRY(t->fbits.ensure(n / 32 + 2));
   if (!d_depths) {
-    SST_CUDA_TRY(t->depth_tmp.ensure(n));
+    SST_CUDA_TRY(t->depth_tmp.exact(n));
     d_depths = t->depth_tmp.p;
   }
   *a = BfsArgs{g->view(),   g->m,       src,         t->bfs_alpha, t->small.p,
@@ -1380,8 +1384,8 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
   if (n == 0) return SST_OK;
   uint32_t *par = d_labels;
   unsigned long long *giant = t->d_small, *err = t->d_small + 1, *hooks = t->d_small + 2;
-  SST_CUDA_TRY(t->qa.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->qb.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->qa.exact((uint64_t)n + 1));
+  SST_CUDA_TRY(t->qb.exact((uint64_t)n + 1));
   SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, (3 + kCcMaxRounds) * 8, s));
   const DGraph dg = g->view();
   SST_LAUNCH_PDL(k_cc_hook_first, blocks_for(n), kTB, 0, s, dg, par, t->qa.p, t->qb.p);
@@ -1426,10 +1430,10 @@ sst_status bc(sst_graph *g, uint32_t src, double *d_dep) {
   if (st != SST_OK) return st;
   TravState *t = g->trav;
   const uint64_t n = g->n;
-  SST_CUDA_TRY(t->sigma.ensure(2 * n));
-  SST_CUDA_TRY(t->ratio.ensure(2 * n));
-  SST_CUDA_TRY(t->levels.ensure(n + 1));
-  SST_CUDA_TRY(t->qb.ensure(n + 1));
+  SST_CUDA_TRY(t->sigma.exact(2 * n));
+  SST_CUDA_TRY(t->ratio.exact(2 * n));
+  SST_CUDA_TRY(t->levels.exact(n + 1));
+  SST_CUDA_TRY(t->qb.ensure(t->nbig + 1));
   // a hub's chunks of kBcLeaves leaves are at most its chunks in the lists
   const uint64_t hubs = t->nchunks + 1;
   SST_CUDA_TRY(t->hub.ensure(2 * hubs));
@@ -1456,7 +1460,7 @@ sst_status tc(sst_graph *g, uint64_t *total, uint64_t *d_pv) {
   SST_CUDA_TRY(t->tlcnt.ensure(nl + 1));
   SST_CUDA_TRY(t->tlpre.ensure(nl + 1));
   SST_CUDA_TRY(t->tmask.ensure(nl + 1));
-  SST_CUDA_TRY(t->toff.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->toff.exact((uint64_t)n + 1));
   g->arena.reset();
   SST_CUDA_TRY(g->arena.reserve(scan_scratch_bytes(nl + 1, 8) + 4096));
   const uint64_t tc_warps = (nl + kTcLeaves - 1) / kTcLeaves;
@@ -1873,14 +1877,14 @@ sst_status bfs_multi(sst_graph *g, const uint32_t *h_srcs, uint32_t k,
     }
   }
   const unsigned long long full = k == 64 ? ~0ull : (1ull << k) - 1;
-  SST_CUDA_TRY(t->mvis.ensure(n));
-  SST_CUDA_TRY(t->mfr.ensure(n));
-  SST_CUDA_TRY(t->mfr2.ensure(n));
-  SST_CUDA_TRY(t->mnx.ensure(n));
-  SST_CUDA_TRY(t->qa.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->qb.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->icnt.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->ioff.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->mvis.exact(n));
+  SST_CUDA_TRY(t->mfr.exact(n));
+  SST_CUDA_TRY(t->mfr2.exact(n));
+  SST_CUDA_TRY(t->mnx.exact(n));
+  SST_CUDA_TRY(t->qa.exact((uint64_t)n + 1));
+  SST_CUDA_TRY(t->qb.exact((uint64_t)n + 1));
+  SST_CUDA_TRY(t->icnt.exact((uint64_t)n + 1));
+  SST_CUDA_TRY(t->ioff.exact((uint64_t)n + 1));
   SST_CUDA_TRY(t->msrc.ensure(2 * (uint64_t)sv.size()));
   SST_CUDA_TRY(cudaMemsetAsync(t->mvis.p, 0, (uint64_t)n * 8, s));
   SST_CUDA_TRY(cudaMemsetAsync(t->mfr.p, 0, (uint64_t)n * 8, s));
@@ -2338,11 +2342,11 @@ sst_status bellman_ford(sst_graph *g, uint32_t src, int32_t *d_out) {
   const uint32_t n = g->n;
   if (n == 0) return SST_OK;
   SST_CUDA_TRY(t->msrc.ensure(n));  // 64-bit distances
-  SST_CUDA_TRY(t->qa.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->qb.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->qa.exact((uint64_t)n + 1));
+  SST_CUDA_TRY(t->qb.exact((uint64_t)n + 1));
   SST_CUDA_TRY(t->fbits.ensure((uint64_t)n + 1));  // round stamps
-  SST_CUDA_TRY(t->icnt.ensure((uint64_t)n + 1));
-  SST_CUDA_TRY(t->ioff.ensure((uint64_t)n + 1));
+  SST_CUDA_TRY(t->icnt.exact((uint64_t)n + 1));
+  SST_CUDA_TRY(t->ioff.exact((uint64_t)n + 1));
   unsigned long long *dist = t->msrc.p;
   uint32_t *stamp = t->fbits.p;
   SST_LAUNCH(k_bf_init, blocks_for(n), kTB, 0, s, dist, stamp, n, src);

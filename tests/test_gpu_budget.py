@@ -59,3 +59,25 @@ def test_batches_of_any_form(sg, b, least, plan):
     g.insert_batch(e)
     assert g.M() > b // 2
     g.close()
+
+
+# What each traversal keeps on an RMAT graph of 2^18 vertices and 2^21 drawn
+# edges, when its levels were launches of their own.
+@pytest.mark.parametrize("name,most", [("bfs", 22572280), ("pr", 23662752), ("cc", 15095800),
+                                       ("bc", 29828512), ("tc", 41834720)])
+def test_traversal_buffers(sg, name, most):
+    import torch
+    run = {"bfs": lambda: sg.BFS(g, 1), "pr": lambda: sg.PR_S(g, 2), "cc": lambda: sg.CC(g),
+           "bc": lambda: sg.BC(g, 1), "tc": lambda: sg.TC(g)}[name]
+    e = torch.empty((8 << 18, 2), dtype=torch.int32, device="cuda")
+    sg.gen_rmat(18, 8 << 18, out=e)
+    torch.cuda.synchronize()
+    e = torch.cat([e, e.flip(1)]).contiguous()
+    torch.cuda.synchronize()
+    g = sg.SparseMatrixV(1 << 18)
+    g.insert_batch(e)
+    g.release_scratch()
+    before = g.get_memory_size()
+    run()
+    assert g.get_memory_size() - before <= most
+    g.close()
