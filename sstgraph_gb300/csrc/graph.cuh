@@ -73,6 +73,7 @@ struct sst_graph {
   bool keep_loops = false;  // inserts keep (v, v) (per-row sets)
 
   uint64_t *d_base = nullptr;
+  void *d_words = nullptr;  // d_cap to d_scan_epoch, where not in d_base's allocation
   uint32_t *d_cap = nullptr;
   uint32_t *d_deg = nullptr;
   uint32_t *d_slots = nullptr;

@@ -102,3 +102,20 @@ def test_load_as_the_general_path_does(sg, loops):
     assert np.array_equal(g.degrees(), w.degrees())
     g.close()
     w.close()
+
+
+# the records in one allocation, in two, and in one again
+@pytest.mark.parametrize("n", [1, 63000, 66000, 120000, 132000])
+def test_records_of_any_size(sg, n):
+    e = np.array([[0, n - 1], [n // 2, 0], [n - 1, n - 1], [n - 1, n // 3]], np.uint32)
+    e = e[e[:, 0] != e[:, 1]]
+    for _ in range(3):
+        g = sg.SparseMatrixV(n)
+        o = oracle.OracleGraph(n)
+        if len(e):
+            assert g.insert_batch(e) == 0
+            o.insert_batch(e)
+        h = g.copy()
+        g.close()
+        same(h, o)
+        h.close()
