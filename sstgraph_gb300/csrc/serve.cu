@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "graph.cuh"
+#include "tcvrule.h"
 #include "traverse.cuh"
 
 using Clock = std::chrono::steady_clock;
@@ -80,22 +81,6 @@ sst_status graph_copy_into(sst_graph *dst, sst_graph *src) {
 // A pair of two long lists spreads over as many lane groups as the shorter one
 // has chunks, so none walks a long list alone.
 namespace {
-// Leaves a chunk, by the pair slots of the call.  A few queries, whose chunks are
-// all in flight at once, end when the longest chunk does (2 to 3 us a leaf of
-// dependent probes); many have chunks to spare and pay for each one's search among
-// the pairs.  The sum of the chunks has to stay below 2^32: 2^22 slots would need
-// as many lists of 8192 leaves to pass it in chunks of 8, more than fits the
-// device, and beyond that the chunks are long.  Pass 3 at RMAT scale 18 (us, by
-// leaves a chunk; last, a warp a chunk of 32):
-//   vertices    1     2     4     8    32    warp
-//   100        17    23    34    51    81     42
-//   1,000      62    56    57    72   141     91
-//   10,000    650   526   483   508   668    699
-//   100,000  5255  4184  3722  3724  4653   5366
-inline uint32_t tcv_chunk_leaves(uint64_t nslots) {
-  return nslots <= 1 << 17 ? 2 : nslots <= 1 << 20 ? 4 : nslots <= 1 << 22 ? 8 : 32;
-}
-
 __device__ __forceinline__ uint32_t leaves_of(uint32_t cap) {
   return cap == 0 ? 0 : (cap <= kLeaf ? 1 : cap >> kLeafLog);
 }
@@ -110,11 +95,13 @@ __global__ void k_tcv_leaves(DGraph g, const uint32_t *__restrict__ vs,
   out[i] = 0;
 }
 
-// pass 2: warp per leaf item; lane = pair slot
+// pass 2: warp per leaf item; lane = pair slot.  Off: the type of the chunk counts
+// and offsets (tcvrule.h)
+template <typename Off>
 __global__ void k_tcv_pairs(DGraph g, const uint32_t *__restrict__ vs, uint64_t k,
                             const uint64_t *__restrict__ loff, uint64_t items,
                             uint32_t chunk, uint32_t *__restrict__ pq,
-                            uint32_t *__restrict__ pw, uint32_t *__restrict__ cost) {
+                            uint32_t *__restrict__ pw, Off *__restrict__ cost) {
   const int lane = threadIdx.x & 31;
   const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t wi = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -147,9 +134,10 @@ __global__ void k_tcv_pairs(DGraph g, const uint32_t *__restrict__ vs, uint64_t 
 // and a chunk is a chain of dependent loads, so four chunks share a warp, and a
 // lane searches for its up to four ids of a leaf together (the longer list is the
 // same, so the searches take the same steps).
+template <typename Off>
 __global__ void __launch_bounds__(256)
 k_tcv_count(DGraph g, const uint32_t *__restrict__ vs, const uint32_t *__restrict__ pq,
-            const uint32_t *__restrict__ pw, const uint32_t *__restrict__ coff, uint64_t nslots,
+            const uint32_t *__restrict__ pw, const Off *__restrict__ coff, uint64_t nslots,
             uint64_t nchunks, uint32_t chunk, unsigned long long *__restrict__ out) {
   const uint32_t sub = threadIdx.x & 7;
   const int shift = threadIdx.x & 24;
@@ -233,40 +221,43 @@ sst_status tc_vertices(sst_graph *g, const uint32_t *d_vs, uint64_t k,
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(&items, tot, 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  // pass 2: pair slots and their chunk counts
-  uint32_t *pq = nullptr, *pw = nullptr, *cost = nullptr, *coff = nullptr;
-  const uint64_t nslots = items * 32;
-  const uint32_t chunk = tcv_chunk_leaves(nslots);
-  uint32_t nchunks = 0;
-  if (e == cudaSuccess && items) {
-    e = cudaMallocAsync(&pq, items * 4, s);
-    if (e == cudaSuccess) e = cudaMallocAsync(&pw, nslots * 4, s);
-    if (e == cudaSuccess) e = cudaMallocAsync(&cost, nslots * 4, s);
-    if (e == cudaSuccess) e = cudaMallocAsync(&coff, nslots * 4, s);
-    if (e == cudaSuccess) {
-      g->arena.reset();
-      e = g->arena.reserve(scan_scratch_bytes(nslots, 4) + 4096);
-    }
-    uint32_t *ctot = e == cudaSuccess ? g->arena.take<uint32_t>(1) : nullptr;
-    if (e == cudaSuccess && !ctot) e = cudaErrorMemoryAllocation;
-    if (e == cudaSuccess) {
-      SST_LAUNCH(k_tcv_pairs, (unsigned)std::min<uint64_t>((items * 32 + tb - 1) / tb, cap_blocks),
-                 tb, 0, s, g->view(), d_vs, k, loff, items, chunk, pq, pw, cost);
-      e = scan<uint32_t, OpAdd>(cost, coff, nslots, 0u, OpAdd{}, true, false, ctot,
-                                g->arena, s);
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&nchunks, ctot, 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    // pass 3
-    if (e == cudaSuccess && nchunks) {
-      SST_LAUNCH(k_tcv_count,
-                 (unsigned)std::min<uint64_t>(((uint64_t)nchunks * 8 + tb - 1) / tb, cap_blocks),
-                 tb, 0, s, g->view(), d_vs, pq, pw, coff, nslots, nchunks, chunk, out);
-      SST_LAUNCH(k_tcv_half, (unsigned)((k + tb - 1) / tb), tb, 0, s, out, k);
-      e = cudaGetLastError();
-    }
-  }
-  for (void *p : {(void *)loff, (void *)pq, (void *)pw, (void *)cost, (void *)coff})
+  // passes 2 and 3
+  uint32_t *pq = nullptr, *pw = nullptr;
+  void *cost = nullptr, *coff = nullptr;
+  auto pairs = [&](auto zero) -> cudaError_t {
+    using Off = decltype(zero);
+    const uint64_t nslots = items * 32;
+    const uint32_t chunk = tcv_chunk_leaves(nslots);
+    cudaError_t r = cudaMallocAsync(&pq, items * 4, s);
+    if (r == cudaSuccess) r = cudaMallocAsync(&pw, nslots * 4, s);
+    if (r == cudaSuccess) r = cudaMallocAsync(&cost, nslots * sizeof(Off), s);
+    if (r == cudaSuccess) r = cudaMallocAsync(&coff, nslots * sizeof(Off), s);
+    if (r != cudaSuccess) return r;
+    Off *const n1 = static_cast<Off *>(cost), *const at = static_cast<Off *>(coff);
+    g->arena.reset();
+    r = g->arena.reserve(scan_scratch_bytes(nslots, sizeof(Off)) + 4096);
+    if (r != cudaSuccess) return r;
+    Off *ctot = g->arena.take<Off>(1);
+    if (!ctot) return cudaErrorMemoryAllocation;
+    SST_LAUNCH(k_tcv_pairs<Off>,
+               (unsigned)std::min<uint64_t>((items * 32 + tb - 1) / tb, cap_blocks), tb, 0, s,
+               g->view(), d_vs, k, loff, items, chunk, pq, pw, n1);
+    r = scan<Off, OpAdd>(n1, at, nslots, Off{0}, OpAdd{}, true, false, ctot, g->arena, s);
+    Off nchunks = 0;
+    if (r == cudaSuccess)
+      r = cudaMemcpyAsync(&nchunks, ctot, sizeof(Off), cudaMemcpyDeviceToHost, s);
+    if (r == cudaSuccess) r = cudaStreamSynchronize(s);
+    if (r != cudaSuccess || !nchunks) return r;
+    // (no more blocks than the cap for any count of chunks)
+    const uint64_t blocks = std::min<uint64_t>(((uint64_t)nchunks + tb / 8 - 1) / (tb / 8), cap_blocks);
+    SST_LAUNCH(k_tcv_count<Off>, (unsigned)blocks, tb, 0, s, g->view(), d_vs, pq, pw, at, nslots,
+               (uint64_t)nchunks, chunk, out);
+    SST_LAUNCH(k_tcv_half, (unsigned)((k + tb - 1) / tb), tb, 0, s, out, k);
+    return cudaGetLastError();
+  };
+  if (e == cudaSuccess && items)
+    e = tcv_wide(items * 32) ? pairs(uint64_t{0}) : pairs(uint32_t{0});
+  for (void *p : {(void *)loff, (void *)pq, (void *)pw, cost, coff})
     if (p) cudaFreeAsync(p, s);
   SST_CUDA_TRY(e);
   return SST_OK;

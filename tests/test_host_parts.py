@@ -3,8 +3,9 @@
 The search kernels' grid barrier: a search of more levels than 32 bits of
 arrivals count (15 million, a path) still waits at every barrier.  The words
 that every traversal uses: an allocation that fails leaves none of them.  The
-PageRank kernels' inline loads: volatile, or nothing keeps them after the wait
-for the kernel whose results they read."""
+chunks of triangles at listed vertices: their sum fits its type.  The PageRank
+kernels' inline loads: volatile, or nothing keeps them after the wait for the
+kernel whose results they read."""
 import os
 import re
 import subprocess
@@ -15,7 +16,8 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.mark.parametrize("name,says", [("barrier_check", "barrier ok"),
-                                       ("travwords_check", "words ok")])
+                                       ("travwords_check", "words ok"),
+                                       ("tcvrule_check", "rule ok")])
 def test_part(tmp_path, name, says):
     out = os.path.join(str(tmp_path), name)
     subprocess.run(["g++", "-std=c++17", "-O1", os.path.join(ROOT, "tests", "cpp", name + ".cpp"),
