@@ -2650,6 +2650,99 @@ static sst_status read_plan(sst_graph *g, PlanSummary *ps) {
   return SST_OK;
 }
 
+// the streams and events of an update's parallel branches
+static sst_status update_streams(sst_graph *g) {
+  if (!g->side) {
+    SST_CUDA_TRY(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
+    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->fork_ev, cudaEventDisableTiming));
+    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->merge_done, cudaEventDisableTiming));
+  }
+  if (!g->aux_fork) {
+    for (int k = 0; k < 2; k++) {
+      SST_CUDA_TRY(cudaStreamCreateWithFlags(&g->aux[k], cudaStreamNonBlocking));
+      SST_CUDA_TRY(cudaEventCreateWithFlags(&g->aux_join[k], cudaEventDisableTiming));
+    }
+    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->aux_fork, cudaEventDisableTiming));
+  }
+  return SST_OK;
+}
+
+// run k independent pieces of work on aux[0..k-1] beside the stream
+static cudaError_t aux_fork(sst_graph *g, cudaStream_t from, int k) {
+  cudaError_t e = cudaEventRecord(g->aux_fork, from);
+  for (int i = 0; i < k && e == cudaSuccess; i++)
+    e = cudaStreamWaitEvent(g->aux[i], g->aux_fork, 0);
+  return e;
+}
+static cudaError_t aux_join(sst_graph *g, cudaStream_t to, int k) {
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < k && e == cudaSuccess; i++) {
+    e = cudaEventRecord(g->aux_join[i], g->aux[i]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(to, g->aux_join[i], 0);
+  }
+  return e;
+}
+
+// 9b: a plan's window / resize tasks, with their staging
+static sst_status apply_tasks(sst_graph *g, Tasks T, const PlanSummary &ps, bool insert,
+                              const uint64_t *p_ul, const uint32_t *p_x, uint32_t *itask,
+                              const ClassStarts &cstart) {
+  cudaStream_t s = g->stream;
+  const DGraph dg = g->view();
+  // staging for window / resize tasks
+  size_t wneed = ps.task_elems * (g->weighted ? 8 : 4) + ps.src_leaves * 20 +
+                 ps.dst_leaves * 4 + scan_scratch_bytes(ps.src_leaves, 8) + 4096;
+  if (wneed > g->work.cap) {
+    sst_status st = budget_check(g, wneed - g->work.cap);
+    if (st != SST_OK) return st;
+  }
+  SST_CUDA_TRY(g->work.reserve(wneed));
+  g->work.reset();
+  uint32_t *stage = g->work.take<uint32_t>(ps.task_elems);
+  if (g->weighted) T.stage_v = g->work.take<uint32_t>(ps.task_elems);
+  uint64_t *scnt = g->work.take<uint64_t>(ps.src_leaves);
+  uint64_t *spre = g->work.take<uint64_t>(ps.src_leaves);
+  uint32_t *stask = g->work.take<uint32_t>(ps.src_leaves);
+  uint32_t *dtask = g->work.take<uint32_t>(ps.dst_leaves);
+  uint32_t *const titem = insert && ps.n_tasks && ps.n_items ? itask : nullptr;
+  if (!ps.n_tasks) return SST_OK;
+  // eight lanes a task (k_task_index) and a leaf (k_gather_old,
+  // k_task_scatter); the new ids' gather writes other staging slots than
+  // the old ids', so it runs beside it on an aux stream
+  SST_LAUNCH_PDL(k_task_index, blocks_for(8 * (uint64_t)ps.n_tasks), kTB, 0, s, dg, T,
+             ps.n_tasks, stask, dtask, titem, scnt);
+  if (ps.src_leaves)
+    SST_CUDA_TRY((scan<uint64_t, OpAdd>(scnt, spre, ps.src_leaves, 0ull,
+                                        OpAdd{}, true, false, nullptr,
+                                        g->work, s)));
+  const bool gnew = insert && ps.n_items;
+  if (gnew && ps.src_leaves) {
+    SST_CUDA_TRY(aux_fork(g, s, 1));
+    SST_LAUNCH_PDL(k_gather_new, blocks_for(ps.n_items), kTB, 0, g->aux[0], dg, T,
+               ps.n_tasks, spre, p_ul, p_x, ps.n_items, stage, titem);
+  } else if (gnew) {
+    SST_LAUNCH_PDL(k_gather_new, blocks_for(ps.n_items), kTB, 0, s, dg, T,
+               ps.n_tasks, spre, p_ul, p_x, ps.n_items, stage, titem);
+  }
+  if (ps.src_leaves)
+    SST_LAUNCH_PDL(k_gather_old, blocks_for(8 * ps.src_leaves), kTB, 0, s, dg, T,
+               ps.n_tasks, ps.src_leaves, spre, p_x, stage, stask);
+  if (gnew && ps.src_leaves) SST_CUDA_TRY(aux_join(g, s, 1));
+  if (ps.dst_leaves)
+    SST_LAUNCH_PDL(k_task_scatter, blocks_for(8 * ps.dst_leaves), kTB, 0, s, dg, T,
+               ps.n_tasks, ps.dst_leaves, cstart, stage, dtask);
+  SST_LAUNCH_PDL(k_finalize, blocks_for(ps.n_tasks), kTB, 0, s, dg, T, ps.n_tasks,
+             cstart);
+  return SST_OK;
+}
+
+// Leaves that a small batch's tasks may read and write in the cluster that applies
+// it: beyond, a task's eight lanes, which add up its leaves one after another, and
+// eight blocks take longer than the general sequence's six launches.  One batch that
+// resizes a row of 16,384 leaves: by the cluster 489 us, by grids 224 (the general
+// sequence 263); of 4,096 leaves 163 and 101; of 512 leaves 100 either way.
+constexpr uint64_t kSmallLeaves = 1024;
+
 // One pass of up to kSmallBatch raw pairs on an unweighted graph, in three
 // launches (see k_small_locate); same result as run_pipeline.
 static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, bool insert,
@@ -2697,17 +2790,23 @@ static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, b
   sst_status rst = read_plan(g, &ps);
   if (rst != SST_OK) return rst;
   if (n_invalid) *n_invalid = ps.invalid;
-  const size_t wneed = ps.task_elems * 4 + ps.src_leaves * 12 + ps.dst_leaves * 4 + 4096;
-  if (wneed > g->work.cap) {
-    sst_status st = budget_check(g, wneed - g->work.cap);
-    if (st != SST_OK) return st;
+  // long rows: the tasks take the general sequence's grids (see kSmallLeaves)
+  const bool grids = ps.src_leaves + ps.dst_leaves > kSmallLeaves;
+  uint32_t *stage = nullptr, *stask = nullptr, *dtask = nullptr;
+  uint64_t *spre = nullptr;
+  if (!grids) {
+    const size_t wneed = ps.task_elems * 4 + ps.src_leaves * 12 + ps.dst_leaves * 4 + 4096;
+    if (wneed > g->work.cap) {
+      sst_status st = budget_check(g, wneed - g->work.cap);
+      if (st != SST_OK) return st;
+    }
+    SST_CUDA_TRY(g->work.reserve(wneed));
+    g->work.reset();
+    stage = g->work.take<uint32_t>(ps.task_elems);
+    spre = g->work.take<uint64_t>(ps.src_leaves);
+    stask = g->work.take<uint32_t>(ps.src_leaves);
+    dtask = g->work.take<uint32_t>(ps.dst_leaves);
   }
-  SST_CUDA_TRY(g->work.reserve(wneed));
-  g->work.reset();
-  uint32_t *stage = g->work.take<uint32_t>(ps.task_elems);
-  uint64_t *spre = g->work.take<uint64_t>(ps.src_leaves);
-  uint32_t *stask = g->work.take<uint32_t>(ps.src_leaves);
-  uint32_t *dtask = g->work.take<uint32_t>(ps.dst_leaves);
   auto apply = [&](uint32_t nmerge, uint32_t ntasks, const ClassStarts &cs) {
     SST_LAUNCH_PDL(k_small_apply, kApplyCtas, kSmallThreads, 0, s, g->view(), T, cs, nmerge,
                    ntasks, ps.n_items, (uint32_t)ps.src_leaves, (uint32_t)ps.dst_leaves, p_ul,
@@ -2723,7 +2822,13 @@ static sst_status run_small(sst_graph *g, const uint32_t *d_pairs, uint32_t b, b
     if (st != SST_OK) return st;
   }
   const ClassStarts cs = plan_class_starts(g, ps);
-  if (nmerge || ps.n_tasks) apply(nmerge, ps.n_tasks, cs);
+  const uint32_t ntasks = grids ? 0 : ps.n_tasks;
+  if (nmerge || ntasks) apply(nmerge, ntasks, cs);
+  if (grids) {
+    sst_status st = update_streams(g);
+    if (st == SST_OK) st = apply_tasks(g, T, ps, insert, p_ul, p_x, itask, cs);
+    if (st != SST_OK) return st;
+  }
   SST_CUDA_TRY(cudaGetLastError());
   if (insert)
     g->m += ps.n_items;
@@ -2940,33 +3045,10 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
     join.ev = g->merge_done;
     return SST_OK;
   };
-  if (!g->side) {
-    SST_CUDA_TRY(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
-    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->fork_ev, cudaEventDisableTiming));
-    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->merge_done, cudaEventDisableTiming));
-  }
-  if (!g->aux_fork) {
-    for (int k = 0; k < 2; k++) {
-      SST_CUDA_TRY(cudaStreamCreateWithFlags(&g->aux[k], cudaStreamNonBlocking));
-      SST_CUDA_TRY(cudaEventCreateWithFlags(&g->aux_join[k], cudaEventDisableTiming));
-    }
-    SST_CUDA_TRY(cudaEventCreateWithFlags(&g->aux_fork, cudaEventDisableTiming));
-  }
-  // run k independent pieces of work on aux[0..k-1] beside the stream
-  auto fork_aux = [&](cudaStream_t from, int k) -> cudaError_t {
-    cudaError_t e = cudaEventRecord(g->aux_fork, from);
-    for (int i = 0; i < k && e == cudaSuccess; i++)
-      e = cudaStreamWaitEvent(g->aux[i], g->aux_fork, 0);
-    return e;
-  };
-  auto join_aux = [&](cudaStream_t to, int k) -> cudaError_t {
-    cudaError_t e = cudaSuccess;
-    for (int i = 0; i < k && e == cudaSuccess; i++) {
-      e = cudaEventRecord(g->aux_join[i], g->aux[i]);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(to, g->aux_join[i], 0);
-    }
-    return e;
-  };
+  sst_status ust = update_streams(g);
+  if (ust != SST_OK) return ust;
+  auto fork_aux = [&](cudaStream_t from, int k) { return aux_fork(g, from, k); };
+  auto join_aux = [&](cudaStream_t to, int k) { return aux_join(g, to, k); };
 
   // 2-8: sort to plan.  For a given batch size and graph layout this is a
   // fixed sequence of launches over device-resident counts; `fork` starts
@@ -3124,53 +3206,9 @@ static sst_status run_pipeline(sst_graph *g, const uint32_t *d_pairs,
   }
   const ClassStarts cstart = plan_class_starts(g, ps);
 
-  // staging for window / resize tasks
-  size_t wneed = ps.task_elems * (g->weighted ? 8 : 4) + ps.src_leaves * 20 +
-                 ps.dst_leaves * 4 + scan_scratch_bytes(ps.src_leaves, 8) + 4096;
-  if (wneed > g->work.cap) {
-    sst_status st = budget_check(g, wneed - g->work.cap);
-    if (st != SST_OK) return st;
-  }
-  SST_CUDA_TRY(g->work.reserve(wneed));
-  g->work.reset();
-  uint32_t *stage = g->work.take<uint32_t>(ps.task_elems);
-  if (g->weighted) T.stage_v = g->work.take<uint32_t>(ps.task_elems);
-  uint64_t *scnt = g->work.take<uint64_t>(ps.src_leaves);
-  uint64_t *spre = g->work.take<uint64_t>(ps.src_leaves);
-  uint32_t *stask = g->work.take<uint32_t>(ps.src_leaves);
-  uint32_t *dtask = g->work.take<uint32_t>(ps.dst_leaves);
-  uint32_t *const titem = insert && ps.n_tasks && ps.n_items ? itask : nullptr;
-
   // 9b: apply the window / resize tasks
-  if (ps.n_tasks) {
-    // eight lanes a task (k_task_index) and a leaf (k_gather_old,
-    // k_task_scatter); the new ids' gather writes other staging slots than
-    // the old ids', so it runs beside it on an aux stream
-    SST_LAUNCH_PDL(k_task_index, blocks_for(8 * (uint64_t)ps.n_tasks), kTB, 0, s, dg, T,
-               ps.n_tasks, stask, dtask, titem, scnt);
-    if (ps.src_leaves)
-      SST_CUDA_TRY((scan<uint64_t, OpAdd>(scnt, spre, ps.src_leaves, 0ull,
-                                          OpAdd{}, true, false, nullptr,
-                                          g->work, s)));
-    const bool gnew = insert && ps.n_items;
-    if (gnew && ps.src_leaves) {
-      SST_CUDA_TRY(fork_aux(s, 1));
-      SST_LAUNCH_PDL(k_gather_new, blocks_for(ps.n_items), kTB, 0, g->aux[0], dg, T,
-                 ps.n_tasks, spre, p_ul, p_x, ps.n_items, stage, titem);
-    } else if (gnew) {
-      SST_LAUNCH_PDL(k_gather_new, blocks_for(ps.n_items), kTB, 0, s, dg, T,
-                 ps.n_tasks, spre, p_ul, p_x, ps.n_items, stage, titem);
-    }
-    if (ps.src_leaves)
-      SST_LAUNCH_PDL(k_gather_old, blocks_for(8 * ps.src_leaves), kTB, 0, s, dg, T,
-                 ps.n_tasks, ps.src_leaves, spre, p_x, stage, stask);
-    if (gnew && ps.src_leaves) SST_CUDA_TRY(join_aux(s, 1));
-    if (ps.dst_leaves)
-      SST_LAUNCH_PDL(k_task_scatter, blocks_for(8 * ps.dst_leaves), kTB, 0, s, dg, T,
-                 ps.n_tasks, ps.dst_leaves, cstart, stage, dtask);
-    SST_LAUNCH_PDL(k_finalize, blocks_for(ps.n_tasks), kTB, 0, s, dg, T, ps.n_tasks,
-               cstart);
-  }
+  ust = apply_tasks(g, T, ps, insert, p_ul, p_x, itask, cstart);
+  if (ust != SST_OK) return ust;
   join.wait();
   // the staging-rank check of this batch is read back with the next plan
   // (or by sst_sync), so a batch ends without a second host synchronisation

@@ -135,3 +135,35 @@ def test_device_and_pinned_pairs(sg, offset):
         g.insert_batch(buf[offset:offset + 2 * b])
         o.insert_batch(e)
         same(g, o)
+
+
+# rows whose tasks the cluster applies, and whose tasks take grids (1024 leaves
+# read and written in all), grown past a resize and shrunk below one
+@pytest.mark.parametrize("cap", [1 << 13, 1 << 14, 1 << 15, 1 << 17])
+def test_long_row(sg, cap):
+    n, b = 2 * cap, 900
+    rng = np.random.default_rng(cap)
+    p = rng.permutation(n).astype(np.uint32)
+    g, o = sg.SparseMatrixV(n), oracle.OracleGraph(n)
+
+    def step(op, cols):
+        e = np.stack([np.full(len(cols), 3, np.uint32), cols], 1)
+        other = rng.integers(0, n, (1000 - b, 2)).astype(np.uint32) if len(cols) <= b else e[:0]
+        e = np.concatenate([e, other])
+        e = e[e[:, 0] != e[:, 1]]
+        for m in (g, o):
+            getattr(m, op)(e)
+
+    at = int(0.84 * cap)
+    step("insert_batch", p[:at])
+    for _ in range(cap // 4 // b + 3 if cap <= 1 << 15 else 4):
+        step("insert_batch", p[at:at + b])
+        at += b
+    same(g, o)
+    keep = int(0.2 * 2 * cap) + 2 * b
+    step("remove_batch", p[keep:at])
+    for _ in range(4):
+        step("remove_batch", p[keep - b:keep])
+        keep -= b
+    same(g, o)
+    g.close()
