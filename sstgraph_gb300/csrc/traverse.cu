@@ -1327,6 +1327,8 @@ static sst_status coop_grid(const sst_graph *g, const void *kernel, uint64_t thr
   return SST_OK;
 }
 
+constexpr uint32_t kVertsPerThread = 8;
+
 // A search's arguments over the graph's work lists, and its grid (see
 // bfslevels.cuh).  d_depths may be null (a temporary), d_parents too (none).
 static sst_status bfs_setup(sst_graph *g, uint32_t src, int32_t *d_parents, int32_t *d_depths,
@@ -1350,7 +1352,12 @@ static sst_status bfs_setup(sst_graph *g, uint32_t src, int32_t *d_parents, int3
                d_depths,    d_parents,  t->fbits.p,  t->qa.p,      t->qitems.p,
                max_items,   reinterpret_cast<BfsCtl *>(t->d_bfs),
                reinterpret_cast<unsigned long long *>(t->h_small)};
-  return coop_grid(g, kernel, std::max(t->nsmall, 32 * t->nchunks), grid);
+  // and a thread for eight vertices: the search clears and scans arrays of all
+  // vertices, whatever the rows hold (2,000 rows in use of 2^24: BFS 1.3 ms by the
+  // five blocks that the rows alone ask for, 0.12 by these; 4 to 32 vertices a thread
+  // alike)
+  const uint64_t work = std::max<uint64_t>({t->nsmall, 32 * t->nchunks, n / kVertsPerThread});
+  return coop_grid(g, kernel, work, grid);
 }
 
 // waits for a search and reports its error
