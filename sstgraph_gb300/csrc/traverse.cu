@@ -1437,8 +1437,11 @@ sst_status bc(sst_graph *g, uint32_t src, double *d_dep) {
   if (st != SST_OK) return st;
   TravState *t = g->trav;
   const uint64_t n = g->n;
-  SST_CUDA_TRY(t->sigma.exact(2 * n));
-  SST_CUDA_TRY(t->ratio.exact(2 * n));
+  for (DevBuf<double> *buf : {&t->sigma, &t->ratio}) {
+    if (buf->cap >= 2 * n) continue;
+    SST_CUDA_TRY(buf->exact(2 * n));
+    SST_CUDA_TRY(cudaMemsetAsync(buf->p, 0, 16 * n, g->stream));
+  }
   SST_CUDA_TRY(t->levels.exact(n + 1));
   SST_CUDA_TRY(t->qb.ensure(t->nbig + 1));
   // a hub's chunks of kBcLeaves leaves are at most its chunks in the lists
@@ -1449,7 +1452,8 @@ sst_status bc(sst_graph *g, uint32_t src, double *d_dep) {
   const BcArgs b{t->sigma.p,    t->ratio.p,        d_dep,        t->big.p,
                  t->nbig,       hubs,              t->hub.p,     t->hub.p + hubs,
                  t->partial.p,  t->hub_done.p,     t->qb.p,
-                 reinterpret_cast<BcCtl *>(a.ctl + 1), t->levels.p};
+                 reinterpret_cast<BcCtl *>(a.ctl + 1),
+                 bc_few(t->nsmall + t->nbig, n),   t->levels.p};
   SST_CUDA_TRY(launch_coop("k_bc_levels", k_bc_levels, grid, kCoopThreads, g->stream, a, b));
   return bfs_finish(g, "BC");
 }

@@ -1,6 +1,7 @@
 """Searches of graphs most of whose vertices have no edge: the arrays of all
-vertices are cleared and read whatever the rows in use.  Against the CPU oracle,
-before and after updates that fill the rows and back."""
+vertices are cleared and read whatever the rows in use, and where those are few
+(below an eighth) BC clears theirs alone.  Against the CPU oracle, before and
+after updates that take the graph past that share and back."""
 import numpy as np
 import pytest
 
