@@ -116,16 +116,18 @@ __global__ void __launch_bounds__(1024) k_cc_giant(const uint32_t *__restrict__ 
 // ancestor): most chains end at one hot root, and loads of it past L1 queue at
 // its L2 slice (2e6 vertices already compressed: 16 us that way, 8 us
 // this way).
+__device__ __forceinline__ void cc_compress(uint32_t *par, uint32_t v) {
+  const uint32_t p = par[v];
+  uint32_t x = p, q;
+  while ((q = par[x]) != x) x = q;
+  if (x != p) par[v] = x;
+}
 __global__ void k_cc_compress(uint32_t *par, uint32_t n,
                               const unsigned long long *__restrict__ hooks) {
   pdl_wait();
   if (hooks && *hooks == 0) return;
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  const uint32_t p = par[v];
-  uint32_t x = p, q;
-  while ((q = par[x]) != x) x = q;
-  if (x != p) par[v] = x;
+  if (v < n) cc_compress(par, v);
 }
 
 }  // namespace

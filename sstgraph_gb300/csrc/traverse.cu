@@ -731,15 +731,36 @@ __global__ void k_front_expand(const uint32_t *__restrict__ q, uint32_t qn,
 // and 14e6 stored edges, where a whole call takes 172 us now.  The rounds
 // are bound by scattered 32-byte sectors: a row's first ids (read once, here),
 // and two parents a vertex and round.
+// The passes go over all vertices, or, where fewer than half of them have a row,
+// over the work lists' entries (a vertex without a row is its own root from the
+// start).  Of 2^24 vertices 2,000 with a row: 474 us over all, 91 over those (the
+// sampled links by find before took 309); of 2^22 one in 16 with a row 167 and 116,
+// one in 4 200 and 160, one in 2 247 and 233, nearly all alike.
+struct CcVerts {
+  const uint32_t *small, *big;  // null: every vertex
+  uint32_t nsmall, count;
+  __device__ __forceinline__ uint32_t operator[](uint32_t i) const {
+    return !small ? i : i < nsmall ? small[i] : big[i - nsmall];
+  }
+};
+__global__ void k_cc_compress_some(CcVerts vs, uint32_t *par,
+                                   const unsigned long long *__restrict__ hooks) {
+  pdl_wait();
+  if (hooks && *hooks == 0) return;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < vs.count) cc_compress(par, vs[i]);
+}
+
 // The start: every vertex below its smallest neighbour (rows ascend), if that
 // is smaller.  A parent is smaller than its child, so the links are a forest.
 // nb1 and nb2 keep what is left of its first two neighbours' edges for the rounds
 // (kEmpty: none): the second, and the smallest if it is larger than u.
-__global__ void k_cc_hook_first(DGraph g, uint32_t *__restrict__ par,
+__global__ void k_cc_hook_first(DGraph g, CcVerts vs, uint32_t *__restrict__ par,
                                 uint32_t *__restrict__ nb1, uint32_t *__restrict__ nb2) {
   pdl_wait();
-  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= g.n) return;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= vs.count) return;
+  const uint32_t u = vs[i];
   const uint32_t cap = g.cap[u];
   uint4 x = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
   if (cap >= 4) {  // starts on a 16-byte boundary; slots past the ids hold kEmpty
@@ -750,8 +771,8 @@ __global__ void k_cc_hook_first(DGraph g, uint32_t *__restrict__ par,
     if (cap > 1) x.y = p[1];
   }
   par[u] = min(u, x.x);
-  nb1[u] = x.y;
-  nb2[u] = x.x > u ? x.x : kEmpty;
+  nb1[i] = x.y;
+  nb2[i] = x.x > u ? x.x : kEmpty;
 }
 
 // A round, after a compression: of the roots of u and its two kept neighbours
@@ -771,20 +792,21 @@ __global__ void k_cc_hook_first(DGraph g, uint32_t *__restrict__ par,
 // once.
 // The parents come through L1: nearly all are one hot root, whose loads would
 // queue at one L2 slice, and a stale one is an ancestor too.
+constexpr uint32_t kCcFew = 2;  // fewer rows than one vertex in 2: over the lists
 constexpr uint32_t kCcSampledN = 1u << 17;
 constexpr int kCcMaxRounds = 3;
 constexpr uint32_t kCcStride[2][kCcMaxRounds] = {{1, 0, 0}, {1, 32, 512}};
-__global__ void k_cc_hook(const uint32_t *__restrict__ nb1, const uint32_t *__restrict__ nb2,
-                          uint32_t n, uint32_t stride, uint32_t *par,
+__global__ void k_cc_hook(CcVerts vs, const uint32_t *__restrict__ nb1,
+                          const uint32_t *__restrict__ nb2, uint32_t stride, uint32_t *par,
                           const unsigned long long *__restrict__ before,
                           unsigned long long *__restrict__ hooks) {
   pdl_wait();
   if (before && *before == 0) return;
-  const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * stride;
+  const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * stride;
   bool hooked = false;
-  if (u < n) {
-    const uint32_t x = nb1[u], y = nb2[u];
-    const uint32_t a = par[u];
+  if (i < vs.count) {
+    const uint32_t x = nb1[i], y = nb2[i];
+    const uint32_t a = par[vs[(uint32_t)i]];
     const uint32_t b = x != kEmpty ? par[x] : a;
     const uint32_t c = y != kEmpty ? par[y] : a;
     const uint32_t m = min(a, min(b, c));
@@ -799,14 +821,15 @@ __global__ void k_cc_hook(const uint32_t *__restrict__ nb1, const uint32_t *__re
 // The kept edges that the rounds have not joined, by find and compare-and-swap:
 // afterwards the trees are the components of every vertex's first two edges, in
 // whatever order the hooks went.
-__global__ void k_cc_link_kept(const uint32_t *__restrict__ nb1, const uint32_t *__restrict__ nb2,
-                               uint32_t n, uint32_t *par, unsigned long long *__restrict__ hooks,
+__global__ void k_cc_link_kept(CcVerts vs, const uint32_t *__restrict__ nb1,
+                               const uint32_t *__restrict__ nb2, uint32_t *par,
+                               unsigned long long *__restrict__ hooks,
                                unsigned long long *__restrict__ err) {
   pdl_wait();
-  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   bool linked = false;
-  if (u < n) {
-    const uint32_t x = nb1[u], y = nb2[u], a = par[u];
+  if (i < vs.count) {
+    const uint32_t u = vs[i], x = nb1[i], y = nb2[i], a = par[u];
     const uint32_t b = x != kEmpty ? par[x] : a, c = y != kEmpty ? par[y] : a;
     if (b != a) cc_link(par, u, x, err);
     if (c != a) cc_link(par, u, y, err);
@@ -1395,20 +1418,29 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
   SST_CUDA_TRY(t->qb.exact((uint64_t)n + 1));
   SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, (3 + kCcMaxRounds) * 8, s));
   const DGraph dg = g->view();
-  SST_LAUNCH_PDL(k_cc_hook_first, blocks_for(n), kTB, 0, s, dg, par, t->qa.p, t->qb.p);
-  SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n,
-                 static_cast<const unsigned long long *>(nullptr));
-  const bool sampled = n >= kCcSampledN;
+  const uint64_t rows = t->nsmall + t->nbig;
+  const bool few = rows < n / kCcFew;
+  const CcVerts vs = few ? CcVerts{t->small.p, t->big.p, (uint32_t)t->nsmall, (uint32_t)rows}
+                         : CcVerts{nullptr, nullptr, 0, n};
+  auto compress = [&](const unsigned long long *if_set) {
+    if (few)
+      SST_LAUNCH_PDL(k_cc_compress_some, blocks_for(vs.count), kTB, 0, s, vs, par, if_set);
+    else
+      SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, if_set);
+  };
+  if (few) SST_LAUNCH(k_iota, blocks_for(n), kTB, 0, s, par, n);
+  SST_LAUNCH_PDL(k_cc_hook_first, blocks_for(vs.count), kTB, 0, s, dg, vs, par, t->qa.p, t->qb.p);
+  compress(nullptr);
+  const bool sampled = vs.count >= kCcSampledN;
   for (int r = 0; r < (sampled ? kCcMaxRounds : 1); r++) {
     const uint32_t stride = kCcStride[sampled][r];
-    SST_LAUNCH_PDL(k_cc_hook, blocks_for((n + stride - 1) / stride), kTB, 0, s, t->qa.p,
-                   t->qb.p, n, stride, par, r ? hooks + std::min(r - 1, 1) : nullptr,
-                   hooks + r);
-    SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, hooks + r);
+    SST_LAUNCH_PDL(k_cc_hook, blocks_for((vs.count + stride - 1) / stride), kTB, 0, s, vs, t->qa.p,
+                   t->qb.p, stride, par, r ? hooks + std::min(r - 1, 1) : nullptr, hooks + r);
+    compress(hooks + r);
   }
-  SST_LAUNCH_PDL(k_cc_link_kept, blocks_for(n), kTB, 0, s, t->qa.p, t->qb.p, n, par,
+  SST_LAUNCH_PDL(k_cc_link_kept, blocks_for(vs.count), kTB, 0, s, vs, t->qa.p, t->qb.p, par,
                  hooks + kCcMaxRounds, err);
-  SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, hooks + kCcMaxRounds);
+  compress(hooks + kCcMaxRounds);
   SST_LAUNCH_PDL(k_cc_giant, 1, 1024, 0, s, par, n, giant);
   if (t->nsmall)
     SST_LAUNCH_PDL(k_cc_rest_small, blocks_for(t->nsmall), kTB, 0, s, dg, t->sdesc.p,
@@ -1416,8 +1448,7 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
   if (t->nchunks)
     SST_LAUNCH_PDL(k_cc_rest_chunks, warp_blocks(t->nchunks), kTB, 0, s, dg, t->cdesc.p,
                t->cv.p, t->nchunks, giant, par, err);
-  SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n,
-                 static_cast<const unsigned long long *>(nullptr));
+  compress(nullptr);
   SST_CUDA_TRY(cudaMemcpyAsync(t->h_small, t->d_small, 16, cudaMemcpyDeviceToHost, s));
   SST_CUDA_TRY(cudaStreamSynchronize(s));
   SST_CUDA_TRY(cudaGetLastError());

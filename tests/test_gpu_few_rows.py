@@ -1,7 +1,8 @@
 """Searches of graphs most of whose vertices have no edge: the arrays of all
 vertices are cleared and read whatever the rows in use, and where those are few
-(below an eighth) BC clears theirs alone.  Against the CPU oracle, before and
-after updates that take the graph past that share and back."""
+(below an eighth) BC clears theirs alone and (below a half) components pass over
+them alone.  Against the CPU oracle, before and after updates that take the graph
+past those shares and back."""
 import numpy as np
 import pytest
 
@@ -27,12 +28,12 @@ def compare(sg, g, o, srcs):
     assert np.array_equal(sg.CC(g), o.cc())
 
 
-# rows in use of all: none, one edge, below an eighth, just above
+# rows in use of all: none, one edge, one in 40, below and above an eighth and a half
 @pytest.mark.parametrize("n", [4096, (1 << 17) - 1, (1 << 18) + 7])
-@pytest.mark.parametrize("share", [0, 2, 40, 9, 7])
+@pytest.mark.parametrize("share", [0, 2, 40, 9, 7, 1.9, 1.1])
 def test_share_in_use(sg, n, share):
-    rng = np.random.default_rng(n + share)
-    used = rng.permutation(n)[: (0 if share == 0 else 2 if share == 2 else n // share)]
+    rng = np.random.default_rng(n + int(10 * share))
+    used = rng.permutation(n)[: (0 if share == 0 else 2 if share == 2 else int(n / share))]
     g, o = sg.SparseMatrixV(n), oracle.OracleGraph(n)
     idle = int(np.setdiff1d(np.arange(n), used)[0])
 
