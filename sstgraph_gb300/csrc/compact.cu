@@ -775,11 +775,13 @@ __global__ void k_ctc_fill(const uint32_t *__restrict__ cols, const uint32_t *__
   if (e < m && keep[e]) adj[pos[e]] = cols[e];
 }
 
-// a row's oriented list starts where its first kept id lands
-__global__ void k_ctc_off(const uint64_t *__restrict__ off, const uint32_t *__restrict__ pos,
-                          uint32_t n, uint64_t m, uint64_t *__restrict__ doff) {
+// a row's oriented list (tcshared.cuh) starts where its first kept id lands
+__global__ void k_ctc_desc(const uint64_t *__restrict__ off, const uint32_t *__restrict__ pos,
+                           uint32_t n, uint64_t m, uint64_t *__restrict__ desc) {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v <= n) doff[v] = pos[off[v] < m ? off[v] : m];
+  if (v >= n) return;
+  const uint64_t b = pos[off[v] < m ? off[v] : m], e = pos[off[v + 1] < m ? off[v + 1] : m];
+  desc[v] = b << kTcLenBits | (e - b);
 }
 
 // ---- betweenness (Brandes) over the decoded rows, level by level
@@ -1228,22 +1230,21 @@ sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) 
     set_error_message("sst_compact_tc: more than 2^32 stored edges");
     return SST_EINVAL;
   }
-  uint64_t *off = nullptr, *doff = nullptr;
+  uint64_t *off = nullptr, *desc = nullptr, *items = nullptr;
   uint32_t *cols = nullptr, *keep = nullptr, *pos = nullptr, *adj = nullptr;
   uint32_t *icnt = nullptr, *ioff = nullptr;
-  uint64_t *items = nullptr, *desc = nullptr;
   cudaError_t e = cudaMalloc(&off, ((uint64_t)n + 1) * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&doff, ((uint64_t)n + 1) * 8);
+  if (e == cudaSuccess) e = cudaMalloc(&desc, (uint64_t)n * 8);
   if (e == cudaSuccess) e = cudaMalloc(&cols, m * 4);
   if (e == cudaSuccess) e = cudaMalloc(&keep, m * 4);
   if (e == cudaSuccess) e = cudaMalloc(&pos, (m + 1) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&adj, m * 4);
   if (e == cudaSuccess) e = cudaMalloc(&icnt, ((uint64_t)n + 1) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&ioff, ((uint64_t)n + 1) * 4);
-  // an item per started batch of 32 of a row
-  const uint64_t max_items = m / kTcBatch + n;
+  // an item per started batch of 32 of a row with entries (the oriented lists have
+  // fewer)
+  const uint64_t max_items = m / kTcBatch + std::min<uint64_t>(n, m) + 1;
   if (e == cudaSuccess) e = cudaMalloc(&items, max_items * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&desc, (uint64_t)n * 8);
   if (e == cudaSuccess) {
     st = compact_to_csr(c, off, cols);
     if (st == SST_OK) {
@@ -1257,18 +1258,31 @@ sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) 
         e = scan<uint32_t, OpAdd>(keep, pos, m, 0u, OpAdd{}, true, false, pos + m, A, s);
         if (e == cudaSuccess) {
           SST_LAUNCH(k_ctc_fill, blocks_for(m), kTB, 0, s, cols, keep, pos, m, adj);
-          SST_LAUNCH(k_ctc_off, blocks_for((uint64_t)n + 1), kTB, 0, s, off, pos, n, m, doff);
+          SST_LAUNCH(k_ctc_desc, blocks_for(n), kTB, 0, s, off, pos, n, m, desc);
           e = cudaMemsetAsync(c->d_cnt, 0, 16, s);  // count, work cursor
           A.reset();
-          if (e == cudaSuccess) {
-            SST_LAUNCH(k_tc_desc, blocks_for(n), kTB, 0, s, doff, n, desc);
+          bool by_rows = tc_few_items(max_items);
+          if (e == cudaSuccess && !by_rows) {
+            unsigned long long est[kTcSampleWords] = {};
+            unsigned long long *d_est = A.take<unsigned long long>(kTcSampleWords);
+            tc_sample_launch(TcKeptLists{desc, adj, n}, desc, d_pv != nullptr, nullptr, d_est, s);
+            e = cudaMemcpyAsync(est, d_est, sizeof(est), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            by_rows = tc_by_rows(est);
+          }
+          unsigned long long *const pv = reinterpret_cast<unsigned long long *>(d_pv);
+          if (e == cudaSuccess && by_rows) {
             SST_LAUNCH(k_tc_items_count, blocks_for(n), kTB, 0, s, off, desc, n, icnt);
             e = scan<uint32_t, OpAdd>(icnt, ioff, n, 0u, OpAdd{}, true, false, ioff + n, A, s);
-          }
-          if (e == cudaSuccess) {
-            SST_LAUNCH(k_tc_items_fill, blocks_for(n), kTB, 0, s, icnt, ioff, n, items);
-            e = tc_count_launch(TcRows{off, cols, items, ioff + n}, desc, adj, c->d_cnt,
-                                reinterpret_cast<unsigned long long *>(d_pv), sms, s);
+            if (e == cudaSuccess) {
+              SST_LAUNCH(k_tc_items_fill, blocks_for(n), kTB, 0, s, icnt, ioff, n, items);
+              e = tc_count_launch(TcRows{off, cols, items, ioff + n}, desc, adj, c->d_cnt, pv, sms,
+                                  s);
+            }
+          } else if (e == cudaSuccess) {
+            TcLists lists;
+            e = tc_list_items(desc, adj, n, m, icnt, ioff, items, A, s, &lists);
+            if (e == cudaSuccess) e = tc_count_launch(lists, desc, adj, c->d_cnt, pv, sms, s);
           }
           if (e == cudaSuccess)
             e = cudaMemcpyAsync(c->h_cnt, c->d_cnt, 8, cudaMemcpyDeviceToHost, s);
@@ -1278,7 +1292,7 @@ sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) 
       }
     }
   }
-  for (void *p : {(void *)off, (void *)doff, (void *)cols, (void *)keep, (void *)pos,
+  for (void *p : {(void *)off, (void *)cols, (void *)keep, (void *)pos,
                   (void *)adj, (void *)icnt, (void *)ioff, (void *)items, (void *)desc})
     if (p) cudaFree(p);
   if (st != SST_OK) return st;

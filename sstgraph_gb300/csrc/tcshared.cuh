@@ -117,11 +117,6 @@ constexpr int kTcLenBits = 24;
 __device__ __forceinline__ uint32_t tc_len(uint64_t d) {
   return (uint32_t)d & ((1u << kTcLenBits) - 1);
 }
-__global__ void k_tc_desc(const uint64_t *__restrict__ off, uint32_t n,
-                          uint64_t *__restrict__ desc) {
-  const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < n) desc[v] = (off[v] << kTcLenBits) | (off[v + 1] - off[v]);
-}
 
 // Which end of an edge takes the set: the one with the larger (key, id); a
 // list that does not fit a set comes last.
@@ -131,6 +126,7 @@ __device__ __forceinline__ uint32_t tc_key(uint32_t len) {
 
 // Work items over the leaves of a graph's leaf directory: an item is a leaf.
 struct TcLeaves {
+  static constexpr bool kOriented = false;
   const uint32_t *slots, *owner, *cnt;
   const uint64_t *slot;
   uint64_t n;
@@ -148,6 +144,7 @@ struct TcLeaves {
 // Work items over the rows of a CSR: an item is a batch of a row, listed as
 // (batch << 32) | row; rows without an oriented list have none.
 struct TcRows {
+  static constexpr bool kOriented = false;
   const uint64_t *off;
   const uint32_t *cols;
   const uint64_t *items;
@@ -166,13 +163,39 @@ struct TcRows {
   __device__ __forceinline__ uint32_t id(uint64_t at) const { return cols[at]; }
 };
 
-// per row: its number of work items
+// Work items over the oriented lists: an item is a batch of one, listed likewise;
+// lists of one entry have none (no triangle has its lowest vertex there).
+struct TcLists {
+  static constexpr bool kOriented = true;
+  const uint64_t *desc;
+  const uint32_t *adj;
+  const uint64_t *items;
+  const uint32_t *nitems;
+  struct Item {
+    uint32_t x, cnt;
+    uint64_t at;
+  };
+  __device__ __forceinline__ uint64_t count() const { return *nitems; }
+  __device__ __forceinline__ Item item(uint64_t k) const {
+    const uint64_t it = items[k];
+    const uint32_t x = (uint32_t)it, b = (uint32_t)(it >> 32) * kTcBatch;
+    const uint64_t d = desc[x];
+    const uint32_t left = tc_len(d) - b;
+    return Item{x, left < kTcBatch ? left : kTcBatch, (d >> kTcLenBits) + b};
+  }
+  __device__ __forceinline__ uint32_t id(uint64_t at) const { return adj[at]; }
+};
+
+// per row: its number of work items, of its own entries or (off null) of its
+// oriented list's
 __global__ void k_tc_items_count(const uint64_t *__restrict__ off,
                                  const uint64_t *__restrict__ desc, uint32_t n,
                                  uint32_t *__restrict__ cnt) {
   const uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n) return;
-  cnt[u] = tc_len(desc[u]) ? (uint32_t)((off[u + 1] - off[u] + kTcBatch - 1) / kTcBatch) : 0u;
+  const uint32_t len = tc_len(desc[u]);
+  const uint64_t entries = off ? off[u + 1] - off[u] : len;
+  cnt[u] = len >= (off ? 1u : 2u) ? (uint32_t)((entries + kTcBatch - 1) / kTcBatch) : 0u;
 }
 
 // per row: its items at its exclusive prefix ioff[u]
@@ -183,6 +206,104 @@ __global__ void k_tc_items_fill(const uint32_t *__restrict__ cnt,
   if (u >= n) return;
   const uint32_t c = cnt[u], o = ioff[u];
   for (uint32_t j = 0; j < c; j++) items[(uint64_t)o + j] = ((uint64_t)j << 32) | u;
+}
+
+// The two forms of the count.  By lists, the items are the oriented lists N+(u) and
+// the streams N+(v) of their entries v: every edge once, from its lower end.  By
+// rows, the items are whole rows, every edge is met from both ends, and the end with
+// the longer list takes the set: the streams are shorter, but the items are more than
+// twice as many.  Which is less work depends on whether the two lists differ: on
+// uniform graphs the upper end's is the shorter already.  So a sample of the kept
+// edges adds up what either would stream.  Times by rows / by lists (us), and the
+// rows' share of the lists' streams:
+//   RMAT a = .57, 2^18 vertices    494   773   .48     a = .40, 2^20    2265  2129   .72
+//   a = .45, 2^18                  336   354   .63     a = .35, 2^18     286   271   .83
+//   uniform 1e5, 6.4e6 stored      461   414   .99     2^22, 6.7e7      3412  3144   .97
+//   path of 2e6 (no stream)        501   325    -      complete, 1500   5566 12231  1.68
+// A probe of a list too long for the set is a binary search, some 20 times a hashed
+// one's time (the complete graph's share, weighed so, is .52); with counts by
+// vertex the atomics hide most of that (47.5 / 37.0 ms).
+constexpr uint32_t kTcSortedCost = 16, kTcSortedCostPv = 4;
+
+// the kept edges (x, y), x the lower end, of a graph's leaves and of oriented lists
+struct TcKeptLeaves {
+  const uint32_t *slots, *owner;
+  const uint64_t *slot;
+  const uint32_t *kmask;
+  uint64_t n;
+  template <class F>
+  __device__ __forceinline__ void each(uint64_t k, int lane, F f) const {
+    if ((kmask[k] >> lane) & 1u) f(owner[k], slots[slot[k] + lane]);
+  }
+};
+struct TcKeptLists {
+  const uint64_t *desc;
+  const uint32_t *adj;
+  uint64_t n;
+  template <class F>
+  __device__ __forceinline__ void each(uint64_t k, int lane, F f) const {
+    const uint64_t d = desc[k];
+    for (uint32_t i = lane; i < tc_len(d); i += 32) f((uint32_t)k, adj[(d >> kTcLenBits) + i]);
+  }
+};
+
+// Block b: est[2b] = the cost of the rows' form over the edges of its items, est[2b + 1]
+// = the lists' form's; est[2 * kTcSampleBlocks] = *also, a word the host reads with them.
+// A warp an item, every step-th one; sums a block, as atomics on one address queue.
+constexpr int kTcSampleBlocks = 28, kTcSampleThreads = 1024;
+constexpr uint64_t kTcSamples = kTcSampleBlocks * (kTcSampleThreads / 32);
+constexpr int kTcSampleWords = 2 * kTcSampleBlocks + 1;
+template <class Kept>
+__global__ void __launch_bounds__(kTcSampleThreads)
+k_tc_sample(Kept src, const uint64_t *__restrict__ desc, uint64_t step, uint32_t sorted_cost,
+            const uint64_t *__restrict__ also, unsigned long long *__restrict__ est) {
+  __shared__ unsigned long long s_est[2];
+  if (threadIdx.x < 2) s_est[threadIdx.x] = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const uint64_t k = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * step;
+  unsigned long long rows = 0, lists = 0;
+  if (k < src.n)
+    src.each(k, lane, [&](uint32_t x, uint32_t y) {
+      const uint32_t lx = tc_len(desc[x]), ly = tc_len(desc[y]);
+      auto cost = [&](uint32_t set, uint32_t stream) {
+        return (unsigned long long)stream * (tc_key(set) ? 1u : sorted_cost);
+      };
+      if (lx < 2) return;
+      lists += cost(lx, ly);
+      const uint32_t kx = tc_key(lx), ky = tc_key(ly);
+      const bool by_x = kx > ky || (kx == ky && x > y);
+      if (ly) rows += by_x ? cost(lx, ly) : cost(ly, lx);
+    });
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    rows += __shfl_xor_sync(0xffffffffu, rows, d);
+    lists += __shfl_xor_sync(0xffffffffu, lists, d);
+  }
+  if (lane == 0 && lists) {
+    atomicAdd(&s_est[0], rows);
+    atomicAdd(&s_est[1], lists);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) est[2 * blockIdx.x + threadIdx.x] = s_est[threadIdx.x];
+  if (blockIdx.x == 0 && threadIdx.x == 2 && also) est[2 * kTcSampleBlocks] = *also;
+}
+template <class Kept>
+inline void tc_sample_launch(const Kept &src, const uint64_t *desc, bool pv, const uint64_t *also,
+                             unsigned long long *est, cudaStream_t s) {
+  SST_LAUNCH(k_tc_sample<Kept>, kTcSampleBlocks, kTcSampleThreads, 0, s, src, desc,
+             (src.n + kTcSamples - 1) / kTcSamples, pv ? kTcSortedCostPv : kTcSortedCost, also, est);
+}
+// Whether a count of so many items by rows (leaves, or rows and started batches) takes
+// the rows' form unseen: it is done in the time of the launches that list the oriented
+// lists' items.
+inline bool tc_few_items(uint64_t items) { return items <= 1u << 14; }
+// Whether the rows' form is the one to take, by the sample's sums (host memory).
+template <class Word>
+inline bool tc_by_rows(const Word *est) {
+  uint64_t rows = 0, lists = 0;
+  for (int b = 0; b < kTcSampleBlocks; b++) rows += est[2 * b], lists += est[2 * b + 1];
+  return rows < lists / 100 * 68;
 }
 
 // items a warp takes per visit to the cursor; their descriptors load in
@@ -231,12 +352,12 @@ k_tc_count(Items src, const uint64_t *__restrict__ desc, const uint32_t *__restr
     // The item's y (stage 1) and their lists (stage 2) load ahead: y two items
     // before the item's turn, the lists one item before (they need y), so a
     // small item's three dependent loads overlap earlier items.  An x without
-    // a list has nothing to load.
+    // a list (of two entries, if it is the lower end) has nothing to load.
     auto load_y = [&](int g, bool &ok) -> uint32_t {
       const uint64_t at = __shfl_sync(full, my.at, g & 31);
       const uint32_t c = __shfl_sync(full, my.cnt, g & 31);
       const uint64_t d = __shfl_sync(full, my_d, g & 31);
-      ok = g < ng && (uint32_t)lane < c && tc_len(d);
+      ok = g < ng && (uint32_t)lane < c && tc_len(d) >= (Items::kOriented ? 2u : 1u);
       return ok ? src.id(at + lane) : 0u;
     };
     bool ok_n1 = false, ok_n2 = false;
@@ -248,13 +369,17 @@ k_tc_count(Items src, const uint64_t *__restrict__ desc, const uint32_t *__restr
       const uint64_t ud = __shfl_sync(full, my_d, gi);
       const uint32_t na = tc_len(ud);
       const uint32_t *A = adj + (ud >> kTcLenBits);
-      // this lane's y and its list, loaded ahead; x counts the edge if its own
-      // list is the set's
+      // this lane's y and its list, loaded ahead; of rows, x counts the edge if its
+      // own list is the set's
       uint32_t v = v_n1;
       uint64_t b0 = d_n1 >> kTcLenBits;
       uint32_t len = ok_n1 ? tc_len(d_n1) : 0u;
-      const uint32_t kx = tc_key(na), ky = tc_key(len);
-      if (ky > kx || (ky == kx && v >= u)) len = 0;  // v == u: a stored self-loop
+      if (!Items::kOriented) {
+        const uint32_t kx = tc_key(na), ky = tc_key(len);
+        if (ky > kx || (ky == kx && v >= u)) len = 0;  // v == u: a stored self-loop
+        // the lower end's list holds the other end and, in a triangle, one more
+        if (na < 2 && len < 2) len = 0;
+      }
       // the next items' loads go out before this item's work
       bool ok_n3 = false;
       const uint32_t v_n3 = load_y(gi + 2, ok_n3);
@@ -265,8 +390,8 @@ k_tc_count(Items src, const uint64_t *__restrict__ desc, const uint32_t *__restr
       v_n2 = v_n3;
       const uint32_t act = __ballot_sync(full, len != 0);
       if (!act) continue;
-      {  // the edges that x counts to the front: the stream's cursor steps over
-         // no empty list
+      if (!Items::kOriented) {  // the edges that x counts to the front: the stream's
+                                // cursor steps over no empty list
         const int from = tc_nth_bit(act, lane);
         v = __shfl_sync(full, v, from & 31);
         b0 = __shfl_sync(full, b0, from & 31);
@@ -350,6 +475,27 @@ k_tc_count(Items src, const uint64_t *__restrict__ desc, const uint32_t *__restr
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) local += __shfl_down_sync(full, local, d);
   if (lane == 0 && local) atomicAdd(total, local);
+}
+
+// an item per started batch of 32 of a list: sum ceil(len / 32) <= madj / 32 + n,
+// and, of lists of two entries or more, <= madj / 2
+inline uint64_t tc_items_bound(uint32_t n, uint64_t madj) {
+  return std::min<uint64_t>(madj / kTcBatch + n, madj / 2) + 1;
+}
+
+// The items of the oriented lists (madj entries in all): cnt and ioff hold n + 1
+// entries each, items tc_items_bound(n, madj); the arena scan_scratch_bytes(n + 1, 4).
+inline cudaError_t tc_list_items(const uint64_t *desc, const uint32_t *adj, uint32_t n,
+                                 uint64_t madj, uint32_t *cnt, uint32_t *ioff, uint64_t *items,
+                                 Arena &arena, cudaStream_t s, TcLists *out) {
+  if (tc_items_bound(n, madj) >= (1ull << 32)) return cudaErrorInvalidValue;
+  const unsigned blocks = (unsigned)(((uint64_t)n + 255) / 256);
+  SST_LAUNCH(k_tc_items_count, blocks, 256, 0, s, (const uint64_t *)nullptr, desc, n, cnt);
+  cudaError_t e = scan<uint32_t, OpAdd>(cnt, ioff, n, 0u, OpAdd{}, true, false, ioff + n, arena, s);
+  if (e != cudaSuccess) return e;
+  SST_LAUNCH(k_tc_items_fill, blocks, 256, 0, s, cnt, ioff, n, items);
+  *out = TcLists{desc, adj, items, ioff + n};
+  return cudaSuccess;
 }
 
 // Counts the triangles of the oriented lists desc[n] / adj over the items of

@@ -97,7 +97,7 @@ struct TravState : TravWords {
   // cc
   DevBuf<uint32_t> par;
   // tc
-  DevBuf<uint64_t> toff, tlpre, tlcnt;
+  DevBuf<uint64_t> toff, tlpre, tlcnt, titems;
   DevBuf<uint32_t> tadj, tmask;
   // multi-source bfs: per-vertex source masks (visited, frontier, next)
   DevBuf<unsigned long long> mvis, mfr, mfr2, mnx, msrc;
@@ -149,6 +149,7 @@ static void trav_buffers_release(TravState *t) {
   t->toff.release();
   t->tlpre.release();
   t->tlcnt.release();
+  t->titems.release();
   t->tadj.release();
   t->tmask.release();
   t->mvis.release();
@@ -209,7 +210,7 @@ uint64_t trav_device_bytes(const sst_graph *g) {
   add(t->il0.cap, 4); add(t->depth_tmp.cap, 4); add(t->parent_tmp.cap, 4);
   add(t->sigma.cap, 8); add(t->ratio.cap, 8); add(t->levels.cap, 8);
   add(t->hub.cap, 8); add(t->hub_done.cap, 4); add(t->par.cap, 4); add(t->toff.cap, 8); add(t->tlpre.cap, 8);
-  add(t->tlcnt.cap, 8); add(t->tadj.cap, 4); add(t->tmask.cap, 4);
+  add(t->tlcnt.cap, 8); add(t->titems.cap, 8); add(t->tadj.cap, 4); add(t->tmask.cap, 4);
   add(t->mvis.cap, 8); add(t->mfr.cap, 8);
   add(t->mfr2.cap, 8); add(t->mnx.cap, 8); add(t->msrc.cap, 8); add(t->mdepth.cap, 4);
   add(t->msig.cap, 8); add(t->mrat.cap, 8); add(t->mpart.cap, 8); add(t->mlist.cap, 4);
@@ -1511,20 +1512,41 @@ sst_status tc(sst_graph *g, uint64_t *total, uint64_t *d_pv) {
                D.slot, D.cnt, nl, g->d_deg, t->tlcnt.p, t->tmask.p);
   SST_CUDA_TRY((scan<uint64_t, OpAdd>(t->tlcnt.p, t->tlpre.p, nl, 0ull, OpAdd{},
                                       true, false, t->tlpre.p + nl, g->arena, s)));
+  const TcLeaves leaves{g->d_slots, D.owner, D.cnt, D.slot, nl};
+  const bool few = tc_few_items(nl);
+  SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, 16, s));  // count, work cursor
+  if (n) SST_LAUNCH(k_tc_lists, blocks_for(n), kTB, 0, s, D.vleaf, t->tlpre.p, n, t->toff.p);
   uint64_t madj = 0;
-  SST_CUDA_TRY(cudaMemcpyAsync(&madj, t->tlpre.p + nl, 8, cudaMemcpyDeviceToHost, s));
+  if (few) {
+    SST_CUDA_TRY(cudaMemcpyAsync(&madj, t->tlpre.p + nl, 8, cudaMemcpyDeviceToHost, s));
+  } else {
+    static_assert(2 + kTcSampleWords <= (int)kTravWords, "the estimates fit the traversal words");
+    tc_sample_launch(TcKeptLeaves{g->d_slots, D.owner, D.slot, t->tmask.p, nl}, t->toff.p,
+                     d_pv != nullptr, t->tlpre.p + nl, t->d_small + 2, s);
+    SST_CUDA_TRY(cudaMemcpyAsync(t->h_small, t->d_small + 2, kTcSampleWords * 8,
+                                 cudaMemcpyDeviceToHost, s));
+  }
   SST_CUDA_TRY(cudaStreamSynchronize(s));
+  if (!few) madj = t->h_small[kTcSampleWords - 1];
   SST_CUDA_TRY(t->tadj.ensure(madj + 1));
   if (nl)
     SST_LAUNCH(k_tc_fill, warp_blocks(tc_warps), kTB, 0, s, g->d_slots, D.slot, nl,
                t->tmask.p, t->tlpre.p, t->tadj.p);
-  if (n) SST_LAUNCH(k_tc_lists, blocks_for(n), kTB, 0, s, D.vleaf, t->tlpre.p, n, t->toff.p);
-  SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, 16, s));  // count, work cursor
   if (d_pv) SST_CUDA_TRY(cudaMemsetAsync(d_pv, 0, (uint64_t)n * 8, s));
-  if (nl)
-    SST_CUDA_TRY(tc_count_launch(TcLeaves{g->d_slots, D.owner, D.cnt, D.slot, nl}, t->toff.p,
-                                 t->tadj.p, t->d_small,
-                                 reinterpret_cast<unsigned long long *>(d_pv), g->sms, s));
+  unsigned long long *const pv = reinterpret_cast<unsigned long long *>(d_pv);
+  if (nl && (few || tc_by_rows(t->h_small))) {
+    SST_CUDA_TRY(tc_count_launch(leaves, t->toff.p, t->tadj.p, t->d_small, pv, g->sms, s));
+  } else if (nl) {
+    SST_CUDA_TRY(t->icnt.exact((uint64_t)n + 1));
+    SST_CUDA_TRY(t->ioff.exact((uint64_t)n + 1));
+    SST_CUDA_TRY(t->titems.ensure(tc_items_bound(n, madj)));
+    g->arena.reset();
+    SST_CUDA_TRY(g->arena.reserve(scan_scratch_bytes((uint64_t)n + 1, 4) + 4096));
+    TcLists lists;
+    SST_CUDA_TRY(tc_list_items(t->toff.p, t->tadj.p, n, madj, t->icnt.p, t->ioff.p, t->titems.p,
+                               g->arena, s, &lists));
+    SST_CUDA_TRY(tc_count_launch(lists, t->toff.p, t->tadj.p, t->d_small, pv, g->sms, s));
+  }
   SST_CUDA_TRY(cudaMemcpyAsync(t->h_small, t->d_small, 8, cudaMemcpyDeviceToHost, s));
   SST_CUDA_TRY(cudaStreamSynchronize(s));
   SST_CUDA_TRY(cudaGetLastError());

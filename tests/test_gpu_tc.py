@@ -2,11 +2,15 @@
 snapshot, against counts known in closed form or from the adjacency matrix:
 rows of one and of many leaves, oriented lists that fit the hash set on both
 ends of an edge, on one and on none, with and without stored self-loops.  (A
-loop belongs to no triangle; loops once matched a vertex's list against itself.)"""
+loop belongs to no triangle; loops once matched a vertex's list against itself.)
+The count's two forms: by rows (up to 16,384 items, or where lists differ in
+length, as a skewed graph's do) and by oriented lists."""
 import math
 
 import numpy as np
 import pytest
+
+import oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -72,3 +76,29 @@ def test_clique(sg, k, loops):
 def test_random(sg, n, m, loops):
     e = random(n, m, n)
     check(sg, n, e, loops, *by_matrix(n, e))
+
+
+# items below and above the 16,384 that are counted by rows unseen; uniform graphs
+# (by lists) and skewed ones (by rows); a path and a star, whose lists hold one entry
+@pytest.mark.parametrize("loops", [False, True])
+@pytest.mark.parametrize("shape", ["er16000", "er16400", "er40000", "rmat14", "rmat16", "path", "star"])
+def test_forms(sg, shape, loops):
+    rng = np.random.default_rng(5)
+    if shape == "path":
+        n = 30000
+        e = both(np.arange(n - 1), np.arange(1, n))
+    elif shape == "star":
+        n = 30000
+        e = np.concatenate([both(np.full(n - 1, 7), np.setdiff1d(np.arange(n), [7])), both([1], [2])])
+    elif shape[:2] == "er":
+        n = int(shape[2:])
+        e = rng.integers(0, n, (8 * n, 2))
+        e = both(*e[e[:, 0] != e[:, 1]].T)
+    else:
+        n = 1 << int(shape[4:])
+        e = oracle.symmetrize(oracle.rmat(int(shape[4:]), 8 * n, seed=4))
+        e = e[e[:, 0] != e[:, 1]]
+    o = oracle.OracleGraph(n)
+    o.insert_batch(e)
+    total, pv = o.tc(per_vertex=True)
+    check(sg, n, e, loops, total, np.asarray(pv).astype(np.int64))
