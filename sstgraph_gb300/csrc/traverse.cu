@@ -360,17 +360,13 @@ __global__ void k_pr_start(const uint32_t *__restrict__ deg, uint32_t n,
   pdl_wait();
   uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n) return;
-  uint32_t d = deg[v];
-  unsigned long long rd;
-  if (fresh) {
-    rd = pr_rdeg_of(d);
-    rdeg[v] = rd;
-  } else {
-    rd = rdeg[v];
-  }
-  contrib[v] = d ? contrib_of(r0, d, rd) : 0ull;
-  if (d == 0) {
-    contrib2[v] = 0ull;
+  const uint32_t d = deg[v];
+  if (d) {
+    const unsigned long long rd = fresh ? pr_rdeg_of(d) : rdeg[v];
+    if (fresh) rdeg[v] = rd;
+    contrib[v] = contrib_of(r0, d, rd);
+  } else {  // (its reciprocal is not read either)
+    contrib[v] = contrib2[v] = 0ull;
     rank[v] = base;  // no in-edges: constant term only
   }
 }
