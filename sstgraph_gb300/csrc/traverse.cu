@@ -1018,18 +1018,26 @@ __global__ void k_tc_lists(const uint64_t *__restrict__ vleaf,
 // Common neighbours of pairs: every id of the shorter row is looked up in the
 // longer one.  On a skewed graph one pair of hubs holds more leaves than all
 // the rest (a thread per pair, the form before this, spent its time in the one
-// thread that walked the longest row: 7.26 ms for 20,000 pairs of an RMAT
-// scale-18 graph, half of them edges; this form 0.136 ms).  So a
+// thread that walked the longest row: 14.5 ms for 20,000 edges of an RMAT
+// scale-18 graph, 0.18 ms this way).  So a
 // cluster of kCommonCtas blocks takes its pairs together: each block lists its
 // share with the leaf counts of the shorter rows in its shared memory, and the
 // cluster's warps split the cluster's leaves evenly, reading the pair
-// descriptors of the other blocks through distributed shared memory.  The
+// descriptors of the other blocks through distributed shared memory.  Two rows of one
+// leaf each and few ids in all (kCommonMerged) are merged by the thread that lists
+// the pair: a warp a leaf would leave most lanes idle (100,000 pairs of rows of four
+// ids 64 us, so 36, by a thread a pair 30; of eight ids 62, 42 and 39).  The
 // split needs no scratch and no readback, so the call stays one launch that
 // neither allocates nor synchronises.  Bound by the chain of dependent loads
 // of a lookup and the L1 rate of its scattered sectors.
 constexpr int kCommonCtas = 8;       // blocks of a cluster (the portable size)
 constexpr int kCommonThreads = 512;  // 128 warps to a cluster
-constexpr uint32_t kCommonPairs = 64;  // pairs of a block, at most
+constexpr uint32_t kCommonPairs = kCommonThreads;  // pairs of a block, at most
+// ids of both rows that a thread merges: while the blocks all run at once a merge is
+// the longer chain (20,000 pairs of an RMAT scale-18 graph 55.6 us with 16, 58.2 with
+// 32; of rows of four ids 29 and 27), and later rounds wait for threads (100,000 pairs
+// of rows of eight ids 54 and 42)
+constexpr uint32_t kCommonMerged = 16, kCommonMergedOfMany = 32;
 
 struct CommonPair {
   uint64_t sbase, obase;  // the shorter and the longer row
@@ -1037,48 +1045,74 @@ struct CommonPair {
   uint32_t lim;  // ids from here on do not count (early end)
 };
 
+// common ids below lim of two rows of one leaf each, na and nb ids: one merge, after
+// a load of every sector of both (a merge alone would wait for them one by one)
+__device__ __forceinline__ uint32_t common_merged(const uint32_t *pa, uint32_t na,
+                                                  const uint32_t *pb, uint32_t nb, uint32_t lim) {
+  if (!na || !nb) return 0;
+  uint32_t i = 0, j = 0, count = 0, x = pa[0], y = pb[0], t = 0;
+#pragma unroll
+  for (uint32_t k = 8; k < kLeaf; k += 8) {
+    if (k < na) t |= pa[k];
+    if (k < nb) t |= pb[k];
+  }
+  asm volatile("" ::"r"(t));
+  while (x < lim && y < lim) {
+    const bool ax = x <= y, by = y <= x;
+    count += ax && by;
+    if (ax) x = ++i < na ? pa[i] : kEmpty;
+    if (by) y = ++j < nb ? pb[j] : kEmpty;
+  }
+  return count;
+}
+
 __global__ void __cluster_dims__(kCommonCtas, 1, 1) __launch_bounds__(kCommonThreads, 2)
 k_common(DGraph g, const uint32_t *__restrict__ pairs, uint64_t n, uint32_t per_cta,
-         bool early, unsigned long long *__restrict__ out) {
+         uint32_t merged, bool early, unsigned long long *__restrict__ out) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   __shared__ CommonPair s_pair[kCommonPairs];
   __shared__ uint64_t s_pre[kCommonPairs + 1];  // leaves of the shorter rows before pair j
-  const int lane = threadIdx.x & 31;
+  __shared__ uint64_t s_warp[kCommonThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t full = 0xffffffffu;
   const uint64_t cta0 = (uint64_t)blockIdx.x - cl.block_rank();  // the cluster's first block
-  if (threadIdx.x < kCommonPairs) {
+  {
     const uint32_t j = threadIdx.x;
     const uint64_t i = (uint64_t)blockIdx.x * per_cta + j;
     uint64_t leaves = 0;
     if (j < per_cta && i < n) {
       const uint32_t a = pairs[2 * i], b = pairs[2 * i + 1];
-      out[i] = 0;
+      unsigned long long count = 0;
       if (a < g.n && b < g.n) {
         const uint32_t da = g.deg[a], db = g.deg[b];
         const uint32_t s = da <= db ? a : b, o = s == a ? b : a;
-        const uint32_t scap = g.cap[s];
-        s_pair[j] = CommonPair{g.base[s],   g.base[o], scap,
-                               min(da, db), g.cap[o],  early ? min(a, b) : kEmpty};
-        leaves = scap ? nleaves_of(scap) : 0;
+        const uint32_t scap = g.cap[s], ocap = g.cap[o], sdeg = min(da, db);
+        const uint32_t lim = early ? min(a, b) : kEmpty;
+        const uint64_t sbase = g.base[s], obase = g.base[o];
+        if (scap <= kLeaf && ocap <= kLeaf && da + db <= merged) {
+          count = common_merged(g.slots + sbase, sdeg, g.slots + obase, max(da, db), lim);
+        } else if (scap) {
+          s_pair[j] = CommonPair{sbase, obase, scap, sdeg, ocap, lim};
+          leaves = nleaves_of(scap);
+        }
       }
+      out[i] = count;
     }
-    s_pre[j + 1] = leaves;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {  // inclusive prefix of the 64 counts, two a lane
-    const uint64_t x0 = s_pre[2 * lane + 1], x1 = s_pre[2 * lane + 2];
-    uint64_t inc = x0 + x1;
+    // inclusive prefix over the block
+    uint64_t inc = leaves;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const uint64_t y = __shfl_up_sync(full, inc, d);
       if (lane >= d) inc += y;
     }
-    s_pre[2 * lane + 1] = inc - x1;
-    s_pre[2 * lane + 2] = inc;
-    if (lane == 0) s_pre[0] = 0;
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    for (int w = 0; w < warp; w++) inc += s_warp[w];
+    if (j < kCommonPairs) s_pre[j + 1] = inc;
+    if (j == 0) s_pre[0] = 0;
   }
-  cl.sync();  // every block's pairs are listed, and their outputs zeroed
+  cl.sync();  // every block's pairs are listed, and their outputs set
   // lane c < kCommonCtas: the leaves of block c, then their inclusive prefix
   uint64_t ctot = lane < kCommonCtas ? cl.map_shared_rank(s_pre, lane)[kCommonPairs] : 0;
   uint64_t cinc = ctot;
@@ -1089,15 +1123,17 @@ k_common(DGraph g, const uint32_t *__restrict__ pairs, uint64_t n, uint32_t per_
   }
   const uint64_t total = __shfl_sync(full, cinc, kCommonCtas - 1);
   constexpr uint32_t kWarps = kCommonCtas * (kCommonThreads / 32);
-  const uint32_t w = cl.block_rank() * (kCommonThreads / 32) + (threadIdx.x >> 5);
+  const uint32_t w = cl.block_rank() * (kCommonThreads / 32) + warp;
   const uint64_t hi = total * (w + 1) / kWarps;
   for (uint64_t at = total * w / kWarps; at < hi;) {
-    // block c and pair j of leaf `at` (empty rows own no leaf)
+    // block c and pair j of leaf `at` (empty rows own no leaf): the pairs before it
+    // by runs of 32, then within the run
     const int c = __popc(__ballot_sync(full, lane < kCommonCtas && cinc <= at));
     const uint64_t rem = at - __shfl_sync(full, cinc - ctot, c);
     const uint64_t *pre = cl.map_shared_rank(s_pre, c);
-    const uint32_t j = __popc(__ballot_sync(full, pre[lane + 1] <= rem)) +
-                       __popc(__ballot_sync(full, pre[lane + 33] <= rem));
+    const uint32_t j0 = 32 * __popc(__ballot_sync(
+        full, lane < (int)kCommonPairs / 32 && pre[min(32u * (lane + 1), kCommonPairs)] <= rem));
+    const uint32_t j = j0 + __popc(__ballot_sync(full, pre[j0 + lane + 1] <= rem));
     const CommonPair q = cl.map_shared_rank(s_pair, c)[j];
     const uint32_t l0 = (uint32_t)(rem - pre[j]);
     const uint64_t left = min(pre[j + 1] - rem, hi - at);
@@ -1553,13 +1589,19 @@ sst_status tc(sst_graph *g, uint64_t *total, uint64_t *d_pv) {
 sst_status common_neighbors_batch(sst_graph *g, const uint32_t *d_pairs,
                                   uint64_t n, bool early_end, uint64_t *d_out) {
   if (n == 0) return SST_OK;
-  // pairs of a block: few, so that a small call spreads over every cluster
-  // that fits at once (two blocks to an SM); at most kCommonPairs
+  // pairs of a block: few, so that a small call spreads over every cluster that fits
+  // at once (two blocks to an SM); beyond 80, 64 of them, so that a block has few long
+  // rows, or as many as make two and a half rounds of blocks (100,000 edges at RMAT
+  // scale 18 by 64, 132, 256 and 512: 553, 577, 686 and 763 us; pairs of short rows
+  // 50, 36, 33 and 34); at most kCommonPairs
   const uint64_t slots = std::max(1, 2 * g->sms / kCommonCtas) * (uint64_t)kCommonCtas;
-  const uint32_t per = (uint32_t)std::min<uint64_t>((n + slots - 1) / slots, kCommonPairs);
+  const uint64_t one = (n + slots - 1) / slots, rounds = (2 * n + 5 * slots - 1) / (5 * slots);
+  const uint64_t want = one <= 80 ? one : std::max<uint64_t>(64, rounds);
+  const uint32_t per = (uint32_t)std::min<uint64_t>(want, kCommonPairs);
   const uint64_t per_cluster = (uint64_t)per * kCommonCtas;
   SST_LAUNCH(k_common, (unsigned)((n + per_cluster - 1) / per_cluster) * kCommonCtas,
-             kCommonThreads, 0, g->stream, g->view(), d_pairs, n, per, early_end,
+             kCommonThreads, 0, g->stream, g->view(), d_pairs, n, per,
+             one <= 160 ? kCommonMerged : kCommonMergedOfMany, early_end,
              reinterpret_cast<unsigned long long *>(d_out));
   SST_CUDA_TRY(cudaGetLastError());
   return SST_OK;

@@ -60,6 +60,22 @@ def test_common_neighbors(graph, n, early):
     assert np.array_equal(got, np.array(exp, np.uint64))
 
 
+# blocks of 64 pairs, of two and a half rounds, of as many as they hold (512)
+@pytest.mark.parametrize("n", [48640, 48641, 100003, 389121])
+def test_common_neighbors_of_many(graph, n):
+    g, o = graph
+    p = pairs_of(n)
+    off, cols = o.csr()
+    a = np.zeros((N, N), bool)
+    a[np.repeat(np.arange(N), np.diff(off.astype(np.int64))), cols] = True
+    bits = np.packbits(a, axis=1)
+    ones = np.unpackbits(np.arange(256, dtype=np.uint8)[:, None], axis=1).sum(1).astype(np.uint16)
+    got = np.asarray(g.common_neighbors_batch(p))
+    for i in range(0, n, 20000):
+        both = bits[p[i:i + 20000, 0]] & bits[p[i:i + 20000, 1]]
+        assert np.array_equal(got[i:i + 20000], ones[both].sum(1))
+
+
 @pytest.mark.parametrize("n", [1, 255, 256, 257, 20011])
 def test_has_batch(graph, n):
     """Lookups in rows of every capacity, at and beside the ids they hold."""
