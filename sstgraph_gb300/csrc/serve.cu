@@ -222,18 +222,16 @@ sst_status tc_vertices(sst_graph *g, const uint32_t *d_vs, uint64_t k,
   if (e == cudaSuccess) e = cudaMemcpyAsync(&items, tot, 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   // passes 2 and 3
-  uint32_t *pq = nullptr, *pw = nullptr;
-  void *cost = nullptr, *coff = nullptr;
+  void *slots = nullptr;
   auto pairs = [&](auto zero) -> cudaError_t {
     using Off = decltype(zero);
     const uint64_t nslots = items * 32;
     const uint32_t chunk = tcv_chunk_leaves(nslots);
-    cudaError_t r = cudaMallocAsync(&pq, items * 4, s);
-    if (r == cudaSuccess) r = cudaMallocAsync(&pw, nslots * 4, s);
-    if (r == cudaSuccess) r = cudaMallocAsync(&cost, nslots * sizeof(Off), s);
-    if (r == cudaSuccess) r = cudaMallocAsync(&coff, nslots * sizeof(Off), s);
+    // a slot's chunks, their offset and its neighbour; an item's query
+    cudaError_t r = cudaMallocAsync(&slots, nslots * (2 * sizeof(Off) + 4) + items * 4, s);
     if (r != cudaSuccess) return r;
-    Off *const n1 = static_cast<Off *>(cost), *const at = static_cast<Off *>(coff);
+    Off *const n1 = static_cast<Off *>(slots), *const at = n1 + nslots;
+    uint32_t *const pw = reinterpret_cast<uint32_t *>(at + nslots), *const pq = pw + nslots;
     g->arena.reset();
     r = g->arena.reserve(scan_scratch_bytes(nslots, sizeof(Off)) + 4096);
     if (r != cudaSuccess) return r;
@@ -257,7 +255,7 @@ sst_status tc_vertices(sst_graph *g, const uint32_t *d_vs, uint64_t k,
   };
   if (e == cudaSuccess && items)
     e = tcv_wide(items * 32) ? pairs(uint64_t{0}) : pairs(uint32_t{0});
-  for (void *p : {(void *)loff, (void *)pq, (void *)pw, cost, coff})
+  for (void *p : {(void *)loff, slots})
     if (p) cudaFreeAsync(p, s);
   SST_CUDA_TRY(e);
   return SST_OK;
