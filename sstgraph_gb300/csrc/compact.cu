@@ -1214,6 +1214,46 @@ sst_status compact_bfs(sst_compact *c, uint32_t src, int32_t *d_depth) {
   return SST_OK;
 }
 
+// The device arrays of one call: a single allocation where they are large (30 us
+// each otherwise, and as much to free), else one each (up to some 4 MB they are
+// carved from memory that the driver holds).
+struct CallArrays {
+  struct Array {
+    void **p;
+    uint64_t bytes;
+  };
+  std::vector<Array> all;
+  void *block = nullptr;
+  template <typename T>
+  void add(T **p, uint64_t n) {
+    all.push_back({reinterpret_cast<void **>(p), (n * sizeof(T) + 255) & ~uint64_t(255)});
+  }
+  cudaError_t alloc() {
+    uint64_t total = 0;
+    for (const Array &a : all) total += a.bytes;
+    if (total > (4ull << 20) && cudaMalloc(&block, total) == cudaSuccess) {
+      char *at = static_cast<char *>(block);
+      for (const Array &a : all) *a.p = at, at += a.bytes;
+      return cudaSuccess;
+    }
+    cudaGetLastError();  // not in one piece: perhaps in several
+    block = nullptr;
+    for (const Array &a : all) {
+      const cudaError_t e = a.bytes ? cudaMalloc(a.p, a.bytes) : cudaSuccess;
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  }
+  void release() {
+    if (block) cudaFree(block);
+    for (const Array &a : all) {
+      if (!block && *a.p) cudaFree(*a.p);
+      *a.p = nullptr;
+    }
+    block = nullptr;
+  }
+};
+
 // TC(g) on the snapshot: triangles (each once); d_pv (may be null) gets
 // the triangles containing each vertex
 sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) {
@@ -1230,21 +1270,23 @@ sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) 
     set_error_message("sst_compact_tc: more than 2^32 stored edges");
     return SST_EINVAL;
   }
-  uint64_t *off = nullptr, *desc = nullptr, *items = nullptr;
-  uint32_t *cols = nullptr, *keep = nullptr, *pos = nullptr, *adj = nullptr;
-  uint32_t *icnt = nullptr, *ioff = nullptr;
-  cudaError_t e = cudaMalloc(&off, ((uint64_t)n + 1) * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&desc, (uint64_t)n * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&cols, m * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&keep, m * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&pos, (m + 1) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&adj, m * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&icnt, ((uint64_t)n + 1) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&ioff, ((uint64_t)n + 1) * 4);
   // an item per started batch of 32 of a row with entries (the oriented lists have
   // fewer)
   const uint64_t max_items = m / kTcBatch + std::min<uint64_t>(n, m) + 1;
-  if (e == cudaSuccess) e = cudaMalloc(&items, max_items * 8);
+  uint64_t *off = nullptr, *desc = nullptr, *items = nullptr;
+  uint32_t *cols = nullptr, *keep = nullptr, *pos = nullptr, *adj = nullptr;
+  uint32_t *icnt = nullptr, *ioff = nullptr;
+  CallArrays arrays;
+  arrays.add(&off, (uint64_t)n + 1);
+  arrays.add(&desc, n);
+  arrays.add(&cols, m);
+  arrays.add(&keep, m);
+  arrays.add(&pos, m + 1);
+  arrays.add(&adj, m);
+  arrays.add(&icnt, (uint64_t)n + 1);
+  arrays.add(&ioff, (uint64_t)n + 1);
+  arrays.add(&items, max_items);
+  cudaError_t e = arrays.alloc();
   if (e == cudaSuccess) {
     st = compact_to_csr(c, off, cols);
     if (st == SST_OK) {
@@ -1292,9 +1334,7 @@ sst_status compact_tc(sst_compact *c, uint64_t *total, uint64_t *d_pv, int sms) 
       }
     }
   }
-  for (void *p : {(void *)off, (void *)cols, (void *)keep, (void *)pos,
-                  (void *)adj, (void *)icnt, (void *)ioff, (void *)items, (void *)desc})
-    if (p) cudaFree(p);
+  arrays.release();
   if (st != SST_OK) return st;
   SST_CUDA_TRY(e);
   SST_CUDA_TRY(cudaGetLastError());
