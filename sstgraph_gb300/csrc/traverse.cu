@@ -1545,11 +1545,12 @@ sst_status tc(sst_graph *g, uint64_t *total, uint64_t *d_pv) {
   SST_CUDA_TRY((scan<uint64_t, OpAdd>(t->tlcnt.p, t->tlpre.p, nl, 0ull, OpAdd{},
                                       true, false, t->tlpre.p + nl, g->arena, s)));
   const TcLeaves leaves{g->d_slots, D.owner, D.cnt, D.slot, nl};
-  const bool few = tc_few_items(nl);
+  // few items: by rows; rows of four ids on average: by lists; else by a sample
+  const bool few = tc_few_items(nl), sample = !few && g->m > 4 * nl;
   SST_CUDA_TRY(cudaMemsetAsync(t->d_small, 0, 16, s));  // count, work cursor
   if (n) SST_LAUNCH(k_tc_lists, blocks_for(n), kTB, 0, s, D.vleaf, t->tlpre.p, n, t->toff.p);
   uint64_t madj = 0;
-  if (few) {
+  if (!sample) {
     SST_CUDA_TRY(cudaMemcpyAsync(&madj, t->tlpre.p + nl, 8, cudaMemcpyDeviceToHost, s));
   } else {
     static_assert(2 + kTcSampleWords <= (int)kTravWords, "the estimates fit the traversal words");
@@ -1559,14 +1560,14 @@ sst_status tc(sst_graph *g, uint64_t *total, uint64_t *d_pv) {
                                  cudaMemcpyDeviceToHost, s));
   }
   SST_CUDA_TRY(cudaStreamSynchronize(s));
-  if (!few) madj = t->h_small[kTcSampleWords - 1];
+  if (sample) madj = t->h_small[kTcSampleWords - 1];
   SST_CUDA_TRY(t->tadj.ensure(madj + 1));
   if (nl)
     SST_LAUNCH(k_tc_fill, warp_blocks(tc_warps), kTB, 0, s, g->d_slots, D.slot, nl,
                t->tmask.p, t->tlpre.p, t->tadj.p);
   if (d_pv) SST_CUDA_TRY(cudaMemsetAsync(d_pv, 0, (uint64_t)n * 8, s));
   unsigned long long *const pv = reinterpret_cast<unsigned long long *>(d_pv);
-  if (nl && (few || tc_by_rows(t->h_small))) {
+  if (nl && (few || (sample && tc_by_rows(t->h_small)))) {
     SST_CUDA_TRY(tc_count_launch(leaves, t->toff.p, t->tadj.p, t->d_small, pv, g->sms, s));
   } else if (nl) {
     SST_CUDA_TRY(t->icnt.exact((uint64_t)n + 1));
