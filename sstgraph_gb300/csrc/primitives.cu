@@ -1,10 +1,9 @@
 // Stable LSD radix sort of 64-bit keys (8-bit digits) and the launch
-// counter.  Each pass: per-tile digit counts, their exclusive scan over
-// (digit, tile), then a stable scatter in which every warp ranks its own
-// contiguous slice of the tile (a digit match from ballots, warp-private
-// counters), the tile is reordered in shared memory and leaves in runs of
-// one digit.  Sorts of up to 256 tiles fold the scan and the next pass's
-// counts into the scatter: one launch a pass.
+// counter.  A pass ranks a tile's keys -- every warp its own contiguous slice,
+// by a match word and a counter a digit in shared memory -- reorders the tile in
+// shared memory and writes it in runs of one digit.  Up to 4096 keys sort in one
+// block; up to 2^30 a pass is one launch, whose tiles add up the counts of the
+// tiles before them; longer sorts count and scan in launches of their own.
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
@@ -186,13 +185,8 @@ constexpr uint64_t kSmallTileKeys = 256ull * kThreads * kSmallItems;  // 2^18, n
 constexpr int kMidItems = 8;
 constexpr uint64_t kMidTileKeys = 448ull * kThreads * kMidItems;  // 7 * 2^17
 constexpr int kRadix = 256;
+constexpr uint64_t kOneSweepKeys = 1ull << 30;  // longer sorts count and scan in launches
 constexpr uint32_t kNoDigit = 0xffffffffu;  // an item past the end
-// Sorts of at most this many tiles run one launch per pass: every block
-// prefixes the raw tile counts itself (reading all of them: the cost grows
-// with the square of the tiles) and counts the next pass's digits as it
-// scatters.  Larger sorts count and scan in separate launches.
-constexpr uint32_t kFuseHistBlocks = 256;  // 1M keys
-
 // Offset of this thread's item `it` in a warp-contiguous tile of ITEMS items
 // per thread: warp w owns [w * ITEMS * 32, (w + 1) * ITEMS * 32), item it of
 // lane l sits at w * ITEMS * 32 + it * 32 + l.  Loads stay coalesced, and a
@@ -260,50 +254,36 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *wsum) 
   return off + inc - v;
 }
 
-// Per-tile digit counts at hist[d * dstride + tile * bstride]: digit-major
-// (dstride = tiles, bstride = 1) for the scanned form, tile-major
-// (dstride = 1, bstride = 256) for the fused one.  With `zero` the blocks
-// also clear that table at the same indices.
-template <int IT>
+// Per-tile digit counts, digit-major: hist[digit * tiles + tile].
 __global__ void __launch_bounds__(kThreads)
 k_hist(const uint64_t *__restrict__ keys, uint64_t n, int shift,
-       uint32_t *__restrict__ hist, uint32_t dstride, uint32_t bstride,
-       uint32_t *__restrict__ zero, const uint32_t *__restrict__ d_n) {
+       uint32_t *__restrict__ hist, const uint32_t *__restrict__ d_n) {
   pdl_wait();
   if (d_n && *d_n < n) n = *d_n;
   __shared__ uint32_t h[kRadix];
   h[threadIdx.x] = 0;
   __syncthreads();
-  const uint64_t t0 = (uint64_t)blockIdx.x * (kThreads * IT);
+  const uint64_t t0 = (uint64_t)blockIdx.x * kTile;
 #pragma unroll 4
-  for (int it = 0; it < IT; it++) {
+  for (int it = 0; it < kItems; it++) {
     uint64_t i = t0 + (uint64_t)it * kThreads + threadIdx.x;
     if (i < n) atomicAdd(&h[(keys[i] >> shift) & 0xff], 1u);
   }
   __syncthreads();
-  const uint64_t at = (uint64_t)threadIdx.x * dstride + (uint64_t)blockIdx.x * bstride;
-  hist[at] = h[threadIdx.x];
-  if (zero) zero[at] = 0;
+  hist[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
 }
 
-// One pass's stable scatter of a tile.  The warps rank their slices, the
-// tile is laid out in shared memory in (digit, index) order, and the block
-// writes it out in that order, so the keys of one digit leave as one run of
-// consecutive addresses (whole sectors, not one 8-byte write per lane).
-//  raw: hist holds the raw tile-major counts (hist[tile * 256 + d]); every
-//    block prefixes them itself (all digits below d over all tiles, plus
-//    digit d over the tiles before its own), counts the next pass's digit
-//    of each key into its destination tile's counter of hist_next (zero on
-//    entry) and clears hist_zero (the counters of the pass after next).
-//  otherwise: hist holds the scanned digit-major offsets.
-// Dynamic shared memory: scatter_smem_bytes<KV, IT>(), IT items per thread.
-// The staging area (keys and values of the tile) also holds the raw form's
-// two [kWarps][kRadix] partial-sum tables before the ranking.
+// One pass's stable scatter of a tile, for sorts too long for the one-sweep form.
+// The warps rank their slices, the tile is laid out in shared memory in (digit,
+// index) order, and the block writes it out in that order, so the keys of one digit
+// leave as one run of consecutive addresses (whole sectors, not one 8-byte write per
+// lane).  hist holds the scanned digit-major counts.
+// Dynamic shared memory: scatter_smem_bytes<KV, IT>(), IT items per thread; the
+// staging area (keys and values of the tile) also holds the match words of the ranking.
 template <bool KV, int IT>
 constexpr size_t scatter_stage_bytes() {
-  return (size_t)kThreads * IT * (KV ? 12 : 8) > (size_t)2 * kWarps * kRadix * 4
-             ? (size_t)kThreads * IT * (KV ? 12 : 8)
-             : (size_t)2 * kWarps * kRadix * 4;
+  static_assert(kThreads * IT * 8 >= kWarps * kRadix * 4, "the match words fit");
+  return (size_t)kThreads * IT * (KV ? 12 : 8);
 }
 template <bool KV, int IT>
 constexpr size_t scatter_smem_bytes() {
@@ -311,16 +291,14 @@ constexpr size_t scatter_smem_bytes() {
          kWarps * 4;
 }
 
-template <bool KV, int IT>
+template <bool KV>
 __global__ void __launch_bounds__(kThreads, 2)
 k_scatter(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
           uint64_t n, int shift, const uint32_t *__restrict__ hist,
-          uint32_t nblocks, bool raw, const uint32_t *__restrict__ vin,
-          uint32_t *__restrict__ vout, uint32_t *__restrict__ hist_next,
-          int next_shift, uint32_t *__restrict__ hist_zero,
+          const uint32_t *__restrict__ vin, uint32_t *__restrict__ vout,
           const uint32_t *__restrict__ d_n) {
   pdl_wait();
-  constexpr int TILE = kThreads * IT;
+  constexpr int IT = kItems, TILE = kTile;
   if (d_n && *d_n < n) n = *d_n;
   extern __shared__ __align__(16) unsigned char smem[];
   uint64_t *skeys = reinterpret_cast<uint64_t *>(smem);
@@ -344,50 +322,10 @@ k_scatter(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
     if (KV) vv[it] = i < n ? vin[i] : 0u;
     dg[it] = i < n ? (uint32_t)(kk[it] >> shift) & 0xff : kNoDigit;
   }
-  // gbase: output position of this tile's first key of digit threadIdx.x
-  uint32_t gbase;
-  if (raw) {
-    // the tiles' counts summed by the block's warps: warp w takes every
-    // kWarps-th tile row from w, each lane eight consecutive digits through
-    // two 16-byte loads; the partial sums meet in shared memory (the key
-    // staging area, unused until the write-out)
-    const int lane = threadIdx.x & 31;
-    uint32_t bef[8], tot[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) bef[k] = tot[k] = 0;
-#pragma unroll 4
-    for (uint32_t b = warp; b < nblocks; b += kWarps) {
-      const uint4 *row = reinterpret_cast<const uint4 *>(hist + (uint64_t)b * kRadix) + lane * 2;
-      const uint4 x0 = row[0], x1 = row[1];
-      const uint32_t v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-      const bool below = b < blockIdx.x;
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        tot[k] += v[k];
-        bef[k] += below ? v[k] : 0u;
-      }
-    }
-    uint32_t *pb = reinterpret_cast<uint32_t *>(smem);  // [kWarps][kRadix]
-    uint32_t *pt = pb + kWarps * kRadix;                // [kWarps][kRadix]
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      pb[warp * kRadix + lane * 8 + k] = bef[k];
-      pt[warp * kRadix + lane * 8 + k] = tot[k];
-    }
-    __syncthreads();
-    uint32_t before = 0, total = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) {
-      before += pb[w * kRadix + threadIdx.x];
-      total += pt[w * kRadix + threadIdx.x];
-    }
-    gbase = block_excl_scan(total, wsum) + before;
-  } else {
-    gbase = hist[(uint64_t)threadIdx.x * nblocks + blockIdx.x];
-    __syncthreads();
-  }
-  // the match words sit in the staging area, free until the reorder (the
-  // raw form's partial-sum tables there are read: barrier above)
+  // output position of this tile's first key of digit threadIdx.x
+  const uint32_t gbase = hist[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x];
+  __syncthreads();
+  // the match words sit in the staging area, free until the reorder
   uint32_t *wm = reinterpret_cast<uint32_t *>(smem) + warp * kRadix;
   clear_match_words(wm);
   uint32_t lr[IT];
@@ -415,17 +353,12 @@ k_scatter(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
     if (KV) svals[lp] = vv[it];
   }
   __syncthreads();
-  if (hist_zero) hist_zero[(uint64_t)blockIdx.x * kRadix + threadIdx.x] = 0;
   const uint32_t tn = t0 >= n ? 0u : (uint32_t)(n - t0 < (uint64_t)TILE ? n - t0 : TILE);
   for (uint32_t j = threadIdx.x; j < tn; j += kThreads) {
     const uint64_t key = skeys[j];
     const uint32_t pos = adj[(key >> shift) & 0xff] + j;
     out[pos] = key;
     if (KV) vout[pos] = svals[j];
-    if (hist_next)
-      atomicAdd(&hist_next[(uint64_t)(pos / TILE) * kRadix +
-                           ((key >> next_shift) & 0xff)],
-                1u);
   }
 }
 
@@ -446,7 +379,7 @@ k_scatter(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
 constexpr uint32_t kOsAgg = 1u << 30, kOsMask = kOsAgg - 1;
 constexpr int kOsPolls = 1 << 14;
 constexpr int kOsLog = 3, kOsGroup = 1 << kOsLog;
-// levels of groups above nt tiles (fewer than 2^18): the last has at most
+// levels of groups above nt tiles (at most 2^18): the last has at most
 // kOsGroup words
 __host__ __device__ inline int os_levels(uint32_t nt) {
   int l = 0;
@@ -653,7 +586,7 @@ cudaError_t scatter_smem_optin() {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 64 && ((done.load(std::memory_order_relaxed) >> dev) & 1)) return cudaSuccess;
-  e = cudaFuncSetAttribute(k_scatter<true, kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  e = cudaFuncSetAttribute(k_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)scatter_smem_bytes<true, kItems>());
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_scatter_os<true, kItems>,
@@ -856,23 +789,13 @@ size_t radix_sort_scratch_bytes(uint64_t n) {
   uint64_t nblocks = (n + tile - 1) / tile;
   uint64_t hn = nblocks * kRadix;
   // the one-sweep form: digit totals and up to eight passes' tile status;
-  // the counting forms: three count tables or counts and their scan
+  // the longer sorts' counts and their scan
   const size_t os = 8 * kRadix * 4 + 8 * os_status_words((uint32_t)nblocks) * 4 + 512;
-  const size_t cnt = 3 * ((hn * 4 + 255) & ~size_t(255)) + scan_scratch_bytes(hn, 4) + 512;
+  const size_t cnt = 2 * ((hn * 4 + 255) & ~size_t(255)) + scan_scratch_bytes(hn, 4) + 512;
   return os > cnt ? os : cnt;
 }
 
-// profiler name of a scatter pass, by its tile size
-template <bool KV, int IT>
-constexpr const char *scatter_name() {
-  if constexpr (IT == kSmallItems)
-    return KV ? "(k_scatter<true, 4>)" : "(k_scatter<false, 4>)";
-  else if constexpr (IT == kMidItems)
-    return KV ? "(k_scatter<true, 8>)" : "(k_scatter<false, 8>)";
-  else
-    return KV ? "(k_scatter<true, 16>)" : "(k_scatter<false, 16>)";
-}
-
+// profiler name of a one-sweep pass, by its tile size
 template <bool KV, int IT>
 constexpr const char *scatter_os_name() {
   if constexpr (IT == kSmallItems)
@@ -892,18 +815,14 @@ static cudaError_t radix_sort_tiles(uint64_t *keys, uint64_t *tmp, uint32_t *val
                                     const SortDigits *pre) {
   constexpr int TILE = kThreads * IT;
   const uint32_t nblocks = (uint32_t)((n + TILE - 1) / TILE);
-  const uint64_t hn = (uint64_t)nblocks * kRadix;
   if (vals) {
     cudaError_t e = scatter_smem_optin();
     if (e != cudaSuccess) return e;
   }
   uint64_t *src = keys, *dst = tmp;
   uint32_t *vsrc = vals, *vdst = vtmp;
-  // every scatter reads and writes keys (and values) and reads the counts
-  const uint64_t hist_bytes = 8 * n + 4 * hn;
-  const uint64_t scatter_bytes = (vals ? 24 : 16) * n + 8 * hn;
   const int passes = (bits + 7) / 8;
-  if (n < (1ull << 30) && passes <= 8) {
+  if (n < kOneSweepKeys) {
     // one sweep: all passes' digit totals in one read, then one launch a
     // pass whose tiles find their offsets by looking back
     uint32_t *totals, *status;
@@ -935,59 +854,36 @@ static cudaError_t radix_sort_tiles(uint64_t *keys, uint64_t *tmp, uint32_t *val
       std::swap(src, dst);
       std::swap(vsrc, vdst);
     }
-  } else if (nblocks <= kFuseHistBlocks) {
-    // three tile-major count tables in rotation: pass p reads table p % 3,
-    // counts into (p + 1) % 3 and clears (p + 2) % 3
-    uint32_t *h[3];
-    for (auto &t : h)
-      if (!(t = arena.take<uint32_t>(hn))) return cudaErrorMemoryAllocation;
-    SST_LAUNCH_PDL_B(hist_bytes, k_hist<IT>, nblocks, kThreads, 0, s, src, n, lo, h[0],
-                 1u, (uint32_t)kRadix, h[1], d_n);
-    int p = 0;
-    for (int shift = lo; shift < lo + bits; shift += 8, p++) {
-      const bool more = shift + 8 < lo + bits;
-      uint32_t *nx = more ? h[(p + 1) % 3] : nullptr;
-      uint32_t *zr = more ? h[(p + 2) % 3] : nullptr;
-      if (vals)
-        SST_LAUNCH_PDL_NB((scatter_name<true, IT>()), scatter_bytes, (k_scatter<true, IT>), nblocks, kThreads,
-                     (scatter_smem_bytes<true, IT>()), s, src,
-                     dst, n, shift, h[p % 3], nblocks, true, vsrc, vdst, nx,
-                     shift + 8, zr, d_n);
-      else
-        SST_LAUNCH_PDL_NB((scatter_name<false, IT>()), scatter_bytes, (k_scatter<false, IT>), nblocks, kThreads,
-                     (scatter_smem_bytes<false, IT>()), s, src,
-                     dst, n, shift, h[p % 3], nblocks, true, vsrc, vdst, nx,
-                     shift + 8, zr, d_n);
-      std::swap(src, dst);
-      std::swap(vsrc, vdst);
-    }
-  } else {
+  } else if constexpr (IT == kItems) {
     // counts and their scan in separate tables (the single-pass scan runs
     // out of place)
+    const uint64_t hn = (uint64_t)nblocks * kRadix;
+    // every scatter reads and writes keys (and values) and reads the counts
+    const uint64_t hist_bytes = 8 * n + 4 * hn;
+    const uint64_t scatter_bytes = (vals ? 24 : 16) * n + 8 * hn;
     uint32_t *cnts = arena.take<uint32_t>(hn);
     uint32_t *hist = arena.take<uint32_t>(hn);
     if (!cnts || !hist) return cudaErrorMemoryAllocation;
     for (int shift = lo; shift < lo + bits; shift += 8) {
-      SST_LAUNCH_PDL_B(hist_bytes, k_hist<IT>, nblocks, kThreads, 0, s, src, n, shift,
-                   cnts, nblocks, 1u, (uint32_t *)nullptr, d_n);
+      SST_LAUNCH_PDL_B(hist_bytes, k_hist, nblocks, kThreads, 0, s, src, n, shift, cnts, d_n);
       size_t mark = arena.used;
       cudaError_t e = scan<uint32_t, OpAdd>(cnts, hist, hn, 0u, OpAdd{}, true,
                                             false, nullptr, arena, s);
       arena.used = mark;
       if (e != cudaSuccess) return e;
       if (vals)
-        SST_LAUNCH_PDL_NB((scatter_name<true, IT>()), scatter_bytes, (k_scatter<true, IT>), nblocks, kThreads,
-                     (scatter_smem_bytes<true, IT>()), s, src,
-                     dst, n, shift, hist, nblocks, false, vsrc, vdst,
-                     (uint32_t *)nullptr, 0, (uint32_t *)nullptr, d_n);
+        SST_LAUNCH_PDL_B(scatter_bytes, k_scatter<true>, nblocks, kThreads,
+                         (scatter_smem_bytes<true, kItems>()), s, src, dst, n, shift, hist, vsrc,
+                         vdst, d_n);
       else
-        SST_LAUNCH_PDL_NB((scatter_name<false, IT>()), scatter_bytes, (k_scatter<false, IT>), nblocks, kThreads,
-                     (scatter_smem_bytes<false, IT>()), s, src,
-                     dst, n, shift, hist, nblocks, false, vsrc, vdst,
-                     (uint32_t *)nullptr, 0, (uint32_t *)nullptr, d_n);
+        SST_LAUNCH_PDL_B(scatter_bytes, k_scatter<false>, nblocks, kThreads,
+                         (scatter_smem_bytes<false, kItems>()), s, src, dst, n, shift, hist, vsrc,
+                         vdst, d_n);
       std::swap(src, dst);
       std::swap(vsrc, vdst);
     }
+  } else {
+    return cudaErrorInvalidValue;  // shorter sorts take the one-sweep form
   }
   *result = src;
   if (vresult) *vresult = vsrc;
@@ -1010,7 +906,7 @@ static int sort_form(uint64_t n, int bits, bool vals) {
 bool radix_sort_digits(uint64_t n, int bits, Arena &arena, SortDigits *d) {
   const int form = sort_form(n, bits, false);
   const int passes = (bits + 7) / 8;
-  if (form < 2 || n >= (1ull << 30) || passes > 8) return false;
+  if (form < 2 || n >= kOneSweepKeys) return false;
   const uint64_t tile = (uint64_t)kThreads * sort_items(n, false);
   const uint64_t sw = os_status_words((uint32_t)((n + tile - 1) / tile));
   d->totals = arena.take<uint32_t>(8 * kRadix);

@@ -89,7 +89,7 @@ struct TravState : TravWords {
   // bfs
   DevBuf<uint32_t> qa, qb, fbits, icnt, ioff, iv, il0;
   DevBuf<unsigned long long> qitems;
-  DevBuf<int32_t> depth_tmp, parent_tmp;
+  DevBuf<int32_t> depth_tmp;
   // bc
   DevBuf<double> sigma, ratio;
   DevBuf<uint2> levels, hub;
@@ -139,7 +139,6 @@ static void trav_buffers_release(TravState *t) {
   t->iv.release();
   t->il0.release();
   t->depth_tmp.release();
-  t->parent_tmp.release();
   t->sigma.release();
   t->ratio.release();
   t->levels.release();
@@ -207,7 +206,7 @@ uint64_t trav_device_bytes(const sst_graph *g) {
   add(t->lsum.cap, 4); add(t->inv_deg.cap, 8); add(t->ca.cap, 8);
   add(t->cb.cap, 8); add(t->partial.cap, 8); add(t->qa.cap, 4); add(t->qb.cap, 4);
   add(t->fbits.cap, 4); add(t->qitems.cap, 8); add(t->icnt.cap, 4); add(t->ioff.cap, 4); add(t->iv.cap, 4);
-  add(t->il0.cap, 4); add(t->depth_tmp.cap, 4); add(t->parent_tmp.cap, 4);
+  add(t->il0.cap, 4); add(t->depth_tmp.cap, 4);
   add(t->sigma.cap, 8); add(t->ratio.cap, 8); add(t->levels.cap, 8);
   add(t->hub.cap, 8); add(t->hub_done.cap, 4); add(t->par.cap, 4); add(t->toff.cap, 8); add(t->tlpre.cap, 8);
   add(t->tlcnt.cap, 8); add(t->titems.cap, 8); add(t->tadj.cap, 4); add(t->tmask.cap, 4);
