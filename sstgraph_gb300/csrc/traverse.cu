@@ -729,9 +729,11 @@ __global__ void k_front_expand(const uint32_t *__restrict__ q, uint32_t qn,
 // and two parents a vertex and round.
 // The passes go over all vertices, or, where fewer than half of them have a row,
 // over the work lists' entries (a vertex without a row is its own root from the
-// start).  Of 2^24 vertices 2,000 with a row: 474 us over all, 91 over those (the
-// sampled links by find before took 309); of 2^22 one in 16 with a row 167 and 116,
-// one in 4 200 and 160, one in 2 247 and 233, nearly all alike.
+// start; where edges are stored one way it may be linked from another's row, so the
+// compressions before the largest tree is sampled and at the end take all vertices).
+// Of 2^24 vertices 2,000 with a row: 474 us over all, 158 over those (the sampled links
+// by find before took 309); of 2^22 one in 16 with a row 167 and 133, one in 4 200 and
+// 171, one in 2 247 and 238.
 struct CcVerts {
   const uint32_t *small, *big;  // null: every vertex
   uint32_t nsmall, count;
@@ -1460,6 +1462,7 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
     else
       SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, if_set);
   };
+  const unsigned long long *const none = nullptr;
   if (few) SST_LAUNCH(k_iota, blocks_for(n), kTB, 0, s, par, n);
   SST_LAUNCH_PDL(k_cc_hook_first, blocks_for(vs.count), kTB, 0, s, dg, vs, par, t->qa.p, t->qb.p);
   compress(nullptr);
@@ -1472,7 +1475,10 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
   }
   SST_LAUNCH_PDL(k_cc_link_kept, blocks_for(vs.count), kTB, 0, s, vs, t->qa.p, t->qb.p, par,
                  hooks + kCcMaxRounds, err);
-  compress(hooks + kCcMaxRounds);
+  if (few)
+    SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, none);
+  else
+    compress(hooks + kCcMaxRounds);
   SST_LAUNCH_PDL(k_cc_giant, 1, 1024, 0, s, par, n, giant);
   if (t->nsmall)
     SST_LAUNCH_PDL(k_cc_rest_small, blocks_for(t->nsmall), kTB, 0, s, dg, t->sdesc.p,
@@ -1480,7 +1486,7 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
   if (t->nchunks)
     SST_LAUNCH_PDL(k_cc_rest_chunks, warp_blocks(t->nchunks), kTB, 0, s, dg, t->cdesc.p,
                t->cv.p, t->nchunks, giant, par, err);
-  compress(nullptr);
+  SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, none);
   SST_CUDA_TRY(cudaMemcpyAsync(t->h_small, t->d_small, 16, cudaMemcpyDeviceToHost, s));
   SST_CUDA_TRY(cudaStreamSynchronize(s));
   SST_CUDA_TRY(cudaGetLastError());

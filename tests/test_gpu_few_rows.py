@@ -58,3 +58,20 @@ def test_share_in_use(sg, n, share):
     step("remove_batch", more)
     compare(sg, g, o, srcs)
     g.close()
+
+
+@pytest.mark.parametrize("n,rows,m", [(1000, 100, 1500), (200000, 50000, 300000), (200000, 90000, 200000),
+                                      (1 << 20, 3000, 200000)])
+def test_one_way_edges(sg, n, rows, m):
+    """Edges stored in one direction, to vertices most of which have no row: the
+    same labels at every call, and those of the byte-width snapshot."""
+    rng = np.random.default_rng(m)
+    e = np.stack([rng.permutation(n)[:rows][rng.integers(0, rows, m)], rng.integers(0, n, m)], 1)
+    g = sg.SparseMatrixV(n)
+    g.insert_batch(e.astype(np.uint32))
+    c = sg.CompactGraph(g)
+    want = np.asarray(c.cc())
+    for _ in range(3):
+        assert np.array_equal(np.asarray(sg.CC(g)), want)
+    c.close()
+    g.close()
