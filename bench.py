@@ -718,19 +718,36 @@ def main():
             off, cols = gg.csr()
             deg = np.diff(off.astype(np.int64))
             rows = np.repeat(np.arange(nn, dtype=np.int64), deg)
-            # TC reads: every stored id once (orientation), the oriented
-            # lists N+ written and read back into the per-u sets, and every
-            # entry of N+(v) for each oriented edge (u, v) probed once;
-            # the orientation keeps an edge at its lower (degree, id) rank
+            # TC reads, by the form that the count takes: every stored id
+            # once (orientation), the oriented lists N+ (an edge at its lower
+            # (degree, id) rank) written and read back into the sets, and
+            # then by rows every id again with its list's descriptor and the
+            # shorter list of each edge's two (one above 1024 ids fits no
+            # set and is streamed), by lists a descriptor an entry and the
+            # upper end's list.  Rows where their streams cost below 0.68 of
+            # the lists', a search of a list without a set counted 16 times.
             c64 = cols.astype(np.int64)
-            rank_r = deg[rows] * nn + rows
-            rank_c = deg[c64] * nn + c64
-            up = rank_c > rank_r
-            dplus = np.bincount(rows[up], minlength=nn).astype(np.int64)
-            m_plus = int(up.sum())
-            probes = int(dplus[c64[up]].sum())
-            tc_bytes = 4 * m + 8 * m_plus + 4 * probes
-            del off, cols, rows, c64, rank_r, rank_c, up, dplus
+            up = deg[c64] * nn + c64 > deg[rows] * nn + rows
+            u, v = rows[up], c64[up]
+            dplus = np.bincount(u, minlength=nn).astype(np.int64)
+            m_plus = len(u)
+            some = dplus[u] >= 2
+            u, v = u[some], v[some]
+            lu, lv = dplus[u], dplus[v]
+            ku, kv = np.where(lu <= 1024, lu, 0), np.where(lv <= 1024, lv, 0)
+            by_u = (ku > kv) | ((ku == kv) & (u > v))
+            s_rows = np.where(lv > 0, np.where(by_u, lv, lu), 0)
+            k_set = np.where(by_u, ku, kv)
+            cost_rows = int((s_rows * np.where(k_set > 0, 1, 16)).sum())
+            cost_lists = int((lv * np.where(ku > 0, 1, 16)).sum())
+            if cost_rows < cost_lists // 100 * 68:
+                probes = int(s_rows.sum())
+                tc_bytes = 4 * m + 8 * m_plus + 12 * m + 4 * probes
+            else:
+                probes = int(lv.sum())
+                tc_bytes = 4 * m + 8 * m_plus + 8 * m_plus + 4 * probes
+            del u, v, some, lu, lv, ku, kv, by_u, s_rows, k_set
+            del off, cols, rows, c64, up, dplus
             dep = torch.empty(nn, dtype=torch.int32, device="cuda")
             pr = torch.empty(nn, dtype=torch.float64, device="cuda")
             lab = torch.empty(nn, dtype=torch.int32, device="cuda")
@@ -808,7 +825,7 @@ def main():
         out["bytes"] = {"bfs": "4 m_r + 12 n", "pagerank20": "20 (4 m + 24 n)",
                         "cc": "4 m + 8 n (one pass over the edges and labels)",
                         "bc": "8 m_r + 28 n",
-                        "tc": "sum over (u, v), v < u of 4 (d<(u) + d<(v)) + 4 m"}
+                        "tc": "4 m + 8 m+ (orientation, lists written and read) + by rows 12 m, by lists 8 m+ (ids and descriptors) + 4 a streamed entry"}
         return out
 
     def measure_multi():

@@ -704,9 +704,10 @@ __device__ __forceinline__ void bc_finish(const BfsArgs &a, const BcArgs &b, uin
 // accumulator j's sum, each the same sum as shuffling it down by 16, 8, 4, 2, 1
 // (an addition's two sides may change places).  The first log2(R) steps halve
 // the accumulators, so R of them take R - 1 + 5 - log2(R) additions, not 5R: a
-// warp's FP64 addition takes about 15 cycles of this device's pipe, which is
-// what bounds the wide levels (with a reduction and a division a row, by one
-// lane, the pipe was busy for 255 of 700 us at RMAT scale 20).
+// warp's FP64 addition takes about 15 cycles of this device's pipe.  With a reduction
+// and a division a row, by one lane, the pipe was busy for 255 of 700 us at RMAT scale
+// 20, with this for 36% of 510: the rest is the gathers' latency with half of the SM's
+// warps (64 registers a thread) and blocks that wait at the grid barrier for others.
 template <int R>
 __device__ __forceinline__ double bc_reduce(double (&acc)[R]) {
   const int lane = threadIdx.x & 31;

@@ -2,7 +2,7 @@
 //
 // A batch (insert or remove) runs as:
 //   1. keys      (row << dbits | col) per pair; self-loops (insert) and ids
-//                out of range become a sentinel that sorts last
+//                out of range take a key that no other pair has
 //   2. sort      stable LSD radix sort of the keys (primitives.cu)
 //   3. locate    per unique key: the leaf of its row's PMA where it belongs
 //                (binary search over leaf heads) and whether it is present
@@ -1904,9 +1904,9 @@ k_mid_out(Tasks t, PlanSummary *P, const unsigned long long *__restrict__ err,
 // located, merged or moved, so the sorted keys alone give each row's size and
 // each id's place: three reads of the keys and two of the rows' ranges, where the
 // general sequence makes about twenty passes over them, with 311 B of scratch a pair.
-// Bound by the key sort (250 of 374 us; 27 MB of slab and 38 MB of pairs take 10).
-// 4.8M pairs of 300,000 rows: kernels 890 -> 374 us, and with the scratch's and the
-// graph's allocation and freeing 3.00 -> 1.08 ms.
+// Bound by the key sort (161 of 272 us; 27 MB of slab and 38 MB of pairs take 10).
+// 4.8M pairs of 300,000 rows: kernels 890 -> 272 us, and with the scratch's and the
+// graph's allocation and freeing 3.04 -> 0.87 ms.
 
 // Ranks of the kept keys (the first of each run of equal ones) among a tile of
 // sorted keys: a warp takes kLoadRows runs of 32 neighbouring keys, a vote gives

@@ -1838,7 +1838,8 @@ __global__ void k_msbc_sigma_small(DGraph g, const uint32_t *__restrict__ list,
   const uint32_t *p = g.slots + g.base[v];
   uint32_t dg = g.deg[v];
   double acc = 0.0;
-  for (uint32_t k0 = 0; k0 < dg; k0 += kBcAhead) {  // as in k_sigma_small
+  // neighbours in order, kBcAhead in flight
+  for (uint32_t k0 = 0; k0 < dg; k0 += kBcAhead) {
     uint32_t u[kBcAhead];
     bool on[kBcAhead];
 #pragma unroll
@@ -1935,7 +1936,8 @@ __global__ void k_msbc_delta_small(DGraph g, const uint32_t *__restrict__ list,
   const uint32_t *p = g.slots + g.base[v];
   uint32_t dg = g.deg[v];
   double acc = 0.0;
-  for (uint32_t k0 = 0; k0 < dg; k0 += kBcAhead) {  // as in k_sigma_small
+  // neighbours in order, kBcAhead in flight
+  for (uint32_t k0 = 0; k0 < dg; k0 += kBcAhead) {
     uint32_t w[kBcAhead];
     bool on[kBcAhead];
 #pragma unroll
