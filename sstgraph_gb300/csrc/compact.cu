@@ -1231,13 +1231,15 @@ struct CallArrays {
   cudaError_t alloc() {
     uint64_t total = 0;
     for (const Array &a : all) total += a.bytes;
-    if (total > (4ull << 20) && cudaMalloc(&block, total) == cudaSuccess) {
-      char *at = static_cast<char *>(block);
-      for (const Array &a : all) *a.p = at, at += a.bytes;
-      return cudaSuccess;
+    if (total > (4ull << 20)) {
+      if (cudaMalloc(&block, total) == cudaSuccess) {
+        char *at = static_cast<char *>(block);
+        for (const Array &a : all) *a.p = at, at += a.bytes;
+        return cudaSuccess;
+      }
+      cudaGetLastError();  // not in one piece: perhaps in several
+      block = nullptr;
     }
-    cudaGetLastError();  // not in one piece: perhaps in several
-    block = nullptr;
     for (const Array &a : all) {
       const cudaError_t e = a.bytes ? cudaMalloc(a.p, a.bytes) : cudaSuccess;
       if (e != cudaSuccess) return e;

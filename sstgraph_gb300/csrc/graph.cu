@@ -1903,7 +1903,7 @@ k_mid_out(Tasks t, PlanSummary *P, const unsigned long long *__restrict__ err,
 // Pairs loaded into a graph that holds no segment: no row has anything to be
 // located, merged or moved, so the sorted keys alone give each row's size and
 // each id's place: three reads of the keys and two of the rows' ranges, where the
-// general sequence makes about twenty passes over them, with 311 B of scratch a pair.
+// general sequence makes about twenty passes over them, with 295 B of scratch a pair.
 // Bound by the key sort (161 of 272 us; 27 MB of slab and 38 MB of pairs take 10).
 // 4.8M pairs of 300,000 rows: kernels 890 -> 272 us, and with the scratch's and the
 // graph's allocation and freeing 3.04 -> 0.87 ms.

@@ -1572,7 +1572,9 @@ sst_status tc(sst_graph *g, uint64_t *total, uint64_t *d_pv) {
                t->tmask.p, t->tlpre.p, t->tadj.p);
   if (d_pv) SST_CUDA_TRY(cudaMemsetAsync(d_pv, 0, (uint64_t)n * 8, s));
   unsigned long long *const pv = reinterpret_cast<unsigned long long *>(d_pv);
-  if (nl && (few || (sample && tc_by_rows(t->h_small)))) {
+  // (more batches of the lists than 32 bits count: by rows)
+  const bool by_rows = few || tc_items_bound(n, madj) >> 32 || (sample && tc_by_rows(t->h_small));
+  if (nl && by_rows) {
     SST_CUDA_TRY(tc_count_launch(leaves, t->toff.p, t->tadj.p, t->d_small, pv, g->sms, s));
   } else if (nl) {
     SST_CUDA_TRY(t->icnt.exact((uint64_t)n + 1));
