@@ -779,6 +779,10 @@ __global__ void k_cc_hook_first(DGraph g, CcVerts vs, uint32_t *__restrict__ par
 // either way a tree only moves below a vertex of its own component with a
 // smaller id.  A hook that another one replaces is linked later, by
 // k_cc_link_kept.
+// Only what was a root at the launch may be offered to: of any other vertex the
+// parent may stand for a first edge, which is not kept.  A neighbour without a row
+// is not in the lists, so after the first round the compressions have left it where
+// that put it, and its root is looked up.
 // The first round, of every vertex, leaves 5e3 trees on that uniform graph.
 // Their roots would get hundreds of offers each, and atomics on one address
 // wait for each other (25 ns apiece: a second round of every vertex takes 240
@@ -805,8 +809,12 @@ __global__ void k_cc_hook(CcVerts vs, const uint32_t *__restrict__ nb1,
   if (i < vs.count) {
     const uint32_t x = nb1[i], y = nb2[i];
     const uint32_t a = par[vs[(uint32_t)i]];
-    const uint32_t b = x != kEmpty ? par[x] : a;
-    const uint32_t c = y != kEmpty ? par[y] : a;
+    uint32_t b = x != kEmpty ? par[x] : a;
+    uint32_t c = y != kEmpty ? par[y] : a;
+    if (vs.small && before) {
+      for (uint32_t q; (q = par[b]) != b;) b = q;
+      for (uint32_t q; (q = par[c]) != c;) c = q;
+    }
     const uint32_t m = min(a, min(b, c));
     // a look (past L1) before an atomic: an offer that is no better costs less
     if (a > m && ld_par(par, a) > m) hooked |= atomicMin(&par[a], m) > m;

@@ -75,3 +75,21 @@ def test_one_way_edges(sg, n, rows, m):
         assert np.array_equal(np.asarray(sg.CC(g)), want)
     c.close()
     g.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("seed", range(4))
+@pytest.mark.parametrize("n,rows,m", [(300007, 300007, 196000), (1 << 20, 400000, 600000),
+                                      (1 << 20, 200000, 220000)])
+def test_one_way_edges_over_the_rounds(sg, n, rows, m, seed):
+    """Enough rows for the sampled rounds, yet fewer than half of the vertices:
+    what one round has joined the later ones keep, also behind vertices without a
+    row."""
+    rng = np.random.default_rng([m, seed])
+    e = np.stack([rng.permutation(n)[:rows][rng.integers(0, rows, m)], rng.integers(0, n, m)], 1)
+    g = sg.SparseMatrixV(n)
+    g.insert_batch(e.astype(np.uint32))
+    c = sg.CompactGraph(g)
+    assert np.array_equal(np.asarray(sg.CC(g)), np.asarray(c.cc()))
+    c.close()
+    g.close()
