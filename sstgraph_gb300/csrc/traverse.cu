@@ -786,16 +786,25 @@ __global__ void k_cc_hook_first(DGraph g, CcVerts vs, uint32_t *__restrict__ par
 // The first round, of every vertex, leaves 5e3 trees on that uniform graph.
 // Their roots would get hundreds of offers each, and atomics on one address
 // wait for each other (25 ns apiece: a second round of every vertex takes 240
-// us, of every 8th 74 us).  So on a large graph the second round takes every
-// 32nd vertex and the third every 512th, which joins the two or three trees that
-// then hold most vertices and leaves few edges to k_cc_link_kept.  Below
-// kCcSampledN there are too few vertices for that, and launches cost more than
-// the atomics.  When the second round finds nothing to hook the third returns at
-// once.
+// us, of every 8th 74 us).  So the second round takes every 32nd vertex and the
+// third every 512th, which joins the two or three trees that then hold most
+// vertices and leaves few edges to k_cc_link_kept.  When the second round finds
+// nothing to hook the third returns at once.
+// Without those two, k_cc_link_kept's compare-and-swaps wait for each other at the
+// same roots: uniform graphs of 16,000, 65,536, 131,000 and 300,000 vertices with
+// 4 edges each take 98, 330, 650 and 900 us, and with them 73, 86, 130 and 118; grids,
+// stars and skewed graphs, which the first round all but finishes, pay 4-6 us for the
+// launches (R-MAT, 65,536 vertices, 59 -> 64).  Below kCcSampledN rows there is too
+// little to wait for (10,000: 70 and 63 us with 10 edges each, 55 and 63 with 40).
+// Below kCcSampledM[0] / kCcSampledM[1] edges a row the first two edges are most of
+// what there is and leave many small trees, to which few wait: of 300,000 vertices
+// with 2.7 edges each 350 us without and 600 with them, with 3.16 each 520 and 950,
+// with 3.25 each 490 and 340.
 // The parents come through L1: nearly all are one hot root, whose loads would
 // queue at one L2 slice, and a stale one is an ancestor too.
 constexpr uint32_t kCcFew = 2;  // fewer rows than one vertex in 2: over the lists
-constexpr uint32_t kCcSampledN = 1u << 17;
+constexpr uint32_t kCcSampledN = 1u << 14;
+constexpr uint64_t kCcSampledM[2] = {16, 5};
 constexpr int kCcMaxRounds = 3;
 constexpr uint32_t kCcStride[2][kCcMaxRounds] = {{1, 0, 0}, {1, 32, 512}};
 __global__ void k_cc_hook(CcVerts vs, const uint32_t *__restrict__ nb1,
@@ -1474,7 +1483,7 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
   if (few) SST_LAUNCH(k_iota, blocks_for(n), kTB, 0, s, par, n);
   SST_LAUNCH_PDL(k_cc_hook_first, blocks_for(vs.count), kTB, 0, s, dg, vs, par, t->qa.p, t->qb.p);
   compress(nullptr);
-  const bool sampled = vs.count >= kCcSampledN;
+  const bool sampled = rows >= kCcSampledN && g->m * kCcSampledM[1] >= rows * kCcSampledM[0];
   for (int r = 0; r < (sampled ? kCcMaxRounds : 1); r++) {
     const uint32_t stride = kCcStride[sampled][r];
     SST_LAUNCH_PDL(k_cc_hook, blocks_for((vs.count + stride - 1) / stride), kTB, 0, s, vs, t->qa.p,

@@ -53,3 +53,28 @@ def test_one_way_edges(sg, n, m):
         assert np.array_equal(np.asarray(sg.CC(g)), want)
     c.close()
     g.close()
+
+
+@pytest.mark.parametrize("n", [16380, 16385, 200005])
+@pytest.mark.parametrize("more", [-2, 0])
+@pytest.mark.parametrize("apart", [1, 1000])
+def test_edges_a_row(sg, n, more, apart):
+    """Below and at the rows and the edges a row from which later rounds follow the
+    first: paths of `apart` parts, ids shuffled, and chords within the parts."""
+    rng = np.random.default_rng(n + apart)
+    id_ = rng.permutation(n)
+    have = {(i, i + apart) for i in range(n - apart)}
+    while 2 * len(have) < 16 * n // 5 + more:
+        for i, k in zip(rng.integers(0, n, n).tolist(), rng.integers(1, max(n // apart, 2), n).tolist()):
+            j = i + k * apart
+            if j < n and 2 * len(have) < 16 * n // 5 + more:
+                have.add((i, j))
+    e = id_[np.array(sorted(have))]
+    g, o = sg.SparseMatrixV(n), oracle.OracleGraph(n)
+    e = oracle.symmetrize(e.astype(np.uint32))
+    g.insert_batch(e)
+    o.insert_batch(e)
+    assert g.M() == 16 * n // 5 + more
+    got = np.asarray(sg.CC(g))
+    assert np.array_equal(got, o.cc()) and len(np.unique(got)) == apart
+    g.close()
