@@ -782,34 +782,45 @@ __global__ void k_cc_hook_first(DGraph g, CcVerts vs, uint32_t *__restrict__ par
 // Only what was a root at the launch may be offered to: of any other vertex the
 // parent may stand for a first edge, which is not kept.  A neighbour without a row
 // is not in the lists, so after the first round the compressions have left it where
-// that put it, and its root is looked up.
+// that put it, and its root is looked up (`walk`).
 // The first round, of every vertex, leaves 5e3 trees on that uniform graph.
 // Their roots would get hundreds of offers each, and atomics on one address
 // wait for each other (25 ns apiece: a second round of every vertex takes 240
-// us, of every 8th 74 us).  So the second round takes every 32nd vertex and the
-// third every 512th, which joins the two or three trees that then hold most
-// vertices and leaves few edges to k_cc_link_kept.  When the second round finds
-// nothing to hook the third returns at once.
-// Without those two, k_cc_link_kept's compare-and-swaps wait for each other at the
-// same roots: uniform graphs of 16,000, 65,536, 131,000 and 300,000 vertices with
-// 4 edges each take 98, 330, 650 and 900 us, and with them 73, 86, 130 and 118; grids,
-// stars and skewed graphs, which the first round all but finishes, pay 4-6 us for the
-// launches (R-MAT, 65,536 vertices, 59 -> 64).  Below kCcSampledN rows there is too
-// little to wait for (10,000: 70 and 63 us with 10 edges each, 55 and 63 with 40).
-// Below kCcSampledM[0] / kCcSampledM[1] edges a row the first two edges are most of
-// what there is and leave many small trees, to which few wait: of 300,000 vertices
-// with 2.7 edges each 350 us without and 600 with them, with 3.16 each 520 and 950,
-// with 3.25 each 490 and 340.
+// us, of every 8th 74 us).  So on a large graph the second round takes every
+// 32nd vertex and the third every 512th, which joins the two or three trees that
+// then hold most vertices and leaves few edges to k_cc_link_kept.  When the second
+// round finds nothing to hook the third returns at once.  Below kCcThirdN vertices
+// the second takes every 8th and is the last, and what follows looks roots up
+// instead of a compression: launches count there.
+// Without later rounds k_cc_link_kept's compare-and-swaps wait for each other at the
+// same roots: uniform graphs of 20,000, 65,536, 131,000 and 300,000 vertices with
+// 4 edges each take 141, 306, 574 and 900 us, and with them 68, 70, 82 and 118; grids,
+// stars and skewed graphs, which the first round all but finishes, pay 2-3 us for the
+// launch (R-MAT, 65,536 vertices, 54 -> 57).  (A second and third round and their
+// compressions below kCcThirdN: 72, 85, 130 and R-MAT 62.)  Below kCcSampledN rows
+// there is too little to wait for (10,000: 70 and 63 us with 10 edges each, 55 and 63
+// with 40).  Below kCcSampledM[0] / kCcSampledM[1] edges a row the first two edges
+// are most of what there is and leave many small trees, to which few wait: of 300,000
+// vertices with 2.7 edges each 350 us without and 600 with them, with 3.16 each 520
+// and 950, with 3.25 each 490 and 340.
 // The parents come through L1: nearly all are one hot root, whose loads would
 // queue at one L2 slice, and a stale one is an ancestor too.
 constexpr uint32_t kCcFew = 2;  // fewer rows than one vertex in 2: over the lists
 constexpr uint32_t kCcSampledN = 1u << 14;
 constexpr uint64_t kCcSampledM[2] = {16, 5};
+constexpr uint32_t kCcThirdN = 1u << 17;
 constexpr int kCcMaxRounds = 3;
-constexpr uint32_t kCcStride[2][kCcMaxRounds] = {{1, 0, 0}, {1, 32, 512}};
+constexpr uint32_t kCcStride[kCcMaxRounds][kCcMaxRounds] = {{1}, {1, 8}, {1, 32, 512}};
+
+// the root of x as far as it is known here: nothing is changed on the way
+__device__ __forceinline__ uint32_t cc_root(const uint32_t *par, uint32_t x) {
+  for (uint32_t p; (p = par[x]) != x;) x = p;
+  return x;
+}
+
 __global__ void k_cc_hook(CcVerts vs, const uint32_t *__restrict__ nb1,
-                          const uint32_t *__restrict__ nb2, uint32_t stride, uint32_t *par,
-                          const unsigned long long *__restrict__ before,
+                          const uint32_t *__restrict__ nb2, uint32_t stride, bool walk,
+                          uint32_t *par, const unsigned long long *__restrict__ before,
                           unsigned long long *__restrict__ hooks) {
   pdl_wait();
   if (before && *before == 0) return;
@@ -817,12 +828,13 @@ __global__ void k_cc_hook(CcVerts vs, const uint32_t *__restrict__ nb1,
   bool hooked = false;
   if (i < vs.count) {
     const uint32_t x = nb1[i], y = nb2[i];
-    const uint32_t a = par[vs[(uint32_t)i]];
+    uint32_t a = par[vs[(uint32_t)i]];
     uint32_t b = x != kEmpty ? par[x] : a;
     uint32_t c = y != kEmpty ? par[y] : a;
-    if (vs.small && before) {
-      for (uint32_t q; (q = par[b]) != b;) b = q;
-      for (uint32_t q; (q = par[c]) != c;) c = q;
+    if (walk) {
+      a = cc_root(par, a);
+      b = cc_root(par, b);
+      c = cc_root(par, c);
     }
     const uint32_t m = min(a, min(b, c));
     // a look (past L1) before an atomic: an offer that is no better costs less
@@ -835,20 +847,28 @@ __global__ void k_cc_hook(CcVerts vs, const uint32_t *__restrict__ nb1,
 
 // The kept edges that the rounds have not joined, by find and compare-and-swap:
 // afterwards the trees are the components of every vertex's first two edges, in
-// whatever order the hooks went.
+// whatever order the hooks went.  After a round that no compression followed the
+// roots are looked up (`walk`) before they are compared.
 __global__ void k_cc_link_kept(CcVerts vs, const uint32_t *__restrict__ nb1,
-                               const uint32_t *__restrict__ nb2, uint32_t *par,
+                               const uint32_t *__restrict__ nb2, bool walk, uint32_t *par,
                                unsigned long long *__restrict__ hooks,
                                unsigned long long *__restrict__ err) {
   pdl_wait();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   bool linked = false;
   if (i < vs.count) {
-    const uint32_t u = vs[i], x = nb1[i], y = nb2[i], a = par[u];
-    const uint32_t b = x != kEmpty ? par[x] : a, c = y != kEmpty ? par[y] : a;
-    if (b != a) cc_link(par, u, x, err);
-    if (c != a) cc_link(par, u, y, err);
-    linked = b != a || c != a;
+    const uint32_t u = vs[i], x = nb1[i], y = nb2[i];
+    uint32_t a = par[u], b = x != kEmpty ? par[x] : a, c = y != kEmpty ? par[y] : a;
+    if (walk) {
+      a = cc_root(par, a);
+      b = cc_root(par, b);
+      c = cc_root(par, c);
+    }
+    // (no neighbour: two walks from one vertex may end apart while others link)
+    const bool join_x = x != kEmpty && b != a, join_y = y != kEmpty && c != a;
+    if (join_x) cc_link(par, u, x, err);
+    if (join_y) cc_link(par, u, y, err);
+    linked = join_x || join_y;
   }
   if (__syncthreads_or(linked) && threadIdx.x == 0) *(volatile unsigned long long *)hooks = 1;
 }
@@ -1483,15 +1503,18 @@ sst_status cc(sst_graph *g, uint32_t *d_labels) {
   if (few) SST_LAUNCH(k_iota, blocks_for(n), kTB, 0, s, par, n);
   SST_LAUNCH_PDL(k_cc_hook_first, blocks_for(vs.count), kTB, 0, s, dg, vs, par, t->qa.p, t->qb.p);
   compress(nullptr);
-  const bool sampled = rows >= kCcSampledN && g->m * kCcSampledM[1] >= rows * kCcSampledM[0];
-  for (int r = 0; r < (sampled ? kCcMaxRounds : 1); r++) {
-    const uint32_t stride = kCcStride[sampled][r];
+  const bool later = rows >= kCcSampledN && g->m * kCcSampledM[1] >= rows * kCcSampledM[0];
+  const int rounds = !later ? 1 : vs.count < kCcThirdN ? 2 : 3;
+  for (int r = 0; r < rounds; r++) {
+    const uint32_t stride = kCcStride[rounds - 1][r];
+    const bool packed = r == 0 || rounds == 3;  // a compression follows
     SST_LAUNCH_PDL(k_cc_hook, blocks_for((vs.count + stride - 1) / stride), kTB, 0, s, vs, t->qa.p,
-                   t->qb.p, stride, par, r ? hooks + std::min(r - 1, 1) : nullptr, hooks + r);
-    compress(hooks + r);
+                   t->qb.p, stride, few && r, par, r ? hooks + r - 1 : nullptr,
+                   hooks + (packed ? r : kCcMaxRounds));
+    if (packed) compress(hooks + r);
   }
-  SST_LAUNCH_PDL(k_cc_link_kept, blocks_for(vs.count), kTB, 0, s, vs, t->qa.p, t->qb.p, par,
-                 hooks + kCcMaxRounds, err);
+  SST_LAUNCH_PDL(k_cc_link_kept, blocks_for(vs.count), kTB, 0, s, vs, t->qa.p, t->qb.p, rounds == 2,
+                 par, hooks + kCcMaxRounds, err);
   if (few)
     SST_LAUNCH_PDL(k_cc_compress, blocks_for(n), kTB, 0, s, par, n, none);
   else
