@@ -295,9 +295,15 @@ inline void tc_sample_launch(const Kept &src, const uint64_t *desc, bool pv, con
              (src.n + kTcSamples - 1) / kTcSamples, pv ? kTcSortedCostPv : kTcSortedCost, also, est);
 }
 // Whether a count of so many items by rows (leaves, or rows and started batches) takes
-// the rows' form unseen: it is done in the time of the launches that list the oriented
-// lists' items.
-inline bool tc_few_items(uint64_t items) { return items <= 1u << 14; }
+// the rows' form unseen: it is done in about the time of the sample and of the launches
+// that list the oriented lists' items (uniform graphs of 22,000, 40,000 and 60,000
+// vertices with 6 edges each: 71, 75 and 84 us by rows and 78, 91 and 93 by lists;
+// of 90,000, 97 and 110, but by vertex 127 and 134 and from there on lists come nearer).
+// Where rows are long the sample sees work that hides in the rows' form (1500 vertices
+// with 350 edges each: 282 us by rows, 416 by the lists that the sample takes); by
+// vertex the lists' fewer atomics count there (698 us, rows 775; 1000 vertices with
+// 550 edges each 2663 and 2992).
+inline bool tc_few_items(uint64_t items) { return items <= 1u << 16; }
 // Whether the rows' form is the one to take, by the sample's sums (host memory).
 template <class Word>
 inline bool tc_by_rows(const Word *est) {

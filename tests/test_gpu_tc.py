@@ -3,7 +3,7 @@ snapshot, against counts known in closed form or from the adjacency matrix:
 rows of one and of many leaves, oriented lists that fit the hash set on both
 ends of an edge, on one and on none, with and without stored self-loops.  (A
 loop belongs to no triangle; loops once matched a vertex's list against itself.)
-The count's two forms: by rows (up to 16,384 items, or where lists differ in
+The count's two forms: by rows (up to 65,536 items, or where lists differ in
 length, as a skewed graph's do) and by oriented lists."""
 import math
 
@@ -78,17 +78,18 @@ def test_random(sg, n, m, loops):
     check(sg, n, e, loops, *by_matrix(n, e))
 
 
-# items below and above the 16,384 that are counted by rows unseen; uniform graphs
+# items below and above the 65,536 that are counted by rows unseen; uniform graphs
 # (by lists) and skewed ones (by rows); a path and a star, whose lists hold one entry
 @pytest.mark.parametrize("loops", [False, True])
-@pytest.mark.parametrize("shape", ["er16000", "er16400", "er40000", "rmat14", "rmat16", "path", "star"])
+@pytest.mark.parametrize("shape", ["er16000", "er16400", "er40000", "rmat14", "rmat16", "path", "star",
+                                   "er65500", "er65600", "er90000", "rmat17", "path90000", "star90000"])
 def test_forms(sg, shape, loops):
     rng = np.random.default_rng(5)
-    if shape == "path":
-        n = 30000
+    if shape[:4] == "path":
+        n = int(shape[4:] or 30000)
         e = both(np.arange(n - 1), np.arange(1, n))
-    elif shape == "star":
-        n = 30000
+    elif shape[:4] == "star":
+        n = int(shape[4:] or 30000)
         e = np.concatenate([both(np.full(n - 1, 7), np.setdiff1d(np.arange(n), [7])), both([1], [2])])
     elif shape[:2] == "er":
         n = int(shape[2:])
